@@ -40,29 +40,8 @@ struct AdjointBatch::Impl {
   std::size_t ringBytes = 0;      // per team, as chosen
   int ringTeams = 0;
 
-  SlotLayout slot_for(int W) const {
-    // the forward slot of a team of W warps, as the batch kernel lays it out for one model
-    const ModelDev& m = *model;
-    SlotLayout L{};
-    std::uint32_t off = 0;
-    const std::size_t nb = sizeof(double) * static_cast<std::size_t>(m.NN);
-    L.vol = take(off, nb); L.level = take(off, nb); L.cx = take(off, nb); L.cy = take(off, nb); L.cz = take(off, nb);
-    L.area = take(off, nb); L.zmax = take(off, nb); L.hEff = take(off, nb); L.aEff = take(off, nb); L.acc = take(off, nb);
-    L.deg = take(off, sizeof(std::int32_t) * static_cast<std::size_t>(m.NN));
-    L.dV = take(off, sizeof(double) * static_cast<std::size_t>(std::max(m.NC, 1)));
-    L.q = take(off, sizeof(double) * static_cast<std::size_t>(std::max(m.NC, 1)));
-    L.tmp = m.NC >= m.NN ? kSlotAliasDV : take(off, nb);
-    L.passes = take(off, 7 * sizeof(double) * static_cast<std::size_t>(m.maxGroup) * static_cast<std::size_t>(W * kMaxLevelGroupsPerWarp));
-    L.hydro = take(off, 8 * 5 * sizeof(double));
-    L.misc = take(off, 4 * sizeof(std::int32_t));
-    L.merged = take(off, static_cast<std::size_t>(std::max(m.NG, 1)));
-    L.pose = take(off, sizeof(Pose));
-    L.buoy = take(off, sizeof(Buoy));
-    L.parked = take(off, sizeof(Parked));
-    L.model = 0;
-    L.bytes = off;
-    return L;
-  }
+  // the forward slot of a team of W warps, as the batch kernel lays it out for one model
+  SlotLayout slot_for(int W) const { return slot_layout(model->NN, model->NC, model->NG, model->maxGroup, W, false); }
 };
 
 AdjointBatch::AdjointBatch(std::shared_ptr<const CompiledShip> ship, const CompiledSim& sim, const AdjointOptions& opt)

@@ -63,12 +63,22 @@ struct AdjTeam {
 // The tape hooks of the forward step (NoTape's counterpart): one lane of a level lane group writes each node pass, the
 // team writes the solved state, the pose and the buoyancy result.
 struct GpuTape {
+  static constexpr bool kLazy = false;
   adj::Tape t;
+  // A unit's start: its first pass's level and extent; the sums stay zero when no pass is made there.
+  __device__ __forceinline__ void start(int n, double h, double zmin, double zmax, const LevelLanes& L) const {
+    if (L.sub != 0) return;
+    double* r = t.pass(n, 0);
+    r[0] = h; r[1] = 0; r[2] = 0; r[3] = 0; r[4] = 0; r[5] = 0; r[6] = zmin; r[7] = zmax;
+    t.i[t.L.npass + n] = 1;
+  }
   __device__ __forceinline__ void pass(int n, int k, double h, const PassR& p, const LevelLanes& L) const {
     if (L.sub != 0) return;
     if (k < adj::kMaxPasses) {
+      const double* r0 = t.pass(n, 0);
+      const double zmin = r0[6], zmax = r0[7];
       double* r = t.pass(n, k);
-      r[0] = h; r[1] = p.vol; r[2] = p.dv; r[3] = p.mx; r[4] = p.my; r[5] = p.mz; r[6] = p.zmin; r[7] = p.zmax;
+      r[0] = h; r[1] = p.vol; r[2] = p.dv; r[3] = p.mx; r[4] = p.my; r[5] = p.mz; r[6] = zmin; r[7] = zmax;
     }
     t.i[t.L.npass + n] = k + 1;
   }
@@ -88,6 +98,11 @@ struct GpuTape {
       t.d[L.buoy] = b.V; t.d[L.buoy + 1] = b.x; t.d[L.buoy + 2] = b.y; t.d[L.buoy + 3] = b.z;
     }
   }
+};
+
+// A forward step without a record; its levels are all formed (checkpoints keep them).
+struct NoRecord : NoTape {
+  static constexpr bool kLazy = false;
 };
 
 // Instance fields for team_step: the connection fields of the instance; events go nowhere (the adjoint runs keep no
@@ -165,9 +180,12 @@ __device__ __forceinline__ void load_state(const double* c, SimRegs& R, Slot& S,
   for (int n = T.rank; n < nn; n += 32 * W) {
     S.vol[n] = c[7 + n]; S.level[n] = c[7 + nn + n]; S.cx[n] = c[7 + 2 * nn + n]; S.cy[n] = c[7 + 3 * nn + n]; S.cz[n] = c[7 + 4 * nn + n];
     S.area[n] = 0; S.zmax[n] = 0; S.hEff[n] = 0; S.aEff[n] = 0; S.acc[n] = 0; S.deg[n] = 0;
+    S.dry[n] = 0;
   }
   for (int g = T.rank; g < M.ng; g += 32 * W) S.merged[g] = 0;
   for (int c2 = T.rank; c2 < M.nc; c2 += 32 * W) { S.dV[c2] = 0; S.q[c2] = 0; }
+  T.sync();
+  if (T.warp == W - 1) list_groups<false>(M, S, T.lane);  // every group, for the whole run
   T.sync();
 }
 
@@ -311,11 +329,11 @@ __global__ void __launch_bounds__(W * 32) adjoint_batch(DevModel M, AdjRun B, Sl
   for (;;) {
     if (T.leader()) {
       const int q = atomicAdd(B.queue, 1);
-      S.misc[0] = B.order == nullptr || q >= B.count ? q : B.order[q];
-      S.misc[2] = W * (32 / kLevelLanes<false>);  // the level solve's group counter for the first step (team_step resets it)
+      S.misc[kMiscInstance] = B.order == nullptr || q >= B.count ? q : B.order[q];
+      S.misc[kMiscTaken] = W * (32 / kLevelLanes<false>);  // the level solve's list counter for the first step (team_step resets it)
     }
     T.sync();
-    const int inst = S.misc[0];
+    const int inst = S.misc[kMiscInstance];
     T.sync();
     if (inst >= B.count) return;
     const long long tStart = global_ns();
@@ -373,7 +391,7 @@ __global__ void __launch_bounds__(W * 32) adjoint_batch(DevModel M, AdjRun B, Sl
         if (T.leader()) rb[s] = static_cast<std::int32_t>(bytes);
         v += static_cast<long long>(bytes);
       } else {
-        team_step<false, W>(M, F, R, S, I, T);
+        team_step<false, W>(M, F, R, S, I, T, NoRecord{});
       }
       F = make_pose(M, R.zO, R.pitch, R.roll);
     }

@@ -56,31 +56,7 @@ struct Batch::Impl {
   const ModelDev& m0() const { return *models.front(); }
   const ModelDev& model(std::size_t inst) const { return *models[static_cast<std::size_t>(instModel[inst])]; }
 
-  // The shared-memory slot of one simulation stepped by a team of W warps: per-node state and scratch, per-connection
-  // dV and q, the group-pass buffers, the buoyancy tree results, the pose, buoyancy result and parked run values, and
-  // in a fleet the team's copy of its instance's model. The loads' sixth scratch column reuses dV when there are at
-  // least as many connections as nodes.
-  SlotLayout layout_for(int W) const {
-    SlotLayout L{};
-    std::uint32_t off = 0;
-    const std::size_t nb = sizeof(double) * static_cast<std::size_t>(NN);
-    L.vol = take(off, nb); L.level = take(off, nb); L.cx = take(off, nb); L.cy = take(off, nb); L.cz = take(off, nb);
-    L.area = take(off, nb); L.zmax = take(off, nb); L.hEff = take(off, nb); L.aEff = take(off, nb); L.acc = take(off, nb);
-    L.deg = take(off, sizeof(std::int32_t) * static_cast<std::size_t>(NN));
-    L.dV = take(off, sizeof(double) * static_cast<std::size_t>(std::max(NC, 1)));
-    L.q = take(off, sizeof(double) * static_cast<std::size_t>(std::max(NC, 1)));
-    L.tmp = NC >= NN ? kSlotAliasDV : take(off, nb);
-    L.passes = take(off, 7 * sizeof(double) * static_cast<std::size_t>(maxGroup) * static_cast<std::size_t>(W * kMaxLevelGroupsPerWarp));
-    L.hydro = take(off, 8 * 5 * sizeof(double));
-    L.misc = take(off, 4 * sizeof(std::int32_t));
-    L.merged = take(off, static_cast<std::size_t>(std::max(NG, 1)));
-    L.pose = take(off, sizeof(Pose));
-    L.buoy = take(off, sizeof(Buoy));
-    L.parked = take(off, sizeof(Parked));
-    L.model = fleet() ? take(off, sizeof(DevModel)) : 0u;
-    L.bytes = off;
-    return L;
-  }
+  SlotLayout layout_for(int W) const { return slot_layout(NN, NC, NG, maxGroup, W, fleet()); }
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   std::vector<cudaEvent_t> phaseEv;           // launch phase k ends at phaseEv[k + 1]; phaseEv[0] starts a round

@@ -81,8 +81,9 @@ __device__ const unsigned char* stage_column_table(const typename Vec2<T>::type*
   return dst;
 }
 
-template <int W>
-__device__ __forceinline__ void write_record(double* rec, const SimRegs& R, const Slot& S, int nn, const Team<W>& T) {
+template <bool MIXED, int W>
+__device__ __forceinline__ void write_record(double* rec, const SimRegs& R, const DevModel& M, const Slot& S, const Team<W>& T) {
+  const int nn = M.nn;
   if (T.warp != 0) return;
   const int lane = T.lane;
   if (lane == 0) {
@@ -92,7 +93,7 @@ __device__ __forceinline__ void write_record(double* rec, const SimRegs& R, cons
   double* p = rec + 10;
   for (int n = lane; n < nn; n += kLanes) {
     p[n] = S.vol[n];
-    p[nn + n] = S.level[n];
+    p[nn + n] = stale_level<MIXED>(M, S, n);
     p[2 * nn + n] = S.cx[n];
     p[3 * nn + n] = S.cy[n];
     p[4 * nn + n] = S.cz[n];
@@ -121,9 +122,12 @@ __device__ bool run_instance(const DevModel& M, const DevBatch& B, Slot& S, int 
     S.vol[n] = B.vol[iN + n]; S.level[n] = B.level[iN + n];
     S.cx[n] = B.cx[iN + n]; S.cy[n] = B.cy[iN + n]; S.cz[n] = B.cz[iN + n];
     S.area[n] = 0; S.zmax[n] = 0; S.hEff[n] = 0; S.aEff[n] = 0; S.acc[n] = 0; S.deg[n] = 0;
+    S.dry[n] = 0;
   }
   for (int g = rank; g < M.ng; g += kStride) S.merged[g] = 0;
   for (int c = rank; c < M.nc; c += kStride) { S.dV[c] = 0; S.q[c] = 0; }
+  T.sync();
+  if (T.warp == W - 1) list_groups<true>(M, S, T.lane);
   T.sync();
 
   long long done = B.steps[inst];
@@ -145,8 +149,8 @@ __device__ bool run_instance(const DevModel& M, const DevBatch& B, Slot& S, int 
     const Pose F0 = make_pose(M, R.zO, R.pitch, R.roll);
     const Buoy hb = buoyancy<MIXED, W>(M, F0, T, S.hydro, S.cols);
     R.inflow = 0; R.Vb = hb.V; R.hullTop = hb.top; R.bx = hb.x; R.by = hb.y; R.bz = hb.z;
-    write_record(denseBase, R, S, M.nn, T);
-    write_record(sampleBase, R, S, M.nn, T);
+    write_record<MIXED>(denseBase, R, M, S, T);
+    write_record<MIXED>(sampleBase, R, M, S, T);
     denseCount = 1; sampleCount = 1; nextSample = B.sampleEvery;
     T.sync();
   }
@@ -154,14 +158,14 @@ __device__ bool run_instance(const DevModel& M, const DevBatch& B, Slot& S, int 
   int stop = kRunning;
   bool paused = false;
   // every thread of the team stores the same pose; no thread reads the previous one after the step's last barrier
-  Pose& F = *S.pose;
-  F = make_pose(M, R.zO, R.pitch, R.roll);
+  // (the two poses change places at the end of a step, so the last solve's stays for stale_level)
+  *S.pose = make_pose(M, R.zO, R.pitch, R.roll);
   for (long long s = 0; s < B.maxSteps; ++s) {
     if (R.foundered || R.t >= B.tMax) break;
     if (B.yieldBelow > 0 && s > 0 && (s % kYieldCheckEvery) == 0) {
-      if (T.leader()) S.misc[1] = *reinterpret_cast<volatile int*>(B.remaining) <= B.yieldBelow ? 1 : 0;
+      if (T.leader()) S.misc[kMiscYield] = *reinterpret_cast<volatile int*>(B.remaining) <= B.yieldBelow ? 1 : 0;
       T.sync();
-      const bool y = S.misc[1] != 0;
+      const bool y = S.misc[kMiscYield] != 0;
       T.sync();
       if (y) { paused = true; break; }
     }
@@ -177,13 +181,17 @@ __device__ bool run_instance(const DevModel& M, const DevBatch& B, Slot& S, int 
       ++curveCount;
       nextCurve += B.curveEvery;
     }
-    team_step<MIXED, W>(M, F, R, S, I, T);
+    team_step<MIXED, W>(M, *S.pose, R, S, I, T);
     ++done;
+    Pose* const last = S.pose;
+    S.pose = S.prev;
+    S.prev = last;
+    Pose& F = *S.pose;
     F = make_pose(M, R.zO, R.pitch, R.roll);
     if (traced) {
-      if (done <= B.denseSteps) write_record(denseBase + static_cast<std::size_t>(denseCount++) * B.recSize, R, S, M.nn, T);
+      if (done <= B.denseSteps) write_record<MIXED>(denseBase + static_cast<std::size_t>(denseCount++) * B.recSize, R, M, S, T);
       if (R.t >= nextSample - 1e-9 && sampleCount < B.maxSamples) {
-        write_record(sampleBase + static_cast<std::size_t>(sampleCount++) * B.recSize, R, S, M.nn, T);
+        write_record<MIXED>(sampleBase + static_cast<std::size_t>(sampleCount++) * B.recSize, R, M, S, T);
         nextSample += B.sampleEvery;
       }
     }
@@ -207,7 +215,7 @@ __device__ bool run_instance(const DevModel& M, const DevBatch& B, Slot& S, int 
   // store the instance
   T.sync();
   for (int n = rank; n < M.nn; n += kStride) {
-    B.vol[iN + n] = S.vol[n]; B.level[iN + n] = S.level[n];
+    B.vol[iN + n] = S.vol[n]; B.level[iN + n] = stale_level<MIXED>(M, S, n);
     B.cx[iN + n] = S.cx[n]; B.cy[iN + n] = S.cy[n]; B.cz[iN + n] = S.cz[n];
   }
   if (T.leader()) {
@@ -262,11 +270,11 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, kMinBlocksPerSM) run_b
   for (;;) {
     if (T.leader()) {
       const int q = atomicAdd(B.queue, 1);
-      S.misc[0] = B.order == nullptr ? q : (q < *B.orderCount ? B.order[q] : B.count);
-      S.misc[2] = W * (32 / kLevelLanes<MIXED>);  // the level solve's group counter for the first step (team_step resets it)
+      S.misc[kMiscInstance] = B.order == nullptr ? q : (q < *B.orderCount ? B.order[q] : B.count);
+      S.misc[kMiscTaken] = W * (32 / kLevelLanes<MIXED>);  // the level solve's list counter for the first step (team_step resets it)
     }
     T.sync();
-    const int inst = S.misc[0];
+    const int inst = S.misc[kMiscInstance];
     T.sync();
     if (inst >= B.count) return;
     if constexpr (FLEET) {

@@ -35,6 +35,13 @@ struct DevModel {
   const double* segAr;
   const float2 *segXYf, *segLHf;
   const float* segArf;
+  // extent lists (extents.h) of the nodes' segments and, as set nn, of the hull columns' tops: 8 (nn + 1) + 1 starts and
+  // the listed points' coordinates, (x, y) and z
+  const std::int32_t* exStart;
+  const double2* exXY;
+  const double* exZ;
+  const float2* exXYf;
+  const float* exZf;
   // nodes
   std::int32_t nn;
   const double *mu, *vmax, *amin, *aov;
@@ -202,14 +209,15 @@ constexpr int kMaxLevelGroupsPerWarp = 32 / (kLevelLanes<false> < kLevelLanes<tr
 
 // Byte offsets of one simulation slot (one team of warps) in dynamic shared memory; `bytes` is the slot stride.
 // passes holds maxGroup node-pass results per level lane group of the team (up to kMaxLevelGroupsPerWarp per warp); hydro the
-// eight buoyancy tree results; misc two ints the team broadcasts (the claimed instance, the yield decision); pose and
-// buoy the step's pose and buoyancy result, which every phase reads (kept here rather than in each thread's registers);
-// parked the run's values during the hydrostatic phases; model (fleets only) the team's copy of its instance's model.
-// tmp is the sixth column of the loads' per-node terms (the other five reuse area, zmax, hEff, aEff and acc, which
-// are dead by then); kSlotAliasDV places it on dV when there are at least as many connections as nodes.
+// eight buoyancy tree results; misc the team's small broadcast values and counters (MiscSlot); dry a flag byte per node and
+// list the groups the next level solve visits (warp_step.cuh); pose (this step's and the last one's) and buoy the step's
+// pose and buoyancy result, which every phase reads (kept here rather than in each thread's registers); parked the run's
+// values during the hydrostatic phases; model (fleets only) the team's copy of its instance's model. tmp is the sixth
+// column of the loads' per-node terms (the other five reuse area, zmax, hEff, aEff and acc, which are dead by then) and,
+// between the level solve and the heads, of the passes' sums.
 struct SlotLayout {
-  std::uint32_t vol, level, cx, cy, cz, area, zmax, hEff, aEff, acc, deg, dV, q, tmp, passes, hydro, misc, merged, pose, buoy, parked, model, bytes;
+  std::uint32_t vol, level, cx, cy, cz, area, zmax, hEff, aEff, acc, deg, dV, q, tmp, passes, hydro, misc, merged, dry, list, pose, buoy, parked,
+      model, bytes;
 };
-constexpr std::uint32_t kSlotAliasDV = 0xFFFFFFFFu;
 
 }  // namespace ssb

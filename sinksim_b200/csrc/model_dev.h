@@ -3,6 +3,7 @@
 // and the adjoint engine (adjoint.cpp).
 #pragma once
 
+#include <algorithm>
 #include <cmath>
 #include <memory>
 #include <stdexcept>
@@ -12,6 +13,7 @@
 #include <cuda_runtime.h>
 
 #include "device_model.h"
+#include "extents.h"
 #include "model.h"
 
 namespace ssb {
@@ -64,6 +66,34 @@ inline std::uint32_t take(std::uint32_t& off, std::size_t bytes) {
   return at;
 }
 
+// The shared-memory slot of one simulation of a model of these sizes, stepped by a team of W warps: per-node state and
+// scratch, per-connection dV and q, the group-pass buffers, the buoyancy tree results, the poses, buoyancy result and
+// parked run values, and in a fleet the team's copy of its instance's model.
+inline SlotLayout slot_layout(std::int32_t NN, std::int32_t NC, std::int32_t NG, std::int32_t maxGroup, int W, bool fleet) {
+  SlotLayout L{};
+  std::uint32_t off = 0;
+  const std::size_t nb = sizeof(double) * static_cast<std::size_t>(NN);
+  const std::size_t cb = sizeof(double) * static_cast<std::size_t>(std::max(NC, 1));
+  L.vol = take(off, nb); L.level = take(off, nb); L.cx = take(off, nb); L.cy = take(off, nb); L.cz = take(off, nb);
+  L.area = take(off, nb); L.zmax = take(off, nb); L.hEff = take(off, nb); L.aEff = take(off, nb); L.acc = take(off, nb);
+  L.deg = take(off, sizeof(std::int32_t) * static_cast<std::size_t>(NN));
+  L.dV = take(off, cb);
+  L.q = take(off, cb);
+  L.tmp = take(off, nb);
+  L.passes = take(off, 5 * sizeof(double) * static_cast<std::size_t>(maxGroup) * static_cast<std::size_t>(W * kMaxLevelGroupsPerWarp));
+  L.hydro = take(off, 8 * 5 * sizeof(double));
+  L.misc = take(off, 4 * sizeof(std::int32_t));
+  L.merged = take(off, static_cast<std::size_t>(std::max(NG, 1)));
+  L.dry = take(off, static_cast<std::size_t>(std::max(NN, 1)));
+  L.list = take(off, sizeof(std::uint16_t) * static_cast<std::size_t>(std::max(NG, 1)));
+  L.pose = take(off, 2 * sizeof(Pose));
+  L.buoy = take(off, sizeof(Buoy));
+  L.parked = take(off, sizeof(Parked));
+  L.model = fleet ? take(off, sizeof(DevModel)) : 0u;
+  L.bytes = off;
+  return L;
+}
+
 // One compiled model on the device: its geometry in the kernel's layout (paired fields, the segment -> column gather
 // resolved, float copies), its node, group, connection, incidence, monitor and mark tables, and the DevModel that
 // points into them.
@@ -73,11 +103,11 @@ struct ModelDev {
   Incidence inc;
   MonitorLists mons;
   std::int32_t NN = 0, NC = 0, NG = 0, nmon = 0, nmark = 0, evCap = 0, maxGroup = 0;
-  DevBuf<double2> colXY, colLH, segXY, segLH;
-  DevBuf<float2> colXYf, colLHf, segXYf, segLHf;
-  DevBuf<float> colAf, segArf;
-  DevBuf<double> colA, segAr, mu, vmax, amin, aov;
-  DevBuf<std::int32_t> segStart, segCount, gStart, gCount, gNodes, ca, cb, skip, incStart, incCount, incConn, sea, monStart, monCount, monConn;
+  DevBuf<double2> colXY, colLH, segXY, segLH, exXY;
+  DevBuf<float2> colXYf, colLHf, segXYf, segLHf, exXYf;
+  DevBuf<float> colAf, segArf, exZf;
+  DevBuf<double> colA, segAr, exZ, mu, vmax, amin, aov;
+  DevBuf<std::int32_t> exStart, segStart, segCount, gStart, gCount, gNodes, ca, cb, skip, incStart, incCount, incConn, sea, monStart, monCount, monConn;
   DevBuf<std::uint8_t> gMode, law, incSide, mkWhen;
   DevBuf<double> gpx, gpy, gpz, kx, ky, kz, coef, mkx, mky, mkz;
   DevModel dm{};
@@ -120,6 +150,29 @@ struct ModelDev {
       colXYf.upload(cxyf, s); colLHf.upload(clhf, s); colAf.upload(caf, s);
       segXY.upload(sxy, s); segLH.upload(slh, s); segAr.upload(sa, s);
       segXYf.upload(sxyf, s); segLHf.upload(slhf, s); segArf.upload(saf, s);
+      // extent lists: set n < NN the segments of node n, set NN the hull's columns (points ns and up; tops only)
+      std::vector<std::int32_t> first(S.segStart), number(S.segCount);
+      first.push_back(static_cast<std::int32_t>(ns));
+      number.push_back(static_cast<std::int32_t>(nc));
+      auto xy = [&](std::int32_t i) { const auto k = static_cast<std::size_t>(i); return k < ns ? sxy[k] : cxy[k - ns]; };
+      auto lh = [&](std::int32_t i) { const auto k = static_cast<std::size_t>(i); return k < ns ? slh[k] : clh[k - ns]; };
+      const ExtentLists lists = extent_lists(
+          first, number, [&](std::int32_t i) { return xy(i).x; }, [&](std::int32_t i) { return xy(i).y; },
+          [&](std::int32_t i) { return lh(i).x; }, [&](std::int32_t i) { return lh(i).y; });
+      std::vector<double2> exy(lists.idx.size());
+      std::vector<float2> exyf(lists.idx.size());
+      std::vector<double> ez(lists.idx.size());
+      std::vector<float> ezf(lists.idx.size());
+      for (std::size_t l = 0; l + 1 < lists.start.size(); ++l) {
+        const bool top = (l / first.size()) & 1;
+        for (auto k = static_cast<std::size_t>(lists.start[l]); k < static_cast<std::size_t>(lists.start[l + 1]); ++k) {
+          exy[k] = xy(lists.idx[k]);
+          ez[k] = top ? lh(lists.idx[k]).y : lh(lists.idx[k]).x;
+          exyf[k] = float2{static_cast<float>(exy[k].x), static_cast<float>(exy[k].y)};
+          ezf[k] = static_cast<float>(ez[k]);
+        }
+      }
+      exStart.upload(lists.start, s); exXY.upload(exy, s); exZ.upload(ez, s); exXYf.upload(exyf, s); exZf.upload(ezf, s);
       check(cudaStreamSynchronize(s), "stream sync");
     }
     mu.upload(S.mu, s); vmax.upload(S.vmax, s); amin.upload(S.amin, s); aov.upload(S.aov, s);
@@ -146,6 +199,7 @@ struct ModelDev {
     d.nseg = S.segments();
     d.segXY = segXY.get(); d.segLH = segLH.get(); d.segAr = segAr.get();
     d.segXYf = segXYf.get(); d.segLHf = segLHf.get(); d.segArf = segArf.get();
+    d.exStart = exStart.get(); d.exXY = exXY.get(); d.exZ = exZ.get(); d.exXYf = exXYf.get(); d.exZf = exZf.get();
     d.nn = NN;
     d.mu = mu.get(); d.vmax = vmax.get(); d.amin = amin.get(); d.aov = aov.get();
     d.segStart = segStart.get(); d.segCount = segCount.get();

@@ -1,4 +1,4 @@
-// One time step of one simulation, computed by a team of W warps (W = 1, 2, 4 or 8). The physics is the reference's
+// One time step of one simulation, computed by a team of W warps (W = 1, 2, 4, 8 or 16). The physics is the reference's
 // kernel::step in the "portable" (double precision) and "portable32" (single-precision column partials) numerics
 // (engine/include/sinksim/kernel/step.hpp:41-54), reproduced bit for bit:
 //
@@ -7,7 +7,8 @@
 //     results in order (kernel/reduce.hpp:12-79, hydro.hpp:241-258). The team's warps share the eight groups: lane l
 //     holds partial w*32+l of group w, and a shuffle butterfly performs the tree, each pair combined as (lower, upper);
 //   * a node pass keeps the reference's 32 lane partials over strided segments and the same tree
-//     (hydro.hpp:305-316, reduce.hpp:52-71); a group of kLevelLanes lanes forms them, each lane combining several
+//     (hydro.hpp:305-316, reduce.hpp:52-71), except the lowest and highest point, which have the same bits however they
+//     are found (extents.h); a group of kLevelLanes lanes forms them, each lane combining several
 //     tree lanes' partials in the tree's order before the shuffles, so a warp solves 32 / kLevelLanes groups at once;
 //   * every other reduction (group sums, incidence gathers, sea inflow, excess, loads, monitors, water) runs in
 //     the reference's serial order, and every expression keeps its operation order (no contraction: -fmad=false).
@@ -61,14 +62,6 @@ template <class T>
 __device__ __forceinline__ T bsum(T v, int off, unsigned mask = kFull) { return v + __shfl_xor_sync(mask, v, off); }
 
 template <class T>
-__device__ __forceinline__ T bmin(T v, int off, int lane, unsigned mask = kFull) {
-  const T o = __shfl_xor_sync(mask, v, off);
-  const bool lower = (lane & off) == 0;
-  const T a = lower ? v : o, b = lower ? o : v;
-  return (b < a) ? b : a;
-}
-
-template <class T>
 __device__ __forceinline__ T bmax(T v, int off, int lane, unsigned mask = kFull) {
   const T o = __shfl_xor_sync(mask, v, off);
   const bool lower = (lane & off) == 0;
@@ -111,28 +104,22 @@ __device__ __forceinline__ void clip_column(T x, T y, T lo, T hi, T A, T R20, T 
   p.V += v; p.Mx += v * x; p.My += v * y; p.Mz += v * (lo + T(0.5) * s);
 }
 
-// One segment into a node-pass partial (kernel/reduce.hpp:52-71 in double, :144-164 in float).
+// One segment into a node-pass partial (kernel/reduce.hpp:52-71 in double, :144-164 in float) without the pass's world
+// extent, which comes from the extent lists (node_extreme). A dry segment adds zeros, which leaves every sum as it is
+// (a sum is never -0), so the lanes of a warp stay together.
 template <class T>
 struct SegPartial {
-  T vol, dv, mx, my, mz, zmin, zmax;
+  T vol, dv, mx, my, mz;
 };
 
 template <class T>
-__device__ __forceinline__ void clip_segment(T x, T y, T a, T b, T A, T R20, T R21, T R22, T tz, T iR, T h, SegPartial<T>& p) {
+__device__ __forceinline__ void clip_segment(T x, T y, T a, T b, T A, T R20, T R21, T tz, T iR, T h, SegPartial<T>& p) {
   const T base = R20 * x + R21 * y + tz;
-  const T wa = base + R22 * a, wb = base + R22 * b;
-  if (wa < p.zmin) p.zmin = wa;
-  if (wb > p.zmax) p.zmax = wb;
   const T zp = (h - base) * iR;
-  if (zp <= a) return;
-  T L;
-  if (zp >= b) {
-    L = b - a;
-  } else {
-    L = zp - a;
-    p.dv += A;
-  }
+  const bool dry = zp <= a, full = zp >= b;
+  const T L = dry ? T(0) : (full ? b - a : zp - a);
   const T v = A * L;
+  p.dv += (dry || full) ? T(0) : A;
   p.vol += v; p.mx += v * x; p.my += v * y; p.mz += v * (a + T(0.5) * L);
 }
 
@@ -258,10 +245,83 @@ __device__ __forceinline__ Buoy buoyancy(const DevModel& M, const Pose& F, const
   return buoyancy_finish(trees);
 }
 
+// ----------------------------------------------------------------------------- world extents
+
+// The lowest bottom (MAX false) or highest top (MAX true) of set n in the world: a node's segments, or the hull's
+// columns for n == M.nn (tops only). Scanned over the set's extent list for the signs of R20 and R21 (extents.h: the
+// same bits as over the whole set, for 4 to 10 points instead of 136), by `lanes` threads, this one taking every
+// lanes-th point from `sub`; the caller combines them. An attitude beyond a quarter turn (R22 < 0, only from a restored
+// state: the step clamps pitch and roll) scans the whole set.
+template <bool MIXED>
+struct Prec;
+template <>
+struct Prec<false> {
+  using T = double;
+  using V2 = double2;
+  static __device__ __forceinline__ const V2* exXY(const DevModel& M) { return M.exXY; }
+  static __device__ __forceinline__ const T* exZ(const DevModel& M) { return M.exZ; }
+  static __device__ __forceinline__ const V2* segXY(const DevModel& M) { return M.segXY; }
+  static __device__ __forceinline__ const V2* segLH(const DevModel& M) { return M.segLH; }
+  static __device__ __forceinline__ const T* segAr(const DevModel& M) { return M.segAr; }
+  static __device__ __forceinline__ const V2* colXY(const DevModel& M) { return M.colXY; }
+  static __device__ __forceinline__ const V2* colLH(const DevModel& M) { return M.colLH; }
+  static __device__ __forceinline__ T R20(const Pose& F) { return F.R20; }
+  static __device__ __forceinline__ T R21(const Pose& F) { return F.R21; }
+  static __device__ __forceinline__ T R22(const Pose& F) { return F.R22; }
+  static __device__ __forceinline__ T tz(const Pose& F) { return F.tz; }
+  static __device__ __forceinline__ T iR(const Pose& F) { return F.iR; }
+};
+template <>
+struct Prec<true> {
+  using T = float;
+  using V2 = float2;
+  static __device__ __forceinline__ const V2* exXY(const DevModel& M) { return M.exXYf; }
+  static __device__ __forceinline__ const T* exZ(const DevModel& M) { return M.exZf; }
+  static __device__ __forceinline__ const V2* segXY(const DevModel& M) { return M.segXYf; }
+  static __device__ __forceinline__ const V2* segLH(const DevModel& M) { return M.segLHf; }
+  static __device__ __forceinline__ const T* segAr(const DevModel& M) { return M.segArf; }
+  static __device__ __forceinline__ const V2* colXY(const DevModel& M) { return M.colXYf; }
+  static __device__ __forceinline__ const V2* colLH(const DevModel& M) { return M.colLHf; }
+  static __device__ __forceinline__ T R20(const Pose& F) { return F.fR20; }
+  static __device__ __forceinline__ T R21(const Pose& F) { return F.fR21; }
+  static __device__ __forceinline__ T R22(const Pose& F) { return F.fR22; }
+  static __device__ __forceinline__ T tz(const Pose& F) { return F.ftz; }
+  static __device__ __forceinline__ T iR(const Pose& F) { return F.fiR; }
+};
+
+template <bool MIXED, bool MAX>
+__device__ __forceinline__ typename Prec<MIXED>::T node_extreme(const DevModel& M, const Pose& F, int n, int sub, int lanes) {
+  using P = Prec<MIXED>;
+  using T = typename P::T;
+  const T R20 = P::R20(F), R21 = P::R21(F), R22 = P::R22(F), tz = P::tz(F);
+  const typename P::V2* xy = P::exXY(M);
+  const T* z = P::exZ(M);
+  int j, end, zs = 1;
+  if (F.R22 >= 0) {
+    const int list = ((F.R20 < 0 ? 2 : 0) + (F.R21 < 0 ? 4 : 0) + (MAX ? 1 : 0)) * (M.nn + 1) + n;
+    j = __ldg(M.exStart + list);
+    end = __ldg(M.exStart + list + 1);
+  } else {
+    const bool hull = n == M.nn;
+    xy = hull ? P::colXY(M) : P::segXY(M);
+    z = reinterpret_cast<const T*>(hull ? P::colLH(M) : P::segLH(M)) + (MAX ? 1 : 0);
+    zs = 2;
+    j = hull ? 0 : __ldg(M.segStart + n);
+    end = j + (hull ? M.ncol : __ldg(M.segCount + n));
+  }
+  T best = MAX ? T(-1e9) : T(1e9);
+  for (j += sub; j < end; j += lanes) {
+    const auto p = __ldg(xy + j);
+    const T w = R20 * p.x + R21 * p.y + tz + R22 * __ldg(z + static_cast<std::size_t>(j) * zs);
+    if (MAX ? w > best : w < best) best = w;
+  }
+  return best;
+}
+
 // ----------------------------------------------------------------------------- node pass (tree order)
 
 struct PassR {
-  double vol, dv, mx, my, mz, zmin, zmax;
+  double vol, dv, mx, my, mz;
 };
 
 // The kLevelLanes<MIXED> consecutive lanes of a warp that solve one group of nodes: `lane` is the lane in the warp, `sub` the
@@ -271,45 +331,26 @@ struct LevelLanes {
   unsigned mask;
 };
 
-// The partial of one lane of the 32-lane tree (the lane whose first segment is `first`): segments first + 32 k in
-// increasing k, two at a time.
-template <class T>
-__device__ __forceinline__ SegPartial<T> segment_partial(const typename Vec2<T>::type* xy, const typename Vec2<T>::type* ab, const T* area,
-                                                         int first, int end, T R20, T R21, T R22, T tz, T iR, T h) {
-  SegPartial<T> p{T(0), T(0), T(0), T(0), T(0), T(1e9), T(-1e9)};
-  int j = first;
-  for (; j + kLanes < end; j += 2 * kLanes) {
-    const auto a0 = __ldg(xy + j), b0 = __ldg(ab + j), a1 = __ldg(xy + j + kLanes), b1 = __ldg(ab + j + kLanes);
-    const T A0 = __ldg(area + j), A1 = __ldg(area + j + kLanes);
-    clip_segment<T>(a0.x, a0.y, b0.x, b0.y, A0, R20, R21, R22, tz, iR, h, p);
-    clip_segment<T>(a1.x, a1.y, b1.x, b1.y, A1, R20, R21, R22, tz, iR, h, p);
-  }
-  if (j < end) {
-    const auto a0 = __ldg(xy + j), b0 = __ldg(ab + j);
-    clip_segment<T>(a0.x, a0.y, b0.x, b0.y, __ldg(area + j), R20, R21, R22, tz, iR, h, p);
-  }
-  return p;
-}
-
-// The partials of two tree lanes 16 apart (first segments fa and fa + 16), in one loop: each iteration takes the next
-// segment of each, so the two accumulation chains run side by side; each keeps its own segments' order. fa's lane has
-// at most one segment more than the other's.
-template <class T>
-__device__ __forceinline__ void segment_pair(const typename Vec2<T>::type* xy, const typename Vec2<T>::type* ab, const T* area, int fa,
-                                             int end, T R20, T R21, T R22, T tz, T iR, T h, SegPartial<T>& pa, SegPartial<T>& pb) {
-  pa = SegPartial<T>{T(0), T(0), T(0), T(0), T(0), T(1e9), T(-1e9)};
+// The partials of two tree lanes OFF apart (first segments fa and fa + OFF; OFF 16, or 32 for fa's lane alone: then only
+// pa is formed, two of its segments per iteration), in one loop: each iteration takes the next segment of each, so the
+// two accumulation chains run side by side; each keeps its own segments' order.
+template <class T, bool PAIR>
+__device__ __forceinline__ void segment_partials(const typename Vec2<T>::type* xy, const typename Vec2<T>::type* ab, const T* area, int fa,
+                                                 int end, T R20, T R21, T tz, T iR, T h, SegPartial<T>& pa, SegPartial<T>& pb) {
+  constexpr int kStep = PAIR ? kLanes : 2 * kLanes, kOff = PAIR ? kLanes / 2 : kLanes;
+  pa = SegPartial<T>{T(0), T(0), T(0), T(0), T(0)};
   pb = pa;
   int ja = fa;
-  for (; ja + 16 < end; ja += kLanes) {
-    const int jb = ja + 16;
+  for (; ja + kOff < end; ja += kStep) {
+    const int jb = ja + kOff;
     const auto a0 = __ldg(xy + ja), b0 = __ldg(ab + ja), a1 = __ldg(xy + jb), b1 = __ldg(ab + jb);
     const T A0 = __ldg(area + ja), A1 = __ldg(area + jb);
-    clip_segment<T>(a0.x, a0.y, b0.x, b0.y, A0, R20, R21, R22, tz, iR, h, pa);
-    clip_segment<T>(a1.x, a1.y, b1.x, b1.y, A1, R20, R21, R22, tz, iR, h, pb);
+    clip_segment<T>(a0.x, a0.y, b0.x, b0.y, A0, R20, R21, tz, iR, h, pa);
+    clip_segment<T>(a1.x, a1.y, b1.x, b1.y, A1, R20, R21, tz, iR, h, PAIR ? pb : pa);
   }
   if (ja < end) {
     const auto a0 = __ldg(xy + ja), b0 = __ldg(ab + ja);
-    clip_segment<T>(a0.x, a0.y, b0.x, b0.y, __ldg(area + ja), R20, R21, R22, tz, iR, h, pa);
+    clip_segment<T>(a0.x, a0.y, b0.x, b0.y, __ldg(area + ja), R20, R21, tz, iR, h, pa);
   }
 }
 
@@ -318,58 +359,48 @@ __device__ __forceinline__ void segment_pair(const typename Vec2<T>::type* xy, c
 template <class T>
 __device__ __forceinline__ void tree_pair(SegPartial<T>& lo, const SegPartial<T>& up) {
   lo.vol = lo.vol + up.vol; lo.dv = lo.dv + up.dv; lo.mx = lo.mx + up.mx; lo.my = lo.my + up.my; lo.mz = lo.mz + up.mz;
-  lo.zmin = (up.zmin < lo.zmin) ? up.zmin : lo.zmin;
-  lo.zmax = (up.zmax > lo.zmax) ? up.zmax : lo.zmax;
 }
 
 // The node pass of node n at world level h: the 32 lane partials, the halving tree and the permeability scaling
-// (hydro.hpp:295-316 / 338-349). Lane `sub` of a group of LANES lanes forms the partials of tree lanes sub + LANES j
-// and combines them over the tree's upper levels (offsets 16 down to LANES) in registers; the lower levels are
-// shuffles inside the group. Every lane of the group ends with the bits of tree lane 0.
-template <class T, int LANES>
-__device__ __forceinline__ PassR node_pass_body(const int* segStart, const int* segCount, const double* muArr, const typename Vec2<T>::type* xy,
-                                                const typename Vec2<T>::type* ab, const T* area, T R20, T R21, T R22, T tz, T iR, double iRd,
-                                                int n, double h, const LevelLanes& L) {
-  const int s0 = __ldg(segStart + n), s1 = s0 + __ldg(segCount + n);
+// (hydro.hpp:295-316 / 338-349). Lane `sub` of a group of kLevelLanes lanes forms the partials of tree lanes
+// sub + kLevelLanes j and combines them over the tree's upper levels (offsets 16 down to kLevelLanes) in registers; the
+// lower levels are shuffles inside the group. Every lane of the group ends with the bits of tree lane 0. Every lane of
+// the warp calls it (n < 0: a group without a node, which sums nothing), so the groups' passes run side by side.
+template <bool MIXED>
+__device__ __forceinline__ PassR node_pass(const DevModel& M, const Pose& F, int n, double h, const LevelLanes& L) {
+  using P = Prec<MIXED>;
+  using T = typename P::T;
+  constexpr int LANES = kLevelLanes<MIXED>;
+  const int s0 = n < 0 ? 0 : __ldg(M.segStart + n), s1 = n < 0 ? 0 : s0 + __ldg(M.segCount + n);
   const T hT = static_cast<T>(h);
   const int f = s0 + L.sub;
-  SegPartial<T> p;
+  const T R20 = P::R20(F), R21 = P::R21(F), tz = P::tz(F), iR = P::iR(F);
+  const typename P::V2 *xy = P::segXY(M), *ab = P::segLH(M);
+  const T* area = P::segAr(M);
+  SegPartial<T> p, b;
   if constexpr (LANES == 32) {
-    p = segment_partial<T>(xy, ab, area, f, s1, R20, R21, R22, tz, iR, hT);
-  } else if constexpr (LANES == 16) {
-    SegPartial<T> b;
-    segment_pair<T>(xy, ab, area, f, s1, R20, R21, R22, tz, iR, hT, p, b);   // tree lanes sub and sub + 16
+    segment_partials<T, false>(xy, ab, area, f, s1, R20, R21, tz, iR, hT, p, b);
+  } else {
+    segment_partials<T, true>(xy, ab, area, f, s1, R20, R21, tz, iR, hT, p, b);  // tree lanes sub and sub + 16
     tree_pair(p, b);
-  } else if constexpr (LANES == 8) {
-    SegPartial<T> b, q, d;
-    segment_pair<T>(xy, ab, area, f, s1, R20, R21, R22, tz, iR, hT, p, b);      // sub and sub + 16
-    tree_pair(p, b);
-    segment_pair<T>(xy, ab, area, f + 8, s1, R20, R21, R22, tz, iR, hT, q, d);  // sub + 8 and sub + 24
-    tree_pair(q, d);
-    tree_pair(p, q);
+    if constexpr (LANES == 8) {
+      SegPartial<T> q;
+      segment_partials<T, true>(xy, ab, area, f + 8, s1, R20, R21, tz, iR, hT, q, b);  // sub + 8 and sub + 24
+      tree_pair(q, b);
+      tree_pair(p, q);
+    }
   }
 #pragma unroll
   for (int off = LANES / 2; off > 0; off >>= 1) {
-    p.vol = bsum(p.vol, off, L.mask); p.dv = bsum(p.dv, off, L.mask); p.mx = bsum(p.mx, off, L.mask);
-    p.my = bsum(p.my, off, L.mask); p.mz = bsum(p.mz, off, L.mask);
-    p.zmin = bmin(p.zmin, off, L.lane, L.mask); p.zmax = bmax(p.zmax, off, L.lane, L.mask);
+    p.vol = bsum(p.vol, off); p.dv = bsum(p.dv, off); p.mx = bsum(p.mx, off);
+    p.my = bsum(p.my, off); p.mz = bsum(p.mz, off);
   }
-  const double mu = __ldg(muArr + n);
+  const double mu = n < 0 ? 0.0 : __ldg(M.mu + n);
   PassR r;
   r.vol = static_cast<double>(p.vol) * mu;
-  r.dv = static_cast<double>(p.dv) * mu * iRd;
+  r.dv = static_cast<double>(p.dv) * mu * F.iR;
   r.mx = static_cast<double>(p.mx) * mu; r.my = static_cast<double>(p.my) * mu; r.mz = static_cast<double>(p.mz) * mu;
-  r.zmin = static_cast<double>(p.zmin); r.zmax = static_cast<double>(p.zmax);
   return r;
-}
-
-template <bool MIXED>
-__device__ __forceinline__ PassR node_pass(const DevModel& M, const Pose& F, int n, double h, const LevelLanes& L) {
-  if constexpr (!MIXED)
-    return node_pass_body<double, kLevelLanes<false>>(M.segStart, M.segCount, M.mu, M.segXY, M.segLH, M.segAr, F.R20, F.R21, F.R22, F.tz, F.iR, F.iR, n, h, L);
-  else
-    return node_pass_body<float, kLevelLanes<true>>(M.segStart, M.segCount, M.mu, M.segXYf, M.segLHf, M.segArf, F.fR20, F.fR21, F.fR22, F.ftz, F.fiR, F.iR, n, h,
-                                 L);
 }
 
 // ----------------------------------------------------------------------------- per-warp view of the slot in shared memory
@@ -380,7 +411,10 @@ struct Slot {
   int* misc;
   PassR* passes;
   std::uint8_t* merged;
-  Pose* pose;
+  std::uint8_t* dry;          // NodeFlag bits
+  std::uint16_t* list;        // the groups the next level solve visits, misc[kMiscListed] of them
+  Pose* pose;                 // the current step's pose, and
+  Pose* prev;                 // the last step's (that of the last level solve, between steps)
   Buoy* buoy;
   Parked* parked;
   const unsigned char* cols;  // the column table staged in the block's shared memory, or null (read from global)
@@ -400,13 +434,16 @@ __device__ __forceinline__ Slot carve_slot(unsigned char* base, const SlotLayout
   s.acc = reinterpret_cast<double*>(base + L.acc);
   s.dV = reinterpret_cast<double*>(base + L.dV);
   s.q = reinterpret_cast<double*>(base + L.q);
-  s.tmp = L.tmp == kSlotAliasDV ? s.dV : reinterpret_cast<double*>(base + L.tmp);
+  s.tmp = reinterpret_cast<double*>(base + L.tmp);
   s.deg = reinterpret_cast<int*>(base + L.deg);
   s.hydro = reinterpret_cast<double*>(base + L.hydro);
   s.misc = reinterpret_cast<int*>(base + L.misc);
   s.passes = reinterpret_cast<PassR*>(base + L.passes);
   s.merged = base + L.merged;
+  s.dry = base + L.dry;
+  s.list = reinterpret_cast<std::uint16_t*>(base + L.list);
   s.pose = reinterpret_cast<Pose*>(base + L.pose);
+  s.prev = s.pose + 1;
   s.buoy = reinterpret_cast<Buoy*>(base + L.buoy);
   s.parked = reinterpret_cast<Parked*>(base + L.parked);
   s.cols = nullptr;
@@ -414,147 +451,113 @@ __device__ __forceinline__ Slot carve_slot(unsigned char* base, const SlotLayout
 }
 
 // ----------------------------------------------------------------------------- free-surface levels (kernel/levels.hpp)
-// Group-uniform: the lanes of a level lane group run the solver on identical pass results and store identical values.
-// Each solver is a loop around its one node-pass call site, in stages: the passes at the starting level, then either
-// the passes at the top of a full node or group (for the centroids) or the passes of the bracketed Newton iteration.
+// What bounds the solve is the number of instructions a step issues, so it visits only the groups that hold water: at
+// the end of a step one warp lists them (list_groups), and the lane groups of the team take them from the list. An
+// empty node's level is its lowest segment bottom at the pose of the solve, which nothing reads before the node gets
+// water or is written out; it is formed then (stale_level), from the pose kept for that. A listed unit (a merged group
+// or one node) takes its world extent from the extent lists first, so the pass the reference makes only for the extent
+// of a full node, or of one whose starting level lies outside it, is not made. Every pass of a warp's lane groups runs
+// through one call site under a warp-wide loop: two half-warps in different solvers would otherwise issue everything
+// twice. Centroids are divided node by node afterwards, a thread per node (team_step).
+// Measured on B200: 2,048 titanic64 instances of the uneven batch to 20 min 512 ms (805 ms with a pass over every
+// segment of every node, a divergent solver per half-warp and the extents in the pass), 264 liner runs to 15 min 119 ms
+// (152), one titanic64 run to 5 min 35.1 ms (40.5).
 
-__device__ __forceinline__ void set_centroid(Slot& S, int n, const PassR& p) {
-  if (p.vol > kCentroidMinVolume) { S.cx[n] = p.mx / p.vol; S.cy[n] = p.my / p.vol; S.cz[n] = p.mz / p.vol; }
-}
+// S.dry[n].
+enum NodeFlag : std::uint8_t {
+  kStale = 1,      // empty at the last level solve: S.level[n] is not formed yet
+  kEmptyNode = 2,  // empty at the coming one
+  kZeroVolume = 4, // ... in a merged group, which empties its members
+  kSolved = 8      // passes were made for it at this one
+};
 
-enum SolveStage { kStageFirst, kStageFull, kStageNewton };
+// S.misc: the claimed instance, the yield flag, the level solve's counter of list entries taken, the list's length.
+enum MiscSlot { kMiscInstance = 0, kMiscYield = 1, kMiscTaken = 2, kMiscListed = 3 };
 
-// Where a step's forward computation records what its reverse (the adjoint, adjoint_kernel.cu) needs: every node pass of
-// the level solve (node, pass number within the node's solve, level, result) and the solved levels. The batch kernels
-// pass NoTape, whose hooks are empty and compile away.
+// Where a step's forward computation records what its reverse (the adjoint, adjoint_kernel.cu) needs: every unit's start
+// (starting level and world extent), every node pass of the level solve (node, pass number within the node's solve,
+// level, result) and the solved levels. kLazy: empty nodes are left out of the solve, their levels formed on demand.
+// The batch kernels pass NoTape, whose hooks are empty and compile away.
 struct NoTape {
+  static constexpr bool kLazy = true;
+  __device__ __forceinline__ void start(int, double, double, double, const LevelLanes&) const {}
   __device__ __forceinline__ void pass(int, int, double, const PassR&, const LevelLanes&) const {}
   template <int W>
   __device__ __forceinline__ void solved(const DevModel&, const Slot&, const Team<W>&) const {}
 };
 
-// One node (levels.hpp:13-49).
-template <bool MIXED, class Tape>
-__device__ __forceinline__ void solve_single(const DevModel& M, const Pose& F, Slot& S, int n, const LevelLanes& L, const Tape& tape) {
-  const double V = S.vol[n], Vmax = __ldg(M.vmax + n);
-  const double tol = jmax(1e-3 * Vmax, 0.5);
-  double h = S.level[n];
-  double hi = 0, a = 0, b = 0;
-  int stage = kStageFirst, it = 0, slot = 0;
-  PassR p;
-  for (;;) {
-    p = node_pass<MIXED>(M, F, n, h, L);
-    tape.pass(n, slot++, h, p, L);
-    if (stage == kStageFirst) {
-      const double lo = p.zmin;
-      hi = p.zmax;
-      S.zmax[n] = hi;
-      if (V <= kEmptyVolume) { S.level[n] = lo; S.area[n] = 0; return; }
-      if (V >= Vmax * kFullFraction) { stage = kStageFull; h = hi; continue; }
-      stage = kStageNewton;
-      a = lo; b = hi;
-      if (h < lo || h > hi) { h = jmin(hi, jmax(lo, h)); continue; }
-    } else if (stage == kStageFull) {
-      const double aov = __ldg(M.aov + n);
-      S.level[n] = hi + jmax(0.0, V - Vmax) / aov;
-      S.area[n] = aov;
-      set_centroid(S, n, p);
-      return;
+// Lists the groups the next level solve visits, in increasing order, and flags the nodes of the others; one warp calls
+// it. A group is left out (kLazy) when neither its members nor their sum exceed the empty volume: then the solve would
+// find it empty merged or not.
+template <bool LAZY>
+__device__ __forceinline__ void list_groups(const DevModel& M, Slot& S, int lane) {
+  int count = 0;
+  for (int g0 = 0; g0 < M.ng; g0 += kLanes) {
+    const int g = g0 + lane;
+    bool live = false;
+    if (g < M.ng) {
+      const int N = __ldg(M.gCount + g);
+      const int* m = M.gNodes + __ldg(M.gStart + g);
+      double V = 0;
+      live = !LAZY;
+      for (int k = 0; k < N; ++k) {
+        const double v = S.vol[__ldg(m + k)];
+        V += v;
+        if (!(v <= kEmptyVolume)) live = true;
+      }
+      if (!(V <= kEmptyVolume)) live = true;
+      if (!live) {
+        const bool merged = N >= 2 && __ldg(M.gMode + g) == 1;
+        S.merged[g] = merged ? 1 : 0;
+        for (int k = 0; k < N; ++k) S.dry[__ldg(m + k)] |= kEmptyNode | (merged ? kZeroVolume : 0);
+      }
     }
-    // Newton: p is the pass at h, the it-th of at most kNewtonFast after the starting one
-    if (it == kNewtonFast) break;
-    const double err = p.vol - V;
-    if (fabs(err) < tol) break;
-    if (err > 0) b = h; else a = h;
-    double hn = p.dv > kSlopeMin ? h - err / p.dv : 0.5 * (a + b);
-    if (!(hn > a && hn < b)) hn = 0.5 * (a + b);
-    h = hn;
-    ++it;
+    const unsigned mask = __ballot_sync(kFull, live);
+    if (live) S.list[count + __popc(mask & ((1u << lane) - 1u))] = static_cast<std::uint16_t>(g);
+    count += __popc(mask);
   }
-  S.level[n] = h; S.area[n] = p.dv;
-  set_centroid(S, n, p);
+  if (lane == 0) S.misc[kMiscListed] = count;
 }
 
-// A merged group of N nodes at one common level (levels.hpp:54-162); P holds the members' passes.
-template <bool MIXED, class Tape>
-__device__ __forceinline__ void solve_group(const DevModel& M, const Pose& F, Slot& S, PassR* P, const int* m, int N, const LevelLanes& L,
-                                            const Tape& tape) {
-  double V = 0, Vmax = 0;
-  for (int k = 0; k < N; ++k) { V += S.vol[__ldg(m + k)]; Vmax += __ldg(M.vmax + __ldg(m + k)); }
-  bool allWet = true;
-  int firstWet = -1;
-  for (int k = 0; k < N; ++k) {
-    if (S.vol[__ldg(m + k)] > 0) { if (firstWet < 0) firstWet = k; }
-    else allWet = false;
+// A group's combined value of node_extreme over its lanes.
+template <bool MIXED, bool MAX>
+__device__ __forceinline__ double group_extreme(const DevModel& M, const Pose& F, int n, const LevelLanes& L) {
+  constexpr int LANES = kLevelLanes<MIXED>;
+  auto v = node_extreme<MIXED, MAX>(M, F, n, L.sub, LANES);
+#pragma unroll
+  for (int off = LANES / 2; off > 0; off >>= 1) {
+    const auto o = __shfl_xor_sync(L.mask, v, off);
+    if (MAX ? o > v : o < v) v = o;
   }
-  double h;
-  if (allWet) {
-    double s = 0;
-    for (int k = 0; k < N; ++k) s += S.level[__ldg(m + k)];
-    h = s / static_cast<double>(N);
-  } else {
-    h = S.level[__ldg(m + (firstWet >= 0 ? firstWet : N - 1))];
-  }
-  const double tol = jmax(1e-3 * Vmax, 0.5);
-  double hi = 0, a = 0, b = 0, dh = 0;
-  int stage = kStageFirst, it = 0, slot = 0;
-  for (;;) {
-    for (int k = 0; k < N; ++k) {
-      P[k] = node_pass<MIXED>(M, F, __ldg(m + k), h, L);
-      tape.pass(__ldg(m + k), slot, h, P[k], L);
-    }
-    ++slot;
-    if (stage == kStageFirst) {
-      for (int k = 0; k < N; ++k) S.zmax[__ldg(m + k)] = P[k].zmax;
-      double lo = P[0].zmin;
-      hi = P[0].zmax;
-      for (int k = 1; k < N; ++k) { if (P[k].zmin < lo) lo = P[k].zmin; if (P[k].zmax > hi) hi = P[k].zmax; }
-      if (V <= kEmptyVolume) {
-        for (int k = 0; k < N; ++k) { const int n = __ldg(m + k); S.vol[n] = 0; S.level[n] = P[k].zmin; S.area[n] = 0; }
-        return;
-      }
-      if (V >= Vmax * kFullFraction) {
-        const double over = jmax(0.0, V - Vmax);
-        double aSum = 0;
-        for (int k = 0; k < N; ++k) aSum += __ldg(M.aov + __ldg(m + k));
-        dh = over / aSum;
-        double assigned = 0;
-        for (int k = 0; k < N - 1; ++k) {
-          const int n = __ldg(m + k);
-          const double v = __ldg(M.vmax + n) + dh * __ldg(M.aov + n);
-          S.vol[n] = v;
-          assigned += v;
-        }
-        S.vol[__ldg(m + N - 1)] = V - assigned;
-        stage = kStageFull;
-        h = hi;
-        continue;
-      }
-      stage = kStageNewton;
-      a = lo; b = hi;
-      if (!(h >= lo && h <= hi)) { h = jmin(hi, jmax(lo, h)); continue; }
-    } else if (stage == kStageFull) {
-      for (int k = 0; k < N; ++k) {
-        const int n = __ldg(m + k);
-        S.level[n] = hi + dh; S.area[n] = __ldg(M.aov + n);
-        set_centroid(S, n, P[k]);
-      }
-      return;
-    }
-    // Newton on the members' summed volume: P holds the passes at h
-    if (it == kNewtonFast) break;
-    double sum = 0;
-    for (int k = 0; k < N; ++k) sum += P[k].vol;
-    const double err = sum - V;
-    if (fabs(err) < tol) break;
-    if (err > 0) b = h; else a = h;
-    double dvs = 0;
-    for (int k = 0; k < N; ++k) dvs += P[k].dv;
-    double hn = dvs > kSlopeMin ? h - err / dvs : 0.5 * (a + b);
-    if (!(hn > a && hn < b)) hn = 0.5 * (a + b);
-    h = hn;
-    ++it;
-  }
+  return static_cast<double>(v);
+}
+
+// Node n's level as the last solve left it (an empty node's is formed here); one thread, or a lane group.
+template <bool MIXED>
+__device__ __forceinline__ double stale_level(const DevModel& M, const Slot& S, int n) {
+  return (S.dry[n] & kStale) ? static_cast<double>(node_extreme<MIXED, false>(M, *S.prev, n, 0, 1)) : S.level[n];
+}
+
+template <bool MIXED>
+__device__ __forceinline__ double group_level(const DevModel& M, const Slot& S, int n, const LevelLanes& L) {
+  return (S.dry[n] & kStale) ? group_extreme<MIXED, false>(M, *S.prev, n, L) : S.level[n];
+}
+
+// The solved values of a node whose last pass was p: the pass's sums go to scratch arrays that are dead until the heads,
+// where the node's thread divides the centroid (set_centroid).
+__device__ __forceinline__ void store_solved(Slot& S, int n, double level, double area, const PassR& p) {
+  S.level[n] = level; S.area[n] = area;
+  S.acc[n] = p.vol; S.hEff[n] = p.mx; S.aEff[n] = p.my; S.tmp[n] = p.mz;
+}
+
+__device__ __forceinline__ void set_centroid(Slot& S, int n) {
+  const double vol = S.acc[n];
+  if (vol > kCentroidMinVolume) { S.cx[n] = S.hEff[n] / vol; S.cy[n] = S.aEff[n] / vol; S.cz[n] = S.tmp[n] / vol; }
+}
+
+// The volumes and solved values of a merged group of N nodes after its Newton iteration (levels.hpp:113-162); P holds
+// the members' last passes, V their water. One lane.
+__device__ __forceinline__ void share_group(const DevModel& M, Slot& S, const PassR* P, const int* m, int N, double V, double h) {
   double tot = 0;
   for (int k = 0; k < N; ++k) tot += P[k].vol;
   double assigned = 0;
@@ -589,16 +592,13 @@ __device__ __forceinline__ void solve_group(const DevModel& M, const Pose& F, Sl
     for (int k = 0; k < N - 1; ++k) assigned += S.vol[__ldg(m + k)];
   }
   S.vol[__ldg(m + N - 1)] = V - assigned;
-  for (int k = 0; k < N; ++k) {
-    const int n = __ldg(m + k);
-    S.level[n] = h; S.area[n] = P[k].dv;
-    set_centroid(S, n, P[k]);
-  }
+  for (int k = 0; k < N; ++k) store_solved(S, __ldg(m + k), h, P[k].dv, P[k]);
 }
 
-// Groups are independent (a group's solve reads and writes only its members), so the team's level lane groups take
-// them in turn: lane group u of the team (32 / kLevelLanes<MIXED> per warp) solves groups u, u + 32 W / kLevelLanes, ...
-// (the reference's block gave them to its eight warps, device_step.cuh:270-281).
+// The level solve of the listed groups (levels.hpp:13-194). Groups are independent (a group's solve reads and writes only
+// its members), so the team's level lane groups (32 / kLevelLanes<MIXED> per warp) take them as they come: each starts
+// with the list entry of its own index, then takes the next one from the team's counter (S.misc[kMiscTaken]); groups
+// take different numbers of passes, and a node's results do not depend on which lane group computes them.
 template <bool MIXED, int W, class Tape>
 __device__ __forceinline__ void solve_levels(const DevModel& M, const Pose& F, Slot& S, const Team<W>& T, const Tape& tape) {
   constexpr int LANES = kLevelLanes<MIXED>, PER_WARP = 32 / LANES;
@@ -609,35 +609,162 @@ __device__ __forceinline__ void solve_levels(const DevModel& M, const Pose& F, S
   if constexpr (LANES == 32) L.mask = kFull;
   else L.mask = ((1u << LANES) - 1u) << (grp * LANES);
   const int unit = T.warp * PER_WARP + grp;
-  PassR* P = S.passes + static_cast<std::size_t>(unit) * M.maxGroup;
-  // each lane group starts with the group of its own index, then takes the next one from the team's counter
-  // (S.misc[2], set to the number of lane groups at the start of the step): the groups take different numbers of
-  // passes, and a node's results do not depend on which lane group computes them
-  for (int g = unit; g < M.ng;) {
-    const int N = __ldg(M.gCount + g);
-    const int* m = M.gNodes + __ldg(M.gStart + g);
-    const int mode = __ldg(M.gMode + g);
-    bool merged = false;
-    if (N >= 2) {
-      if (mode == 1) {
-        merged = true;
-      } else if (mode == 2) {
-        const double zMw = world_z(F, __ldg(M.gpx + g), __ldg(M.gpy + g), __ldg(M.gpz + g));
-        merged = true;
-        for (int k = 0; k < N; ++k) {
-          const int n = __ldg(m + k);
-          if (!(S.vol[n] > kEmptyVolume && S.level[n] > zMw + M.gMargin)) { merged = false; break; }
+  PassR* const P = S.passes + static_cast<std::size_t>(unit) * M.maxGroup;
+  const int listed = S.misc[kMiscListed];
+  int i = unit;                                // the next list entry
+  const int* m = nullptr;                      // the current group's members,
+  int N = 0, j = 0, units = 0;                 // their number, its next unit and its units
+  bool merged = false;
+  // the current unit: nm members from mm, and where its solve is
+  const int* mm = nullptr;
+  int nm = 0, k = 0, slot = 0, it = 0;
+  bool have = false, full = false;
+  double V = 0, tol = 0, h = 0, a = 0, b = 0, sum = 0, dvs = 0;
+  for (;;) {
+    while (!have && (j < units || i < listed)) {
+      if (j >= units) {
+        const int g = S.list[i];
+        int next = 0;
+        if (L.sub == 0) next = atomicAdd(&S.misc[kMiscTaken], 1);
+        i = __shfl_sync(L.mask, next, grp * LANES);
+        N = __ldg(M.gCount + g);
+        m = M.gNodes + __ldg(M.gStart + g);
+        merged = false;
+        if (N >= 2) {
+          const int mode = __ldg(M.gMode + g);
+          if (mode == 1) {
+            merged = true;
+          } else if (mode == 2) {
+            const double zMw = world_z(F, __ldg(M.gpx + g), __ldg(M.gpy + g), __ldg(M.gpz + g));
+            merged = true;
+            for (int q = 0; q < N; ++q) {
+              const int n = __ldg(m + q);
+              if (!(S.vol[n] > kEmptyVolume && group_level<MIXED>(M, S, n, L) > zMw + M.gMargin)) { merged = false; break; }
+            }
+          }
+        }
+        if (L.sub == 0) S.merged[g] = merged ? 1 : 0;
+        units = merged ? 1 : N;
+        j = 0;
+        if (units == 0) continue;  // a group without members
+      }
+      mm = merged ? m : m + j;
+      nm = merged ? N : 1;
+      ++j;
+      double Vmax = 0;
+      V = 0;
+      for (int q = 0; q < nm; ++q) { const int n = __ldg(mm + q); V += S.vol[n]; Vmax += __ldg(M.vmax + n); }
+      const bool empty = V <= kEmptyVolume;
+      if constexpr (Tape::kLazy) {
+        if (empty) {
+          if (L.sub == 0)
+            for (int q = 0; q < nm; ++q) S.dry[__ldg(mm + q)] = (S.dry[__ldg(mm + q)] & kStale) | kEmptyNode | (merged ? kZeroVolume : 0);
+          continue;
         }
       }
+      if (!merged) {
+        h = group_level<MIXED>(M, S, __ldg(mm), L);
+      } else {
+        bool allWet = true;
+        int firstWet = -1;
+        for (int q = 0; q < nm; ++q) {
+          if (S.vol[__ldg(mm + q)] > 0) { if (firstWet < 0) firstWet = q; }
+          else allWet = false;
+        }
+        if (allWet) {
+          double s = 0;
+          for (int q = 0; q < nm; ++q) s += group_level<MIXED>(M, S, __ldg(mm + q), L);
+          h = s / static_cast<double>(nm);
+        } else {
+          h = group_level<MIXED>(M, S, __ldg(mm + (firstWet >= 0 ? firstWet : nm - 1)), L);
+        }
+      }
+      double lo = 0, hi = 0;
+      for (int q = 0; q < nm; ++q) {
+        const int n = __ldg(mm + q);
+        const double zlo = group_extreme<MIXED, false>(M, F, n, L), zhi = group_extreme<MIXED, true>(M, F, n, L);
+        tape.start(n, h, zlo, zhi, L);
+        if (q == 0 || zlo < lo) lo = zlo;
+        if (q == 0 || zhi > hi) hi = zhi;
+        if (L.sub == 0) {
+          S.zmax[n] = zhi;
+          S.dry[n] = empty ? kEmptyNode | (merged ? kZeroVolume : 0) : kSolved;
+          if (empty) S.level[n] = zlo;
+        }
+      }
+      if (empty) continue;
+      full = V >= Vmax * kFullFraction;
+      it = 0; slot = 0; k = 0; sum = 0; dvs = 0;
+      if (full) {
+        // the pass at the top of a full unit, for its centroids; its level and volumes first
+        double dh = 0;
+        if (!merged) {
+          dh = jmax(0.0, V - Vmax) / __ldg(M.aov + __ldg(mm));
+        } else {
+          const double over = jmax(0.0, V - Vmax);
+          double aSum = 0;
+          for (int q = 0; q < nm; ++q) aSum += __ldg(M.aov + __ldg(mm + q));
+          dh = over / aSum;
+          if (L.sub == 0) {
+            double assigned = 0;
+            for (int q = 0; q < nm - 1; ++q) {
+              const int n = __ldg(mm + q);
+              const double v = __ldg(M.vmax + n) + dh * __ldg(M.aov + n);
+              S.vol[n] = v;
+              assigned += v;
+            }
+            S.vol[__ldg(mm + nm - 1)] = V - assigned;
+          }
+        }
+        a = hi + dh;  // the level
+        h = hi;
+        slot = 1;
+      } else {
+        tol = jmax(1e-3 * Vmax, 0.5);
+        a = lo; b = hi;
+        if (merged ? !(h >= lo && h <= hi) : (h < lo || h > hi)) {
+          h = jmin(hi, jmax(lo, h));
+          slot = 1;
+        }
+      }
+      have = true;
     }
-    S.merged[g] = merged ? 1 : 0;
-    if (merged) solve_group<MIXED>(M, F, S, P, m, N, L, tape);
-    else for (int k = 0; k < N; ++k) solve_single<MIXED>(M, F, S, __ldg(m + k), L, tape);
-    int next = 0;
-    if (L.sub == 0) next = atomicAdd(&S.misc[2], 1);
-    g = __shfl_sync(L.mask, next, grp * LANES);
+    if (!__any_sync(kFull, have)) break;
+    const int n = have ? __ldg(mm + k) : -1;
+    const PassR p = node_pass<MIXED>(M, F, n, h, L);
+    if (!have) continue;
+    tape.pass(n, slot, h, p, L);
+    if (full) {
+      if (L.sub == 0) store_solved(S, n, a, __ldg(M.aov + n), p);
+      if (++k == nm) have = false;
+      continue;
+    }
+    sum += p.vol;
+    dvs += p.dv;
+    if (nm > 1) {
+      if (L.sub == 0) P[k] = p;
+      if (++k < nm) continue;
+      k = 0;
+    }
+    ++slot;
+    // Newton on the unit's volume: sum and dvs are its passes at h, the it-th after the starting one
+    const double err = sum - V;
+    if (it < kNewtonFast && !(fabs(err) < tol)) {
+      if (err > 0) b = h; else a = h;
+      double hn = dvs > kSlopeMin ? h - err / dvs : 0.5 * (a + b);
+      if (!(hn > a && hn < b)) hn = 0.5 * (a + b);
+      h = hn;
+      ++it;
+      sum = 0; dvs = 0;
+      continue;
+    }
+    if (L.sub == 0) {
+      if (nm == 1 && !merged) store_solved(S, n, h, p.dv, p);
+      else share_group(M, S, P, mm, nm, V, h);
+    }
+    have = false;
   }
-  __syncwarp();  // the lane groups leave the loop after different numbers of groups
+  __syncwarp();
 }
 
 // ----------------------------------------------------------------------------- flows (kernel/flows.hpp:38-78)
@@ -793,17 +920,26 @@ __device__ __forceinline__ void team_step(const DevModel& M, const Pose& F, SimR
     solve_levels<MIXED, W>(M, F, S, T, tape);
     T.sync();
   }
-  // the group counter for the next step's level solve (read after this step's later barriers)
-  if (T.leader()) S.misc[2] = W * (32 / kLevelLanes<MIXED>);
-  tape.solved(M, S, T);
+  // the list counter for the next step's level solve (read after this step's later barriers)
+  if (T.leader()) S.misc[kMiscTaken] = W * (32 / kLevelLanes<MIXED>);
 
-  // effective heads and areas, then degrees (flows.hpp:15-35)
+  // the solve's ends node by node (an empty node's area, a wet one's centroid), effective heads and areas, then degrees
+  // (flows.hpp:15-35)
   for (int n = rank; n < M.nn; n += kStride) {
+    const int flags = S.dry[n];
+    S.dry[n] = (Tape::kLazy && (flags & kEmptyNode)) ? kStale : 0;
+    if (flags & kEmptyNode) {
+      S.area[n] = 0;
+      if (flags & kZeroVolume) S.vol[n] = 0;
+    } else if (flags & kSolved) {
+      set_centroid(S, n);
+    }
     const double v = S.vol[n];
     S.hEff[n] = v > kEmptyVolume ? S.level[n] : kNoHead;
     S.aEff[n] = v >= __ldg(M.vmax + n) ? __ldg(M.aov + n) : jmax(S.area[n], __ldg(M.amin + n));
     S.deg[n] = 0;
   }
+  tape.solved(M, S, T);  // a thread reads the nodes it has just finished
   T.sync();
   // A node's degree is the number of its incident connections that are enabled and not between two empty spaces. Each
   // such connection counts once at each of its nodes (the incidence lists hold it once at a when a >= 0 and once at b),
@@ -836,7 +972,9 @@ __device__ __forceinline__ void team_step(const DevModel& M, const Pose& F, SimR
     const double vm = __ldg(M.vmax + n);
     double excess = 0;
     if (v > vm) {
-      const double head = jmax(0.0, -S.zmax[n]);
+      // (a node that was empty at the solve has no extent yet)
+      const double zmax = (S.dry[n] & kStale) ? static_cast<double>(node_extreme<MIXED, true>(M, F, n, 0, 1)) : S.zmax[n];
+      const double head = jmax(0.0, -zmax);
       const double cap = vm + __ldg(M.aov + n) * head;
       if (v > cap) { excess = v - cap; v = cap; }
     }
@@ -847,6 +985,9 @@ __device__ __forceinline__ void team_step(const DevModel& M, const Pose& F, SimR
   for (int k = 0; k < M.nsea; ++k) seaIn += S.dV[__ldg(M.sea + k)];
   T.sync();
   unpark(S.parked, R);
+  if constexpr (Tape::kLazy) {
+    if (T.warp == W - 1) list_groups<true>(M, S, lane);
+  }
   // the excess returns to the sea in node order (flows.hpp:114-118)
   for (int n0 = 0; n0 < M.nn; n0 += kLanes) {
     const int n = n0 + lane;
