@@ -209,7 +209,7 @@ constexpr int kMaxLevelGroupsPerWarp = 32 / (kLevelLanes<false> < kLevelLanes<tr
 
 // Byte offsets of one simulation slot (one team of warps) in dynamic shared memory; `bytes` is the slot stride.
 // passes holds maxGroup node-pass results per level lane group of the team (up to kMaxLevelGroupsPerWarp per warp); hydro the
-// eight buoyancy tree results; misc the team's small broadcast values and counters (MiscSlot); dry a flag byte per node and
+// eight buoyancy tree results and the hull top; misc the team's small broadcast values and counters (MiscSlot); dry a flag byte per node and
 // list the groups the next level solve visits (warp_step.cuh); pose (this step's and the last one's) and buoy the step's
 // pose and buoyancy result, which every phase reads (kept here rather than in each thread's registers); parked the run's
 // values during the hydrostatic phases; model (fleets only) the team's copy of its instance's model. tmp is the sixth

@@ -81,7 +81,7 @@ inline SlotLayout slot_layout(std::int32_t NN, std::int32_t NC, std::int32_t NG,
   L.q = take(off, cb);
   L.tmp = take(off, nb);
   L.passes = take(off, 5 * sizeof(double) * static_cast<std::size_t>(maxGroup) * static_cast<std::size_t>(W * kMaxLevelGroupsPerWarp));
-  L.hydro = take(off, 8 * 5 * sizeof(double));
+  L.hydro = take(off, 33 * sizeof(double));
   L.misc = take(off, 4 * sizeof(std::int32_t));
   L.merged = take(off, static_cast<std::size_t>(std::max(NG, 1)));
   L.dry = take(off, static_cast<std::size_t>(std::max(NN, 1)));

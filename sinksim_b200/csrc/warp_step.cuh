@@ -5,7 +5,7 @@
 //   * the buoyancy integral keeps the reference's 256 partial sums (partial p sums columns p, p+256, ... in
 //     order), reduces each group of 32 partials with the halving tree (offsets 16..1) and adds the eight group
 //     results in order (kernel/reduce.hpp:12-79, hydro.hpp:241-258). The team's warps share the eight groups: lane l
-//     holds partial w*32+l of group w, and a shuffle butterfly performs the tree, each pair combined as (lower, upper);
+//     holds partial w*32+l of group w, and a shuffle butterfly performs the tree;
 //   * a node pass keeps the reference's 32 lane partials over strided segments and the same tree
 //     (hydro.hpp:305-316, reduce.hpp:52-71), except the lowest and highest point, which have the same bits however they
 //     are found (extents.h); a group of kLevelLanes lanes forms them, each lane combining several
@@ -55,19 +55,11 @@ __device__ __forceinline__ double world_z(const Pose& F, double x, double y, dou
 
 // ----------------------------------------------------------------------------- butterfly steps of the canonical tree
 // At offset `off` the tree combines partial l (l < off) with partial l + off. With xor shuffles every lane pairs
-// with lane ^ off; sums are exact to swap (IEEE addition is commutative) and the min / max keep the reference's
-// operand order (lower partner first), so every lane ends with the bits of the tree's lane 0.
+// with lane ^ off; sums are exact to swap (IEEE addition is commutative), so every lane ends with the bits of the tree's
+// lane 0.
 
 template <class T>
 __device__ __forceinline__ T bsum(T v, int off, unsigned mask = kFull) { return v + __shfl_xor_sync(mask, v, off); }
-
-template <class T>
-__device__ __forceinline__ T bmax(T v, int off, int lane, unsigned mask = kFull) {
-  const T o = __shfl_xor_sync(mask, v, off);
-  const bool lower = (lane & off) == 0;
-  const T a = lower ? v : o, b = lower ? o : v;
-  return (b > a) ? b : a;
-}
 
 // ----------------------------------------------------------------------------- a team of W warps stepping one simulation
 
@@ -83,23 +75,99 @@ struct Team {
   __device__ __forceinline__ bool leader() const { return rank == 0; }
 };
 
+// ----------------------------------------------------------------------------- world extents
+
+// The lowest bottom (MAX false) or highest top (MAX true) of set n in the world: a node's segments, or the hull's
+// columns for n == M.nn (tops only). Scanned over the set's extent list for the signs of R20 and R21 (extents.h: the
+// same bits as over the whole set, for 4 to 10 points instead of 136), by `lanes` threads, this one taking every
+// lanes-th point from `sub`; the caller combines them. An attitude beyond a quarter turn (R22 < 0, only from a restored
+// state: the step clamps pitch and roll) scans the whole set.
+template <bool MIXED>
+struct Prec;
+template <>
+struct Prec<false> {
+  using T = double;
+  using V2 = double2;
+  static __device__ __forceinline__ const V2* exXY(const DevModel& M) { return M.exXY; }
+  static __device__ __forceinline__ const T* exZ(const DevModel& M) { return M.exZ; }
+  static __device__ __forceinline__ const V2* segXY(const DevModel& M) { return M.segXY; }
+  static __device__ __forceinline__ const V2* segLH(const DevModel& M) { return M.segLH; }
+  static __device__ __forceinline__ const T* segAr(const DevModel& M) { return M.segAr; }
+  static __device__ __forceinline__ const V2* colXY(const DevModel& M) { return M.colXY; }
+  static __device__ __forceinline__ const V2* colLH(const DevModel& M) { return M.colLH; }
+  static __device__ __forceinline__ const T* colAr(const DevModel& M) { return M.colA; }
+  static __device__ __forceinline__ T R20(const Pose& F) { return F.R20; }
+  static __device__ __forceinline__ T R21(const Pose& F) { return F.R21; }
+  static __device__ __forceinline__ T R22(const Pose& F) { return F.R22; }
+  static __device__ __forceinline__ T tz(const Pose& F) { return F.tz; }
+  static __device__ __forceinline__ T iR(const Pose& F) { return F.iR; }
+};
+template <>
+struct Prec<true> {
+  using T = float;
+  using V2 = float2;
+  static __device__ __forceinline__ const V2* exXY(const DevModel& M) { return M.exXYf; }
+  static __device__ __forceinline__ const T* exZ(const DevModel& M) { return M.exZf; }
+  static __device__ __forceinline__ const V2* segXY(const DevModel& M) { return M.segXYf; }
+  static __device__ __forceinline__ const V2* segLH(const DevModel& M) { return M.segLHf; }
+  static __device__ __forceinline__ const T* segAr(const DevModel& M) { return M.segArf; }
+  static __device__ __forceinline__ const V2* colXY(const DevModel& M) { return M.colXYf; }
+  static __device__ __forceinline__ const V2* colLH(const DevModel& M) { return M.colLHf; }
+  static __device__ __forceinline__ const T* colAr(const DevModel& M) { return M.colAf; }
+  static __device__ __forceinline__ T R20(const Pose& F) { return F.fR20; }
+  static __device__ __forceinline__ T R21(const Pose& F) { return F.fR21; }
+  static __device__ __forceinline__ T R22(const Pose& F) { return F.fR22; }
+  static __device__ __forceinline__ T tz(const Pose& F) { return F.ftz; }
+  static __device__ __forceinline__ T iR(const Pose& F) { return F.fiR; }
+};
+
+template <bool MIXED, bool MAX>
+__device__ __forceinline__ typename Prec<MIXED>::T node_extreme(const DevModel& M, const Pose& F, int n, int sub, int lanes) {
+  using P = Prec<MIXED>;
+  using T = typename P::T;
+  const T R20 = P::R20(F), R21 = P::R21(F), R22 = P::R22(F), tz = P::tz(F);
+  const typename P::V2* xy = P::exXY(M);
+  const T* z = P::exZ(M);
+  int j, end, zs = 1;
+  if (F.R22 >= 0) {
+    const int list = ((F.R20 < 0 ? 2 : 0) + (F.R21 < 0 ? 4 : 0) + (MAX ? 1 : 0)) * (M.nn + 1) + n;
+    j = __ldg(M.exStart + list);
+    end = __ldg(M.exStart + list + 1);
+  } else {
+    const bool hull = n == M.nn;
+    xy = hull ? P::colXY(M) : P::segXY(M);
+    z = reinterpret_cast<const T*>(hull ? P::colLH(M) : P::segLH(M)) + (MAX ? 1 : 0);
+    zs = 2;
+    j = hull ? 0 : __ldg(M.segStart + n);
+    end = j + (hull ? M.ncol : __ldg(M.segCount + n));
+  }
+  T best = MAX ? T(-1e9) : T(1e9);
+  for (j += sub; j < end; j += lanes) {
+    const auto p = __ldg(xy + j);
+    const T w = R20 * p.x + R21 * p.y + tz + R22 * __ldg(z + static_cast<std::size_t>(j) * zs);
+    if (MAX ? w > best : w < best) best = w;
+  }
+  return best;
+}
+
 // ----------------------------------------------------------------------------- buoyancy (hydro pass, tree order)
 
 // One column into a buoyancy partial (kernel/reduce.hpp:39-49 in double, :131-142 in float): the same expressions in
-// the same order for T = double (portable) and T = float (portable32).
+// the same order for T = double (portable) and T = float (portable32). The hull's highest point is not formed here but
+// from the columns' extent list (node_extreme: 24 to 41 points on titanic64 for 4,408), and a dry column adds zeros,
+// which leaves every sum as it is. The loop is bound by the instructions it issues; with both out of it, on B200:
+// 2,048 uneven titanic64 runs to 20 min 493 ms against 512, a fleet of 96 ships to 5 min 63.6 against 68.7, one run to
+// 5 min 33.4 against 35.1.
 template <class T>
 struct ColPartial {
-  T V, Mx, My, Mz, top;
+  T V, Mx, My, Mz;
 };
 
 template <class T>
-__device__ __forceinline__ void clip_column(T x, T y, T lo, T hi, T A, T R20, T R21, T R22, T tz, T iR, ColPartial<T>& p) {
+__device__ __forceinline__ void clip_column(T x, T y, T lo, T hi, T A, T R20, T R21, T tz, T iR, ColPartial<T>& p) {
   const T base = R20 * x + R21 * y + tz;
-  const T wt = base + R22 * hi;
-  if (wt > p.top) p.top = wt;
   const T zp = -base * iR;
-  if (zp <= lo) return;
-  const T s = zp >= hi ? hi - lo : zp - lo;
+  const T s = zp <= lo ? T(0) : (zp >= hi ? hi - lo : zp - lo);
   const T v = A * s;
   p.V += v; p.Mx += v * x; p.My += v * y; p.Mz += v * (lo + T(0.5) * s);
 }
@@ -139,18 +207,18 @@ __device__ __forceinline__ P load_col(const P* p) {
 // column issue before the first is clipped; the clips stay in order).
 template <class T, bool SMEM = false>
 __device__ __forceinline__ ColPartial<T> column_partial(const typename Vec2<T>::type* xy, const typename Vec2<T>::type* lh, const T* area,
-                                                        int ncol, int first, T R20, T R21, T R22, T tz, T iR) {
-  ColPartial<T> p{T(0), T(0), T(0), T(0), T(-1e9)};
+                                                        int ncol, int first, T R20, T R21, T tz, T iR) {
+  ColPartial<T> p{T(0), T(0), T(0), T(0)};
   int i = first;
   for (; i + 256 < ncol; i += 512) {
     const auto a0 = load_col<SMEM>(xy + i), b0 = load_col<SMEM>(lh + i), a1 = load_col<SMEM>(xy + i + 256), b1 = load_col<SMEM>(lh + i + 256);
     const T A0 = load_col<SMEM>(area + i), A1 = load_col<SMEM>(area + i + 256);
-    clip_column<T>(a0.x, a0.y, b0.x, b0.y, A0, R20, R21, R22, tz, iR, p);
-    clip_column<T>(a1.x, a1.y, b1.x, b1.y, A1, R20, R21, R22, tz, iR, p);
+    clip_column<T>(a0.x, a0.y, b0.x, b0.y, A0, R20, R21, tz, iR, p);
+    clip_column<T>(a1.x, a1.y, b1.x, b1.y, A1, R20, R21, tz, iR, p);
   }
   if (i < ncol) {
     const auto a0 = load_col<SMEM>(xy + i), b0 = load_col<SMEM>(lh + i);
-    clip_column<T>(a0.x, a0.y, b0.x, b0.y, load_col<SMEM>(area + i), R20, R21, R22, tz, iR, p);
+    clip_column<T>(a0.x, a0.y, b0.x, b0.y, load_col<SMEM>(area + i), R20, R21, tz, iR, p);
   }
   return p;
 }
@@ -175,66 +243,57 @@ __host__ __device__ __forceinline__ StagedColumns<T> staged_columns(int ncol) {
   return c;
 }
 
-// The eight trees are spread over the team's warps (warp v computes trees v, v + W, ...); the tree results meet in
-// shared memory and every thread adds them in the reference's order (trees 0..7).
+// The eight trees are spread over the team's warps (warp v computes trees v, v + W, ...), and the last warp finds the
+// hull's highest point; the results meet in shared memory (four values per tree, then the top) and every thread adds
+// them in the reference's order (trees 0..7).
 template <bool MIXED, int W>
 __device__ __forceinline__ void buoyancy_trees(const DevModel& M, const Pose& F, const Team<W>& T, double* trees, const unsigned char* cols) {
+  using P = Prec<MIXED>;
+  using R = typename P::T;
   const int lane = T.lane;
   for (int w = T.warp; w < 8; w += W) {
-    double g[5];
-    if constexpr (!MIXED) {
-      ColPartial<double> p;
-      if (cols) {
-        const StagedColumns<double> c = staged_columns<double>(M.ncol);
-        p = column_partial<double, true>(reinterpret_cast<const double2*>(cols + c.xy), reinterpret_cast<const double2*>(cols + c.lh),
-                                         reinterpret_cast<const double*>(cols + c.area), M.ncol, w * kLanes + lane, F.R20, F.R21, F.R22, F.tz, F.iR);
-      } else {
-        p = column_partial<double>(M.colXY, M.colLH, M.colA, M.ncol, w * kLanes + lane, F.R20, F.R21, F.R22, F.tz, F.iR);
-      }
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        p.V = bsum(p.V, off); p.Mx = bsum(p.Mx, off); p.My = bsum(p.My, off); p.Mz = bsum(p.Mz, off);
-        p.top = bmax(p.top, off, lane);
-      }
-      g[0] = p.V; g[1] = p.Mx; g[2] = p.My; g[3] = p.Mz; g[4] = p.top;
+    ColPartial<R> p;
+    if (cols) {
+      const StagedColumns<R> c = staged_columns<R>(M.ncol);
+      p = column_partial<R, true>(reinterpret_cast<const typename P::V2*>(cols + c.xy), reinterpret_cast<const typename P::V2*>(cols + c.lh),
+                                  reinterpret_cast<const R*>(cols + c.area), M.ncol, w * kLanes + lane, P::R20(F), P::R21(F), P::tz(F), P::iR(F));
     } else {
-      ColPartial<float> p;
-      if (cols) {
-        const StagedColumns<float> c = staged_columns<float>(M.ncol);
-        p = column_partial<float, true>(reinterpret_cast<const float2*>(cols + c.xy), reinterpret_cast<const float2*>(cols + c.lh),
-                                        reinterpret_cast<const float*>(cols + c.area), M.ncol, w * kLanes + lane, F.fR20, F.fR21, F.fR22, F.ftz, F.fiR);
-      } else {
-        p = column_partial<float>(M.colXYf, M.colLHf, M.colAf, M.ncol, w * kLanes + lane, F.fR20, F.fR21, F.fR22, F.ftz, F.fiR);
-      }
+      p = column_partial<R>(P::colXY(M), P::colLH(M), P::colAr(M), M.ncol, w * kLanes + lane, P::R20(F), P::R21(F), P::tz(F), P::iR(F));
+    }
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        p.V = bsum(p.V, off); p.Mx = bsum(p.Mx, off); p.My = bsum(p.My, off); p.Mz = bsum(p.Mz, off);
-        p.top = bmax(p.top, off, lane);
-      }
-      g[0] = p.V; g[1] = p.Mx; g[2] = p.My; g[3] = p.Mz; g[4] = p.top;
+    for (int off = 16; off > 0; off >>= 1) {
+      p.V = bsum(p.V, off); p.Mx = bsum(p.Mx, off); p.My = bsum(p.My, off); p.Mz = bsum(p.Mz, off);
     }
     if (lane == 0) {
-      double* t = trees + 5 * w;
-      for (int k = 0; k < 5; ++k) t[k] = g[k];
+      double* t = trees + 4 * w;
+      t[0] = p.V; t[1] = p.Mx; t[2] = p.My; t[3] = p.Mz;
     }
+  }
+  if (T.warp == W - 1) {
+    R top = node_extreme<MIXED, true>(M, F, M.nn, lane, kLanes);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      const R o = __shfl_xor_sync(kFull, top, off);
+      if (o > top) top = o;
+    }
+    if (lane == 0) trees[32] = top;
   }
 }
 
 // The buoyancy result from the eight trees (after a team barrier that follows buoyancy_trees): every thread adds
 // them in the reference's order and holds the same values.
 __device__ __forceinline__ Buoy buoyancy_finish(const double* trees) {
-  double V = trees[0], Mx = trees[1], My = trees[2], Mz = trees[3], top = trees[4];
+  double V = trees[0], Mx = trees[1], My = trees[2], Mz = trees[3];
   for (int w = 1; w < 8; ++w) {
-    const double* t = trees + 5 * w;
+    const double* t = trees + 4 * w;
     V += t[0]; Mx += t[1]; My += t[2]; Mz += t[3];
-    if (t[4] > top) top = t[4];
   }
   Buoy b;
   b.V = V;
   b.x = V > 0 ? Mx / V : 0;
   b.y = V > 0 ? My / V : 0;
   b.z = V > 0 ? Mz / V : 0;
-  b.top = top;
+  b.top = trees[32];
   return b;
 }
 
@@ -243,79 +302,6 @@ __device__ __forceinline__ Buoy buoyancy(const DevModel& M, const Pose& F, const
   buoyancy_trees<MIXED, W>(M, F, T, trees, cols);
   T.sync();
   return buoyancy_finish(trees);
-}
-
-// ----------------------------------------------------------------------------- world extents
-
-// The lowest bottom (MAX false) or highest top (MAX true) of set n in the world: a node's segments, or the hull's
-// columns for n == M.nn (tops only). Scanned over the set's extent list for the signs of R20 and R21 (extents.h: the
-// same bits as over the whole set, for 4 to 10 points instead of 136), by `lanes` threads, this one taking every
-// lanes-th point from `sub`; the caller combines them. An attitude beyond a quarter turn (R22 < 0, only from a restored
-// state: the step clamps pitch and roll) scans the whole set.
-template <bool MIXED>
-struct Prec;
-template <>
-struct Prec<false> {
-  using T = double;
-  using V2 = double2;
-  static __device__ __forceinline__ const V2* exXY(const DevModel& M) { return M.exXY; }
-  static __device__ __forceinline__ const T* exZ(const DevModel& M) { return M.exZ; }
-  static __device__ __forceinline__ const V2* segXY(const DevModel& M) { return M.segXY; }
-  static __device__ __forceinline__ const V2* segLH(const DevModel& M) { return M.segLH; }
-  static __device__ __forceinline__ const T* segAr(const DevModel& M) { return M.segAr; }
-  static __device__ __forceinline__ const V2* colXY(const DevModel& M) { return M.colXY; }
-  static __device__ __forceinline__ const V2* colLH(const DevModel& M) { return M.colLH; }
-  static __device__ __forceinline__ T R20(const Pose& F) { return F.R20; }
-  static __device__ __forceinline__ T R21(const Pose& F) { return F.R21; }
-  static __device__ __forceinline__ T R22(const Pose& F) { return F.R22; }
-  static __device__ __forceinline__ T tz(const Pose& F) { return F.tz; }
-  static __device__ __forceinline__ T iR(const Pose& F) { return F.iR; }
-};
-template <>
-struct Prec<true> {
-  using T = float;
-  using V2 = float2;
-  static __device__ __forceinline__ const V2* exXY(const DevModel& M) { return M.exXYf; }
-  static __device__ __forceinline__ const T* exZ(const DevModel& M) { return M.exZf; }
-  static __device__ __forceinline__ const V2* segXY(const DevModel& M) { return M.segXYf; }
-  static __device__ __forceinline__ const V2* segLH(const DevModel& M) { return M.segLHf; }
-  static __device__ __forceinline__ const T* segAr(const DevModel& M) { return M.segArf; }
-  static __device__ __forceinline__ const V2* colXY(const DevModel& M) { return M.colXYf; }
-  static __device__ __forceinline__ const V2* colLH(const DevModel& M) { return M.colLHf; }
-  static __device__ __forceinline__ T R20(const Pose& F) { return F.fR20; }
-  static __device__ __forceinline__ T R21(const Pose& F) { return F.fR21; }
-  static __device__ __forceinline__ T R22(const Pose& F) { return F.fR22; }
-  static __device__ __forceinline__ T tz(const Pose& F) { return F.ftz; }
-  static __device__ __forceinline__ T iR(const Pose& F) { return F.fiR; }
-};
-
-template <bool MIXED, bool MAX>
-__device__ __forceinline__ typename Prec<MIXED>::T node_extreme(const DevModel& M, const Pose& F, int n, int sub, int lanes) {
-  using P = Prec<MIXED>;
-  using T = typename P::T;
-  const T R20 = P::R20(F), R21 = P::R21(F), R22 = P::R22(F), tz = P::tz(F);
-  const typename P::V2* xy = P::exXY(M);
-  const T* z = P::exZ(M);
-  int j, end, zs = 1;
-  if (F.R22 >= 0) {
-    const int list = ((F.R20 < 0 ? 2 : 0) + (F.R21 < 0 ? 4 : 0) + (MAX ? 1 : 0)) * (M.nn + 1) + n;
-    j = __ldg(M.exStart + list);
-    end = __ldg(M.exStart + list + 1);
-  } else {
-    const bool hull = n == M.nn;
-    xy = hull ? P::colXY(M) : P::segXY(M);
-    z = reinterpret_cast<const T*>(hull ? P::colLH(M) : P::segLH(M)) + (MAX ? 1 : 0);
-    zs = 2;
-    j = hull ? 0 : __ldg(M.segStart + n);
-    end = j + (hull ? M.ncol : __ldg(M.segCount + n));
-  }
-  T best = MAX ? T(-1e9) : T(1e9);
-  for (j += sub; j < end; j += lanes) {
-    const auto p = __ldg(xy + j);
-    const T w = R20 * p.x + R21 * p.y + tz + R22 * __ldg(z + static_cast<std::size_t>(j) * zs);
-    if (MAX ? w > best : w < best) best = w;
-  }
-  return best;
 }
 
 // ----------------------------------------------------------------------------- node pass (tree order)
