@@ -30,6 +30,9 @@ HOST_FLAGS = "-fPIC,-ffp-contract=off,-fno-fast-math,-fexcess-precision=standard
 NVCC_FLAGS = ARCH + ["-O3", "-std=c++17", "-fmad=false", "-lineinfo", "-Xptxas", "-v", "-diag-suppress", "222",
                      "-Xcompiler", HOST_FLAGS, "-I" + os.path.join(ROOT, "include"), "-I" + CSRC]
 
+# The batch kernel's instantiations, one unit per team size and per kind of batch (each takes about half a minute).
+INSTANCES = [("batch_kernel_inst.cu", f"batch_kernel_w{w}{'_fleet' if fleet else ''}",
+              [f"-DSSB_INST_WARPS={w}", f"-DSSB_INST_FLEET={'true' if fleet else 'false'}"]) for w in (1, 2, 4, 8, 16) for fleet in (False, True)]
 SOURCES = ["batch_kernel.cu", "adjoint_kernel.cu", "portable_math.cu", "probes.cu", "batch.cpp", "adjoint.cpp", "model.cpp", "json.cpp",
            "sweep.cpp", "capi.cpp"]
 APPS = ["sinksim_cuda_run", "sinksim_sweep"]
@@ -42,8 +45,8 @@ def nvcc():
     raise RuntimeError("nvcc not found")
 
 
-def _compile(src, obj, log):
-    cmd = [nvcc()] + NVCC_FLAGS + ["-x", "cu" if src.endswith(".cu") else "c++", "-c", src, "-o", obj]
+def _compile(src, obj, log, defines=()):
+    cmd = [nvcc()] + NVCC_FLAGS + list(defines) + ["-x", "cu" if src.endswith(".cu") else "c++", "-c", src, "-o", obj]
     if not src.endswith(".cu"):
         # host-only C++ through nvcc: same flags, no device code
         cmd = [nvcc()] + [f for f in NVCC_FLAGS if f not in ("-lineinfo",)] + ["-c", src, "-o", obj]
@@ -68,12 +71,14 @@ def build(jobs=8, force=False, verbose=False):
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]
     headers.append(os.path.join(ROOT, "include", "sinksim_b200.h"))
     objs, todo = [], []
-    for s in SOURCES:
+    # the longest compiles first: the adjoint kernel, then the batch kernel's instantiations
+    for s, name, defines in [(s, s, []) for s in SOURCES if s == "adjoint_kernel.cu"] + INSTANCES + \
+            [(s, s, []) for s in SOURCES if s != "adjoint_kernel.cu"]:
         src = os.path.join(CSRC, s)
-        obj = os.path.join(BUILD, s + ".o")
+        obj = os.path.join(BUILD, name + ".o")
         objs.append(obj)
         if force or _stale(obj, [src] + headers):
-            todo.append((src, obj, os.path.join(BUILD, s + ".log")))
+            todo.append((src, obj, os.path.join(BUILD, name + ".log"), defines))
     with cf.ThreadPoolExecutor(max_workers=jobs) as ex:
         for f in [ex.submit(_compile, *t) for t in todo]:
             f.result()
@@ -92,9 +97,8 @@ def build(jobs=8, force=False, verbose=False):
             if r.returncode != 0:
                 raise RuntimeError(f"building {app} failed:\n{r.stdout}{r.stderr}")
     if verbose:
-        for s in SOURCES:
-            if s.endswith(".cu"):
-                print(open(os.path.join(BUILD, s + ".log")).read())
+        for s in [s for s in SOURCES if s.endswith(".cu")] + [name for _, name, _ in INSTANCES]:
+            print(open(os.path.join(BUILD, s + ".log")).read())
     return LIB
 
 

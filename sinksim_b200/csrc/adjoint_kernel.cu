@@ -183,7 +183,7 @@ __device__ __forceinline__ void load_state(const double* c, SimRegs& R, Slot& S,
     S.dry[n] = 0;
   }
   for (int g = T.rank; g < M.ng; g += 32 * W) S.merged[g] = 0;
-  for (int c2 = T.rank; c2 < M.nc; c2 += 32 * W) { S.dV[c2] = 0; S.q[c2] = 0; }
+  for (int c2 = T.rank; c2 < M.nc; c2 += 32 * W) S.dV[c2] = 0;
   T.sync();
   if (T.warp == W - 1) list_groups<false>(M, S, T.lane);  // every group, for the whole run
   T.sync();

@@ -210,13 +210,13 @@ constexpr int kMaxLevelGroupsPerWarp = 32 / (kLevelLanes<false> < kLevelLanes<tr
 // Byte offsets of one simulation slot (one team of warps) in dynamic shared memory; `bytes` is the slot stride.
 // passes holds maxGroup node-pass results per level lane group of the team (up to kMaxLevelGroupsPerWarp per warp); hydro the
 // eight buoyancy tree results and the hull top; misc the team's small broadcast values and counters (MiscSlot); dry a flag byte per node and
-// list the groups the next level solve visits (warp_step.cuh); pose (this step's and the last one's) and buoy the step's
+// list the groups the next level solve visits, flow the connections that can flow (warp_step.cuh); pose (this step's and the last one's) and buoy the step's
 // pose and buoyancy result, which every phase reads (kept here rather than in each thread's registers); parked the run's
 // values during the hydrostatic phases; model (fleets only) the team's copy of its instance's model. tmp is the sixth
 // column of the loads' per-node terms (the other five reuse area, zmax, hEff, aEff and acc, which are dead by then) and,
 // between the level solve and the heads, of the passes' sums.
 struct SlotLayout {
-  std::uint32_t vol, level, cx, cy, cz, area, zmax, hEff, aEff, acc, deg, dV, q, tmp, passes, hydro, misc, merged, dry, list, pose, buoy, parked,
+  std::uint32_t vol, level, cx, cy, cz, area, zmax, hEff, aEff, acc, deg, dV, flow, tmp, passes, hydro, misc, merged, dry, list, pose, buoy, parked,
       model, bytes;
 };
 

@@ -67,7 +67,7 @@ inline std::uint32_t take(std::uint32_t& off, std::size_t bytes) {
 }
 
 // The shared-memory slot of one simulation of a model of these sizes, stepped by a team of W warps: per-node state and
-// scratch, per-connection dV and q, the group-pass buffers, the buoyancy tree results, the poses, buoyancy result and
+// scratch, the connections' flows and their list, the group-pass buffers, the buoyancy tree results, the poses, buoyancy result and
 // parked run values, and in a fleet the team's copy of its instance's model.
 inline SlotLayout slot_layout(std::int32_t NN, std::int32_t NC, std::int32_t NG, std::int32_t maxGroup, int W, bool fleet) {
   SlotLayout L{};
@@ -78,11 +78,11 @@ inline SlotLayout slot_layout(std::int32_t NN, std::int32_t NC, std::int32_t NG,
   L.area = take(off, nb); L.zmax = take(off, nb); L.hEff = take(off, nb); L.aEff = take(off, nb); L.acc = take(off, nb);
   L.deg = take(off, sizeof(std::int32_t) * static_cast<std::size_t>(NN));
   L.dV = take(off, cb);
-  L.q = take(off, cb);
+  L.flow = take(off, sizeof(std::uint16_t) * static_cast<std::size_t>(std::max(NC, 1)));
   L.tmp = take(off, nb);
   L.passes = take(off, 5 * sizeof(double) * static_cast<std::size_t>(maxGroup) * static_cast<std::size_t>(W * kMaxLevelGroupsPerWarp));
   L.hydro = take(off, 33 * sizeof(double));
-  L.misc = take(off, 4 * sizeof(std::int32_t));
+  L.misc = take(off, 8 * sizeof(std::int32_t));
   L.merged = take(off, static_cast<std::size_t>(std::max(NG, 1)));
   L.dry = take(off, static_cast<std::size_t>(std::max(NN, 1)));
   L.list = take(off, sizeof(std::uint16_t) * static_cast<std::size_t>(std::max(NG, 1)));

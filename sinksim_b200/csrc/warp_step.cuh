@@ -392,13 +392,14 @@ __device__ __forceinline__ PassR node_pass(const DevModel& M, const Pose& F, int
 // ----------------------------------------------------------------------------- per-warp view of the slot in shared memory
 
 struct Slot {
-  double *vol, *level, *cx, *cy, *cz, *area, *zmax, *hEff, *aEff, *acc, *dV, *q, *tmp, *hydro;
+  double *vol, *level, *cx, *cy, *cz, *area, *zmax, *hEff, *aEff, *acc, *dV, *tmp, *hydro;
   int* deg;
   int* misc;
   PassR* passes;
   std::uint8_t* merged;
   std::uint8_t* dry;          // NodeFlag bits
   std::uint16_t* list;        // the groups the next level solve visits, misc[kMiscListed] of them
+  std::uint16_t* flow;        // the connections that can flow in this step (sort_connections)
   Pose* pose;                 // the current step's pose, and
   Pose* prev;                 // the last step's (that of the last level solve, between steps)
   Buoy* buoy;
@@ -419,7 +420,7 @@ __device__ __forceinline__ Slot carve_slot(unsigned char* base, const SlotLayout
   s.aEff = reinterpret_cast<double*>(base + L.aEff);
   s.acc = reinterpret_cast<double*>(base + L.acc);
   s.dV = reinterpret_cast<double*>(base + L.dV);
-  s.q = reinterpret_cast<double*>(base + L.q);
+  s.flow = reinterpret_cast<std::uint16_t*>(base + L.flow);
   s.tmp = reinterpret_cast<double*>(base + L.tmp);
   s.deg = reinterpret_cast<int*>(base + L.deg);
   s.hydro = reinterpret_cast<double*>(base + L.hydro);
@@ -457,8 +458,9 @@ enum NodeFlag : std::uint8_t {
   kSolved = 8      // passes were made for it at this one
 };
 
-// S.misc: the claimed instance, the yield flag, the level solve's counter of list entries taken, the list's length.
-enum MiscSlot { kMiscInstance = 0, kMiscYield = 1, kMiscTaken = 2, kMiscListed = 3 };
+// S.misc: the claimed instance, the yield flag, the level solve's counter of list entries taken, the list's length, the
+// numbers of flows at the front and at the back of their list.
+enum MiscSlot { kMiscInstance = 0, kMiscYield = 1, kMiscTaken = 2, kMiscListed = 3, kMiscFront = 4, kMiscBack = 5, kMiscSlots = 8 };
 
 // Where a step's forward computation records what its reverse (the adjoint, adjoint_kernel.cu) needs: every unit's start
 // (starting level and world extent), every node pass of the level solve (node, pass number within the node's solve,
@@ -754,16 +756,53 @@ __device__ __forceinline__ void solve_levels(const DevModel& M, const Pose& F, S
 }
 
 // ----------------------------------------------------------------------------- flows (kernel/flows.hpp:38-78)
+// Of a hull's connections most join two dry spaces or stand above the water (about 230 of titanic64's 290 early in a
+// run), and a warp of 32 mixed ones issues the orifice's, the weir's and the submerged weir's code (two pow) one after
+// the other. Teams of up to four warps, of which many share an SM and issue slots bound it, therefore sort them first
+// (sort_connections): the ones that can flow go into a list whose front holds orifices and free weirs and whose back
+// holds submerged weirs, the others' flow is zero; then the listed ones are computed, a warp's lanes in one class.
+// Larger teams have a thread for every connection of such a hull and are bound by the chain of dependent steps: they
+// form every flow while they count the degrees, and limit it after the barrier (team_step). A node's reciprocal area is
+// divided once, and a monitor divides the flows it sums itself (the step kept every connection's quotient before).
+// On B200: 2,048 uneven titanic64 runs to 20 min 469 ms against 493 (two-warp teams); one run to 5 min 32.2 against 33.4
+// (the sorted form in its 16-warp team: 35.4), 264 liner runs to 15 min 113 against 114 (sorted: 123).
 
-__device__ __forceinline__ double connection_flow(const DevModel& M, const Pose& F, double t, const Slot& S, const std::uint8_t* en,
-                                                  const double* area, const double* tOn, int c, double& qOut) {
-  if (!__ldg(en + c) || __ldg(tOn + c) > t) { qOut = 0; return 0; }
-  const int sk = __ldg(M.skip + c);
-  if (sk >= 0 && S.merged[sk]) { qOut = 0; return 0; }
+// The heads over connection c's opening at its two ends.
+struct FlowHeads {
+  int a, b;
+  double zo, Ha, Hb;
+};
+
+__device__ __forceinline__ FlowHeads flow_heads(const DevModel& M, const Pose& F, const Slot& S, int c) {
+  FlowHeads f;
+  f.a = __ldg(M.ca + c);
+  f.b = __ldg(M.cb + c);
+  f.zo = F.R20 * __ldg(M.kx + c) + F.R21 * __ldg(M.ky + c) + F.R22 * __ldg(M.kz + c) + F.tz;
+  const double ha = f.a < 0 ? 0.0 : S.hEff[f.a], hb = S.hEff[f.b];
+  f.Ha = ha > f.zo ? ha - f.zo : 0.0;
+  f.Hb = hb > f.zo ? hb - f.zo : 0.0;
+  return f;
+}
+
+// A node's degree is the number of its incident connections that are enabled and not between two empty spaces. Each such
+// connection counts once at each of its nodes (the incidence lists hold it once at a when a >= 0 and once at b), counted
+// per connection with shared-memory atomics: an integer count, the same in any order, and one round of independent loads
+// instead of a walk down every node's incidence list. Returns whether connection c may flow at time t (an uncounted one
+// cannot: both its ends are empty).
+template <class IP>
+__device__ __forceinline__ bool count_degrees(const DevModel& M, double t, Slot& S, const IP& I, int c) {
+  if (!__ldg(I.en() + c)) return false;
   const int a = __ldg(M.ca + c), b = __ldg(M.cb + c);
-  const double zo = F.R20 * __ldg(M.kx + c) + F.R21 * __ldg(M.ky + c) + F.R22 * __ldg(M.kz + c) + F.tz;
-  const double ha = a < 0 ? 0.0 : S.hEff[a], hbv = S.hEff[b];
-  const double Ha = ha > zo ? ha - zo : 0.0, Hb = hbv > zo ? hbv - zo : 0.0;
+  if (a >= 0 && S.hEff[a] < kNoHeadTest && S.hEff[b] < kNoHeadTest) return false;
+  if (a >= 0) atomicAdd(&S.deg[a], 1);
+  atomicAdd(&S.deg[b], 1);
+  const int sk = __ldg(M.skip + c);
+  return !(__ldg(I.tOn() + c) > t) && !(sk >= 0 && S.merged[sk]);
+}
+
+// The volume that connection c's law sends through it in the step, a to b.
+__device__ __forceinline__ double law_volume(const DevModel& M, const FlowHeads& f, const double* area, int c) {
+  const double Ha = f.Ha, Hb = f.Hb;
   double q = 0;
   if (__ldg(M.law + c) == 0) {
     const double d = Ha - Hb;
@@ -772,27 +811,79 @@ __device__ __forceinline__ double connection_flow(const DevModel& M, const Pose&
     const double H1 = Ha > Hb ? Ha : Hb;
     if (H1 > 0) {
       const double H2 = Ha > Hb ? Hb : Ha;
-      double f = 1;
+      double v = 1;
       if (H2 > 0) {
         const double r = H2 / H1;
-        f = pm::pow(jmax(0.0, 1 - pm::pow(r, kWeirExponent)), kVillemonteExponent);
+        v = pm::pow(jmax(0.0, 1 - pm::pow(r, kWeirExponent)), kVillemonteExponent);
       }
-      q = __ldg(M.coef + c) * __ldg(area + c) * kWeirCoefficient * M.sq2g * H1 * pm::sqrt_rn(H1) * f * (Ha >= Hb ? 1.0 : -1.0);
+      q = __ldg(M.coef + c) * __ldg(area + c) * kWeirCoefficient * M.sq2g * H1 * pm::sqrt_rn(H1) * v * (Ha >= Hb ? 1.0 : -1.0);
     }
   }
-  if (q == 0) { qOut = 0; return 0; }
-  double dV = q * M.dt;
-  const int src = dV > 0 ? a : b, dst = dV > 0 ? b : a;
+  return q == 0 ? 0 : q * M.dt;
+}
+
+// The flow dV (not zero) after the limiter. S.aEff holds the reciprocals of the nodes' effective areas.
+__device__ __forceinline__ double limit_volume(const Slot& S, const FlowHeads& f, double dV) {
+  const int src = dV > 0 ? f.a : f.b, dst = dV > 0 ? f.b : f.a;
   const double hs = src < 0 ? 0.0 : S.hEff[src];
   const double hd = dst < 0 ? 0.0 : S.hEff[dst];
-  const double inv = (src < 0 ? 0.0 : 1 / S.aEff[src]) + (dst < 0 ? 0.0 : 1 / S.aEff[dst]);
+  const double inv = (src < 0 ? 0.0 : S.aEff[src]) + (dst < 0 ? 0.0 : S.aEff[dst]);
   const int degRef = src < 0 ? S.deg[dst] : (dst < 0 ? S.deg[src] : (S.deg[src] > S.deg[dst] ? S.deg[src] : S.deg[dst]));
   const double share = kLimiterShare / static_cast<double>(degRef > 1 ? degRef : 1);
-  double lim = inv > 0 ? share * (hs - jmax(hd, zo)) / inv : fabs(dV);
+  double lim = inv > 0 ? share * (hs - jmax(hd, f.zo)) / inv : fabs(dV);
   if (lim < 0) lim = 0;
   if (fabs(dV) > lim) dV = dV > 0 ? lim : -lim;
-  qOut = dV / M.dt;
   return dV;
+}
+
+// Sorts the connections (zero, front or back) and counts the nodes' degrees; the flows follow after a barrier
+// (listed_flows). The order within the list varies, the flows do not depend on it.
+template <int W, class IP>
+__device__ __forceinline__ void sort_connections(const DevModel& M, const Pose& F, double t, Slot& S, const IP& I, const Team<W>& T) {
+#pragma unroll 1
+  for (int c0 = T.warp * kLanes; c0 < M.nc; c0 += kLanes * W) {
+    const int c = c0 + T.lane;
+    int cls = 0;
+    if (c < M.nc) {
+      S.dV[c] = 0;
+      if (count_degrees(M, t, S, I, c)) {
+        const FlowHeads f = flow_heads(M, F, S, c);
+        if (__ldg(M.law + c) == 0) {
+          cls = f.Ha - f.Hb != 0 ? 1 : 0;
+        } else if ((f.Ha > f.Hb ? f.Ha : f.Hb) > 0) {
+          cls = (f.Ha > f.Hb ? f.Hb : f.Ha) > 0 ? 2 : 1;
+        }
+      }
+    }
+    const unsigned front = __ballot_sync(kFull, cls == 1), back = __ballot_sync(kFull, cls == 2);
+    const unsigned before = (1u << T.lane) - 1u;
+    if (front) {
+      int base = 0;
+      if (T.lane == 0) base = atomicAdd(&S.misc[kMiscFront], __popc(front));
+      base = __shfl_sync(kFull, base, 0);
+      if (cls == 1) S.flow[base + __popc(front & before)] = static_cast<std::uint16_t>(c);
+    }
+    if (back) {
+      int base = 0;
+      if (T.lane == 0) base = atomicAdd(&S.misc[kMiscBack], __popc(back));
+      base = __shfl_sync(kFull, base, 0);
+      if (cls == 2) S.flow[M.nc - 1 - (base + __popc(back & before))] = static_cast<std::uint16_t>(c);
+    }
+  }
+}
+
+template <int W, class IP>
+__device__ __forceinline__ void listed_flows(const DevModel& M, const Pose& F, Slot& S, const IP& I, const Team<W>& T) {
+  const int front = S.misc[kMiscFront], back = S.misc[kMiscBack];
+  const int split = (front + kLanes - 1) / kLanes * kLanes;  // the back starts with a new warp
+#pragma unroll 1
+  for (int k = T.rank; k < split + back; k += kLanes * W) {
+    if (k >= front && k < split) continue;
+    const int c = S.flow[k < front ? k : M.nc - 1 - (k - split)];
+    const FlowHeads f = flow_heads(M, F, S, c);
+    const double dV = law_volume(M, f, I.area(), c);
+    S.dV[c] = dV != 0 ? limit_volume(S, f, dV) : dV;
+  }
 }
 
 // Scalars of one simulation: identical in every lane of its warp.
@@ -907,7 +998,11 @@ __device__ __forceinline__ void team_step(const DevModel& M, const Pose& F, SimR
     T.sync();
   }
   // the list counter for the next step's level solve (read after this step's later barriers)
-  if (T.leader()) S.misc[kMiscTaken] = W * (32 / kLevelLanes<MIXED>);
+  if (T.leader()) {
+    S.misc[kMiscTaken] = W * (32 / kLevelLanes<MIXED>);
+    S.misc[kMiscFront] = 0;
+    S.misc[kMiscBack] = 0;
+  }
 
   // the solve's ends node by node (an empty node's area, a wet one's centroid), effective heads and areas, then degrees
   // (flows.hpp:15-35)
@@ -922,27 +1017,25 @@ __device__ __forceinline__ void team_step(const DevModel& M, const Pose& F, SimR
     }
     const double v = S.vol[n];
     S.hEff[n] = v > kEmptyVolume ? S.level[n] : kNoHead;
-    S.aEff[n] = v >= __ldg(M.vmax + n) ? __ldg(M.aov + n) : jmax(S.area[n], __ldg(M.amin + n));
+    S.aEff[n] = 1 / (v >= __ldg(M.vmax + n) ? __ldg(M.aov + n) : jmax(S.area[n], __ldg(M.amin + n)));
     S.deg[n] = 0;
   }
   tape.solved(M, S, T);  // a thread reads the nodes it has just finished
   T.sync();
-  // A node's degree is the number of its incident connections that are enabled and not between two empty spaces. Each
-  // such connection counts once at each of its nodes (the incidence lists hold it once at a when a >= 0 and once at b),
-  // counted per connection with shared-memory atomics: an integer count, the same in any order, and one round of
-  // independent loads instead of a walk down every node's incidence list.
-  for (int c = rank; c < M.nc; c += kStride) {
-    if (!__ldg(I.en() + c)) continue;
-    const int a = __ldg(M.ca + c), b = __ldg(M.cb + c);
-    if (a >= 0 && S.hEff[a] < kNoHeadTest && S.hEff[b] < kNoHeadTest) continue;
-    if (a >= 0) atomicAdd(&S.deg[a], 1);
-    atomicAdd(&S.deg[b], 1);
-  }
-  T.sync();
-  for (int c = rank; c < M.nc; c += kStride) {
-    double q;
-    S.dV[c] = connection_flow(M, F, tNow, S, I.en(), I.area(), I.tOn(), c, q);
-    S.q[c] = q;
+  if constexpr (W <= 4) {
+    sort_connections(M, F, tNow, S, I, T);
+    T.sync();
+    listed_flows(M, F, S, I, T);
+  } else {
+#pragma unroll 1
+    for (int c = rank; c < M.nc; c += kStride)
+      S.dV[c] = count_degrees(M, tNow, S, I, c) ? law_volume(M, flow_heads(M, F, S, c), I.area(), c) : 0;
+    T.sync();
+#pragma unroll 1
+    for (int c = rank; c < M.nc; c += kStride) {
+      const double dV = S.dV[c];
+      if (dV != 0) S.dV[c] = limit_volume(S, flow_heads(M, F, S, c), dV);
+    }
   }
   T.sync();
   // per-node gathers in increasing connection order, then the volume update (flows.hpp:81-111)
@@ -1055,8 +1148,8 @@ __device__ __forceinline__ void team_step(const DevModel& M, const Pose& F, SimR
       const int k0 = __ldg(M.monStart + m), k1 = k0 + __ldg(M.monCount + m);
       double over = 0;
       for (int k = k0; k < k1; ++k) {
-        const double qc = S.q[__ldg(M.monConn + k)];
-        if (qc > 0) over += qc;
+        const double d = S.dV[__ldg(M.monConn + k)];
+        if (d > 0) over += d / M.dt;
       }
       fire = over > M.monThreshold;
       if (fire) I.overT()[m] = R.t;
