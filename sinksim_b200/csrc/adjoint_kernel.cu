@@ -63,17 +63,18 @@ struct AdjTeam {
 // The tape hooks of the forward step (NoTape's counterpart): one lane of a level lane group writes each node pass, the
 // team writes the solved state, the pose and the buoyancy result.
 struct GpuTape {
-  static constexpr bool kLazy = false;
+  static constexpr bool kLazy = false;  // every level is formed: records and checkpoints keep them
   adj::Tape t;
+  bool on;  // false: the step is not recorded
   // A unit's start: its first pass's level and extent; the sums stay zero when no pass is made there.
   __device__ __forceinline__ void start(int n, double h, double zmin, double zmax, const LevelLanes& L) const {
-    if (L.sub != 0) return;
+    if (!on || L.sub != 0) return;
     double* r = t.pass(n, 0);
     r[0] = h; r[1] = 0; r[2] = 0; r[3] = 0; r[4] = 0; r[5] = 0; r[6] = zmin; r[7] = zmax;
     t.i[t.L.npass + n] = 1;
   }
   __device__ __forceinline__ void pass(int n, int k, double h, const PassR& p, const LevelLanes& L) const {
-    if (L.sub != 0) return;
+    if (!on || L.sub != 0) return;
     if (k < adj::kMaxPasses) {
       const double* r0 = t.pass(n, 0);
       const double zmin = r0[6], zmax = r0[7];
@@ -84,6 +85,7 @@ struct GpuTape {
   }
   template <int W>
   __device__ __forceinline__ void solved(const DevModel& M, const Slot& S, const Team<W>& T) const {
+    if (!on) return;
     const adj::TapeLayout& L = t.L;
     for (int n = T.rank; n < M.nn; n += 32 * W) {
       t.d[L.volS + n] = S.vol[n]; t.d[L.levelS + n] = S.level[n]; t.d[L.areaS + n] = S.area[n];
@@ -94,15 +96,10 @@ struct GpuTape {
       const Pose& F = *S.pose;
       const double p[14] = {F.R00, F.R01, F.R02, F.R10, F.R11, F.R12, F.R20, F.R21, F.R22, F.tx, F.ty, F.tz, F.cth, F.iR};
       for (int k = 0; k < 14; ++k) t.d[L.pose + k] = p[k];
-      const Buoy& b = *S.buoy;
+      const Buoy b = buoyancy_finish(S.hydro);
       t.d[L.buoy] = b.V; t.d[L.buoy + 1] = b.x; t.d[L.buoy + 2] = b.y; t.d[L.buoy + 3] = b.z;
     }
   }
-};
-
-// A forward step without a record; its levels are all formed (checkpoints keep them).
-struct NoRecord : NoTape {
-  static constexpr bool kLazy = false;
 };
 
 // Instance fields for team_step: the connection fields of the instance; events go nowhere (the adjoint runs keep no
@@ -303,8 +300,22 @@ __device__ __forceinline__ void add_sample_adjoint(const DevModel& M, double zO,
   adj::pose_reverse(M, F, aP, aSc[0], aSc[1], aSc[2]);
 }
 
+// Sample k of the objective at state s with pose F: its values, their residuals into J, and where it was taken.
+__device__ __forceinline__ void add_sample(const DevModel& M, const Pose& F, double pitch, const AdjRun& B, int inst, int k, long long s,
+                                           const double* trimT, const double* heaveT, double& J, double* sampleS, bool leader) {
+  double tr, hv;
+  adj::trim_heave(M, PoseD{F.R00, F.R01, F.R02, F.R10, F.R11, F.R12, F.R20, F.R21, F.R22, F.tx, F.ty, F.tz, F.cth, F.iR}, pitch, tr, hv);
+  J += (tr - trimT[k]) * (tr - trimT[k]) + (hv - heaveT[k]) * (hv - heaveT[k]);
+  if (leader) {
+    B.trim[static_cast<std::size_t>(inst) * B.nsamples + k] = tr; B.heave[static_cast<std::size_t>(inst) * B.nsamples + k] = hv;
+    sampleS[k] = static_cast<double>(s);
+  }
+}
+
+// 16 warps per SM in all: 128 registers a thread (left to itself the compiler takes 208 for 8-warp teams, and one fits an SM)
 template <int W>
-__global__ void __launch_bounds__(W * 32) adjoint_batch(DevModel M, AdjRun B, SlotLayout SL, AdjLayout AL) {
+__global__ void __launch_bounds__(W * 32, 16 / W) adjoint_batch(const __grid_constant__ DevModel M, const __grid_constant__ AdjRun B, const __grid_constant__ SlotLayout SL,
+                                                       const __grid_constant__ AdjLayout AL) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int team = blockIdx.x;
   Team<W> T;
@@ -337,7 +348,7 @@ __global__ void __launch_bounds__(W * 32) adjoint_batch(DevModel M, AdjRun B, Sl
     T.sync();
     if (inst >= B.count) return;
     const long long tStart = global_ns();
-    long long tRecompute = 0, tReverse = 0, nRecomputed = 0;
+    long long tForward = 0, tRecompute = 0, tReverse = 0, nRecomputed = 0;
     const std::size_t ic = static_cast<std::size_t>(inst) * M.nc;
     const AdjInst I{B.en + ic, B.area + ic, B.tOn + ic, sink, isink, M.nmon};
     // the event bookkeeping sinks: overflow and mark times set (nothing fires), so events never write
@@ -355,96 +366,81 @@ __global__ void __launch_bounds__(W * 32) adjoint_batch(DevModel M, AdjRun B, Sl
       }
       __threadfence_block();
       T.sync();
-      load_state(c, R, S, M, T);
     }
-    // ---- 1. forward with checkpoints, the objective's samples and (tapeForward) every step's record
-    Pose& F = *S.pose;
-    F = make_pose(M, R.zO, R.pitch, R.roll);
     const double* trimT = B.trimT + static_cast<std::size_t>(inst) * NS;
     const double* heaveT = B.heaveT + static_cast<std::size_t>(inst) * NS;
     double J = 0;
-    int k = 0;
-    long long s = 0, v = 0;
-    for (;; ++s) {
-      if (s % B.K == 0 && s > 0) {
-        save_state(ckpt + static_cast<std::size_t>(s / B.K) * recSize, R, S, M.nn, T);
-        T.sync();
-      }
-      if (R.foundered || R.t >= B.tMax || s >= B.maxSteps) break;
-      while (k < NS && R.t >= B.sampleT[k]) {
-        double tr, hv;
-        adj::trim_heave(M, PoseD{F.R00, F.R01, F.R02, F.R10, F.R11, F.R12, F.R20, F.R21, F.R22, F.tx, F.ty, F.tz, F.cth, F.iR}, R.pitch, tr, hv);
-        J += (tr - trimT[k]) * (tr - trimT[k]) + (hv - heaveT[k]) * (hv - heaveT[k]);
-        if (T.leader()) {
-          B.trim[static_cast<std::size_t>(inst) * NS + k] = tr; B.heave[static_cast<std::size_t>(inst) * NS + k] = hv;
-          A.sampleS[k] = static_cast<double>(s);
-        }
-        ++k;
-      }
-      if (B.tapeForward) {
-        tape_inputs(sp, R, S, M.nn, T);
-        team_step<false, W>(M, F, R, S, I, T, GpuTape{sp});
-        T.sync();
-        v = ring_place(v, B.arenaBytes, recMax);
-        if (T.leader()) off[s] = v;
-        const std::size_t bytes = store_record(sp, M.nn, A.poff, ring + v % static_cast<long long>(B.arenaBytes), T);
-        if (T.leader()) rb[s] = static_cast<std::int32_t>(bytes);
-        v += static_cast<long long>(bytes);
-      } else {
-        team_step<false, W>(M, F, R, S, I, T, NoRecord{});
-      }
-      F = make_pose(M, R.zO, R.pitch, R.roll);
-    }
-    const long long S_end = s;
-    // the ring holds the records at virtual offsets >= v - cap: a segment is reversed from the ring when its first
-    // step's record is among them
-    const long long kept = B.tapeForward ? v - static_cast<long long>(B.arenaBytes) : LLONG_MAX;
-    const double zE = R.zO, thE = R.pitch, phE = R.roll;
-    for (; k < NS; ++k) {
-      double tr, hv;
-      adj::trim_heave(M, PoseD{F.R00, F.R01, F.R02, F.R10, F.R11, F.R12, F.R20, F.R21, F.R22, F.tx, F.ty, F.tz, F.cth, F.iR}, R.pitch, tr, hv);
-      J += (tr - trimT[k]) * (tr - trimT[k]) + (hv - heaveT[k]) * (hv - heaveT[k]);
-      if (T.leader()) {
-        B.trim[static_cast<std::size_t>(inst) * NS + k] = tr; B.heave[static_cast<std::size_t>(inst) * NS + k] = hv;
-        A.sampleS[k] = static_cast<double>(S_end);
-      }
-    }
-    __threadfence_block();
-    T.sync();
-    const long long tForward = global_ns() - tStart;
-    // ---- 2. reverse
     double aSc[6] = {0, 0, 0, 0, 0, 0};
-    for (int n = T.rank; n < M.nn; n += 32 * W) { A.as.aVol[n] = 0; A.as.aLevel[n] = 0; A.as.aCx[n] = 0; A.as.aCy[n] = 0; A.as.aCz[n] = 0; }
-    for (int c = T.rank; c < M.nc; c += 32 * W) A.grad[c] = 0;
-    T.sync();
-    // the samples at the final state (the objective's values of the trim and heave, recomputed from the outputs)
-    for (int q = 0; q < NS; ++q)
-      if (static_cast<long long>(A.sampleS[q]) == S_end) {
-        const double tr = B.trim[static_cast<std::size_t>(inst) * NS + q], hv = B.heave[static_cast<std::size_t>(inst) * NS + q];
-        add_sample_adjoint(M, zE, thE, phE, 2 * (tr - trimT[q]), 2 * (hv - heaveT[q]), aSc);
-      }
-    int err = 0;
-    const long long nseg = (S_end + B.K - 1) / B.K;
-    for (long long g = nseg - 1; g >= 0; --g) {
-      const long long s0 = g * B.K, s1 = (s0 + B.K < S_end) ? s0 + B.K : S_end;
+    int k = 0, err = 0;
+    long long S_end = 0, kept = 0;
+    // stretch g = -1: forward from the initial state with checkpoints, the objective's samples and (tapeForward) every
+    // step's record; then the segments, last first: one whose records the ring no longer holds is stepped again from its
+    // checkpoint into the ring (every later segment has been reversed already, so the whole ring is free; it holds K
+    // records of the largest size), and each is reversed. Both kinds of stretch run through one call of the step, of
+    // which three inlined copies and the reverse did not fit the instruction caches.
+    for (long long g = -1;;) {
+      const bool forward = g < 0;
+      const long long s0 = forward ? 0 : g * B.K;
+      const long long s1 = forward ? B.maxSteps : (s0 + B.K < S_end ? s0 + B.K : S_end);
       const long long tSeg = global_ns();
-      if (!(B.tapeForward && off[s0] >= kept)) {
-        // recompute the segment from its checkpoint into the ring (every later segment has been reversed already, so
-        // the whole ring is free; it holds K records of the largest size)
-        load_state(ckpt + static_cast<std::size_t>(g) * recSize, R, S, M, T);
-        F = make_pose(M, R.zO, R.pitch, R.roll);
-        long long w = 0;
-        nRecomputed += s1 - s0;
-        for (long long st = s0; st < s1; ++st) {
-          tape_inputs(sp, R, S, M.nn, T);
-          team_step<false, W>(M, F, R, S, I, T, GpuTape{sp});
-          T.sync();
-          if (T.leader()) off[st] = w;
-          const std::size_t bytes = store_record(sp, M.nn, A.poff, ring + w, T);
-          if (T.leader()) rb[st] = static_cast<std::int32_t>(bytes);
-          w += static_cast<long long>(bytes);
-          F = make_pose(M, R.zO, R.pitch, R.roll);
+      if (forward || !(B.tapeForward && off[s0] >= kept)) {
+        load_state(ckpt + static_cast<std::size_t>(forward ? 0 : g) * recSize, R, S, M, T);
+        *S.pose = make_pose(M, R.zO, R.pitch, R.roll);
+        park(S.parked, R);
+        T.sync();
+        const bool record = !forward || B.tapeForward;
+        long long s = s0, v = 0;
+        for (;; ++s) {
+          if (forward) {
+            if (s % B.K == 0 && s > 0) {
+              save_state(ckpt + static_cast<std::size_t>(s / B.K) * recSize, R, S, M.nn, T);
+              T.sync();
+            }
+            if (R.foundered || R.t >= B.tMax) break;
+          }
+          if (s >= s1) break;
+          while (forward && k < NS && R.t >= B.sampleT[k]) {
+            add_sample(M, *S.pose, R.pitch, B, inst, k, s, trimT, heaveT, J, A.sampleS, T.leader());
+            ++k;
+          }
+          if (record) tape_inputs(sp, R, S, M.nn, T);
+          team_step<false, W>(M, R, S, I, T, GpuTape{sp, record});
+          if (record) {
+            T.sync();
+            v = ring_place(v, B.arenaBytes, recMax);
+            if (T.leader()) off[s] = v;
+            const std::size_t bytes = store_record(sp, M.nn, A.poff, ring + v % static_cast<long long>(B.arenaBytes), T);
+            if (T.leader()) rb[s] = static_cast<std::int32_t>(bytes);
+            v += static_cast<long long>(bytes);
+          }
         }
+        if (forward) {
+          S_end = s;
+          // the ring holds the records at virtual offsets >= v - cap: a segment is reversed from the ring when its first
+          // step's record is among them
+          kept = B.tapeForward ? v - static_cast<long long>(B.arenaBytes) : LLONG_MAX;
+        } else {
+          nRecomputed += s1 - s0;
+        }
+      }
+      if (forward) {
+        for (; k < NS; ++k) add_sample(M, *S.pose, R.pitch, B, inst, k, S_end, trimT, heaveT, J, A.sampleS, T.leader());
+        const double zE = R.zO, thE = R.pitch, phE = R.roll;
+        __threadfence_block();
+        T.sync();
+        tForward = global_ns() - tStart;
+        for (int n = T.rank; n < M.nn; n += 32 * W) { A.as.aVol[n] = 0; A.as.aLevel[n] = 0; A.as.aCx[n] = 0; A.as.aCy[n] = 0; A.as.aCz[n] = 0; }
+        for (int c = T.rank; c < M.nc; c += 32 * W) A.grad[c] = 0;
+        T.sync();
+        // the samples at the final state (the objective's values of the trim and heave, recomputed from the outputs)
+        for (int q = 0; q < NS; ++q)
+          if (static_cast<long long>(A.sampleS[q]) == S_end) {
+            const double tr = B.trim[static_cast<std::size_t>(inst) * NS + q], hv = B.heave[static_cast<std::size_t>(inst) * NS + q];
+            add_sample_adjoint(M, zE, thE, phE, 2 * (tr - trimT[q]), 2 * (hv - heaveT[q]), aSc);
+          }
+        g = (S_end + B.K - 1) / B.K - 1;
+        if (g < 0) break;
+        continue;
       }
       __threadfence_block();
       T.sync();
@@ -487,6 +483,7 @@ __global__ void __launch_bounds__(W * 32) adjoint_batch(DevModel M, AdjRun B, Sl
         T.sync();
       }
       tReverse += global_ns() - tRev;
+      if (--g < 0) break;
     }
     T.sync();
     for (int c = T.rank; c < M.nc; c += 32 * W) B.grad[ic + c] = A.grad[c];

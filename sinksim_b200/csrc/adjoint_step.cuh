@@ -33,8 +33,26 @@
 #include "portable_math.cuh"
 #include "scheme.h"
 
+// Loops whose bodies the compiler would copy four times over, and functions called from several places: the reverse
+// issues a long straight run of code once per step, which has to come from the instruction caches. With one call site of
+// the forward step (adjoint_kernel.cu) the kernel is 310 KB of code instead of 940; on B200 a 64-point gradient on the
+// liner to 400 s takes 107 ms against 111, 3 points on titanic64 51 against 58.
+#if defined(__CUDA_ARCH__)
+#define SSB_ROLLED _Pragma("unroll 1")
+#else
+#define SSB_ROLLED
+#endif
+#if defined(__CUDACC__)
+#define SSB_CALLED static __host__ __device__ __noinline__
+#else
+#define SSB_CALLED inline
+#endif
+
 namespace ssb {
 namespace adj {
+
+SSB_CALLED double pow_of(double x, double y) { return pm::pow(x, y); }
+SSB_CALLED void trig_of(double x, double& s, double& c) { pm::sin_cos(x, s, c); }
 
 // Node passes of one node in one step's level solve, at most: the start, a clamped start or the pass at the top of a
 // full node, and the solver's six Newton iterations.
@@ -115,7 +133,9 @@ SSB_HD PoseD load_pose(const double* p) {
 
 // The forward pose (frame.hpp:9-21) with portable sin / cos: the same operations as the step's.
 SSB_HD PoseD pose_of(const DevModel& M, double zO, double th, double ph) {
-  const double cth = pm::cos(th), sth = pm::sin(th), cph = pm::cos(ph), sph = pm::sin(ph);
+  double cth, sth, cph, sph;
+  trig_of(th, sth, cth);
+  trig_of(ph, sph, cph);
   PoseD F;
   F.R00 = cth; F.R01 = sth * sph; F.R02 = sth * cph;
   F.R10 = 0;   F.R11 = cph;       F.R12 = -sph;
@@ -198,7 +218,7 @@ SSB_HD double lane_sum(double v, int width) {
 // top: each tree lane l scans segments s0 + l + 32 k keeping the first strict improvement, and the tree combines lane l
 // with lane l + off (off = 16 .. 1), the lower lane winning ties (kernel/reduce.hpp:52-71 and :12-37). On the device
 // the warp's lanes are the tree's lanes; on the host the lanes are emulated.
-SSB_HD int pass_extreme(const DevModel& M, const PoseD& F, int n, bool want_min, int lane, int width) {
+SSB_CALLED int pass_extreme(const DevModel& M, const PoseD& F, int n, bool want_min, int lane, int width) {
   const int s0 = M.segStart[n], s1 = s0 + M.segCount[n];
 #if defined(__CUDA_ARCH__)
   if (width == 32) {
@@ -211,6 +231,7 @@ SSB_HD int pass_extreme(const DevModel& M, const PoseD& F, int n, bool want_min,
     };
     // two segments per round, both loaded before either is compared; each lane keeps its segments' order
     int j = s0 + lane;
+    SSB_ROLLED
     for (; j + 32 < s1; j += 64) {
       const double2 xy0 = M.segXY[j], ab0 = M.segLH[j], xy1 = M.segXY[j + 32], ab1 = M.segLH[j + 32];
       seg(xy0, ab0, j);
@@ -235,6 +256,7 @@ SSB_HD int pass_extreme(const DevModel& M, const PoseD& F, int n, bool want_min,
   for (int l = 0; l < 32; ++l) {
     best[l] = want_min ? 1e9 : -1e9;
     idx[l] = -1;
+    SSB_ROLLED
     for (int j = s0 + l; j < s1; j += 32) {
       const double2 xy = M.segXY[j], ab = M.segLH[j];
       const double base = F.R20 * xy.x + F.R21 * xy.y + F.tz;
@@ -263,7 +285,7 @@ SSB_HD void extreme_reverse(const DevModel& M, int j, bool bottom, double a_w, A
 // moments: adds the pose adjoint to aP and returns this lane's share of d(outputs)/d h (sum over the warp's lanes for
 // the total). Only segments the level cuts contribute (kernel/reduce.hpp:52-71: a full segment's height is b - a, a dry
 // one adds nothing).
-SSB_HD double pass_sweep1(const DevModel& M, const PoseD& F, int n, double h, double av, double amx, double amy, double amz, int lane, int width,
+SSB_CALLED double pass_sweep1(const DevModel& M, const PoseD& F, int n, double h, double av, double amx, double amy, double amz, int lane, int width,
                           AdjPose& aP) {
   const int s0 = M.segStart[n], s1 = s0 + M.segCount[n];
   const double mu = M.mu[n];
@@ -281,6 +303,7 @@ SSB_HD double pass_sweep1(const DevModel& M, const PoseD& F, int n, double h, do
   };
   // two segments per round, both loaded before either is used; each lane still visits its segments in order
   int j = s0 + lane;
+  SSB_ROLLED
   for (; j + width < s1; j += 2 * width) {
     const double2 xy0 = M.segXY[j], ab0 = M.segLH[j], xy1 = M.segXY[j + width], ab1 = M.segLH[j + width];
     const double A0 = M.segAr[j], A1 = M.segAr[j + width];
@@ -294,13 +317,14 @@ SSB_HD double pass_sweep1(const DevModel& M, const PoseD& F, int n, double h, do
 
 // The pose adjoint of np passes of node n at levels h[i] whose vol has the adjoint av[i] and whose moments have none
 // (their level adjoints are not needed).
-SSB_HD void pass_sweep_levels(const DevModel& M, const PoseD& F, int n, int np, const double* h, const double* av, int lane, int width,
+SSB_CALLED void pass_sweep_levels(const DevModel& M, const PoseD& F, int n, int np, const double* h, const double* av, int lane, int width,
                               AdjPose& aP) {
   const int s0 = M.segStart[n], s1 = s0 + M.segCount[n];
   const double mu = M.mu[n];
   double aR20 = 0, aR21 = 0, atz = 0, aiR = 0;
   auto seg = [&](const double2 xy, const double2 ab, const double A) {
     const double base = F.R20 * xy.x + F.R21 * xy.y + F.tz;
+    SSB_ROLLED
     for (int i = 0; i < np; ++i) {
       const double zp = (h[i] - base) * F.iR;
       if (!(zp > ab.x && zp < ab.y)) continue;
@@ -311,6 +335,7 @@ SSB_HD void pass_sweep_levels(const DevModel& M, const PoseD& F, int n, int np, 
     }
   };
   int j = s0 + lane;
+  SSB_ROLLED
   for (; j + width < s1; j += 2 * width) {
     const double2 xy0 = M.segXY[j], ab0 = M.segLH[j], xy1 = M.segXY[j + width], ab1 = M.segLH[j + width];
     const double A0 = M.segAr[j], A1 = M.segAr[j + width];
@@ -323,7 +348,7 @@ SSB_HD void pass_sweep_levels(const DevModel& M, const PoseD& F, int n, int np, 
 
 // Reverse of the buoyancy integral (kernel/reduce.hpp:39-49) over this thread's columns first, first + stride, ...: the
 // adjoints of V, Mx, My, Mz into the pose adjoint. A column cut by the waterplane contributes through its wet height.
-SSB_HD void buoyancy_sweep(const DevModel& M, const PoseD& F, double aV, double aMx, double aMy, double aMz, int first, int stride,
+SSB_CALLED void buoyancy_sweep(const DevModel& M, const PoseD& F, double aV, double aMx, double aMy, double aMz, int first, int stride,
                            AdjPose& aP) {
   double aR20 = 0, aR21 = 0, atz = 0, aiR = 0;
   auto col = [&](const double2 xy, const double2 lh, const double A) {
@@ -338,6 +363,7 @@ SSB_HD void buoyancy_sweep(const DevModel& M, const PoseD& F, double aV, double 
   };
   // two columns per round, both loaded before either is used; each thread keeps its columns' order
   int i = first;
+  SSB_ROLLED
   for (; i + stride < M.ncol; i += 2 * stride) {
     const double2 xy0 = M.colXY[i], lh0 = M.colLH[i], xy1 = M.colXY[i + stride], lh1 = M.colLH[i + stride];
     const double A0 = M.colA[i], A1 = M.colA[i + stride];
@@ -383,14 +409,17 @@ SSB_HD void replay_unit(const DevModel& M, const Tape& t, const int* members, in
   r.ok = N <= kMaxMembers;
   r.cs = 0; r.base = 0; r.K = 0; r.startSrc = 0; r.loSrc = 0; r.hiSrc = 0;
   if (!r.ok) return;
+  SSB_ROLLED
   for (int k = 0; k < N; ++k) r.members[k] = members[k];
   const double* volIn = t.d + t.L.volIn;
   const double* levelIn = t.d + t.L.levelIn;
   double V = 0, Vmax = 0;
+  SSB_ROLLED
   for (int k = 0; k < N; ++k) { V += volIn[members[k]]; Vmax += M.vmax[members[k]]; }
   r.V = V; r.Vmax = Vmax;
   bool allWet = true;
   int firstWet = -1;
+  SSB_ROLLED
   for (int k = 0; k < N; ++k) {
     if (volIn[members[k]] > 0) { if (firstWet < 0) firstWet = k; }
     else allWet = false;
@@ -401,6 +430,7 @@ SSB_HD void replay_unit(const DevModel& M, const Tape& t, const int* members, in
     h = levelIn[members[0]];
   } else if (allWet) {
     double s = 0;
+    SSB_ROLLED
     for (int k = 0; k < N; ++k) s += levelIn[members[k]];
     h = s / static_cast<double>(N);
   } else {
@@ -410,6 +440,7 @@ SSB_HD void replay_unit(const DevModel& M, const Tape& t, const int* members, in
   // the extent: the members' start passes
   double lo = rec(t, members[0], 0)[6], hi = rec(t, members[0], 0)[7];
   int loSrc = 0, hiSrc = 0;
+  SSB_ROLLED
   for (int k = 1; k < N; ++k) {
     const double* p = rec(t, members[k], 0);
     if (p[6] < lo) { lo = p[6]; loSrc = k; }
@@ -421,6 +452,7 @@ SSB_HD void replay_unit(const DevModel& M, const Tape& t, const int* members, in
   }
   r.loSrc = loSrc; r.hiSrc = hiSrc;
   bool ok = true;
+  SSB_ROLLED
   for (int k = 0; k < N; ++k) ok = ok && rec(t, members[k], 0)[0] == h;
   if (V <= kEmptyVolume) { r.cs = 0; r.K = 0; r.ok = ok; return; }
   if (V >= Vmax * kFullFraction) { r.cs = 1; r.K = 1; r.ok = ok; return; }
@@ -432,6 +464,7 @@ SSB_HD void replay_unit(const DevModel& M, const Tape& t, const int* members, in
     r.startSrc = h < lo ? kSrcLo : kSrcHi;
     h = hc;
     base = 1;
+    SSB_ROLLED
     for (int k = 0; k < N; ++k) ok = ok && rec(t, members[k], 1)[0] == h;
   }
   r.base = base;
@@ -439,12 +472,15 @@ SSB_HD void replay_unit(const DevModel& M, const Tape& t, const int* members, in
   double a = lo, b = hi;
   int aS = kSrcLo, bS = kSrcHi;
   int k = base;
+  SSB_ROLLED
   for (int it = 0; it < kNewtonFast; ++it) {
     double sum = 0, dvs = 0;
+    SSB_ROLLED
     for (int q = 0; q < N; ++q) sum += rec(t, members[q], k)[1];
     const double err = single ? rec(t, members[0], k)[1] - V : sum - V;
     if (fabs(err) < tol) break;
     if (err > 0) { b = h; bS = k; } else { a = h; aS = k; }
+    SSB_ROLLED
     for (int q = 0; q < N; ++q) dvs += rec(t, members[q], k)[2];
     if (single) dvs = rec(t, members[0], k)[2];
     double hn = dvs > kSlopeMin ? h - err / dvs : 0.5 * (a + b);
@@ -454,6 +490,7 @@ SSB_HD void replay_unit(const DevModel& M, const Tape& t, const int* members, in
     r.aSrc[k] = aS; r.bSrc[k] = bS;
     h = hn;
     ++k;
+    SSB_ROLLED
     for (int q = 0; q < N; ++q) ok = ok && rec(t, members[q], k)[0] == h;
   }
   r.K = k;
@@ -515,7 +552,9 @@ SSB_HD bool unit_reverse(const DevModel& M, const PoseD& F, const Tape& t, UnitW
   const int N = r.N;
   const int K = r.K;
   if (lane == 0) {
+    SSB_ROLLED
     for (int k = 0; k < N; ++k) {
+      SSB_ROLLED
       for (int i = 0; i <= K; ++i) w.av[k][i] = w.adv[k][i] = 0;
       w.amx[k] = w.amy[k] = w.amz[k] = 0;
       w.aZmin0[k] = 0;
@@ -523,11 +562,13 @@ SSB_HD bool unit_reverse(const DevModel& M, const PoseD& F, const Tape& t, UnitW
       w.np[k] = 0;
       u.oVol[k] = u.oLevel[k] = u.oCx[k] = u.oCy[k] = u.oCz[k] = 0;
     }
+    SSB_ROLLED
     for (int i = 0; i <= K; ++i) w.ah[i] = 0;
     w.aV = w.aLo = w.aHi = w.aH0 = 0;
     w.err = 0;
     if (r.cs == 0) {
       // empty: the level is the member's own extent bottom; a group empties its members, a node alone keeps its volume
+      SSB_ROLLED
       for (int k = 0; k < N; ++k) {
         w.aZmin0[k] += u.aLevel[k];
         if (r.single) w.aV += u.aVol[k];
@@ -536,15 +577,19 @@ SSB_HD bool unit_reverse(const DevModel& M, const PoseD& F, const Tape& t, UnitW
     } else if (r.cs == 1) {
       // full: volumes vmax + dh aov (the last takes the rest), level hi + dh, centroids at the top (levels.hpp:29-35, :91-111)
       double aSum = 0;
+      SSB_ROLLED
       for (int k = 0; k < N; ++k) aSum += M.aov[r.members[k]];
       double aDh = 0;
       double aV = u.aVol[N - 1];
+      SSB_ROLLED
       for (int k = 0; k < N - 1; ++k) aDh += (u.aVol[k] - u.aVol[N - 1]) * M.aov[r.members[k]];
       double aHi = 0;
+      SSB_ROLLED
       for (int k = 0; k < N; ++k) { aDh += u.aLevel[k]; aHi += u.aLevel[k]; }
       if (r.V - r.Vmax > 0) aV += aDh / aSum;
       w.aV = aV;
       w.aHi = aHi;
+      SSB_ROLLED
       for (int k = 0; k < N; ++k) {
         const double* p = rec(t, r.members[k], 1);
         centroid_reverse(p, u.aCx[k], u.aCy[k], u.aCz[k], w.av[k][1], w.amx[k], w.amy[k], w.amz[k], u.oCx[k], u.oCy[k], u.oCz[k]);
@@ -552,6 +597,7 @@ SSB_HD bool unit_reverse(const DevModel& M, const PoseD& F, const Tape& t, UnitW
       }
     } else {
       // Newton: level h_K, area and centroid of the final passes, the group's water shared in proportion to them
+      SSB_ROLLED
       for (int k = 0; k < N; ++k) {
         w.ah[K] += u.aLevel[k];
         w.adv[k][K] += u.aArea[k];
@@ -563,9 +609,11 @@ SSB_HD bool unit_reverse(const DevModel& M, const PoseD& F, const Tape& t, UnitW
         w.aV += u.aVol[0];
       } else {
         double tot = 0;
+        SSB_ROLLED
         for (int k = 0; k < N; ++k) tot += rec(t, r.members[k], K)[1];
         double assigned = 0, aTot = 0;
         double aV = u.aVol[N - 1];
+        SSB_ROLLED
         for (int k = 0; k < N - 1; ++k) {
           const double pk = rec(t, r.members[k], K)[1];
           double v = tot > 0 ? r.V * pk / tot : r.V / static_cast<double>(N);
@@ -585,6 +633,7 @@ SSB_HD bool unit_reverse(const DevModel& M, const PoseD& F, const Tape& t, UnitW
         w.aV = aV;
         if (r.V - assigned > M.vmax[r.members[N - 1]]) w.err = kErrCascade;
         else if (aTot != 0)
+          SSB_ROLLED
           for (int k = 0; k < N; ++k) w.av[k][K] += aTot;
       }
     }
@@ -593,6 +642,7 @@ SSB_HD bool unit_reverse(const DevModel& M, const PoseD& F, const Tape& t, UnitW
   if (w.err) { *err |= w.err; return false; }
   // the final passes: their level derivative (volume and moments), before the chain of updates
   if (r.cs != 0)
+    SSB_ROLLED
     for (int k = 0; k < N; ++k) {
       const double a1 = lane_sum(pass_sweep1(M, F, r.members[k], w.hFinal[k], w.av[k][K], w.amx[k], w.amy[k], w.amz[k], lane, width, aP), width);
       if (lane == 0) {
@@ -603,15 +653,18 @@ SSB_HD bool unit_reverse(const DevModel& M, const PoseD& F, const Tape& t, UnitW
   if (lane == 0) {
     if (r.cs == 2) {
       // the updates, last first: h_{j+1} = h_j - err_j / dv_j (Newton) or the bracket's midpoint (bisection)
+      SSB_ROLLED
       for (int j = K - 1; j >= r.base; --j) {
         if (r.newton[j]) {
           double e = 0, dvs = 0;
+          SSB_ROLLED
           for (int k = 0; k < N; ++k) { e += rec(t, r.members[k], j)[1]; dvs += rec(t, r.members[k], j)[2]; }
           e = e - r.V;
           w.ah[j] += w.ah[j + 1];
           const double aErr = -w.ah[j + 1] / dvs;
           const double aDvs = w.ah[j + 1] * e / (dvs * dvs);
           w.aV -= aErr;
+          SSB_ROLLED
           for (int k = 0; k < N; ++k) { w.av[k][j] += aErr; w.adv[k][j] += aDvs; }
         } else {
           const double half = 0.5 * w.ah[j + 1];
@@ -623,6 +676,7 @@ SSB_HD bool unit_reverse(const DevModel& M, const PoseD& F, const Tape& t, UnitW
           }
         }
         // pass j's own level dependence: d vol / d h is its free-surface area, its area does not depend on h
+        SSB_ROLLED
         for (int k = 0; k < N; ++k) w.ah[j] += w.av[k][j] * rec(t, r.members[k], j)[2];
       }
       // the first Newton level: the clamped start (the extent's bottom or top) or the start itself
@@ -632,8 +686,10 @@ SSB_HD bool unit_reverse(const DevModel& M, const PoseD& F, const Tape& t, UnitW
         w.aH0 += w.ah[0];
       }
       // the passes before the final one whose volume the chain reached: their pose adjoints come from a sweep
+      SSB_ROLLED
       for (int k = 0; k < N; ++k) {
         int np = 0;
+        SSB_ROLLED
         for (int j = r.base; j < K; ++j) {
           if (w.av[k][j] == 0) continue;
           w.hs[k][np] = rec(t, r.members[k], j)[0];
@@ -650,9 +706,11 @@ SSB_HD bool unit_reverse(const DevModel& M, const PoseD& F, const Tape& t, UnitW
     }
   }
   warp_sync();
+  SSB_ROLLED
   for (int k = 0; k < N; ++k)
     if (w.np[k]) pass_sweep_levels(M, F, r.members[k], w.np[k], w.hs[k], w.pv[k], lane, width, aP);
   // (every lane finds the same segment; lane 0 alone adds its terms)
+  SSB_ROLLED
   for (int k = 0; k < N; ++k) {
     if (w.aZmin0[k] != 0) {
       const int j = pass_extreme(M, F, r.members[k], true, lane, width);
@@ -666,17 +724,21 @@ SSB_HD bool unit_reverse(const DevModel& M, const PoseD& F, const Tape& t, UnitW
   if (lane == 0) {
     // the free-surface area of every pass: dv = (sum of the cut segments' footprints) mu / R22; lane 0 alone adds it
     // to the pose adjoint, which is summed over the lanes afterwards
+    SSB_ROLLED
     for (int k = 0; k < N; ++k)
+      SSB_ROLLED
       for (int j = 0; j <= K && j < kMaxPasses; ++j)
         if (w.adv[k][j] != 0) aP.iR += w.adv[k][j] * rec(t, r.members[k], j)[2] / F.iR;
     // the start level and the unit's volume
     if (r.single) {
       u.oLevel[0] += w.aH0;
     } else if (r.allWet) {
+      SSB_ROLLED
       for (int k = 0; k < N; ++k) u.oLevel[k] += w.aH0 / static_cast<double>(N);
     } else {
       u.oLevel[r.firstWet >= 0 ? r.firstWet : N - 1] += w.aH0;
     }
+    SSB_ROLLED
     for (int k = 0; k < N; ++k) u.oVol[k] += w.aV;
   }
   return true;
@@ -721,9 +783,9 @@ SSB_HD FlowRec flow_forward(const DevModel& M, const PoseD& F, double t, const s
       f.f = 1;
       if (f.H2 > 0) {
         f.r = f.H2 / f.H1;
-        f.p1 = reuse ? pw[2 * c] : pm::pow(f.r, kWeirExponent);
+        f.p1 = reuse ? pw[2 * c] : pow_of(f.r, kWeirExponent);
         f.g = 1 - f.p1;
-        f.f = reuse ? pw[2 * c + 1] : pm::pow(jmax(0.0, f.g), kVillemonteExponent);
+        f.f = reuse ? pw[2 * c + 1] : pow_of(jmax(0.0, f.g), kVillemonteExponent);
         if (!reuse) { pw[2 * c] = f.p1; pw[2 * c + 1] = f.f; }
       }
       q = M.coef[c] * area[c] * kWeirCoefficient * M.sq2g * f.H1 * pm::sqrt_rn(f.H1) * f.f * (f.Ha >= f.Hb ? 1.0 : -1.0);
@@ -977,6 +1039,7 @@ SSB_HDT bool reverse_step(const T& team, const DevModel& M, const Tape& tp, cons
   const int NN = M.nn, NC = M.nc;
 
   // ---- the step's flows, volume update and loads, recomputed (flows.hpp:15-118, body.hpp:11-40)
+  SSB_ROLLED
   for (int n = team.rank; n < NN; n += team.size) {
     const double v = volS[n];
     S.hEff[n] = v > kEmptyVolume ? levelS[n] : kNoHead;
@@ -984,6 +1047,7 @@ SSB_HDT bool reverse_step(const T& team, const DevModel& M, const Tape& tp, cons
     S.deg[n] = 0;
   }
   team.sync();
+  SSB_ROLLED
   for (int c = team.rank; c < NC; c += team.size) {
     if (!en[c]) continue;
     const int ca = M.ca[c], cb = M.cb[c];
@@ -992,14 +1056,17 @@ SSB_HDT bool reverse_step(const T& team, const DevModel& M, const Tape& tp, cons
     team.add_int(&S.deg[cb], 1);
   }
   team.sync();
+  SSB_ROLLED
   for (int c = team.rank; c < NC; c += team.size)
     S.dV[c] = flow_forward(M, F, t, en, area, tOn, S.hEff, S.aEff, S.deg, merged, c, S.pw, false).dV;
   team.sync();
   LoadSums Ls = loads_buoyancy(M, F, hb);
   double part[6] = {0, 0, 0, 0, 0, 0};
+  SSB_ROLLED
   for (int n = team.rank; n < NN; n += team.size) {
     const int k0 = M.incStart[n], k1 = k0 + M.incCount[n];
     double acc = 0;
+    SSB_ROLLED
     for (int k = k0; k < k1; ++k) {
       const double d = S.dV[M.incConn[k]];
       acc = M.incSide[k] ? acc + d : acc - d;
@@ -1037,6 +1104,7 @@ SSB_HDT bool reverse_step(const T& team, const DevModel& M, const Tape& tp, cons
     if (team.rank == 0)
       for (int k = 0; k < kAdjPoseFields; ++k) fields(aP)[k] += fields(once)[k];
   }
+  SSB_ROLLED
   for (int n = team.rank; n < NN; n += team.size) {
     double aV, ax, ay, az;
     loads_node_reverse(M, F, zO, S.volPost[n], cxS[n], cyS[n], czS[n], aL, F.cth, aV, ax, ay, az, aZo, aP);
@@ -1057,6 +1125,7 @@ SSB_HDT bool reverse_step(const T& team, const DevModel& M, const Tape& tp, cons
   team.sync();
 
   // ---- flows
+  SSB_ROLLED
   for (int c = team.rank; c < NC; c += team.size) {
     const int ca = M.ca[c], cb = M.cb[c];
     const double aDV = S.aAcc[cb] - (ca >= 0 ? S.aAcc[ca] : 0.0);
@@ -1067,9 +1136,11 @@ SSB_HDT bool reverse_step(const T& team, const DevModel& M, const Tape& tp, cons
   }
   team.sync();
   // heads and limiter areas (flows.hpp:15-19): per node, its connections' adjoints in incidence order
+  SSB_ROLLED
   for (int n = team.rank; n < NN; n += team.size) {
     const int k0 = M.incStart[n], k1 = k0 + M.incCount[n];
     double aH = 0, aA = 0;
+    SSB_ROLLED
     for (int k = k0; k < k1; ++k) {
       const int c = M.incConn[k];
       if (M.incSide[k]) { aH += S.faHB[c]; aA += S.faAB[c]; }
@@ -1089,6 +1160,7 @@ SSB_HDT bool reverse_step(const T& team, const DevModel& M, const Tape& tp, cons
   // warps in turn: a warp per merged group or node alone, lane 0 doing its scalar chain in the warp's work area.
   if (team.warp == 0) {
     int base = 0;
+    SSB_ROLLED
     for (int g0 = 0; g0 < M.ng; g0 += team.width) {
       const int g = g0 + team.lane;
       int c = 0;
@@ -1097,6 +1169,7 @@ SSB_HDT bool reverse_step(const T& team, const DevModel& M, const Tape& tp, cons
           c = 1;
         } else {
           const int* mem = M.gNodes + M.gStart[g];
+          SSB_ROLLED
           for (int k = 0; k < M.gCount[g]; ++k) {
             const int n = mem[k];
             S.plain[n] = tp.d[L.volIn + n] <= kEmptyVolume && tp.i[L.npass + n] == 1 && tp.pass(n, 0)[0] == tp.d[L.levelIn + n] &&
@@ -1118,6 +1191,7 @@ SSB_HDT bool reverse_step(const T& team, const DevModel& M, const Tape& tp, cons
           S.units[at] = (g << 16) | 0xffff;
         } else {
           const int* mem = M.gNodes + M.gStart[g];
+          SSB_ROLLED
           for (int k = 0; k < M.gCount[g]; ++k)
             if (!S.plain[mem[k]]) S.units[at++] = (g << 16) | k;
         }
@@ -1129,6 +1203,7 @@ SSB_HDT bool reverse_step(const T& team, const DevModel& M, const Tape& tp, cons
   team.sync();
   const int nu = *S.nunits;
   // every unit's replay at once, a thread per unit (the replay is a chain of scalar decisions over the recorded passes)
+  SSB_ROLLED
   for (int i = team.rank; i < nu; i += team.size) {
     const int e = S.units[i];
     const int g = e >> 16, u = e & 0xffff;
@@ -1137,6 +1212,7 @@ SSB_HDT bool reverse_step(const T& team, const DevModel& M, const Tape& tp, cons
     const int un = isMerged ? M.gCount[g] : 1;
     Replay& r = S.replays[i];
     replay_unit(M, tp, um, un, !isMerged, r);
+    SSB_ROLLED
     for (int k = 0; k < un && k < kMaxMembers; ++k) {
       const int want = r.cs == 0 ? 1 : (r.cs == 1 ? 2 : r.K + 1);
       r.ok = r.ok && tp.i[L.npass + um[k]] == want;
@@ -1145,6 +1221,7 @@ SSB_HDT bool reverse_step(const T& team, const DevModel& M, const Tape& tp, cons
   team.sync();
   bool ok = true;
   UnitWork& w = S.work[team.warp];
+  SSB_ROLLED
   for (int i = team.warp; i < nu; i += team.nwarps) {
     {
       const int e = S.units[i];
@@ -1159,9 +1236,11 @@ SSB_HDT bool reverse_step(const T& team, const DevModel& M, const Tape& tp, cons
       {
         const auto* src = reinterpret_cast<const std::int32_t*>(&S.replays[i]);
         auto* dst = reinterpret_cast<std::int32_t*>(&w.r);
+        SSB_ROLLED
         for (int k = team.lane; k < static_cast<int>(sizeof(Replay) / sizeof(std::int32_t)); k += team.width) dst[k] = src[k];
       }
       if (team.lane == 0) {
+        SSB_ROLLED
         for (int k = 0; k < un; ++k) {
           const int n = um[k];
           w.u.aLevel[k] = S.aLs[n]; w.u.aArea[k] = S.aAs[n]; w.u.aCx[k] = S.aCxs[n]; w.u.aCy[k] = S.aCys[n]; w.u.aCz[k] = S.aCzs[n];
@@ -1182,6 +1261,7 @@ SSB_HDT bool reverse_step(const T& team, const DevModel& M, const Tape& tp, cons
         }
       }
       if (done && team.lane == 0)
+        SSB_ROLLED
         for (int k = 0; k < un; ++k) {
           const int n = um[k];
           a.aVol[n] = w.u.oVol[k]; a.aLevel[n] = w.u.oLevel[k];

@@ -57,10 +57,12 @@ __device__ const unsigned char* stage_column_table(const typename Vec2<T>::type*
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(to), "l"(src[k]),
                      "r"(bulk), "r"(bar)
                      : "memory");
+#pragma unroll 1
       for (std::size_t b = bulk; b < size[k]; ++b) dst[off[k] + b] = src[k][b];
     }
   }
   bool done = false;
+#pragma unroll 1
   for (int it = 0; it < kStageWaitLimit && !done; ++it) {
     unsigned ready;
     asm volatile(
@@ -77,22 +79,28 @@ __device__ const unsigned char* stage_column_table(const typename Vec2<T>::type*
   return dst;
 }
 
+// A trace record: the run's values by the leader, the nodes by the team's lane groups (an empty node's level is formed by
+// a group's lanes side by side).
 template <bool MIXED, int W>
 __device__ __forceinline__ void write_record(double* rec, const SimRegs& R, const DevModel& M, const Slot& S, const Team<W>& T) {
   const int nn = M.nn;
-  if (T.warp != 0) return;
-  const int lane = T.lane;
-  if (lane == 0) {
+  if (T.leader()) {
     rec[0] = R.t; rec[1] = R.zO; rec[2] = R.pitch; rec[3] = R.roll; rec[4] = R.vz; rec[5] = R.wth; rec[6] = R.wph;
     rec[7] = R.inflow; rec[8] = R.Vb; rec[9] = R.hullTop;
   }
+  constexpr int LANES = kLevelLanes<MIXED>, GROUPS = 32 / LANES * W;
+  const LevelLanes L = level_lanes<MIXED>(T.lane);
   double* p = rec + 10;
-  for (int n = lane; n < nn; n += kLanes) {
-    p[n] = S.vol[n];
-    p[nn + n] = stale_level<MIXED>(M, S, n);
-    p[2 * nn + n] = S.cx[n];
-    p[3 * nn + n] = S.cy[n];
-    p[4 * nn + n] = S.cz[n];
+#pragma unroll 1
+  for (int n = T.rank / LANES; n < nn; n += GROUPS) {
+    const double level = group_level<MIXED>(M, S, n, L);
+    if (L.sub == 0) {
+      p[n] = S.vol[n];
+      p[nn + n] = level;
+      p[2 * nn + n] = S.cx[n];
+      p[3 * nn + n] = S.cy[n];
+      p[4 * nn + n] = S.cz[n];
+    }
   }
 }
 
@@ -114,13 +122,16 @@ __device__ bool run_instance(const DevModel& M, const DevBatch& B, Slot& S, int 
     R.founderT = B.founderT[inst];
     R.evCount = B.evCount[inst];
   }
+#pragma unroll 1
   for (int n = rank; n < M.nn; n += kStride) {
     S.vol[n] = B.vol[iN + n]; S.level[n] = B.level[iN + n];
     S.cx[n] = B.cx[iN + n]; S.cy[n] = B.cy[iN + n]; S.cz[n] = B.cz[iN + n];
     S.area[n] = 0; S.zmax[n] = 0; S.hEff[n] = 0; S.aEff[n] = 0; S.acc[n] = 0; S.deg[n] = 0;
     S.dry[n] = 0;
   }
+#pragma unroll 1
   for (int g = rank; g < M.ng; g += kStride) S.merged[g] = 0;
+#pragma unroll 1
   for (int c = rank; c < M.nc; c += kStride) S.dV[c] = 0;
   T.sync();
   if (T.warp == W - 1) list_groups<true>(M, S, T.lane);
@@ -145,17 +156,19 @@ __device__ bool run_instance(const DevModel& M, const DevBatch& B, Slot& S, int 
     const Pose F0 = make_pose(M, R.zO, R.pitch, R.roll);
     const Buoy hb = buoyancy<MIXED, W>(M, F0, T, S.hydro, S.cols);
     R.inflow = 0; R.Vb = hb.V; R.hullTop = hb.top; R.bx = hb.x; R.by = hb.y; R.bz = hb.z;
-    write_record<MIXED>(denseBase, R, M, S, T);
-    write_record<MIXED>(sampleBase, R, M, S, T);
+#pragma unroll 1
+    for (int k = 0; k < 2; ++k) write_record<MIXED>(k == 0 ? denseBase : sampleBase, R, M, S, T);
     denseCount = 1; sampleCount = 1; nextSample = B.sampleEvery;
     T.sync();
   }
 
   int stop = kRunning;
   bool paused = false;
-  // every thread of the team stores the same pose; no thread reads the previous one after the step's last barrier
-  // (the two poses change places at the end of a step, so the last solve's stays for stale_level)
+  // every thread of the team stores the same pose and values; a step replaces them (team_step)
   *S.pose = make_pose(M, R.zO, R.pitch, R.roll);
+  park(S.parked, R);
+  T.sync();
+#pragma unroll 1
   for (long long s = 0; s < B.maxSteps; ++s) {
     if (R.foundered || R.t >= B.tMax) break;
     if (B.yieldBelow > 0 && s > 0 && (s % kYieldCheckEvery) == 0) {
@@ -176,20 +189,24 @@ __device__ bool run_instance(const DevModel& M, const DevBatch& B, Slot& S, int 
       }
       ++curveCount;
       nextCurve += B.curveEvery;
+      T.sync();  // no warp starts the next solve, which changes volumes, while the first still adds them up
     }
-    team_step<MIXED, W>(M, *S.pose, R, S, I, T);
+    team_step<MIXED, W>(M, R, S, I, T);
     ++done;
-    Pose* const last = S.pose;
-    S.pose = S.prev;
-    S.prev = last;
-    Pose& F = *S.pose;
-    F = make_pose(M, R.zO, R.pitch, R.roll);
+    const Pose& F = *S.pose;
     if (traced) {
-      if (done <= B.denseSteps) write_record<MIXED>(denseBase + static_cast<std::size_t>(denseCount++) * B.recSize, R, M, S, T);
-      if (R.t >= nextSample - 1e-9 && sampleCount < B.maxSamples) {
-        write_record<MIXED>(sampleBase + static_cast<std::size_t>(sampleCount++) * B.recSize, R, M, S, T);
-        nextSample += B.sampleEvery;
+#pragma unroll 1
+      for (int k = 0; k < 2; ++k) {
+        double* rec = nullptr;
+        if (k == 0) {
+          if (done <= B.denseSteps) rec = denseBase + static_cast<std::size_t>(denseCount++) * B.recSize;
+        } else if (R.t >= nextSample - 1e-9 && sampleCount < B.maxSamples) {
+          rec = sampleBase + static_cast<std::size_t>(sampleCount++) * B.recSize;
+          nextSample += B.sampleEvery;
+        }
+        if (rec) write_record<MIXED>(rec, R, M, S, T);
       }
+      T.sync();  // no warp starts the next solve while another still reads the nodes
     }
     if (B.stopWhenStable && R.t > 1800) {
       R.calm = (fabs(R.inflow) < 0.02 && fabs(R.wth) < 1e-5 && fabs(R.vz) < 1e-3) ? R.calm + M.dt : 0;
@@ -210,10 +227,12 @@ __device__ bool run_instance(const DevModel& M, const DevBatch& B, Slot& S, int 
 
   // store the instance
   T.sync();
+#pragma unroll 1
   for (int n = rank; n < M.nn; n += kStride) {
     B.vol[iN + n] = S.vol[n]; B.level[iN + n] = stale_level<MIXED>(M, S, n);
     B.cx[iN + n] = S.cx[n]; B.cy[iN + n] = S.cy[n]; B.cz[iN + n] = S.cz[n];
   }
+  if (T.warp == kEventWarp<W> && T.lane == 0) B.evCount[inst] = R.evCount;
   if (T.leader()) {
     double* st = B.st + static_cast<std::size_t>(inst) * 8;
     st[0] = R.t; st[1] = R.zO; st[2] = R.pitch; st[3] = R.roll; st[4] = R.vz; st[5] = R.wth; st[6] = R.wph; st[7] = R.calm;
@@ -221,7 +240,6 @@ __device__ bool run_instance(const DevModel& M, const DevBatch& B, Slot& S, int 
     o[0] = R.inflow; o[1] = R.Vb; o[2] = R.hullTop; o[3] = R.mw; o[4] = R.bx; o[5] = R.by; o[6] = R.bz;
     B.foundered[inst] = R.foundered;
     B.founderT[inst] = R.founderT;
-    B.evCount[inst] = R.evCount;  // the leader is lane 0 of warp 0, which keeps the event log
     B.steps[inst] = done;
     B.stop[inst] = stop;
     if (!(isfinite(R.zO) && isfinite(R.pitch) && isfinite(R.roll) && isfinite(R.vz) && isfinite(R.wth) && isfinite(R.wph)))
@@ -244,7 +262,7 @@ __device__ bool run_instance(const DevModel& M, const DevBatch& B, Slot& S, int 
 // The persistent batch kernel: teams claim instances from the work queue until it runs dry (or the phase yields). In a
 // fleet (FLEET), a team first copies its instance's model description into its slot and steps the instance with it.
 template <bool MIXED, int W, bool FLEET>
-__global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, kMinBlocksPerSM) run_batch(DevModel M, DevBatch B, SlotLayout L) {
+__global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, kMinBlocksPerSM) run_batch(const __grid_constant__ DevModel M, const __grid_constant__ DevBatch B, const __grid_constant__ SlotLayout L) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int warpInBlock = threadIdx.x >> 5;
   const int team = warpInBlock / W;
@@ -278,6 +296,7 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, kMinBlocksPerSM) run_b
       DevModel* const own = reinterpret_cast<DevModel*>(slot + L.model);
       const unsigned* src = reinterpret_cast<const unsigned*>(B.models + B.model[inst]);
       unsigned* dst = reinterpret_cast<unsigned*>(own);
+#pragma unroll 1
       for (int k = T.rank; k < static_cast<int>(sizeof(DevModel) / sizeof(unsigned)); k += 32 * W) dst[k] = src[k];
       T.sync();
       // run_instance ends with a team barrier, so no thread still reads this copy when the next claim overwrites it

@@ -61,6 +61,7 @@ struct DevModel {
   // incidence: per node its connections in increasing order (side 1 at the b end), and the sea connections
   const std::int32_t *incStart, *incCount, *incConn;
   const std::uint8_t* incSide;
+  const std::int32_t* incEdge;  // 2 incConn + incSide
   std::int32_t nsea;
   const std::int32_t* sea;
   // monitors: per monitor its connections in increasing order
@@ -182,10 +183,9 @@ struct Buoy {
   double V, x, y, z, top;
 };
 
-// The run's values that the hydrostatic phases of a step do not read: a team parks them in its slot while those
-// phases run, so that their registers serve the level solve (every thread of the team holds the same values).
+// The run's values, which a team keeps in its slot through a step, so that their registers serve its phases.
 struct Parked {
-  double t, zO, pitch, roll, vz, wth, wph, calm, inflow, Vb, hullTop, mw, bx, by, bz, founderT;
+  double t, zO, pitch, roll, vz, wth, wph, inflow, Vb, hullTop, mw, bx, by, bz, founderT;
   int foundered;
 };
 
@@ -209,14 +209,14 @@ constexpr int kMaxLevelGroupsPerWarp = 32 / (kLevelLanes<false> < kLevelLanes<tr
 
 // Byte offsets of one simulation slot (one team of warps) in dynamic shared memory; `bytes` is the slot stride.
 // passes holds maxGroup node-pass results per level lane group of the team (up to kMaxLevelGroupsPerWarp per warp); hydro the
-// eight buoyancy tree results and the hull top; misc the team's small broadcast values and counters (MiscSlot); dry a flag byte per node and
-// list the groups the next level solve visits, flow the connections that can flow (warp_step.cuh); pose (this step's and the last one's) and buoy the step's
-// pose and buoyancy result, which every phase reads (kept here rather than in each thread's registers); parked the run's
-// values during the hydrostatic phases; model (fleets only) the team's copy of its instance's model. tmp is the sixth
-// column of the loads' per-node terms (the other five reuse area, zmax, hEff, aEff and acc, which are dead by then) and,
-// between the level solve and the heads, of the passes' sums.
+// eight buoyancy tree results and the hull's top; misc the team's small broadcast values and counters (MiscSlot); dry a
+// flag byte per node, list the groups the next level solve visits and flow the connections that can flow
+// (warp_step.cuh); pose this step's pose and the last one's, which every phase reads (kept here rather than in each
+// thread's registers); parked the run's values; model (fleets only) the team's copy of its instance's model. area, zmax,
+// hEff, aEff, tmp and term5 become the six columns of the loads' per-node terms (a fixed stride apart); between the level
+// solve and the heads, acc, hEff, aEff and tmp hold the passes' sums.
 struct SlotLayout {
-  std::uint32_t vol, level, cx, cy, cz, area, zmax, hEff, aEff, acc, deg, dV, flow, tmp, passes, hydro, misc, merged, dry, list, pose, buoy, parked,
+  std::uint32_t vol, level, cx, cy, cz, area, zmax, hEff, aEff, tmp, term5, acc, deg, dV, flow, passes, hydro, misc, merged, dry, list, pose, parked,
       model, bytes;
 };
 

@@ -23,16 +23,16 @@ struct ExtentLists {
   std::vector<std::int32_t> start, idx;
 };
 
-// Appends to out the indices of the points [first, first + n) that no other point beats in all of sx x, sy y, sz z
-// (one of several equal points). x(i), y(i), z(i) give a point's coordinates.
+// Appends to out the points of `from` that no other one beats in all of sx x, sy y, sz z (one of several equal points).
+// x(i), y(i), z(i) give a point's coordinates.
 template <class X, class Y, class Z>
-void append_undominated(std::int32_t first, std::int32_t n, X x, Y y, Z z, double sx, double sy, double sz, std::vector<std::int32_t>& out) {
+void append_undominated(const std::vector<std::int32_t>& from, X x, Y y, Z z, double sx, double sy, double sz, std::vector<std::int32_t>& out) {
   struct P {
     double x, y, z;
     std::int32_t i;
   };
   std::vector<P> kept;
-  for (std::int32_t i = first; i < first + n; ++i) {
+  for (const std::int32_t i : from) {
     const P p{sx * x(i), sy * y(i), sz * z(i), i};
     bool beaten = false;
     for (std::size_t k = 0; k < kept.size(); ++k) {
@@ -50,20 +50,42 @@ void append_undominated(std::int32_t first, std::int32_t n, X x, Y y, Z z, doubl
   for (const P& k : kept) out.push_back(k.i);
 }
 
+// The points of [first, first + n) without those that two neighbours in the array (one or two places away: hulls are
+// stored line by line, some with the sides alternating) beat whatever the signs: the neighbours have the same x and lie on
+// both sides in y, and neither is larger in s z. This leaves the ends of every flat stretch, so the lists are built from a
+// fraction of the points. (Strictly on both sides, so a chain of points that beat one another ends at one that is kept.)
+template <class X, class Y, class Z>
+std::vector<std::int32_t> line_ends(std::int32_t first, std::int32_t n, X x, Y y, Z z, double s) {
+  std::vector<std::int32_t> out;
+  const std::int32_t end = first + n;
+  auto inside = [&](std::int32_t a, std::int32_t b, std::int32_t c) {
+    return a >= first && c < end && x(a) == x(b) && x(b) == x(c) && s * z(a) <= s * z(b) && s * z(c) <= s * z(b) &&
+           ((y(a) < y(b) && y(b) < y(c)) || (y(a) > y(b) && y(b) > y(c)));
+  };
+  for (std::int32_t i = first; i < end; ++i)
+    if (!inside(i - 1, i, i + 1) && !inside(i - 2, i, i + 2)) out.push_back(i);
+  return out;
+}
+
 // The lists of every set n of points [start[n], start[n] + count[n]), with coordinates (x(i), y(i)), bottoms lo(i) and
 // tops hi(i).
 template <class X, class Y, class Lo, class Hi>
 ExtentLists extent_lists(const std::vector<std::int32_t>& start, const std::vector<std::int32_t>& count, X x, Y y, Lo lo, Hi hi) {
   ExtentLists L;
   L.start.push_back(0);
+  std::vector<std::vector<std::int32_t>> ends[2];
+  for (std::size_t n = 0; n < start.size(); ++n) {
+    ends[0].push_back(line_ends(start[n], count[n], x, y, lo, 1.0));
+    ends[1].push_back(line_ends(start[n], count[n], x, y, hi, -1.0));
+  }
   for (int q = 0; q < 4; ++q)
     for (int end = 0; end < 2; ++end)
       for (std::size_t n = 0; n < start.size(); ++n) {
         // the minimum looks for small directed coordinates, the maximum for large ones
         const double s = end == 0 ? 1.0 : -1.0;
         const double sx = (q & 1) ? -s : s, sy = (q & 2) ? -s : s;
-        if (end == 0) append_undominated(start[n], count[n], x, y, lo, sx, sy, s, L.idx);
-        else append_undominated(start[n], count[n], x, y, hi, sx, sy, s, L.idx);
+        if (end == 0) append_undominated(ends[0][n], x, y, lo, sx, sy, s, L.idx);
+        else append_undominated(ends[1][n], x, y, hi, sx, sy, s, L.idx);
         L.start.push_back(static_cast<std::int32_t>(L.idx.size()));
       }
   return L;

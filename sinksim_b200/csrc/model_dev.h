@@ -67,7 +67,7 @@ inline std::uint32_t take(std::uint32_t& off, std::size_t bytes) {
 }
 
 // The shared-memory slot of one simulation of a model of these sizes, stepped by a team of W warps: per-node state and
-// scratch, the connections' flows and their list, the group-pass buffers, the buoyancy tree results, the poses, buoyancy result and
+// scratch, the connections' flows and their list, the group-pass buffers, the buoyancy tree results, the poses and
 // parked run values, and in a fleet the team's copy of its instance's model.
 inline SlotLayout slot_layout(std::int32_t NN, std::int32_t NC, std::int32_t NG, std::int32_t maxGroup, int W, bool fleet) {
   SlotLayout L{};
@@ -75,11 +75,14 @@ inline SlotLayout slot_layout(std::int32_t NN, std::int32_t NC, std::int32_t NG,
   const std::size_t nb = sizeof(double) * static_cast<std::size_t>(NN);
   const std::size_t cb = sizeof(double) * static_cast<std::size_t>(std::max(NC, 1));
   L.vol = take(off, nb); L.level = take(off, nb); L.cx = take(off, nb); L.cy = take(off, nb); L.cz = take(off, nb);
-  L.area = take(off, nb); L.zmax = take(off, nb); L.hEff = take(off, nb); L.aEff = take(off, nb); L.acc = take(off, nb);
+  // six columns that the loads' terms are summed down side by side, so a stride that puts them in different banks
+  const std::size_t column = sizeof(double) * ((static_cast<std::size_t>(NN) + 5) / 8 * 8 + 2);
+  L.area = take(off, column); L.zmax = take(off, column); L.hEff = take(off, column); L.aEff = take(off, column); L.tmp = take(off, column);
+  L.term5 = take(off, column);
+  L.acc = take(off, nb);
   L.deg = take(off, sizeof(std::int32_t) * static_cast<std::size_t>(NN));
   L.dV = take(off, cb);
   L.flow = take(off, sizeof(std::uint16_t) * static_cast<std::size_t>(std::max(NC, 1)));
-  L.tmp = take(off, nb);
   L.passes = take(off, 5 * sizeof(double) * static_cast<std::size_t>(maxGroup) * static_cast<std::size_t>(W * kMaxLevelGroupsPerWarp));
   L.hydro = take(off, 33 * sizeof(double));
   L.misc = take(off, 8 * sizeof(std::int32_t));
@@ -87,7 +90,6 @@ inline SlotLayout slot_layout(std::int32_t NN, std::int32_t NC, std::int32_t NG,
   L.dry = take(off, static_cast<std::size_t>(std::max(NN, 1)));
   L.list = take(off, sizeof(std::uint16_t) * static_cast<std::size_t>(std::max(NG, 1)));
   L.pose = take(off, 2 * sizeof(Pose));
-  L.buoy = take(off, sizeof(Buoy));
   L.parked = take(off, sizeof(Parked));
   L.model = fleet ? take(off, sizeof(DevModel)) : 0u;
   L.bytes = off;
@@ -107,7 +109,7 @@ struct ModelDev {
   DevBuf<float2> colXYf, colLHf, segXYf, segLHf, exXYf;
   DevBuf<float> colAf, segArf, exZf;
   DevBuf<double> colA, segAr, exZ, mu, vmax, amin, aov;
-  DevBuf<std::int32_t> exStart, segStart, segCount, gStart, gCount, gNodes, ca, cb, skip, incStart, incCount, incConn, sea, monStart, monCount, monConn;
+  DevBuf<std::int32_t> exStart, incEdge, segStart, segCount, gStart, gCount, gNodes, ca, cb, skip, incStart, incCount, incConn, sea, monStart, monCount, monConn;
   DevBuf<std::uint8_t> gMode, law, incSide, mkWhen;
   DevBuf<double> gpx, gpy, gpz, kx, ky, kz, coef, mkx, mky, mkz;
   DevModel dm{};
@@ -182,6 +184,9 @@ struct ModelDev {
     ca.upload(M.ca, s); cb.upload(M.cb, s); skip.upload(M.cSkipGroup, s); law.upload(M.cLaw, s);
     kx.upload(M.cx, s); ky.upload(M.cy, s); kz.upload(M.cz, s); coef.upload(M.cCoef, s);
     incStart.upload(inc.start, s); incCount.upload(inc.count, s); incConn.upload(inc.conn, s); incSide.upload(inc.side, s);
+    std::vector<std::int32_t> edge(inc.conn.size());
+    for (std::size_t k = 0; k < edge.size(); ++k) edge[k] = 2 * inc.conn[k] + (inc.side[k] ? 1 : 0);
+    incEdge.upload(edge, s);
     sea.upload(inc.sea.empty() ? std::vector<std::int32_t>{0} : inc.sea, s);
     monStart.upload(mons.start.empty() ? std::vector<std::int32_t>{0} : mons.start, s);
     monCount.upload(mons.count.empty() ? std::vector<std::int32_t>{0} : mons.count, s);
@@ -209,7 +214,7 @@ struct ModelDev {
     d.nc = NC;
     d.ca = ca.get(); d.cb = cb.get(); d.skip = skip.get(); d.law = law.get();
     d.kx = kx.get(); d.ky = ky.get(); d.kz = kz.get(); d.coef = coef.get();
-    d.incStart = incStart.get(); d.incCount = incCount.get(); d.incConn = incConn.get(); d.incSide = incSide.get();
+    d.incStart = incStart.get(); d.incCount = incCount.get(); d.incConn = incConn.get(); d.incSide = incSide.get(); d.incEdge = incEdge.get();
     d.nsea = static_cast<std::int32_t>(inc.sea.size()); d.sea = sea.get();
     d.nmon = nmon; d.monThreshold = M.monitorThreshold;
     d.monStart = monStart.get(); d.monCount = monCount.get(); d.monConn = monConn.get();

@@ -247,6 +247,35 @@ SSB_HD double cos(double x) {
   }
 }
 
+// sin(x) into s and cos(x) into c, from one reduction: the same bits as sin and cos.
+SSB_HD void sin_cos(double x, double& s, double& c) {
+  const std::int32_t ix = high_word(x) & 0x7fffffff;
+  if (ix <= 0x3fe921fb) {
+    s = sin_kernel(x, 0.0, 0);
+    c = cos_kernel(x, 0.0);
+    return;
+  }
+  if (ix >= 0x7ff00000) { s = c = x - x; return; }  // inf or NaN
+  double y0, y1;
+  bool ok;
+  const int n = reduce_half_pi(x, y0, y1, ok);
+  if (!ok) {
+#if defined(__CUDA_ARCH__)
+    s = ::sin(x); c = ::cos(x);
+#else
+    s = std::sin(x); c = std::cos(x);
+#endif
+    return;
+  }
+  const double ks = sin_kernel(y0, y1, 1), kc = cos_kernel(y0, y1);
+  switch (n & 3) {
+    case 0: s = ks; c = kc; break;
+    case 1: s = kc; c = -ks; break;
+    case 2: s = -ks; c = -kc; break;
+    default: s = -kc; c = ks; break;
+  }
+}
+
 // ----------------------------------------------------------------------------- pow (e_pow.c)
 
 // log2(ax) as t1 + t2, t1 with a cleared low word, for |y| <= 2^31 (the general path of e_pow.c step 1).

@@ -30,8 +30,26 @@ namespace ssb {
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kLanes = 32;
 
+// What a step issues must come from the instruction caches: with everything inlined and unrolled the kernel was 396 KB
+// of code, and once the level solve issued a third of its instructions the warps waited for code most of the time (8.8 of
+// 15.8 warps per issue, 1-warp teams). So the portable math, the extremes and the buoyancy are called, and loops that need
+// no overlap are not unrolled: 140 KB, most of it outside the step. Together with the sums a lane per column and one warp
+// for the motion (move_body), on B200: 2,048 uneven titanic64 runs to 20 min 371 ms against 469, a fleet of 96 ships to
+// 5 min 36.5 against 62.4, one run to 5 min 29.1 against 32.2, 48 portable32 runs to 15 min 68 against 83.
+static __device__ __noinline__ double2 trig_of(double x) {
+  double s, c;
+  pm::sin_cos(x, s, c);
+  return double2{s, c};
+}
+static __device__ __noinline__ double pow_of(double x, double y) { return pm::pow(x, y); }
+
+// The pose of (zO, pitch th, roll ph); a whole warp calls it (even lanes take the pitch's sine and cosine, odd lanes the
+// roll's, and they swap).
 __device__ __forceinline__ Pose make_pose(const DevModel& M, double zO, double th, double ph) {
-  const double cth = pm::cos(th), sth = pm::sin(th), cph = pm::cos(ph), sph = pm::sin(ph);
+  const bool odd = threadIdx.x & 1;
+  const double2 t = trig_of(odd ? ph : th);
+  const double os = __shfl_xor_sync(kFull, t.x, 1), oc = __shfl_xor_sync(kFull, t.y, 1);
+  const double sth = odd ? os : t.x, cth = odd ? oc : t.y, sph = odd ? t.x : os, cph = odd ? t.y : oc;
   Pose F;
   F.R00 = cth; F.R01 = sth * sph; F.R02 = sth * cph;
   F.R10 = 0;   F.R11 = cph;       F.R12 = -sph;
@@ -121,8 +139,8 @@ struct Prec<true> {
   static __device__ __forceinline__ T iR(const Pose& F) { return F.fiR; }
 };
 
-template <bool MIXED, bool MAX>
-__device__ __forceinline__ typename Prec<MIXED>::T node_extreme(const DevModel& M, const Pose& F, int n, int sub, int lanes) {
+template <bool MIXED>
+__device__ __noinline__ typename Prec<MIXED>::T node_extreme(const DevModel& M, const Pose& F, int n, bool top, int sub, int lanes) {
   using P = Prec<MIXED>;
   using T = typename P::T;
   const T R20 = P::R20(F), R21 = P::R21(F), R22 = P::R22(F), tz = P::tz(F);
@@ -130,22 +148,23 @@ __device__ __forceinline__ typename Prec<MIXED>::T node_extreme(const DevModel& 
   const T* z = P::exZ(M);
   int j, end, zs = 1;
   if (F.R22 >= 0) {
-    const int list = ((F.R20 < 0 ? 2 : 0) + (F.R21 < 0 ? 4 : 0) + (MAX ? 1 : 0)) * (M.nn + 1) + n;
+    const int list = ((F.R20 < 0 ? 2 : 0) + (F.R21 < 0 ? 4 : 0) + (top ? 1 : 0)) * (M.nn + 1) + n;
     j = __ldg(M.exStart + list);
     end = __ldg(M.exStart + list + 1);
   } else {
     const bool hull = n == M.nn;
     xy = hull ? P::colXY(M) : P::segXY(M);
-    z = reinterpret_cast<const T*>(hull ? P::colLH(M) : P::segLH(M)) + (MAX ? 1 : 0);
+    z = reinterpret_cast<const T*>(hull ? P::colLH(M) : P::segLH(M)) + (top ? 1 : 0);
     zs = 2;
     j = hull ? 0 : __ldg(M.segStart + n);
     end = j + (hull ? M.ncol : __ldg(M.segCount + n));
   }
-  T best = MAX ? T(-1e9) : T(1e9);
+  T best = top ? T(-1e9) : T(1e9);
+#pragma unroll 1
   for (j += sub; j < end; j += lanes) {
     const auto p = __ldg(xy + j);
     const T w = R20 * p.x + R21 * p.y + tz + R22 * __ldg(z + static_cast<std::size_t>(j) * zs);
-    if (MAX ? w > best : w < best) best = w;
+    if (top ? w > best : w < best) best = w;
   }
   return best;
 }
@@ -203,22 +222,27 @@ __device__ __forceinline__ P load_col(const P* p) {
   else return __ldg(p);
 }
 
-// Lane `lane`'s partial of tree w: columns w*32 + lane + 256 k in increasing k, two at a time (loads of the second
-// column issue before the first is clipped; the clips stay in order).
+// Lane `lane`'s partial of tree w: columns w*32 + lane + 256 k in increasing k, four at a time (the loads of all four
+// issue before the first is clipped; the clips stay in order).
 template <class T, bool SMEM = false>
 __device__ __forceinline__ ColPartial<T> column_partial(const typename Vec2<T>::type* xy, const typename Vec2<T>::type* lh, const T* area,
                                                         int ncol, int first, T R20, T R21, T tz, T iR) {
+  constexpr int kAtOnce = 4;
   ColPartial<T> p{T(0), T(0), T(0), T(0)};
-  int i = first;
-  for (; i + 256 < ncol; i += 512) {
-    const auto a0 = load_col<SMEM>(xy + i), b0 = load_col<SMEM>(lh + i), a1 = load_col<SMEM>(xy + i + 256), b1 = load_col<SMEM>(lh + i + 256);
-    const T A0 = load_col<SMEM>(area + i), A1 = load_col<SMEM>(area + i + 256);
-    clip_column<T>(a0.x, a0.y, b0.x, b0.y, A0, R20, R21, tz, iR, p);
-    clip_column<T>(a1.x, a1.y, b1.x, b1.y, A1, R20, R21, tz, iR, p);
-  }
-  if (i < ncol) {
-    const auto a0 = load_col<SMEM>(xy + i), b0 = load_col<SMEM>(lh + i);
-    clip_column<T>(a0.x, a0.y, b0.x, b0.y, load_col<SMEM>(area + i), R20, R21, tz, iR, p);
+#pragma unroll 1
+  for (int i = first; i < ncol; i += kAtOnce * 256) {
+    typename Vec2<T>::type a[kAtOnce], b[kAtOnce];
+    T A[kAtOnce];
+#pragma unroll
+    for (int k = 0; k < kAtOnce; ++k) {
+      // past the table's end: the last column read again with no footprint, which adds zeros
+      const int j = i + 256 * k < ncol ? i + 256 * k : i;
+      a[k] = load_col<SMEM>(xy + j);
+      b[k] = load_col<SMEM>(lh + j);
+      A[k] = i + 256 * k < ncol ? load_col<SMEM>(area + j) : T(0);
+    }
+#pragma unroll
+    for (int k = 0; k < kAtOnce; ++k) clip_column<T>(a[k].x, a[k].y, b[k].x, b[k].y, A[k], R20, R21, tz, iR, p);
   }
   return p;
 }
@@ -247,11 +271,11 @@ __host__ __device__ __forceinline__ StagedColumns<T> staged_columns(int ncol) {
 // hull's highest point; the results meet in shared memory (four values per tree, then the top) and every thread adds
 // them in the reference's order (trees 0..7).
 template <bool MIXED, int W>
-__device__ __forceinline__ void buoyancy_trees(const DevModel& M, const Pose& F, const Team<W>& T, double* trees, const unsigned char* cols) {
+__device__ __noinline__ void buoyancy_trees(const DevModel& M, const Pose& F, int warp, int lane, double* trees, const unsigned char* cols) {
   using P = Prec<MIXED>;
   using R = typename P::T;
-  const int lane = T.lane;
-  for (int w = T.warp; w < 8; w += W) {
+#pragma unroll 1
+  for (int w = warp; w < 8; w += W) {
     ColPartial<R> p;
     if (cols) {
       const StagedColumns<R> c = staged_columns<R>(M.ncol);
@@ -269,8 +293,8 @@ __device__ __forceinline__ void buoyancy_trees(const DevModel& M, const Pose& F,
       t[0] = p.V; t[1] = p.Mx; t[2] = p.My; t[3] = p.Mz;
     }
   }
-  if (T.warp == W - 1) {
-    R top = node_extreme<MIXED, true>(M, F, M.nn, lane, kLanes);
+  if (warp == W - 1) {
+    R top = node_extreme<MIXED>(M, F, M.nn, true, lane, kLanes);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
       const R o = __shfl_xor_sync(kFull, top, off);
@@ -299,7 +323,7 @@ __device__ __forceinline__ Buoy buoyancy_finish(const double* trees) {
 
 template <bool MIXED, int W>
 __device__ __forceinline__ Buoy buoyancy(const DevModel& M, const Pose& F, const Team<W>& T, double* trees, const unsigned char* cols) {
-  buoyancy_trees<MIXED, W>(M, F, T, trees, cols);
+  buoyancy_trees<MIXED, W>(M, F, T.warp, T.lane, trees, cols);
   T.sync();
   return buoyancy_finish(trees);
 }
@@ -317,26 +341,30 @@ struct LevelLanes {
   unsigned mask;
 };
 
-// The partials of two tree lanes OFF apart (first segments fa and fa + OFF; OFF 16, or 32 for fa's lane alone: then only
-// pa is formed, two of its segments per iteration), in one loop: each iteration takes the next segment of each, so the
-// two accumulation chains run side by side; each keeps its own segments' order.
-template <class T, bool PAIR>
+template <bool MIXED>
+__device__ __forceinline__ LevelLanes level_lanes(int lane) {
+  constexpr int LANES = kLevelLanes<MIXED>;
+  return LevelLanes{lane, lane % LANES, (LANES == 32 ? kFull : (1u << (LANES & 31)) - 1u) << (lane / LANES * LANES)};
+}
+
+// The partials of two tree lanes 16 apart (first segments fa and fa + 16; PAIR), or of fa's tree lane alone, two of its
+// segments per iteration, in one loop: each iteration takes the next segment of each, so the two accumulation chains run
+// side by side; each keeps its own segments' order. A missing second segment is the first one again with no footprint,
+// which adds zeros. AHEAD iterations' loads issue together.
+template <class T, bool PAIR, int AHEAD>
 __device__ __forceinline__ void segment_partials(const typename Vec2<T>::type* xy, const typename Vec2<T>::type* ab, const T* area, int fa,
                                                  int end, T R20, T R21, T tz, T iR, T h, SegPartial<T>& pa, SegPartial<T>& pb) {
   constexpr int kStep = PAIR ? kLanes : 2 * kLanes, kOff = PAIR ? kLanes / 2 : kLanes;
   pa = SegPartial<T>{T(0), T(0), T(0), T(0), T(0)};
   pb = pa;
-  int ja = fa;
-  for (; ja + kOff < end; ja += kStep) {
-    const int jb = ja + kOff;
+#pragma unroll AHEAD
+  for (int ja = fa; ja < end; ja += kStep) {
+    const bool two = ja + kOff < end;
+    const int jb = two ? ja + kOff : ja;
     const auto a0 = __ldg(xy + ja), b0 = __ldg(ab + ja), a1 = __ldg(xy + jb), b1 = __ldg(ab + jb);
-    const T A0 = __ldg(area + ja), A1 = __ldg(area + jb);
+    const T A0 = __ldg(area + ja), A1 = two ? __ldg(area + jb) : T(0);
     clip_segment<T>(a0.x, a0.y, b0.x, b0.y, A0, R20, R21, tz, iR, h, pa);
     clip_segment<T>(a1.x, a1.y, b1.x, b1.y, A1, R20, R21, tz, iR, h, PAIR ? pb : pa);
-  }
-  if (ja < end) {
-    const auto a0 = __ldg(xy + ja), b0 = __ldg(ab + ja);
-    clip_segment<T>(a0.x, a0.y, b0.x, b0.y, __ldg(area + ja), R20, R21, tz, iR, h, pa);
   }
 }
 
@@ -352,11 +380,12 @@ __device__ __forceinline__ void tree_pair(SegPartial<T>& lo, const SegPartial<T>
 // sub + kLevelLanes j and combines them over the tree's upper levels (offsets 16 down to kLevelLanes) in registers; the
 // lower levels are shuffles inside the group. Every lane of the group ends with the bits of tree lane 0. Every lane of
 // the warp calls it (n < 0: a group without a node, which sums nothing), so the groups' passes run side by side.
-template <bool MIXED>
+template <bool MIXED, int W>
 __device__ __forceinline__ PassR node_pass(const DevModel& M, const Pose& F, int n, double h, const LevelLanes& L) {
   using P = Prec<MIXED>;
   using T = typename P::T;
   constexpr int LANES = kLevelLanes<MIXED>;
+  constexpr int AHEAD = W >= 8 ? 2 : 1;  // large teams are bound by the loads' latency, small ones by issue slots
   const int s0 = n < 0 ? 0 : __ldg(M.segStart + n), s1 = n < 0 ? 0 : s0 + __ldg(M.segCount + n);
   const T hT = static_cast<T>(h);
   const int f = s0 + L.sub;
@@ -365,13 +394,13 @@ __device__ __forceinline__ PassR node_pass(const DevModel& M, const Pose& F, int
   const T* area = P::segAr(M);
   SegPartial<T> p, b;
   if constexpr (LANES == 32) {
-    segment_partials<T, false>(xy, ab, area, f, s1, R20, R21, tz, iR, hT, p, b);
+    segment_partials<T, false, AHEAD>(xy, ab, area, f, s1, R20, R21, tz, iR, hT, p, b);
   } else {
-    segment_partials<T, true>(xy, ab, area, f, s1, R20, R21, tz, iR, hT, p, b);  // tree lanes sub and sub + 16
+    segment_partials<T, true, AHEAD>(xy, ab, area, f, s1, R20, R21, tz, iR, hT, p, b);  // tree lanes sub and sub + 16
     tree_pair(p, b);
     if constexpr (LANES == 8) {
       SegPartial<T> q;
-      segment_partials<T, true>(xy, ab, area, f + 8, s1, R20, R21, tz, iR, hT, q, b);  // sub + 8 and sub + 24
+      segment_partials<T, true, AHEAD>(xy, ab, area, f + 8, s1, R20, R21, tz, iR, hT, q, b);  // sub + 8 and sub + 24
       tree_pair(q, b);
       tree_pair(p, q);
     }
@@ -392,7 +421,7 @@ __device__ __forceinline__ PassR node_pass(const DevModel& M, const Pose& F, int
 // ----------------------------------------------------------------------------- per-warp view of the slot in shared memory
 
 struct Slot {
-  double *vol, *level, *cx, *cy, *cz, *area, *zmax, *hEff, *aEff, *acc, *dV, *tmp, *hydro;
+  double *vol, *level, *cx, *cy, *cz, *area, *zmax, *hEff, *aEff, *tmp, *term5, *acc, *dV, *hydro;
   int* deg;
   int* misc;
   PassR* passes;
@@ -402,7 +431,6 @@ struct Slot {
   std::uint16_t* flow;        // the connections that can flow in this step (sort_connections)
   Pose* pose;                 // the current step's pose, and
   Pose* prev;                 // the last step's (that of the last level solve, between steps)
-  Buoy* buoy;
   Parked* parked;
   const unsigned char* cols;  // the column table staged in the block's shared memory, or null (read from global)
 };
@@ -422,6 +450,7 @@ __device__ __forceinline__ Slot carve_slot(unsigned char* base, const SlotLayout
   s.dV = reinterpret_cast<double*>(base + L.dV);
   s.flow = reinterpret_cast<std::uint16_t*>(base + L.flow);
   s.tmp = reinterpret_cast<double*>(base + L.tmp);
+  s.term5 = reinterpret_cast<double*>(base + L.term5);
   s.deg = reinterpret_cast<int*>(base + L.deg);
   s.hydro = reinterpret_cast<double*>(base + L.hydro);
   s.misc = reinterpret_cast<int*>(base + L.misc);
@@ -431,7 +460,6 @@ __device__ __forceinline__ Slot carve_slot(unsigned char* base, const SlotLayout
   s.list = reinterpret_cast<std::uint16_t*>(base + L.list);
   s.pose = reinterpret_cast<Pose*>(base + L.pose);
   s.prev = s.pose + 1;
-  s.buoy = reinterpret_cast<Buoy*>(base + L.buoy);
   s.parked = reinterpret_cast<Parked*>(base + L.parked);
   s.cols = nullptr;
   return s;
@@ -480,6 +508,7 @@ struct NoTape {
 template <bool LAZY>
 __device__ __forceinline__ void list_groups(const DevModel& M, Slot& S, int lane) {
   int count = 0;
+#pragma unroll 1
   for (int g0 = 0; g0 < M.ng; g0 += kLanes) {
     const int g = g0 + lane;
     bool live = false;
@@ -488,6 +517,7 @@ __device__ __forceinline__ void list_groups(const DevModel& M, Slot& S, int lane
       const int* m = M.gNodes + __ldg(M.gStart + g);
       double V = 0;
       live = !LAZY;
+#pragma unroll 1
       for (int k = 0; k < N; ++k) {
         const double v = S.vol[__ldg(m + k)];
         V += v;
@@ -497,6 +527,7 @@ __device__ __forceinline__ void list_groups(const DevModel& M, Slot& S, int lane
       if (!live) {
         const bool merged = N >= 2 && __ldg(M.gMode + g) == 1;
         S.merged[g] = merged ? 1 : 0;
+#pragma unroll 1
         for (int k = 0; k < N; ++k) S.dry[__ldg(m + k)] |= kEmptyNode | (merged ? kZeroVolume : 0);
       }
     }
@@ -508,14 +539,14 @@ __device__ __forceinline__ void list_groups(const DevModel& M, Slot& S, int lane
 }
 
 // A group's combined value of node_extreme over its lanes.
-template <bool MIXED, bool MAX>
-__device__ __forceinline__ double group_extreme(const DevModel& M, const Pose& F, int n, const LevelLanes& L) {
+template <bool MIXED>
+__device__ __forceinline__ double group_extreme(const DevModel& M, const Pose& F, int n, bool top, const LevelLanes& L) {
   constexpr int LANES = kLevelLanes<MIXED>;
-  auto v = node_extreme<MIXED, MAX>(M, F, n, L.sub, LANES);
+  auto v = node_extreme<MIXED>(M, F, n, top, L.sub, LANES);
 #pragma unroll
   for (int off = LANES / 2; off > 0; off >>= 1) {
     const auto o = __shfl_xor_sync(L.mask, v, off);
-    if (MAX ? o > v : o < v) v = o;
+    if (top ? o > v : o < v) v = o;
   }
   return static_cast<double>(v);
 }
@@ -523,12 +554,12 @@ __device__ __forceinline__ double group_extreme(const DevModel& M, const Pose& F
 // Node n's level as the last solve left it (an empty node's is formed here); one thread, or a lane group.
 template <bool MIXED>
 __device__ __forceinline__ double stale_level(const DevModel& M, const Slot& S, int n) {
-  return (S.dry[n] & kStale) ? static_cast<double>(node_extreme<MIXED, false>(M, *S.prev, n, 0, 1)) : S.level[n];
+  return (S.dry[n] & kStale) ? static_cast<double>(node_extreme<MIXED>(M, *S.prev, n, false, 0, 1)) : S.level[n];
 }
 
 template <bool MIXED>
 __device__ __forceinline__ double group_level(const DevModel& M, const Slot& S, int n, const LevelLanes& L) {
-  return (S.dry[n] & kStale) ? group_extreme<MIXED, false>(M, *S.prev, n, L) : S.level[n];
+  return (S.dry[n] & kStale) ? group_extreme<MIXED>(M, *S.prev, n, false, L) : S.level[n];
 }
 
 // The solved values of a node whose last pass was p: the pass's sums go to scratch arrays that are dead until the heads,
@@ -547,8 +578,10 @@ __device__ __forceinline__ void set_centroid(Slot& S, int n) {
 // the members' last passes, V their water. One lane.
 __device__ __forceinline__ void share_group(const DevModel& M, Slot& S, const PassR* P, const int* m, int N, double V, double h) {
   double tot = 0;
+#pragma unroll 1
   for (int k = 0; k < N; ++k) tot += P[k].vol;
   double assigned = 0;
+#pragma unroll 1
   for (int k = 0; k < N - 1; ++k) {
     const int n = __ldg(m + k);
     double v = tot > 0 ? V * P[k].vol / tot : V / static_cast<double>(N);
@@ -562,8 +595,10 @@ __device__ __forceinline__ void share_group(const DevModel& M, Slot& S, const Pa
     // the last member would overflow: the ones before it hold V - vmaxLast, filled from the end (levels.hpp:136-155)
     const double need = V - vmaxLast;
     double capped = 0;
+#pragma unroll 1
     for (int k = N - 2; k >= 0; --k) {
       double prior = 0;
+#pragma unroll 1
       for (int j = 0; j < k; ++j) prior += S.vol[__ldg(m + j)];
       const int n = __ldg(m + k);
       const double v = (need - capped) - prior;
@@ -577,9 +612,11 @@ __device__ __forceinline__ void share_group(const DevModel& M, Slot& S, const Pa
       break;
     }
     assigned = 0;
+#pragma unroll 1
     for (int k = 0; k < N - 1; ++k) assigned += S.vol[__ldg(m + k)];
   }
   S.vol[__ldg(m + N - 1)] = V - assigned;
+#pragma unroll 1
   for (int k = 0; k < N; ++k) store_solved(S, __ldg(m + k), h, P[k].dv, P[k]);
 }
 
@@ -590,12 +627,8 @@ __device__ __forceinline__ void share_group(const DevModel& M, Slot& S, const Pa
 template <bool MIXED, int W, class Tape>
 __device__ __forceinline__ void solve_levels(const DevModel& M, const Pose& F, Slot& S, const Team<W>& T, const Tape& tape) {
   constexpr int LANES = kLevelLanes<MIXED>, PER_WARP = 32 / LANES;
-  LevelLanes L;
-  L.lane = T.lane;
-  L.sub = T.lane % LANES;
+  const LevelLanes L = level_lanes<MIXED>(T.lane);
   const int grp = T.lane / LANES;
-  if constexpr (LANES == 32) L.mask = kFull;
-  else L.mask = ((1u << LANES) - 1u) << (grp * LANES);
   const int unit = T.warp * PER_WARP + grp;
   PassR* const P = S.passes + static_cast<std::size_t>(unit) * M.maxGroup;
   const int listed = S.misc[kMiscListed];
@@ -609,6 +642,7 @@ __device__ __forceinline__ void solve_levels(const DevModel& M, const Pose& F, S
   bool have = false, full = false;
   double V = 0, tol = 0, h = 0, a = 0, b = 0, sum = 0, dvs = 0;
   for (;;) {
+#pragma unroll 1
     while (!have && (j < units || i < listed)) {
       if (j >= units) {
         const int g = S.list[i];
@@ -625,6 +659,7 @@ __device__ __forceinline__ void solve_levels(const DevModel& M, const Pose& F, S
           } else if (mode == 2) {
             const double zMw = world_z(F, __ldg(M.gpx + g), __ldg(M.gpy + g), __ldg(M.gpz + g));
             merged = true;
+#pragma unroll 1
             for (int q = 0; q < N; ++q) {
               const int n = __ldg(m + q);
               if (!(S.vol[n] > kEmptyVolume && group_level<MIXED>(M, S, n, L) > zMw + M.gMargin)) { merged = false; break; }
@@ -641,36 +676,41 @@ __device__ __forceinline__ void solve_levels(const DevModel& M, const Pose& F, S
       ++j;
       double Vmax = 0;
       V = 0;
+#pragma unroll 1
       for (int q = 0; q < nm; ++q) { const int n = __ldg(mm + q); V += S.vol[n]; Vmax += __ldg(M.vmax + n); }
       const bool empty = V <= kEmptyVolume;
       if constexpr (Tape::kLazy) {
         if (empty) {
           if (L.sub == 0)
+#pragma unroll 1
             for (int q = 0; q < nm; ++q) S.dry[__ldg(mm + q)] = (S.dry[__ldg(mm + q)] & kStale) | kEmptyNode | (merged ? kZeroVolume : 0);
           continue;
         }
       }
-      if (!merged) {
-        h = group_level<MIXED>(M, S, __ldg(mm), L);
-      } else {
-        bool allWet = true;
-        int firstWet = -1;
-        for (int q = 0; q < nm; ++q) {
-          if (S.vol[__ldg(mm + q)] > 0) { if (firstWet < 0) firstWet = q; }
-          else allWet = false;
-        }
-        if (allWet) {
-          double s = 0;
-          for (int q = 0; q < nm; ++q) s += group_level<MIXED>(M, S, __ldg(mm + q), L);
-          h = s / static_cast<double>(nm);
-        } else {
-          h = group_level<MIXED>(M, S, __ldg(mm + (firstWet >= 0 ? firstWet : nm - 1)), L);
-        }
+      // the starting level: the node's, the mean of a wet group's, or that of the group's first wet member (its last one
+      // when none is)
+      bool allWet = true;
+      int firstWet = -1;
+#pragma unroll 1
+      for (int q = 0; merged && q < nm; ++q) {
+        if (S.vol[__ldg(mm + q)] > 0) { if (firstWet < 0) firstWet = q; }
+        else allWet = false;
       }
+      const int q0 = allWet ? 0 : (firstWet >= 0 ? firstWet : nm - 1), q1 = allWet ? nm : q0 + 1;
+      h = 0;
+#pragma unroll 1
+      for (int q = q0; q < q1; ++q) h += group_level<MIXED>(M, S, __ldg(mm + q), L);
+      if (merged && allWet) h = h / static_cast<double>(nm);
       double lo = 0, hi = 0;
+#pragma unroll 1
       for (int q = 0; q < nm; ++q) {
         const int n = __ldg(mm + q);
-        const double zlo = group_extreme<MIXED, false>(M, F, n, L), zhi = group_extreme<MIXED, true>(M, F, n, L);
+        double zlo = 0, zhi = 0;
+#pragma unroll 1
+        for (int top = 0; top < 2; ++top) {
+          const double z = group_extreme<MIXED>(M, F, n, top != 0, L);
+          if (top) zhi = z; else zlo = z;
+        }
         tape.start(n, h, zlo, zhi, L);
         if (q == 0 || zlo < lo) lo = zlo;
         if (q == 0 || zhi > hi) hi = zhi;
@@ -691,10 +731,12 @@ __device__ __forceinline__ void solve_levels(const DevModel& M, const Pose& F, S
         } else {
           const double over = jmax(0.0, V - Vmax);
           double aSum = 0;
+#pragma unroll 1
           for (int q = 0; q < nm; ++q) aSum += __ldg(M.aov + __ldg(mm + q));
           dh = over / aSum;
           if (L.sub == 0) {
             double assigned = 0;
+#pragma unroll 1
             for (int q = 0; q < nm - 1; ++q) {
               const int n = __ldg(mm + q);
               const double v = __ldg(M.vmax + n) + dh * __ldg(M.aov + n);
@@ -719,7 +761,7 @@ __device__ __forceinline__ void solve_levels(const DevModel& M, const Pose& F, S
     }
     if (!__any_sync(kFull, have)) break;
     const int n = have ? __ldg(mm + k) : -1;
-    const PassR p = node_pass<MIXED>(M, F, n, h, L);
+    const PassR p = node_pass<MIXED, W>(M, F, n, h, L);
     if (!have) continue;
     tape.pass(n, slot, h, p, L);
     if (full) {
@@ -814,7 +856,7 @@ __device__ __forceinline__ double law_volume(const DevModel& M, const FlowHeads&
       double v = 1;
       if (H2 > 0) {
         const double r = H2 / H1;
-        v = pm::pow(jmax(0.0, 1 - pm::pow(r, kWeirExponent)), kVillemonteExponent);
+        v = pow_of(jmax(0.0, 1 - pow_of(r, kWeirExponent)), kVillemonteExponent);
       }
       q = __ldg(M.coef + c) * __ldg(area + c) * kWeirCoefficient * M.sq2g * H1 * pm::sqrt_rn(H1) * v * (Ha >= Hb ? 1.0 : -1.0);
     }
@@ -892,19 +934,20 @@ struct SimRegs {
   double inflow, Vb, hullTop, mw, bx, by, bz;
   int foundered;
   double founderT;
-  int evCount;  // warp 0's count is the log's; the other warps' lag
+  int evCount;  // the event warp's count is the log's; the other warps' lag
 };
 
-// Every thread stores the same values (evCount, which differs between warps, stays in registers).
+// The run's values live in the slot (Parked) through a step, so that their registers serve its phases; the step's first
+// warp moves them on, and every thread takes them at its end. The settle timer and the event count stay in registers.
 __device__ __forceinline__ void park(Parked* P, const SimRegs& R) {
   P->t = R.t; P->zO = R.zO; P->pitch = R.pitch; P->roll = R.roll; P->vz = R.vz; P->wth = R.wth; P->wph = R.wph;
-  P->calm = R.calm; P->inflow = R.inflow; P->Vb = R.Vb; P->hullTop = R.hullTop; P->mw = R.mw; P->bx = R.bx;
+  P->inflow = R.inflow; P->Vb = R.Vb; P->hullTop = R.hullTop; P->mw = R.mw; P->bx = R.bx;
   P->by = R.by; P->bz = R.bz; P->founderT = R.founderT; P->foundered = R.foundered;
 }
 
 __device__ __forceinline__ void unpark(const Parked* P, SimRegs& R) {
   R.t = P->t; R.zO = P->zO; R.pitch = P->pitch; R.roll = P->roll; R.vz = P->vz; R.wth = P->wth; R.wph = P->wph;
-  R.calm = P->calm; R.inflow = P->inflow; R.Vb = P->Vb; R.hullTop = P->hullTop; R.mw = P->mw; R.bx = P->bx;
+  R.inflow = P->inflow; R.Vb = P->Vb; R.hullTop = P->hullTop; R.mw = P->mw; R.bx = P->bx;
   R.by = P->by; R.bz = P->bz; R.founderT = P->founderT; R.foundered = P->foundered;
 }
 
@@ -962,41 +1005,158 @@ struct InstPtrs<true> {
   __device__ __forceinline__ double* markT() const { return markT_; }
 };
 
-// The event log belongs to warp 0 of the team: only its lane 0 writes, only its count is stored.
+// The event log belongs to one warp of the team (not the first where there are two: that one integrates the motion
+// meanwhile); its lane 0 writes, only its count is stored.
+template <int W>
+constexpr int kEventWarp = W > 1 ? 1 : 0;
+
 template <class IP>
-__device__ __forceinline__ void push_event(const DevModel& M, SimRegs& R, const IP& I, int id, int kind, int lane) {
-  if (R.evCount < M.evCap) {
-    if (lane == 0) { I.evT()[R.evCount] = R.t; I.evId()[R.evCount] = id; I.evKind()[R.evCount] = kind; }
-    R.evCount++;
+__device__ __forceinline__ void push_event(const DevModel& M, double t, int& evCount, const IP& I, int id, int kind, int lane) {
+  if (evCount < M.evCap) {
+    if (lane == 0) { I.evT()[evCount] = t; I.evId()[evCount] = id; I.evKind()[evCount] = kind; }
+    evCount++;
   }
+}
+
+// The overflow and mark events of a step that ends at time t (events.hpp:11-38): monitors in order, then marks in order,
+// at the step's pose and flows. One warp.
+template <class IP>
+__device__ __forceinline__ void step_events(const DevModel& M, const Pose& F, double t, int& evCount, const Slot& S, const IP& I, int lane) {
+#pragma unroll 1
+  for (int m0 = 0; m0 < M.nmon; m0 += kLanes) {
+    const int m = m0 + lane;
+    bool fire = false;
+    if (m < M.nmon && I.overT()[m] < 0) {
+      const int k0 = __ldg(M.monStart + m), k1 = k0 + __ldg(M.monCount + m);
+      double over = 0;
+#pragma unroll 1
+      for (int k = k0; k < k1; ++k) {
+        const double d = S.dV[__ldg(M.monConn + k)];
+        if (d > 0) over += d / M.dt;
+      }
+      fire = over > M.monThreshold;
+      if (fire) I.overT()[m] = t;
+    }
+    unsigned mask = __ballot_sync(kFull, fire);
+    while (mask) {
+      const int b = __ffs(mask) - 1;
+      mask &= mask - 1;
+      push_event(M, t, evCount, I, m0 + b, 0, lane);
+    }
+  }
+#pragma unroll 1
+  for (int i0 = 0; i0 < M.nmark; i0 += kLanes) {
+    const int i = i0 + lane;
+    bool fire = false;
+    if (i < M.nmark && I.markT()[i] < 0) {
+      const double wz = world_z(F, __ldg(M.mkx + i), __ldg(M.mky + i), __ldg(M.mkz + i));
+      const bool under = __ldg(M.mkWhen + i) == 0;
+      fire = (under && wz < 0) || (!under && wz > 0);
+      if (fire) I.markT()[i] = t;
+    }
+    unsigned mask = __ballot_sync(kFull, fire);
+    while (mask) {
+      const int b = __ffs(mask) - 1;
+      mask &= mask - 1;
+      push_event(M, t, evCount, I, i0 + b, 1, lane);
+    }
+  }
+}
+
+// The sum of the nonzero values of v over the lanes, in lane order, added to (or, with SUB, taken from) acc; zeros leave
+// a sum as it is.
+template <bool SUB>
+__device__ __forceinline__ double add_in_order(double acc, double v) {
+  unsigned mask = __ballot_sync(kFull, v != 0);
+  while (mask) {
+    const int b = __ffs(mask) - 1;
+    mask &= mask - 1;
+    const double x = __shfl_sync(kFull, v, b);
+    acc = SUB ? acc - x : acc + x;
+  }
+  return acc;
 }
 
 // ----------------------------------------------------------------------------- the step (kernel/step.hpp:41-54)
 // Phases that exchange per-node or per-connection arrays are separated by team barriers; per-node and
-// per-connection work is spread over all 32 W threads of the team; scalars are computed redundantly and identically
-// by every thread, so every decision is uniform across the team.
+// per-connection work is spread over all 32 W threads of the team; the sums over nodes in their serial order, the
+// motion and the next pose are one warp's, while another lists the next solve's groups and a third the events.
 
+// The sums, the motion and the next pose (flows.hpp:114-118, body.hpp:11-57, events.hpp:30-38), by one warp: the load
+// terms of the nodes are in columns a fixed stride apart from S.area (dry nodes hold -0, which leaves every sum as it is),
+// the excess in S.acc. Lanes 0 .. 5 each add one column in node order: a lane reading all six, node by node, took a
+// dependent load and six adds a node.
+__device__ __forceinline__ void move_body(const DevModel& M, const Pose& F, Slot& S, int lane) {
+  double seaIn = 0;
+#pragma unroll 1
+  for (int k0 = 0; k0 < M.nsea; k0 += kLanes) {
+    const int k = k0 + lane;
+    seaIn = add_in_order<false>(seaIn, k < M.nsea ? S.dV[__ldg(M.sea + k)] : 0.0);
+  }
+  // the excess returns to the sea in node order
+#pragma unroll 1
+  for (int n0 = 0; n0 < M.nn; n0 += kLanes) {
+    const int n = n0 + lane;
+    seaIn = add_in_order<true>(seaIn, n < M.nn && S.acc[n] > 0 ? S.acc[n] : 0.0);
+  }
+  Parked& P = *S.parked;
+  const Buoy hb = buoyancy_finish(S.hydro);
+  const double Wg = M.rho * M.g;
+  const double Fb = Wg * hb.V;
+  const double bxw = F.R00 * hb.x + F.R01 * hb.y + F.R02 * hb.z + F.tx;
+  const double byw = F.R10 * hb.x + F.R11 * hb.y + F.R12 * hb.z + F.ty;
+  double sum = 0;
+  if (lane == 0) sum = (byw - M.YO) * Fb;
+  if (lane == 1) sum = -(bxw - M.XO) * Fb;
+  if (lane == 2) sum = Fb - M.g * M.ms;
+  {
+    const double* t = S.area + (lane < 6 ? lane : 5) * (S.zmax - S.area);
+    const int NN = M.nn;
+#pragma unroll 8
+    for (int n = 0; n < NN; ++n) sum += t[n];
+  }
+  const double tauX = __shfl_sync(kFull, sum, 0), tauY = __shfl_sync(kFull, sum, 1), Fz = __shfl_sync(kFull, sum, 2);
+  const double mw = __shfl_sync(kFull, sum, 3), Iw_p = __shfl_sync(kFull, sum, 4), Iw_r = __shfl_sync(kFull, sum, 5);
+  const double Mth = tauY, Mph = tauX * F.cth;
+  const double dt = M.dt;
+  double vz = P.vz, wth = P.wth, wph = P.wph, zO = P.zO, pitch = P.pitch, roll = P.roll;
+  const double mh = M.mh0 + mw;
+  const double Ith = M.Ith0 + Iw_p, Iph = M.Iph0 + Iw_r;
+  const double az = (Fz - M.cDz * vz - M.qz * fabs(vz) * vz) / mh;
+  const double ath = (Mth - M.cDth * wth - M.qth * fabs(wth) * wth) / Ith;
+  const double aph = (Mph - M.cDph * wph - M.qph * fabs(wph) * wph) / Iph;
+  vz += az * dt; wth += ath * dt; wph += aph * dt;
+  zO += vz * dt; pitch += wth * dt; roll += wph * dt;
+  if (pitch > kPitchClamp) { pitch = kPitchClamp; wth = 0; }
+  if (pitch < -kPitchClamp) { pitch = -kPitchClamp; wth = 0; }
+  if (roll > kRollClamp) { roll = kRollClamp; wph = 0; }
+  if (roll < -kRollClamp) { roll = -kRollClamp; wph = 0; }
+  const double t = P.t + dt;
+  __syncwarp();  // the lanes have read the values they now replace
+  P.t = t; P.zO = zO; P.pitch = pitch; P.roll = roll; P.vz = vz; P.wth = wth; P.wph = wph;
+  P.inflow = seaIn / dt; P.Vb = hb.V; P.hullTop = hb.top; P.mw = mw;
+  P.bx = hb.x; P.by = hb.y; P.bz = hb.z;
+  if (!P.foundered && (hb.top < M.hullTopBelow || fabs(pitch) > M.pitchAbsAbove || (hb.V < M.buoyancyBelow && t > M.minT))) {
+    P.foundered = 1;
+    P.founderT = t;
+  }
+  *S.prev = make_pose(M, zO, pitch, roll);
+}
+
+// One step. On entry S.parked holds R's values and S.pose their pose; on return R, S.parked and S.pose are the next ones
+// (S.prev the step's).
 template <bool MIXED, int W, class IP, class Tape = NoTape>
-__device__ __forceinline__ void team_step(const DevModel& M, const Pose& F, SimRegs& R, Slot& S, const IP& I, const Team<W>& T,
-                                          const Tape& tape = Tape{}) {
+__device__ __forceinline__ void team_step(const DevModel& M, SimRegs& R, Slot& S, const IP& I, const Team<W>& T, const Tape& tape = Tape{}) {
   constexpr int kStride = 32 * W;
   const int lane = T.lane, rank = T.rank;
-  const double tNow = R.t;
-  park(S.parked, R);  // until the volume update; no thread reads it before the barrier that ends that phase
-  if constexpr (W > 8) {
-    // The buoyancy's eight trees and the level solve need nothing from each other: the warps without a tree go on to
-    // take node groups, and one barrier ends both (16-warp teams: the tail phase 517 against 534 ms on the bench
-    // batch, the adjoint's forward 125 against 132 team-s per call; in teams of at most 8 warps, where every warp has
-    // trees, the same order made the main phase slower, 2.75 against 2.60 s)
-    buoyancy_trees<MIXED, W>(M, F, T, S.hydro, S.cols);
-    solve_levels<MIXED, W>(M, F, S, T, tape);
-    T.sync();
-    *S.buoy = buoyancy_finish(S.hydro);  // every thread stores the same values
-  } else {
-    *S.buoy = buoyancy<MIXED, W>(M, F, T, S.hydro, S.cols);  // every thread stores the same values
-    solve_levels<MIXED, W>(M, F, S, T, tape);
-    T.sync();
-  }
+  const Pose& F = *S.pose;
+  buoyancy_trees<MIXED, W>(M, F, T.warp, lane, S.hydro, S.cols);
+  // The buoyancy's eight trees and the level solve need nothing from each other: in 16-warp teams the warps without a
+  // tree go on to take list entries, and one barrier ends both. In smaller teams every warp has trees, and a barrier
+  // between keeps the warps in the same tables.
+  if constexpr (W <= 8) T.sync();
+  solve_levels<MIXED, W>(M, F, S, T, tape);
+  T.sync();
   // the list counter for the next step's level solve (read after this step's later barriers)
   if (T.leader()) {
     S.misc[kMiscTaken] = W * (32 / kLevelLanes<MIXED>);
@@ -1006,6 +1166,7 @@ __device__ __forceinline__ void team_step(const DevModel& M, const Pose& F, SimR
 
   // the solve's ends node by node (an empty node's area, a wet one's centroid), effective heads and areas, then degrees
   // (flows.hpp:15-35)
+#pragma unroll 1
   for (int n = rank; n < M.nn; n += kStride) {
     const int flags = S.dry[n];
     S.dry[n] = (Tape::kLazy && (flags & kEmptyNode)) ? kStale : 0;
@@ -1022,6 +1183,7 @@ __device__ __forceinline__ void team_step(const DevModel& M, const Pose& F, SimR
   }
   tape.solved(M, S, T);  // a thread reads the nodes it has just finished
   T.sync();
+  const double tNow = S.parked->t;
   if constexpr (W <= 4) {
     sort_connections(M, F, tNow, S, I, T);
     T.sync();
@@ -1038,158 +1200,71 @@ __device__ __forceinline__ void team_step(const DevModel& M, const Pose& F, SimR
     }
   }
   T.sync();
-  // per-node gathers in increasing connection order, then the volume update (flows.hpp:81-111)
-  for (int n = rank; n < M.nn; n += kStride) {
-    const int k0 = __ldg(M.incStart + n), k1 = k0 + __ldg(M.incCount + n);
-    double acc = 0;
-    for (int k = k0; k < k1; ++k) {
-      const double d = S.dV[__ldg(M.incConn + k)];
-      acc = __ldg(M.incSide + k) ? acc + d : acc - d;
+  // per-node gathers in increasing connection order, the volume update (flows.hpp:81-111) and, by the same thread, the
+  // node's terms of the loads (body.hpp:20-33), which overwrite arrays of which only this node's entries are still read
+  {
+    const double Wg = M.rho * M.g;
+    const double zO = S.parked->zO;
+#pragma unroll 1
+    for (int n = rank; n < M.nn; n += kStride) {
+      const int k0 = __ldg(M.incStart + n), k1 = k0 + __ldg(M.incCount + n);
+      double acc = 0;
+#pragma unroll 4
+      for (int k = k0; k < k1; ++k) {
+        const int e = __ldg(M.incEdge + k);
+        const double d = S.dV[e >> 1];
+        acc = (e & 1) ? acc + d : acc - d;
+      }
+      double v = S.vol[n] + acc;
+      if (v < 0) v = 0;
+      const double vm = __ldg(M.vmax + n);
+      double excess = 0;
+      if (v > vm) {
+        // (a node that was empty at the solve has no extent yet)
+        const double zmax = (S.dry[n] & kStale) ? static_cast<double>(node_extreme<MIXED>(M, F, n, true, 0, 1)) : S.zmax[n];
+        const double head = jmax(0.0, -zmax);
+        const double cap = vm + __ldg(M.aov + n) * head;
+        if (v > cap) { excess = v - cap; v = cap; }
+      }
+      S.acc[n] = excess;
+      S.vol[n] = v;
+      double t0 = -0.0, t1 = -0.0, t2 = -0.0, t3 = -0.0, t4 = -0.0, t5 = -0.0;
+      if (!(v <= 0)) {
+        const double x = S.cx[n], y = S.cy[n], z = S.cz[n];
+        const double wx = F.R00 * x + F.R01 * y + F.R02 * z + F.tx - M.XO;
+        const double wy = F.R10 * x + F.R11 * y + F.R12 * z + F.ty - M.YO;
+        const double wz = F.R20 * x + F.R21 * y + F.R22 * z + F.tz - zO;
+        const double f = -Wg * v;
+        const double m = M.rho * v;
+        t0 = wy * f;
+        t1 = -(wx * f);
+        t2 = f;
+        t3 = m;
+        t4 = m * (wx * wx + wz * wz);
+        t5 = m * (wy * wy + wz * wz);
+      }
+      S.area[n] = t0; S.zmax[n] = t1; S.hEff[n] = t2; S.aEff[n] = t3; S.tmp[n] = t4; S.term5[n] = t5;
     }
-    double v = S.vol[n] + acc;
-    if (v < 0) v = 0;
-    const double vm = __ldg(M.vmax + n);
-    double excess = 0;
-    if (v > vm) {
-      // (a node that was empty at the solve has no extent yet)
-      const double zmax = (S.dry[n] & kStale) ? static_cast<double>(node_extreme<MIXED, true>(M, F, n, 0, 1)) : S.zmax[n];
-      const double head = jmax(0.0, -zmax);
-      const double cap = vm + __ldg(M.aov + n) * head;
-      if (v > cap) { excess = v - cap; v = cap; }
-    }
-    S.acc[n] = excess;
-    S.vol[n] = v;
   }
-  double seaIn = 0;
-  for (int k = 0; k < M.nsea; ++k) seaIn += S.dV[__ldg(M.sea + k)];
   T.sync();
-  unpark(S.parked, R);
+  if (T.warp == 0) move_body(M, F, S, lane);
   if constexpr (Tape::kLazy) {
     if (T.warp == W - 1) list_groups<true>(M, S, lane);
   }
-  // the excess returns to the sea in node order (flows.hpp:114-118)
-  for (int n0 = 0; n0 < M.nn; n0 += kLanes) {
-    const int n = n0 + lane;
-    unsigned mask = __ballot_sync(kFull, n < M.nn && S.acc[n] > 0);
-    while (mask) {
-      const int b = __ffs(mask) - 1;
-      mask &= mask - 1;
-      seaIn -= S.acc[n0 + b];
-    }
-  }
-  R.inflow = seaIn / M.dt;
-  // the loads' per-node terms overwrite area, zmax, hEff, aEff, acc and dV, all read for the last time above
+  if (T.warp == kEventWarp<W>) step_events(M, F, tNow + M.dt, R.evCount, S, I, lane);
   T.sync();
-
-  // loads (body.hpp:11-40): per-node terms in parallel, sums in node order
-  double* const t0 = S.area;
-  double* const t1 = S.zmax;
-  double* const t2 = S.hEff;
-  double* const t3 = S.aEff;
-  double* const t4 = S.acc;
-  double* const t5 = S.tmp;
-  const Buoy hb = *S.buoy;
-  const double Wg = M.rho * M.g;
-  const double Fb = Wg * hb.V;
-  const double bxw = F.R00 * hb.x + F.R01 * hb.y + F.R02 * hb.z + F.tx;
-  const double byw = F.R10 * hb.x + F.R11 * hb.y + F.R12 * hb.z + F.ty;
-  double tauX = (byw - M.YO) * Fb, tauY = -(bxw - M.XO) * Fb;
-  double Fz = Fb - M.g * M.ms;
-  double mw = 0, Iw_p = 0, Iw_r = 0;
-  const int NN = M.nn;
-  for (int n = rank; n < NN; n += kStride) {
-    const double V = S.vol[n];
-    if (V <= 0) continue;
-    const double x = S.cx[n], y = S.cy[n], z = S.cz[n];
-    const double wx = F.R00 * x + F.R01 * y + F.R02 * z + F.tx - M.XO;
-    const double wy = F.R10 * x + F.R11 * y + F.R12 * z + F.ty - M.YO;
-    const double wz = F.R20 * x + F.R21 * y + F.R22 * z + F.tz - R.zO;
-    const double f = -Wg * V;
-    const double m = M.rho * V;
-    t0[n] = wy * f;
-    t1[n] = wx * f;
-    t2[n] = f;
-    t3[n] = m;
-    t4[n] = m * (wx * wx + wz * wz);
-    t5[n] = m * (wy * wy + wz * wz);
-  }
-  T.sync();
-  for (int n = 0; n < NN; ++n) {
-    if (S.vol[n] <= 0) continue;
-    tauX += t0[n]; tauY -= t1[n]; Fz += t2[n];
-    mw += t3[n];
-    Iw_p += t4[n];
-    Iw_r += t5[n];
-  }
-  const double Mth = tauY, Mph = tauX * F.cth;
-  // integrate (body.hpp:42-57)
-  const double dt = M.dt;
-  const double mh = M.mh0 + mw;
-  const double Ith = M.Ith0 + Iw_p, Iph = M.Iph0 + Iw_r;
-  const double az = (Fz - M.cDz * R.vz - M.qz * fabs(R.vz) * R.vz) / mh;
-  const double ath = (Mth - M.cDth * R.wth - M.qth * fabs(R.wth) * R.wth) / Ith;
-  const double aph = (Mph - M.cDph * R.wph - M.qph * fabs(R.wph) * R.wph) / Iph;
-  R.vz += az * dt; R.wth += ath * dt; R.wph += aph * dt;
-  R.zO += R.vz * dt; R.pitch += R.wth * dt; R.roll += R.wph * dt;
-  if (R.pitch > kPitchClamp) { R.pitch = kPitchClamp; R.wth = 0; }
-  if (R.pitch < -kPitchClamp) { R.pitch = -kPitchClamp; R.wth = 0; }
-  if (R.roll > kRollClamp) { R.roll = kRollClamp; R.wph = 0; }
-  if (R.roll < -kRollClamp) { R.roll = -kRollClamp; R.wph = 0; }
-  R.t += dt;
-  R.Vb = hb.V; R.hullTop = hb.top; R.mw = mw;
-  R.bx = hb.x; R.by = hb.y; R.bz = hb.z;
-
-  // events (events.hpp:11-38): monitors in order, marks in order, then the founder rule; warp 0 keeps the log
-  if (T.warp == 0) {
-  for (int m0 = 0; m0 < M.nmon; m0 += kLanes) {
-    const int m = m0 + lane;
-    bool fire = false;
-    if (m < M.nmon && I.overT()[m] < 0) {
-      const int k0 = __ldg(M.monStart + m), k1 = k0 + __ldg(M.monCount + m);
-      double over = 0;
-      for (int k = k0; k < k1; ++k) {
-        const double d = S.dV[__ldg(M.monConn + k)];
-        if (d > 0) over += d / M.dt;
-      }
-      fire = over > M.monThreshold;
-      if (fire) I.overT()[m] = R.t;
-    }
-    unsigned mask = __ballot_sync(kFull, fire);
-    while (mask) {
-      const int b = __ffs(mask) - 1;
-      mask &= mask - 1;
-      push_event(M, R, I, m0 + b, 0, lane);
-    }
-  }
-  for (int i0 = 0; i0 < M.nmark; i0 += kLanes) {
-    const int i = i0 + lane;
-    bool fire = false;
-    if (i < M.nmark && I.markT()[i] < 0) {
-      const double wz = world_z(F, __ldg(M.mkx + i), __ldg(M.mky + i), __ldg(M.mkz + i));
-      const bool under = __ldg(M.mkWhen + i) == 0;
-      fire = (under && wz < 0) || (!under && wz > 0);
-      if (fire) I.markT()[i] = R.t;
-    }
-    unsigned mask = __ballot_sync(kFull, fire);
-    while (mask) {
-      const int b = __ffs(mask) - 1;
-      mask &= mask - 1;
-      push_event(M, R, I, i0 + b, 1, lane);
-    }
-  }
-  }
-  if (!R.foundered && (R.hullTop < M.hullTopBelow || fabs(R.pitch) > M.pitchAbsAbove || (R.Vb < M.buoyancyBelow && R.t > M.minT))) {
-    R.foundered = 1;
-    R.founderT = R.t;
-    if (T.warp == 0) push_event(M, R, I, -1, 2, lane);
-  }
-  T.sync();
+  Pose* const last = S.pose;
+  S.pose = S.prev;
+  S.prev = last;
+  unpark(S.parked, R);
+  if (R.foundered && T.warp == kEventWarp<W>) push_event(M, R.t, R.evCount, I, -1, 2, lane);
 }
 
 // Readouts at the current state (kernel/readouts.hpp:20-36): t, trim, list, water (t), inflow (t/min), draftF, draftA.
 __device__ __forceinline__ void readouts(const DevModel& M, const SimRegs& R, const Slot& S, double* r7) {
   const Pose F = make_pose(M, R.zO, R.pitch, R.roll);
   double water = 0;
+#pragma unroll 1
   for (int n = 0; n < M.nn; ++n) water += S.vol[n];
   r7[0] = R.t;
   r7[1] = R.pitch * 180 / kPi;
