@@ -194,6 +194,7 @@ float AdjointBatch::run() {
   // allows. Unless the caller set a budget: a whole run of records with two passes per node (nodes take about 1.2 on
   // average), within half the device memory free at the first run; the ring is kept for later runs.
   const std::size_t minRing = static_cast<std::size_t>(K) * tapeBytes;
+  const std::size_t usual = (static_cast<std::size_t>(maxSteps) + 1) * adjoint_record_bytes(m.NN, m.NG, 2 * m.NN);
   if (I.ringBytes == 0 || I.ringTeams != teams_) {
     std::size_t perTeam = 0;
     if (I.tapeBudget != 0) {
@@ -201,7 +202,6 @@ float AdjointBatch::run() {
     } else {
       std::size_t freeB = 0, totalB = 0;
       check(cudaMemGetInfo(&freeB, &totalB), "cudaMemGetInfo");
-      const std::size_t usual = (static_cast<std::size_t>(maxSteps) + 1) * adjoint_record_bytes(m.NN, m.NG, 2 * m.NN);
       perTeam = std::min(usual, (freeB + I.arena.bytes()) / 2 / static_cast<std::size_t>(teams_));
     }
     I.ringBytes = std::max(minRing, perTeam) & ~static_cast<std::size_t>(15);
@@ -225,7 +225,10 @@ float AdjointBatch::run() {
   R.K = K; R.maxCkpt = maxCkpt; R.ckpt = I.ckpt.get();
   R.arena = I.arena.get(); R.arenaBytes = I.ringBytes; R.stepOff = I.stepOff.get(); R.recBytes = I.recBytes.get();
   R.stageRecords = stageRecords ? 1 : 0;
-  R.tapeForward = I.ringBytes > minRing ? 1 : 0; R.sink = I.sink.get(); R.isink = I.isink.get();
+  // The forward run records its steps when the ring can keep more than the last segment of them, or a usual whole run (a
+  // short one fits the smallest ring: 320 points on the liner to 150 s took 171 ms stepping everything a second time from
+  // the checkpoints, 123 ms from their records, on B200).
+  R.tapeForward = I.ringBytes > minRing || I.ringBytes >= usual ? 1 : 0; R.sink = I.sink.get(); R.isink = I.isink.get();
   R.phaseNs = I.phase.get();
   R.recomputed = I.recomputed.get();
   check(cudaEventRecord(I.ev0, s), "cudaEventRecord");
