@@ -20,6 +20,13 @@
 
 namespace ssb {
 
+// A group as a step's level solve lists it: its index, its first two members (a group of one: that one twice), their number
+// (255: at least that many) and its merge mode.
+struct alignas(8) Listed {
+  std::uint16_t g, n0, n1;
+  std::uint8_t N, mode;
+};
+
 struct DevModel {
   // columns: (x, y) and (zlo, zhi) pairs, so one 16-byte load fetches two fields, and the footprint dxdy; the float
   // copies are the same values rounded to single precision once on the host (the portable32 column arithmetic
@@ -46,10 +53,12 @@ struct DevModel {
   std::int32_t nn;
   const double *mu, *vmax, *amin, *aov;
   const std::int32_t *segStart, *segCount;
+  const int2* nodeSeg;  // (segStart, segCount)
   // groups
   std::int32_t ng;
   const std::int32_t *gStart, *gCount, *gNodes;
   const std::uint8_t* gMode;
+  const Listed* groupEntry;
   const double *gpx, *gpy, *gpz;
   double gMargin;
   std::int32_t maxGroup;
@@ -210,13 +219,13 @@ constexpr int kMaxLevelGroupsPerWarp = 32 / (kLevelLanes<false> < kLevelLanes<tr
 // Byte offsets of one simulation slot (one team of warps) in dynamic shared memory; `bytes` is the slot stride.
 // passes holds maxGroup node-pass results per level lane group of the team (up to kMaxLevelGroupsPerWarp per warp); hydro the
 // eight buoyancy tree results and the hull's top; misc the team's small broadcast values and counters (MiscSlot); dry a
-// flag byte per node, list the groups the next level solve visits and flow the connections that can flow
+// flag byte per node, wet the numbers of load terms, list the groups the next level solve visits and flow the connections that can flow
 // (warp_step.cuh); pose this step's pose and the last one's, which every phase reads (kept here rather than in each
 // thread's registers); parked the run's values; model (fleets only) the team's copy of its instance's model. area, zmax,
 // hEff, aEff, tmp and term5 become the six columns of the loads' per-node terms (a fixed stride apart); between the level
 // solve and the heads, acc, hEff, aEff and tmp hold the passes' sums.
 struct SlotLayout {
-  std::uint32_t vol, level, cx, cy, cz, area, zmax, hEff, aEff, tmp, term5, acc, deg, dV, flow, passes, hydro, misc, merged, dry, list, pose, parked,
+  std::uint32_t vol, level, cx, cy, cz, area, zmax, hEff, aEff, tmp, term5, acc, deg, dV, flow, passes, hydro, misc, merged, dry, wet, list, pose, parked,
       model, bytes;
 };
 

@@ -47,6 +47,8 @@ void append_undominated(const std::vector<std::int32_t>& from, X x, Y y, Z z, do
     kept.erase(std::remove_if(kept.begin(), kept.end(), [&](const P& k) { return p.x <= k.x && p.y <= k.y && p.z <= k.z; }), kept.end());
     kept.push_back(p);
   }
+  // the lowest (or highest) of them on an even keel first: a look at the first few mostly settles what is asked
+  std::sort(kept.begin(), kept.end(), [](const P& a, const P& b) { return a.z < b.z || (a.z == b.z && a.i < b.i); });
   for (const P& k : kept) out.push_back(k.i);
 }
 

@@ -88,7 +88,8 @@ inline SlotLayout slot_layout(std::int32_t NN, std::int32_t NC, std::int32_t NG,
   L.misc = take(off, 8 * sizeof(std::int32_t));
   L.merged = take(off, static_cast<std::size_t>(std::max(NG, 1)));
   L.dry = take(off, static_cast<std::size_t>(std::max(NN, 1)));
-  L.list = take(off, sizeof(std::uint16_t) * static_cast<std::size_t>(std::max(NG, 1)));
+  L.wet = take(off, static_cast<std::size_t>(NN) / 32 + 1);
+  L.list = take(off, sizeof(Listed) * static_cast<std::size_t>(std::max(NG, 1)));
   L.pose = take(off, 2 * sizeof(Pose));
   L.parked = take(off, sizeof(Parked));
   L.model = fleet ? take(off, sizeof(DevModel)) : 0u;
@@ -110,6 +111,8 @@ struct ModelDev {
   DevBuf<float> colAf, segArf, exZf;
   DevBuf<double> colA, segAr, exZ, mu, vmax, amin, aov;
   DevBuf<std::int32_t> exStart, incEdge, segStart, segCount, gStart, gCount, gNodes, ca, cb, skip, incStart, incCount, incConn, sea, monStart, monCount, monConn;
+  DevBuf<int2> nodeSeg;
+  DevBuf<Listed> groupEntry;
   DevBuf<std::uint8_t> gMode, law, incSide, mkWhen;
   DevBuf<double> gpx, gpy, gpz, kx, ky, kz, coef, mkx, mky, mkz;
   DevModel dm{};
@@ -178,8 +181,20 @@ struct ModelDev {
       check(cudaStreamSynchronize(s), "stream sync");
     }
     mu.upload(S.mu, s); vmax.upload(S.vmax, s); amin.upload(S.amin, s); aov.upload(S.aov, s);
+    std::vector<int2> ns(static_cast<std::size_t>(NN));
+    for (std::size_t n = 0; n < ns.size(); ++n) ns[n] = int2{S.segStart[n], S.segCount[n]};
+    nodeSeg.upload(ns, s);
     segStart.upload(S.segStart, s); segCount.upload(S.segCount, s);
     gStart.upload(M.gNodeStart, s); gCount.upload(M.gNodeCount, s); gNodes.upload(M.gNodes, s); gMode.upload(M.gMode, s);
+    std::vector<Listed> entry(static_cast<std::size_t>(NG));
+    for (std::size_t g = 0; g < entry.size(); ++g) {
+      const std::int32_t* m = M.gNodes.data() + M.gNodeStart[g];
+      const std::int32_t N = M.gNodeCount[g];
+      const std::int32_t first = N > 0 ? m[0] : 0;
+      entry[g] = Listed{static_cast<std::uint16_t>(g), static_cast<std::uint16_t>(first), static_cast<std::uint16_t>(N > 1 ? m[1] : first),
+                        static_cast<std::uint8_t>(std::min(N, 255)), M.gMode[g]};
+    }
+    groupEntry.upload(entry, s);
     gpx.upload(M.gpx, s); gpy.upload(M.gpy, s); gpz.upload(M.gpz, s);
     ca.upload(M.ca, s); cb.upload(M.cb, s); skip.upload(M.cSkipGroup, s); law.upload(M.cLaw, s);
     kx.upload(M.cx, s); ky.upload(M.cy, s); kz.upload(M.cz, s); coef.upload(M.cCoef, s);
@@ -207,9 +222,9 @@ struct ModelDev {
     d.exStart = exStart.get(); d.exXY = exXY.get(); d.exZ = exZ.get(); d.exXYf = exXYf.get(); d.exZf = exZf.get();
     d.nn = NN;
     d.mu = mu.get(); d.vmax = vmax.get(); d.amin = amin.get(); d.aov = aov.get();
-    d.segStart = segStart.get(); d.segCount = segCount.get();
+    d.segStart = segStart.get(); d.segCount = segCount.get(); d.nodeSeg = nodeSeg.get();
     d.ng = NG;
-    d.gStart = gStart.get(); d.gCount = gCount.get(); d.gNodes = gNodes.get(); d.gMode = gMode.get();
+    d.gStart = gStart.get(); d.gCount = gCount.get(); d.gNodes = gNodes.get(); d.gMode = gMode.get(); d.groupEntry = groupEntry.get();
     d.gpx = gpx.get(); d.gpy = gpy.get(); d.gpz = gpz.get(); d.gMargin = M.gMargin; d.maxGroup = maxGroup;
     d.nc = NC;
     d.ca = ca.get(); d.cb = cb.get(); d.skip = skip.get(); d.law = law.get();

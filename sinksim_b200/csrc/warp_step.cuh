@@ -139,8 +139,11 @@ struct Prec<true> {
   static __device__ __forceinline__ T iR(const Pose& F) { return F.fiR; }
 };
 
+// With `first` only the first point of this thread is looked at, and `whole` is cleared when the list has more than the
+// threads' first ones.
 template <bool MIXED>
-__device__ __noinline__ typename Prec<MIXED>::T node_extreme(const DevModel& M, const Pose& F, int n, bool top, int sub, int lanes) {
+__device__ __noinline__ typename Prec<MIXED>::T scan_extreme(const DevModel& M, const Pose& F, int n, bool top, int sub, int lanes, bool first,
+                                                              bool& whole) {
   using P = Prec<MIXED>;
   using T = typename P::T;
   const T R20 = P::R20(F), R21 = P::R21(F), R22 = P::R22(F), tz = P::tz(F);
@@ -159,14 +162,22 @@ __device__ __noinline__ typename Prec<MIXED>::T node_extreme(const DevModel& M, 
     j = hull ? 0 : __ldg(M.segStart + n);
     end = j + (hull ? M.ncol : __ldg(M.segCount + n));
   }
+  whole = !first || end - j <= lanes;
+  if (!whole) end = j + lanes;
   T best = top ? T(-1e9) : T(1e9);
-#pragma unroll 1
+#pragma unroll 2
   for (j += sub; j < end; j += lanes) {
     const auto p = __ldg(xy + j);
     const T w = R20 * p.x + R21 * p.y + tz + R22 * __ldg(z + static_cast<std::size_t>(j) * zs);
     if (top ? w > best : w < best) best = w;
   }
   return best;
+}
+
+template <bool MIXED>
+__device__ __forceinline__ typename Prec<MIXED>::T node_extreme(const DevModel& M, const Pose& F, int n, bool top, int sub, int lanes) {
+  bool whole;
+  return scan_extreme<MIXED>(M, F, n, top, sub, lanes, false, whole);
 }
 
 // ----------------------------------------------------------------------------- buoyancy (hydro pass, tree order)
@@ -214,35 +225,60 @@ template <class T> struct Vec2;
 template <> struct Vec2<double> { using type = double2; };
 template <> struct Vec2<float> { using type = float2; };
 
-// A load of the column table: through the read-only data cache from global memory, or from shared memory (SMEM: the
-// table staged there).
-template <bool SMEM, class P>
+// A load of the column table: from shared memory (kStaged: the table staged there), or through the read-only data cache
+// from global memory; kStreamed: without a place in L1, which a lone simulation's step would sweep clean with the 176 KB
+// it reads once, while the segments and the small tables are read again.
+enum ColumnSource { kCached, kStreamed, kStaged };
+
+__device__ __forceinline__ double2 load_streamed(const double2* p) {
+  double2 v;
+  asm("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double load_streamed(const double* p) {
+  double v;
+  asm("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float2 load_streamed(const float2* p) {
+  float2 v;
+  asm("ld.global.nc.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float load_streamed(const float* p) {
+  float v;
+  asm("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+
+template <ColumnSource SRC, class P>
 __device__ __forceinline__ P load_col(const P* p) {
-  if constexpr (SMEM) return *p;
+  if constexpr (SRC == kStaged) return *p;
+  else if constexpr (SRC == kStreamed) return load_streamed(p);
   else return __ldg(p);
 }
 
-// Lane `lane`'s partial of tree w: columns w*32 + lane + 256 k in increasing k, four at a time (the loads of all four
-// issue before the first is clipped; the clips stay in order).
-template <class T, bool SMEM = false>
+// Lane `lane`'s partial of tree w: columns w*32 + lane + 256 k in increasing k, AT_ONCE at a time (the loads of
+// all issue before the first is clipped; the clips stay in order). Large teams wait for the loads and take four; small
+// ones share an SM with others that fill the wait, and two need less code and pad less.
+template <class T, ColumnSource SRC, int AT_ONCE>
 __device__ __forceinline__ ColPartial<T> column_partial(const typename Vec2<T>::type* xy, const typename Vec2<T>::type* lh, const T* area,
                                                         int ncol, int first, T R20, T R21, T tz, T iR) {
-  constexpr int kAtOnce = 4;
   ColPartial<T> p{T(0), T(0), T(0), T(0)};
 #pragma unroll 1
-  for (int i = first; i < ncol; i += kAtOnce * 256) {
-    typename Vec2<T>::type a[kAtOnce], b[kAtOnce];
-    T A[kAtOnce];
+  for (int i = first; i < ncol; i += AT_ONCE * 256) {
+    typename Vec2<T>::type a[AT_ONCE], b[AT_ONCE];
+    T A[AT_ONCE];
 #pragma unroll
-    for (int k = 0; k < kAtOnce; ++k) {
+    for (int k = 0; k < AT_ONCE; ++k) {
       // past the table's end: the last column read again with no footprint, which adds zeros
       const int j = i + 256 * k < ncol ? i + 256 * k : i;
-      a[k] = load_col<SMEM>(xy + j);
-      b[k] = load_col<SMEM>(lh + j);
-      A[k] = i + 256 * k < ncol ? load_col<SMEM>(area + j) : T(0);
+      a[k] = load_col<SRC>(xy + j);
+      b[k] = load_col<SRC>(lh + j);
+      A[k] = i + 256 * k < ncol ? load_col<SRC>(area + j) : T(0);
     }
 #pragma unroll
-    for (int k = 0; k < kAtOnce; ++k) clip_column<T>(a[k].x, a[k].y, b[k].x, b[k].y, A[k], R20, R21, tz, iR, p);
+    for (int k = 0; k < AT_ONCE; ++k) clip_column<T>(a[k].x, a[k].y, b[k].x, b[k].y, A[k], R20, R21, tz, iR, p);
   }
   return p;
 }
@@ -279,10 +315,10 @@ __device__ __noinline__ void buoyancy_trees(const DevModel& M, const Pose& F, in
     ColPartial<R> p;
     if (cols) {
       const StagedColumns<R> c = staged_columns<R>(M.ncol);
-      p = column_partial<R, true>(reinterpret_cast<const typename P::V2*>(cols + c.xy), reinterpret_cast<const typename P::V2*>(cols + c.lh),
+      p = column_partial<R, kStaged, 2>(reinterpret_cast<const typename P::V2*>(cols + c.xy), reinterpret_cast<const typename P::V2*>(cols + c.lh),
                                   reinterpret_cast<const R*>(cols + c.area), M.ncol, w * kLanes + lane, P::R20(F), P::R21(F), P::tz(F), P::iR(F));
     } else {
-      p = column_partial<R>(P::colXY(M), P::colLH(M), P::colAr(M), M.ncol, w * kLanes + lane, P::R20(F), P::R21(F), P::tz(F), P::iR(F));
+      p = column_partial<R, (W >= 8 ? kStreamed : kCached), (W >= 8 ? 4 : 2)>(P::colXY(M), P::colLH(M), P::colAr(M), M.ncol, w * kLanes + lane, P::R20(F), P::R21(F), P::tz(F), P::iR(F));
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
@@ -375,18 +411,17 @@ __device__ __forceinline__ void tree_pair(SegPartial<T>& lo, const SegPartial<T>
   lo.vol = lo.vol + up.vol; lo.dv = lo.dv + up.dv; lo.mx = lo.mx + up.mx; lo.my = lo.my + up.my; lo.mz = lo.mz + up.mz;
 }
 
-// The node pass of node n at world level h: the 32 lane partials, the halving tree and the permeability scaling
-// (hydro.hpp:295-316 / 338-349). Lane `sub` of a group of kLevelLanes lanes forms the partials of tree lanes
-// sub + kLevelLanes j and combines them over the tree's upper levels (offsets 16 down to kLevelLanes) in registers; the
-// lower levels are shuffles inside the group. Every lane of the group ends with the bits of tree lane 0. Every lane of
-// the warp calls it (n < 0: a group without a node, which sums nothing), so the groups' passes run side by side.
+// The pass over a node's segments [s0, s1) with permeability mu at world level h: the 32 lane partials, the halving tree
+// and the permeability scaling (hydro.hpp:295-316 / 338-349). Lane `sub` of a group of kLevelLanes lanes forms the partials
+// of tree lanes sub + kLevelLanes j and combines them over the tree's upper levels (offsets 16 down to kLevelLanes) in
+// registers; the lower levels are shuffles inside the group. Every lane of the group ends with the bits of tree lane 0.
+// Every lane of the warp calls it (an empty range for a group without a node), so the groups' passes run side by side.
 template <bool MIXED, int W>
-__device__ __forceinline__ PassR node_pass(const DevModel& M, const Pose& F, int n, double h, const LevelLanes& L) {
+__device__ __forceinline__ PassR node_pass(const DevModel& M, const Pose& F, int s0, int s1, double mu, double h, const LevelLanes& L) {
   using P = Prec<MIXED>;
   using T = typename P::T;
   constexpr int LANES = kLevelLanes<MIXED>;
   constexpr int AHEAD = W >= 8 ? 2 : 1;  // large teams are bound by the loads' latency, small ones by issue slots
-  const int s0 = n < 0 ? 0 : __ldg(M.segStart + n), s1 = n < 0 ? 0 : s0 + __ldg(M.segCount + n);
   const T hT = static_cast<T>(h);
   const int f = s0 + L.sub;
   const T R20 = P::R20(F), R21 = P::R21(F), tz = P::tz(F), iR = P::iR(F);
@@ -410,7 +445,6 @@ __device__ __forceinline__ PassR node_pass(const DevModel& M, const Pose& F, int
     p.vol = bsum(p.vol, off); p.dv = bsum(p.dv, off); p.mx = bsum(p.mx, off);
     p.my = bsum(p.my, off); p.mz = bsum(p.mz, off);
   }
-  const double mu = n < 0 ? 0.0 : __ldg(M.mu + n);
   PassR r;
   r.vol = static_cast<double>(p.vol) * mu;
   r.dv = static_cast<double>(p.dv) * mu * F.iR;
@@ -427,7 +461,8 @@ struct Slot {
   PassR* passes;
   std::uint8_t* merged;
   std::uint8_t* dry;          // NodeFlag bits
-  std::uint16_t* list;        // the groups the next level solve visits, misc[kMiscListed] of them
+  Listed* list;               // the groups the next level solve visits, misc[kMiscListed] of them
+  std::uint8_t* wet;          // per 32 nodes, the flooded ones among them (their load terms)
   std::uint16_t* flow;        // the connections that can flow in this step (sort_connections)
   Pose* pose;                 // the current step's pose, and
   Pose* prev;                 // the last step's (that of the last level solve, between steps)
@@ -457,7 +492,8 @@ __device__ __forceinline__ Slot carve_slot(unsigned char* base, const SlotLayout
   s.passes = reinterpret_cast<PassR*>(base + L.passes);
   s.merged = base + L.merged;
   s.dry = base + L.dry;
-  s.list = reinterpret_cast<std::uint16_t*>(base + L.list);
+  s.wet = base + L.wet;
+  s.list = reinterpret_cast<Listed*>(base + L.list);
   s.pose = reinterpret_cast<Pose*>(base + L.pose);
   s.prev = s.pose + 1;
   s.parked = reinterpret_cast<Parked*>(base + L.parked);
@@ -474,16 +510,20 @@ __device__ __forceinline__ Slot carve_slot(unsigned char* base, const SlotLayout
 // of a full node, or of one whose starting level lies outside it, is not made. Every pass of a warp's lane groups runs
 // through one call site under a warp-wide loop: two half-warps in different solvers would otherwise issue everything
 // twice. Centroids are divided node by node afterwards, a thread per node (team_step).
-// Measured on B200: 2,048 titanic64 instances of the uneven batch to 20 min 512 ms (805 ms with a pass over every
-// segment of every node, a divergent solver per half-warp and the extents in the pass), 264 liner runs to 15 min 119 ms
-// (152), one titanic64 run to 5 min 35.1 ms (40.5).
+// Measured on B200 when it came, with the step as it then was: 2,048 titanic64 instances of the uneven batch to 20 min
+// 512 ms (805 ms with a pass over every segment of every node, a divergent solver per half-warp and the extents in the
+// pass), 264 liner runs to 15 min 119 ms (152), one titanic64 run to 5 min 35.1 ms (40.5). The first look at the extent
+// lists, members side by side, list entries that carry the members, the pair's sharing in all lanes and the columns past
+// L1 in large teams: 192 runs to 1 h 264 ms (353 before), one run 21.7 (29.1), 264 liner runs 95 (108), 2,048 uneven runs
+// 348 (371).
 
 // S.dry[n].
 enum NodeFlag : std::uint8_t {
   kStale = 1,      // empty at the last level solve: S.level[n] is not formed yet
   kEmptyNode = 2,  // empty at the coming one
   kZeroVolume = 4, // ... in a merged group, which empties its members
-  kSolved = 8      // passes were made for it at this one
+  kSolved = 8,     // passes were made for it at this one
+  kNoTop = 16      // ... without its highest point: S.zmax[n] is not formed
 };
 
 // S.misc: the claimed instance, the yield flag, the level solve's counter of list entries taken, the list's length, the
@@ -504,35 +544,50 @@ struct NoTape {
 
 // Lists the groups the next level solve visits, in increasing order, and flags the nodes of the others; one warp calls
 // it. A group is left out (kLazy) when neither its members nor their sum exceed the empty volume: then the solve would
-// find it empty merged or not.
+// find it empty merged or not. An entry, made with the model, carries what the solve would otherwise fetch in three
+// dependent loads.
 template <bool LAZY>
 __device__ __forceinline__ void list_groups(const DevModel& M, Slot& S, int lane) {
   int count = 0;
 #pragma unroll 1
   for (int g0 = 0; g0 < M.ng; g0 += kLanes) {
-    const int g = g0 + lane;
-    bool live = false;
-    if (g < M.ng) {
-      const int N = __ldg(M.gCount + g);
+    const bool any = g0 + lane < M.ng;
+    const int g = any ? g0 + lane : g0;
+    const uint2 bits = __ldg(reinterpret_cast<const uint2*>(M.groupEntry) + g);
+    const int n0 = bits.x >> 16, n1 = bits.y & 0xffff, N = (bits.y >> 16) & 0xff;
+    const double v0 = S.vol[n0], v1 = S.vol[n1];  // (n1 is n0 in a group of one)
+    double V = v0;
+    bool live = !LAZY || !(v0 <= kEmptyVolume);
+    if (N >= 2) {
+      V += v1;
+      live = live || !(v1 <= kEmptyVolume);
+    }
+    if (N > 2) {
       const int* m = M.gNodes + __ldg(M.gStart + g);
-      double V = 0;
-      live = !LAZY;
+      const int all = __ldg(M.gCount + g);
 #pragma unroll 1
-      for (int k = 0; k < N; ++k) {
+      for (int k = 2; k < all; ++k) {
         const double v = S.vol[__ldg(m + k)];
         V += v;
-        if (!(v <= kEmptyVolume)) live = true;
+        live = live || !(v <= kEmptyVolume);
       }
-      if (!(V <= kEmptyVolume)) live = true;
-      if (!live) {
-        const bool merged = N >= 2 && __ldg(M.gMode + g) == 1;
-        S.merged[g] = merged ? 1 : 0;
+    }
+    live = any && (live || !(V <= kEmptyVolume));
+    if (any && !live) {
+      const bool merged = N >= 2 && (bits.y >> 24) == 1;
+      const int flags = kEmptyNode | (merged ? kZeroVolume : 0);
+      S.merged[g] = merged ? 1 : 0;
+      S.dry[n0] |= flags;
+      if (N >= 2) S.dry[n1] |= flags;
+      if (N > 2) {
+        const int* m = M.gNodes + __ldg(M.gStart + g);
+        const int all = __ldg(M.gCount + g);
 #pragma unroll 1
-        for (int k = 0; k < N; ++k) S.dry[__ldg(m + k)] |= kEmptyNode | (merged ? kZeroVolume : 0);
+        for (int k = 2; k < all; ++k) S.dry[__ldg(m + k)] |= flags;
       }
     }
     const unsigned mask = __ballot_sync(kFull, live);
-    if (live) S.list[count + __popc(mask & ((1u << lane) - 1u))] = static_cast<std::uint16_t>(g);
+    if (live) reinterpret_cast<uint2*>(S.list)[count + __popc(mask & ((1u << lane) - 1u))] = bits;
     count += __popc(mask);
   }
   if (lane == 0) S.misc[kMiscListed] = count;
@@ -560,6 +615,36 @@ __device__ __forceinline__ double stale_level(const DevModel& M, const Slot& S, 
 template <bool MIXED>
 __device__ __forceinline__ double group_level(const DevModel& M, const Slot& S, int n, const LevelLanes& L) {
   return (S.dry[n] & kStale) ? group_extreme<MIXED>(M, *S.prev, n, false, L) : S.level[n];
+}
+
+// A first look at the world extents of one node, or of two side by side, by a lane group: z[0] and z[1] the lowest bottom
+// and highest top of n0, z[2] and z[3] those of n1, over the first points of their lists. Each quarter of the lanes looks
+// at one list (with one node, two quarters share each); `whole` says whether that was all of every list.
+struct Extents {
+  double z[4];
+  bool whole;
+};
+
+template <bool MIXED>
+__device__ __forceinline__ Extents first_extents(const DevModel& M, const Pose& F, int n0, int n1, bool two, const LevelLanes& L) {
+  constexpr int LANES = kLevelLanes<MIXED>, Q = LANES / 4;
+  const int quarter = L.sub / Q, at = L.sub % Q;
+  const bool top = quarter & 1;
+  bool whole = true;
+  auto v = scan_extreme<MIXED>(M, F, two && quarter >= 2 ? n1 : n0, top, two ? at : (quarter >> 1) * Q + at, two ? Q : 2 * Q, true, whole);
+#pragma unroll
+  for (int off = Q / 2; off > 0; off >>= 1) {
+    const auto o = __shfl_xor_sync(L.mask, v, off);
+    if (top ? o > v : o < v) v = o;
+  }
+  const auto o = __shfl_xor_sync(L.mask, v, 2 * Q);
+  if (!two && (top ? o > v : o < v)) v = o;
+  Extents e;
+  const int base = L.lane - L.sub;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) e.z[k] = static_cast<double>(__shfl_sync(L.mask, v, base + k * Q));
+  e.whole = (__ballot_sync(L.mask, whole) & L.mask) == L.mask;
+  return e;
 }
 
 // The solved values of a node whose last pass was p: the pass's sums go to scratch arrays that are dead until the heads,
@@ -620,70 +705,108 @@ __device__ __forceinline__ void share_group(const DevModel& M, Slot& S, const Pa
   for (int k = 0; k < N; ++k) store_solved(S, __ldg(m + k), h, P[k].dv, P[k]);
 }
 
+// share_group for a group of two, by all lanes of its group: p0 the first member's pass, p1 the second's, tot their volume.
+__device__ __forceinline__ void share_pair(Slot& S, const PassR& p0, const PassR& p1, int n0, int n1, double vmax0, double vmax1, double tot,
+                                           double V, double h, int sub) {
+  double v = tot > 0 ? V * p0.vol / tot : 0.5 * V;
+  if (v > vmax0) v = vmax0;
+  if (V - v > vmax1) v = V - vmax1;
+  if (sub == 0) {
+    S.vol[n0] = v;
+    S.vol[n1] = V - v;
+    store_solved(S, n0, h, p0.dv, p0);
+    store_solved(S, n1, h, p1.dv, p1);
+  }
+}
+
 // The level solve of the listed groups (levels.hpp:13-194). Groups are independent (a group's solve reads and writes only
 // its members), so the team's level lane groups (32 / kLevelLanes<MIXED> per warp) take them as they come: each starts
 // with the list entry of its own index, then takes the next one from the team's counter (S.misc[kMiscTaken]); groups
-// take different numbers of passes, and a node's results do not depend on which lane group computes them.
+// take different numbers of passes, and a node's results do not depend on which lane group computes them. In 16-warp teams
+// the upper warps, which have no buoyancy tree, start with the first entries.
+//
+// A unit needs its world extent to see that its starting level lies inside, and as the ends of the Newton bracket. Both are
+// comparisons, which the first points of the extent lists mostly decide: a level above one of the bottoms is above the
+// lowest, an iterate below one of the tops is below the highest. The rest of the lists are scanned only when they leave
+// the question open or a bisection needs the ends themselves (and with a tape, which records the extent). A lane group's
+// solver is a small machine (Phase) around one place for each of its parts.
 template <bool MIXED, int W, class Tape>
 __device__ __forceinline__ void solve_levels(const DevModel& M, const Pose& F, Slot& S, const Team<W>& T, const Tape& tape) {
   constexpr int LANES = kLevelLanes<MIXED>, PER_WARP = 32 / LANES;
+  enum Phase { kIdle, kStart, kUpdate, kPass };
   const LevelLanes L = level_lanes<MIXED>(T.lane);
   const int grp = T.lane / LANES;
-  const int unit = T.warp * PER_WARP + grp;
-  PassR* const P = S.passes + static_cast<std::size_t>(unit) * M.maxGroup;
+  PassR* const P = S.passes + static_cast<std::size_t>(T.warp * PER_WARP + grp) * M.maxGroup;
   const int listed = S.misc[kMiscListed];
-  int i = unit;                                // the next list entry
-  const int* m = nullptr;                      // the current group's members,
+  int i = (W == 16 ? T.warp ^ 8 : T.warp) * PER_WARP + grp;   // the next list entry
+  Listed e{};                                  // the current group,
+  const int* m = nullptr;                      // its members when there are more than two,
   int N = 0, j = 0, units = 0;                 // their number, its next unit and its units
   bool merged = false;
-  // the current unit: nm members from mm, and where its solve is
-  const int* mm = nullptr;
-  int nm = 0, k = 0, slot = 0, it = 0;
-  bool have = false, full = false;
-  double V = 0, tol = 0, h = 0, a = 0, b = 0, sum = 0, dvs = 0;
+  // the current unit: nm members, n0 and n1 first (the others from m) with their segments
+  int n0 = 0, n1 = 0, nm = 0;
+  int2 seg0{}, seg1{};
+  // (phase is made opaque between the parts, or the compiler copies them for each phase they can follow: 3% of a full
+  // load's time in code)
+  // where its solve is: the member of the pass, the pass's tape slot, the Newton update, what is known of the extent
+  int phase = kIdle;
+  int k = 0, slot = 0, it = 0;
+  bool full = false, empty = false, inside = false;
+  bool aKnown = false, bKnown = false;  // a (b) is an iterate or the unit's whole extent's end, not just a first look's
+  double V = 0, Vmax = 0, vmax1 = 0, h = 0, a = 0, b = 0, sum = 0, dvs = 0;
+  auto member = [&](int q) { return q == 0 ? n0 : (q == 1 ? n1 : __ldg(m + q)); };
+#pragma unroll 1
   for (;;) {
 #pragma unroll 1
-    while (!have && (j < units || i < listed)) {
+    while (phase == kIdle && (j < units || i < listed)) {
       if (j >= units) {
-        const int g = S.list[i];
+        e = S.list[i];
         int next = 0;
         if (L.sub == 0) next = atomicAdd(&S.misc[kMiscTaken], 1);
         i = __shfl_sync(L.mask, next, grp * LANES);
-        N = __ldg(M.gCount + g);
-        m = M.gNodes + __ldg(M.gStart + g);
+        N = e.N;
+        m = nullptr;
+        if (N > 2) {
+          if (N == 255) N = __ldg(M.gCount + e.g);
+          m = M.gNodes + __ldg(M.gStart + e.g);
+        }
         merged = false;
         if (N >= 2) {
-          const int mode = __ldg(M.gMode + g);
-          if (mode == 1) {
+          if (e.mode == 1) {
             merged = true;
-          } else if (mode == 2) {
-            const double zMw = world_z(F, __ldg(M.gpx + g), __ldg(M.gpy + g), __ldg(M.gpz + g));
+          } else if (e.mode == 2) {
+            const double zMw = world_z(F, __ldg(M.gpx + e.g), __ldg(M.gpy + e.g), __ldg(M.gpz + e.g));
             merged = true;
 #pragma unroll 1
             for (int q = 0; q < N; ++q) {
-              const int n = __ldg(m + q);
+              const int n = q == 0 ? e.n0 : (q == 1 ? e.n1 : __ldg(m + q));
               if (!(S.vol[n] > kEmptyVolume && group_level<MIXED>(M, S, n, L) > zMw + M.gMargin)) { merged = false; break; }
             }
           }
         }
-        if (L.sub == 0) S.merged[g] = merged ? 1 : 0;
+        if (L.sub == 0) S.merged[e.g] = merged ? 1 : 0;
         units = merged ? 1 : N;
         j = 0;
         if (units == 0) continue;  // a group without members
       }
-      mm = merged ? m : m + j;
+      n0 = j == 0 ? e.n0 : (j == 1 ? e.n1 : __ldg(m + j));
       nm = merged ? N : 1;
+      n1 = nm > 1 ? e.n1 : n0;
       ++j;
-      double Vmax = 0;
-      V = 0;
+      // everything the unit needs of its nodes' table, in one round of loads
+      seg0 = __ldg(M.nodeSeg + n0); seg1 = __ldg(M.nodeSeg + n1);
+      Vmax = __ldg(M.vmax + n0);
+      V = S.vol[n0];
+      vmax1 = __ldg(M.vmax + n1);
+      if (nm > 1) { V += S.vol[n1]; Vmax += vmax1; }
 #pragma unroll 1
-      for (int q = 0; q < nm; ++q) { const int n = __ldg(mm + q); V += S.vol[n]; Vmax += __ldg(M.vmax + n); }
-      const bool empty = V <= kEmptyVolume;
+      for (int q = 2; q < nm; ++q) { const int n = __ldg(m + q); V += S.vol[n]; Vmax += __ldg(M.vmax + n); }
+      empty = V <= kEmptyVolume;
       if constexpr (Tape::kLazy) {
         if (empty) {
           if (L.sub == 0)
 #pragma unroll 1
-            for (int q = 0; q < nm; ++q) S.dry[__ldg(mm + q)] = (S.dry[__ldg(mm + q)] & kStale) | kEmptyNode | (merged ? kZeroVolume : 0);
+            for (int q = 0; q < nm; ++q) { const int n = member(q); S.dry[n] = (S.dry[n] & kStale) | kEmptyNode | (merged ? kZeroVolume : 0); }
           continue;
         }
       }
@@ -693,80 +816,129 @@ __device__ __forceinline__ void solve_levels(const DevModel& M, const Pose& F, S
       int firstWet = -1;
 #pragma unroll 1
       for (int q = 0; merged && q < nm; ++q) {
-        if (S.vol[__ldg(mm + q)] > 0) { if (firstWet < 0) firstWet = q; }
+        if (S.vol[member(q)] > 0) { if (firstWet < 0) firstWet = q; }
         else allWet = false;
       }
       const int q0 = allWet ? 0 : (firstWet >= 0 ? firstWet : nm - 1), q1 = allWet ? nm : q0 + 1;
       h = 0;
 #pragma unroll 1
-      for (int q = q0; q < q1; ++q) h += group_level<MIXED>(M, S, __ldg(mm + q), L);
-      if (merged && allWet) h = h / static_cast<double>(nm);
+      for (int q = q0; q < q1; ++q) h += group_level<MIXED>(M, S, member(q), L);
+      if (merged && allWet) h = nm == 2 ? 0.5 * h : h / static_cast<double>(nm);
+      full = V >= Vmax * kFullFraction;
+      inside = aKnown = bKnown = false;
+      if (nm <= 2) {
+        const Extents x = first_extents<MIXED>(M, F, n0, n1, nm == 2, L);
+        a = nm == 2 && x.z[2] < x.z[0] ? x.z[2] : x.z[0];
+        b = nm == 2 && x.z[3] > x.z[1] ? x.z[3] : x.z[1];
+        inside = Tape::kLazy && !full && h >= a && h <= b;
+        aKnown = bKnown = x.whole;
+        if (inside || x.whole) {
+          tape.start(n0, h, x.z[0], x.z[1], L);
+          if (nm == 2) tape.start(n1, h, x.z[2], x.z[3], L);
+          if (L.sub == 0) {
+            const int flags = !Tape::kLazy && empty ? kEmptyNode | (merged ? kZeroVolume : 0) : kSolved | (x.whole ? 0 : kNoTop);
+            S.zmax[n0] = x.z[1];
+            S.dry[n0] = flags;
+            if (nm == 2) { S.zmax[n1] = x.z[3]; S.dry[n1] = flags; }
+            if (!Tape::kLazy && empty) { S.level[n0] = x.z[0]; if (nm == 2) S.level[n1] = x.z[2]; }
+          }
+        }
+      }
+      phase = kStart;
+      break;
+    }
+    asm volatile("" : "+r"(phase));
+    // an update's Newton iterate: sum and dvs are the unit's passes at h, the it-th after the starting one
+    double hn = 0;
+    if (phase == kUpdate) {
+      const double err = sum - V;
+      if (err > 0) { b = h; bKnown = true; } else { a = h; aKnown = true; }
+      hn = h - err / dvs;
+    }
+    asm volatile("" : "+r"(phase));
+    // the whole extent, where the first look leaves the start or an update open
+    if ((phase == kStart && !inside && !aKnown) || (phase == kUpdate && !(aKnown && bKnown) && !(dvs > kSlopeMin && hn > a && hn < b))) {
       double lo = 0, hi = 0;
 #pragma unroll 1
       for (int q = 0; q < nm; ++q) {
-        const int n = __ldg(mm + q);
+        const int n = member(q);
         double zlo = 0, zhi = 0;
 #pragma unroll 1
         for (int top = 0; top < 2; ++top) {
           const double z = group_extreme<MIXED>(M, F, n, top != 0, L);
           if (top) zhi = z; else zlo = z;
         }
-        tape.start(n, h, zlo, zhi, L);
         if (q == 0 || zlo < lo) lo = zlo;
         if (q == 0 || zhi > hi) hi = zhi;
+        if (phase == kStart) tape.start(n, h, zlo, zhi, L);
         if (L.sub == 0) {
           S.zmax[n] = zhi;
-          S.dry[n] = empty ? kEmptyNode | (merged ? kZeroVolume : 0) : kSolved;
-          if (empty) S.level[n] = zlo;
+          S.dry[n] = !Tape::kLazy && empty ? kEmptyNode | (merged ? kZeroVolume : 0) : kSolved;
+          if (!Tape::kLazy && empty) S.level[n] = zlo;
         }
       }
-      if (empty) continue;
-      full = V >= Vmax * kFullFraction;
+      if (!aKnown) a = lo;
+      if (!bKnown) b = hi;
+      aKnown = bKnown = true;
+    }
+    asm volatile("" : "+r"(phase));
+    if (phase == kStart) {
       it = 0; slot = 0; k = 0; sum = 0; dvs = 0;
-      if (full) {
+      phase = kPass;
+      if (!Tape::kLazy && empty) {
+        phase = kIdle;
+      } else if (full) {
         // the pass at the top of a full unit, for its centroids; its level and volumes first
         double dh = 0;
         if (!merged) {
-          dh = jmax(0.0, V - Vmax) / __ldg(M.aov + __ldg(mm));
+          dh = jmax(0.0, V - Vmax) / __ldg(M.aov + n0);
         } else {
           const double over = jmax(0.0, V - Vmax);
           double aSum = 0;
 #pragma unroll 1
-          for (int q = 0; q < nm; ++q) aSum += __ldg(M.aov + __ldg(mm + q));
+          for (int q = 0; q < nm; ++q) aSum += __ldg(M.aov + member(q));
           dh = over / aSum;
           if (L.sub == 0) {
             double assigned = 0;
 #pragma unroll 1
             for (int q = 0; q < nm - 1; ++q) {
-              const int n = __ldg(mm + q);
+              const int n = member(q);
               const double v = __ldg(M.vmax + n) + dh * __ldg(M.aov + n);
               S.vol[n] = v;
               assigned += v;
             }
-            S.vol[__ldg(mm + nm - 1)] = V - assigned;
+            S.vol[member(nm - 1)] = V - assigned;
           }
         }
-        a = hi + dh;  // the level
-        h = hi;
+        h = b;
+        a = b + dh;  // the level
         slot = 1;
-      } else {
-        tol = jmax(1e-3 * Vmax, 0.5);
-        a = lo; b = hi;
-        if (merged ? !(h >= lo && h <= hi) : (h < lo || h > hi)) {
-          h = jmin(hi, jmax(lo, h));
-          slot = 1;
-        }
+      } else if (!inside && (merged ? !(h >= a && h <= b) : (h < a || h > b))) {
+        h = jmin(b, jmax(a, h));
+        slot = 1;
       }
-      have = true;
+    } else if (phase == kUpdate) {
+      if (!(dvs > kSlopeMin && hn > a && hn < b)) hn = 0.5 * (a + b);
+      h = hn;
+      ++it;
+      sum = 0; dvs = 0;
+      phase = kPass;
     }
-    if (!__any_sync(kFull, have)) break;
-    const int n = have ? __ldg(mm + k) : -1;
-    const PassR p = node_pass<MIXED, W>(M, F, n, h, L);
-    if (!have) continue;
+    asm volatile("" : "+r"(phase));
+    if (!__any_sync(kFull, phase == kPass)) {
+      if (!__any_sync(kFull, j < units || i < listed)) break;
+      continue;
+    }
+    int2 sg = k == 0 ? seg0 : seg1;
+    int n = k == 0 ? n0 : n1;
+    if (k > 1) { n = __ldg(m + k); sg = __ldg(M.nodeSeg + n); }
+    if (phase != kPass) sg = int2{0, 0};
+    const PassR p = node_pass<MIXED, W>(M, F, sg.x, sg.x + sg.y, __ldg(M.mu + n), h, L);
+    if (phase != kPass) continue;
     tape.pass(n, slot, h, p, L);
     if (full) {
       if (L.sub == 0) store_solved(S, n, a, __ldg(M.aov + n), p);
-      if (++k == nm) have = false;
+      if (++k == nm) { phase = kIdle; k = 0; }
       continue;
     }
     sum += p.vol;
@@ -777,22 +949,18 @@ __device__ __forceinline__ void solve_levels(const DevModel& M, const Pose& F, S
       k = 0;
     }
     ++slot;
-    // Newton on the unit's volume: sum and dvs are its passes at h, the it-th after the starting one
-    const double err = sum - V;
-    if (it < kNewtonFast && !(fabs(err) < tol)) {
-      if (err > 0) b = h; else a = h;
-      double hn = dvs > kSlopeMin ? h - err / dvs : 0.5 * (a + b);
-      if (!(hn > a && hn < b)) hn = 0.5 * (a + b);
-      h = hn;
-      ++it;
-      sum = 0; dvs = 0;
+    if (it < kNewtonFast && !(fabs(sum - V) < jmax(1e-3 * Vmax, 0.5))) {
+      phase = kUpdate;
       continue;
     }
-    if (L.sub == 0) {
-      if (nm == 1 && !merged) store_solved(S, n, h, p.dv, p);
-      else share_group(M, S, P, mm, nm, V, h);
+    if (nm == 2) {
+      __syncwarp(L.mask);
+      share_pair(S, P[0], p, n0, n1, __ldg(M.vmax + n0), vmax1, sum, V, h, L.sub);
+    } else if (L.sub == 0) {
+      if (nm == 1) store_solved(S, n, h, p.dv, p);
+      else share_group(M, S, P, m, nm, V, h);
     }
-    have = false;
+    phase = kIdle;
   }
   __syncwarp();
 }
@@ -1082,23 +1250,61 @@ __device__ __forceinline__ double add_in_order(double acc, double v) {
 // per-connection work is spread over all 32 W threads of the team; the sums over nodes in their serial order, the
 // motion and the next pose are one warp's, while another lists the next solve's groups and a third the events.
 
-// The sums, the motion and the next pose (flows.hpp:114-118, body.hpp:11-57, events.hpp:30-38), by one warp: the load
-// terms of the nodes are in columns a fixed stride apart from S.area (dry nodes hold -0, which leaves every sum as it is),
-// the excess in S.acc. Lanes 0 .. 5 each add one column in node order: a lane reading all six, node by node, took a
-// dependent load and six adds a node.
-__device__ __forceinline__ void move_body(const DevModel& M, const Pose& F, Slot& S, int lane) {
+// The inflow from the sea in the step that just flowed (flows.hpp:114-118): the sea connections in order, less the excess
+// that returns, in node order. Nothing in the motion needs it, so another warp forms it meanwhile.
+__device__ __forceinline__ void sea_inflow(const DevModel& M, Slot& S, int lane) {
   double seaIn = 0;
 #pragma unroll 1
   for (int k0 = 0; k0 < M.nsea; k0 += kLanes) {
     const int k = k0 + lane;
     seaIn = add_in_order<false>(seaIn, k < M.nsea ? S.dV[__ldg(M.sea + k)] : 0.0);
   }
-  // the excess returns to the sea in node order
 #pragma unroll 1
   for (int n0 = 0; n0 < M.nn; n0 += kLanes) {
     const int n = n0 + lane;
     seaIn = add_in_order<true>(seaIn, n < M.nn && S.acc[n] > 0 ? S.acc[n] : 0.0);
   }
+  if (lane == 0) S.parked->inflow = seaIn / M.dt;
+}
+
+// The semi-implicit motion (body.hpp:42-57) and the founder rule (events.hpp:30-38) on the run's values, by the lanes of one
+// warp alike; returns (zO, pitch, roll).
+struct MotionIn {
+  double tauX, tauY, Fz, mw, Iwp, Iwr, cth;
+};
+
+__device__ __forceinline__ double3 integrate_motion(const DevModel& M, Parked& P, const MotionIn& I, const Buoy& hb) {
+  const double Mth = I.tauY, Mph = I.tauX * I.cth;
+  const double dt = M.dt;
+  double vz = P.vz, wth = P.wth, wph = P.wph, zO = P.zO, pitch = P.pitch, roll = P.roll;
+  const double mh = M.mh0 + I.mw;
+  const double Ith = M.Ith0 + I.Iwp, Iph = M.Iph0 + I.Iwr;
+  const double az = (I.Fz - M.cDz * vz - M.qz * fabs(vz) * vz) / mh;
+  const double ath = (Mth - M.cDth * wth - M.qth * fabs(wth) * wth) / Ith;
+  const double aph = (Mph - M.cDph * wph - M.qph * fabs(wph) * wph) / Iph;
+  vz += az * dt; wth += ath * dt; wph += aph * dt;
+  zO += vz * dt; pitch += wth * dt; roll += wph * dt;
+  if (pitch > kPitchClamp) { pitch = kPitchClamp; wth = 0; }
+  if (pitch < -kPitchClamp) { pitch = -kPitchClamp; wth = 0; }
+  if (roll > kRollClamp) { roll = kRollClamp; wph = 0; }
+  if (roll < -kRollClamp) { roll = -kRollClamp; wph = 0; }
+  const double t = P.t + dt;
+  __syncwarp();  // the lanes have read the values they now replace
+  P.t = t; P.zO = zO; P.pitch = pitch; P.roll = roll; P.vz = vz; P.wth = wth; P.wph = wph;
+  P.Vb = hb.V; P.hullTop = hb.top; P.mw = I.mw;
+  P.bx = hb.x; P.by = hb.y; P.bz = hb.z;
+  if (!P.foundered && (hb.top < M.hullTopBelow || fabs(pitch) > M.pitchAbsAbove || (hb.V < M.buoyancyBelow && t > M.minT))) {
+    P.foundered = 1;
+    P.founderT = t;
+  }
+  return double3{zO, pitch, roll};
+}
+
+// The load sums, the motion and the next pose (body.hpp:11-57, events.hpp:30-38), by one warp. The load terms of the
+// flooded nodes are in six columns a fixed stride apart from S.area, in node order, 32 nodes' at the front of their 32
+// places and their number in S.wet (team_step). Lanes 0 .. 5 each add one column: a lane reading all six, node by node,
+// took a dependent load and six adds for each of all the nodes, and an add takes 23 cycles.
+__device__ __forceinline__ void move_body(const DevModel& M, const Pose& F, Slot& S, int lane) {
   Parked& P = *S.parked;
   const Buoy hb = buoyancy_finish(S.hydro);
   const double Wg = M.rho * M.g;
@@ -1111,36 +1317,18 @@ __device__ __forceinline__ void move_body(const DevModel& M, const Pose& F, Slot
   if (lane == 2) sum = Fb - M.g * M.ms;
   {
     const double* t = S.area + (lane < 6 ? lane : 5) * (S.zmax - S.area);
-    const int NN = M.nn;
-#pragma unroll 8
-    for (int n = 0; n < NN; ++n) sum += t[n];
+#pragma unroll 1
+    for (int n0 = 0; n0 < M.nn; n0 += kLanes) {
+      const int wet = S.wet[n0 / kLanes];
+#pragma unroll 4
+      for (int k = 0; k < wet; ++k) sum += t[n0 + k];
+    }
   }
   const double tauX = __shfl_sync(kFull, sum, 0), tauY = __shfl_sync(kFull, sum, 1), Fz = __shfl_sync(kFull, sum, 2);
   const double mw = __shfl_sync(kFull, sum, 3), Iw_p = __shfl_sync(kFull, sum, 4), Iw_r = __shfl_sync(kFull, sum, 5);
-  const double Mth = tauY, Mph = tauX * F.cth;
-  const double dt = M.dt;
-  double vz = P.vz, wth = P.wth, wph = P.wph, zO = P.zO, pitch = P.pitch, roll = P.roll;
-  const double mh = M.mh0 + mw;
-  const double Ith = M.Ith0 + Iw_p, Iph = M.Iph0 + Iw_r;
-  const double az = (Fz - M.cDz * vz - M.qz * fabs(vz) * vz) / mh;
-  const double ath = (Mth - M.cDth * wth - M.qth * fabs(wth) * wth) / Ith;
-  const double aph = (Mph - M.cDph * wph - M.qph * fabs(wph) * wph) / Iph;
-  vz += az * dt; wth += ath * dt; wph += aph * dt;
-  zO += vz * dt; pitch += wth * dt; roll += wph * dt;
-  if (pitch > kPitchClamp) { pitch = kPitchClamp; wth = 0; }
-  if (pitch < -kPitchClamp) { pitch = -kPitchClamp; wth = 0; }
-  if (roll > kRollClamp) { roll = kRollClamp; wph = 0; }
-  if (roll < -kRollClamp) { roll = -kRollClamp; wph = 0; }
-  const double t = P.t + dt;
-  __syncwarp();  // the lanes have read the values they now replace
-  P.t = t; P.zO = zO; P.pitch = pitch; P.roll = roll; P.vz = vz; P.wth = wth; P.wph = wph;
-  P.inflow = seaIn / dt; P.Vb = hb.V; P.hullTop = hb.top; P.mw = mw;
-  P.bx = hb.x; P.by = hb.y; P.bz = hb.z;
-  if (!P.foundered && (hb.top < M.hullTopBelow || fabs(pitch) > M.pitchAbsAbove || (hb.V < M.buoyancyBelow && t > M.minT))) {
-    P.foundered = 1;
-    P.founderT = t;
-  }
-  *S.prev = make_pose(M, zO, pitch, roll);
+  const MotionIn in{tauX, tauY, Fz, mw, Iw_p, Iw_r, F.cth};
+  const double3 at = integrate_motion(M, P, in, hb);
+  *S.prev = make_pose(M, at.x, at.y, at.z);
 }
 
 // One step. On entry S.parked holds R's values and S.pose their pose; on return R, S.parked and S.pose are the next ones
@@ -1169,7 +1357,7 @@ __device__ __forceinline__ void team_step(const DevModel& M, SimRegs& R, Slot& S
 #pragma unroll 1
   for (int n = rank; n < M.nn; n += kStride) {
     const int flags = S.dry[n];
-    S.dry[n] = (Tape::kLazy && (flags & kEmptyNode)) ? kStale : 0;
+    S.dry[n] = Tape::kLazy ? ((flags & kEmptyNode) ? kStale : flags & kNoTop) : 0;
     if (flags & kEmptyNode) {
       S.area[n] = 0;
       if (flags & kZeroVolume) S.vol[n] = 0;
@@ -1201,13 +1389,15 @@ __device__ __forceinline__ void team_step(const DevModel& M, SimRegs& R, Slot& S
   }
   T.sync();
   // per-node gathers in increasing connection order, the volume update (flows.hpp:81-111) and, by the same thread, the
-  // node's terms of the loads (body.hpp:20-33), which overwrite arrays of which only this node's entries are still read
+  // node's terms of the loads (body.hpp:20-33), which overwrite arrays of which only these 32 nodes' entries are still read
+  // (and those before the ballot)
   {
     const double Wg = M.rho * M.g;
     const double zO = S.parked->zO;
 #pragma unroll 1
-    for (int n = rank; n < M.nn; n += kStride) {
-      const int k0 = __ldg(M.incStart + n), k1 = k0 + __ldg(M.incCount + n);
+    for (int n0 = T.warp * kLanes; n0 < M.nn; n0 += kStride) {
+      const int n = n0 + lane < M.nn ? n0 + lane : n0;
+      const int k0 = __ldg(M.incStart + n), k1 = n0 + lane < M.nn ? k0 + __ldg(M.incCount + n) : k0;
       double acc = 0;
 #pragma unroll 4
       for (int k = k0; k < k1; ++k) {
@@ -1220,30 +1410,34 @@ __device__ __forceinline__ void team_step(const DevModel& M, SimRegs& R, Slot& S
       const double vm = __ldg(M.vmax + n);
       double excess = 0;
       if (v > vm) {
-        // (a node that was empty at the solve has no extent yet)
-        const double zmax = (S.dry[n] & kStale) ? static_cast<double>(node_extreme<MIXED>(M, F, n, true, 0, 1)) : S.zmax[n];
+        // (a node that was empty at the solve, or whose solve did not need it, has no highest point yet)
+        const double zmax = (S.dry[n] & (kStale | kNoTop)) ? static_cast<double>(node_extreme<MIXED>(M, F, n, true, 0, 1)) : S.zmax[n];
         const double head = jmax(0.0, -zmax);
         const double cap = vm + __ldg(M.aov + n) * head;
         if (v > cap) { excess = v - cap; v = cap; }
       }
-      S.acc[n] = excess;
-      S.vol[n] = v;
-      double t0 = -0.0, t1 = -0.0, t2 = -0.0, t3 = -0.0, t4 = -0.0, t5 = -0.0;
-      if (!(v <= 0)) {
+      const bool mine = n0 + lane < M.nn, wet = mine && !(v <= 0);
+      const unsigned mask = __ballot_sync(kFull, wet);
+      if (lane == 0) S.wet[n0 / kLanes] = static_cast<std::uint8_t>(__popc(mask));
+      if (mine) {
+        S.acc[n] = excess;
+        S.vol[n] = v;
+      }
+      if (wet) {
         const double x = S.cx[n], y = S.cy[n], z = S.cz[n];
         const double wx = F.R00 * x + F.R01 * y + F.R02 * z + F.tx - M.XO;
         const double wy = F.R10 * x + F.R11 * y + F.R12 * z + F.ty - M.YO;
         const double wz = F.R20 * x + F.R21 * y + F.R22 * z + F.tz - zO;
         const double f = -Wg * v;
         const double m = M.rho * v;
-        t0 = wy * f;
-        t1 = -(wx * f);
-        t2 = f;
-        t3 = m;
-        t4 = m * (wx * wx + wz * wz);
-        t5 = m * (wy * wy + wz * wz);
+        const int at = n0 + __popc(mask & ((1u << lane) - 1u));
+        S.area[at] = wy * f;
+        S.zmax[at] = -(wx * f);
+        S.hEff[at] = f;
+        S.aEff[at] = m;
+        S.tmp[at] = m * (wx * wx + wz * wz);
+        S.term5[at] = m * (wy * wy + wz * wz);
       }
-      S.area[n] = t0; S.zmax[n] = t1; S.hEff[n] = t2; S.aEff[n] = t3; S.tmp[n] = t4; S.term5[n] = t5;
     }
   }
   T.sync();
@@ -1252,6 +1446,7 @@ __device__ __forceinline__ void team_step(const DevModel& M, SimRegs& R, Slot& S
     if (T.warp == W - 1) list_groups<true>(M, S, lane);
   }
   if (T.warp == kEventWarp<W>) step_events(M, F, tNow + M.dt, R.evCount, S, I, lane);
+  if (T.warp == (W > 2 ? 2 : W - 1)) sea_inflow(M, S, lane);
   T.sync();
   Pose* const last = S.pose;
   S.pose = S.prev;
