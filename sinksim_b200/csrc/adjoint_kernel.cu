@@ -43,18 +43,35 @@ struct AdjTeam {
     else asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(W * 32) : "memory");
   }
   __device__ __forceinline__ void add_int(int* p, int v) const { atomicAdd(p, v); }
-  // team-wide sums of K values (K <= 16), every thread receives them: each warp's sums in shared memory, then lane k
-  // of every warp adds value k over the warps (in warp order) and the lanes pass the K totals round by shuffles
-  __device__ __forceinline__ void reduce(double* v, int K, double* red) const {
-    for (int k = 0; k < K; ++k) {
-      double x = v[k];
-      for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
-      if (lane == 0) red[warp * 16 + k] = x;
+  // team-wide sums of K values (K <= 16), every thread receives them. The lanes' butterfly (offsets 16 .. 1) halves the
+  // values a lane carries at each of its first four offsets, so 31 exchanges do for 16 values instead of 80, with the same
+  // pairs at every offset and so the same bits; each warp's sums go through shared memory, lane k of every warp adds value
+  // k over the warps (in warp order) and the lanes pass the K totals round.
+  template <int K>
+  __device__ __forceinline__ void reduce(double (&v)[K], int, double* red) const {
+    static_assert(K <= 16, "at most 16 values");
+    double x[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) x[k] = k < K ? v[k] : 0.0;
+    int mine = 0;  // the value this lane ends with
+#pragma unroll
+    for (int off = 16, n = 16; off > 1; off >>= 1, n >>= 1) {
+      const bool upper = (lane & off) != 0;
+#pragma unroll
+      for (int k = 0; k < n / 2; ++k) {
+        const double keep = upper ? x[k + n / 2] : x[k], give = upper ? x[k] : x[k + n / 2];
+        x[k] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+      }
+      if (upper) mine += n / 2;
     }
+    x[0] += __shfl_xor_sync(0xffffffffu, x[0], 1);
+    if (mine < K && (lane & 1) == 0) red[warp * 16 + mine] = x[0];
     sync();
     double s = 0;
     if (lane < K)
-      for (int w = 0; w < nwarps; ++w) s += red[w * 16 + lane];
+#pragma unroll 4
+      for (int w = 0; w < W; ++w) s += red[w * 16 + lane];
+#pragma unroll
     for (int k = 0; k < K; ++k) v[k] = __shfl_sync(0xffffffffu, s, k);
     sync();
   }
@@ -232,34 +249,44 @@ __device__ __forceinline__ std::size_t store_record(const adj::Tape& tp, int nn,
   for (int n = T.rank; n <= nn; n += 32 * W) di[L.ints + n] = poff[n];
   double* dd = reinterpret_cast<double*>(dst + record_ints_bytes(L, nn));
   for (std::size_t i = T.rank; i < L.passes; i += 32 * W) dd[i] = tp.d[i];
-  constexpr int kPerNode = adj::kMaxPasses * adj::kPassFields;
-  for (int i = T.rank; i < nn * kPerNode; i += 32 * W) {
-    const int n = i / kPerNode, k = (i / adj::kPassFields) % adj::kMaxPasses, f = i % adj::kPassFields;
-    if (k < tp.i[L.npass + n]) dd[L.passes + static_cast<std::size_t>(poff[n] + k) * adj::kPassFields + f] = tp.d[L.passes + i];
+  // a round per pass number: nodes take one or two passes, so later rounds are empty and end the loop
+  for (int k = 0;; ++k) {
+    bool more = false;
+    for (int i = T.rank; i < nn * adj::kPassFields; i += 32 * W) {
+      const int n = i / adj::kPassFields, f = i % adj::kPassFields;
+      const int np = min(tp.i[L.npass + n], adj::kMaxPasses);
+      if (k < np) dd[L.passes + static_cast<std::size_t>(poff[n] + k) * adj::kPassFields + f] = tp.pass(n, k)[f];
+      more = more || k + 1 < np;
+    }
+    if (!__any_sync(0xffffffffu, more)) break;
   }
   const std::size_t bytes = record_bytes(L, nn, poff[nn]);
   T.sync();
   return bytes;
 }
 
-// Unpacks a record (global) into the step's tape in shared memory, in one round of loads and one barrier: the pass
-// records go to their slots by the record's own offsets; slots the step did not use are left as they are (the replay
-// reads only the used ones).
-template <int W>
-__device__ __forceinline__ void load_record(const unsigned char* src, const adj::Tape& tp, int nn, const Team<W>& T) {
-  const adj::TapeLayout& L = tp.L;
-  const std::int32_t* si = reinterpret_cast<const std::int32_t*>(src);
-  const std::int32_t* soff = si + L.ints;
-  for (std::size_t i = T.rank; i < L.ints; i += 32 * W) tp.i[i] = si[i];
-  const double* sd = reinterpret_cast<const double*>(src + record_ints_bytes(L, nn));
-  for (std::size_t i = T.rank; i < L.passes; i += 32 * W) tp.d[i] = sd[i];
-  constexpr int kPerNode = adj::kMaxPasses * adj::kPassFields;
-  for (int i = T.rank; i < nn * kPerNode; i += 32 * W) {
-    const int n = i / kPerNode, k = (i / adj::kPassFields) % adj::kMaxPasses, f = i % adj::kPassFields;
-    if (k < si[L.npass + n]) tp.d[L.passes + i] = sd[L.passes + static_cast<std::size_t>(soff[n] + k) * adj::kPassFields + f];
-  }
-  T.sync();
+// A packed record in memory as a tape.
+__device__ __forceinline__ adj::Tape packed_tape(unsigned char* rec, const adj::TapeLayout& L, int nn) {
+  adj::Tape t;
+  t.i = reinterpret_cast<std::int32_t*>(rec);
+  t.d = reinterpret_cast<double*>(rec + record_ints_bytes(L, nn));
+  t.L = L;
+  t.first = t.i + L.ints;
+  return t;
 }
+
+// Starts copying a record of `bytes` (global, 16-byte aligned, as is its size) into shared memory: 16-byte asynchronous
+// copies spread over the team. copies_done, then a team barrier, make it visible.
+template <int W>
+__device__ __forceinline__ void copy_record(const unsigned char* src, int bytes, unsigned char* dst, const Team<W>& T) {
+  const auto to = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+#pragma unroll 1
+  for (int k = T.rank * 16; k < bytes; k += 32 * W * 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + k), "l"(src + k) : "memory");
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // The step's inputs into its tape, before the step: the scalars and every node's state, pass counts cleared.
 template <int W>
@@ -446,41 +473,32 @@ __global__ void __launch_bounds__(W * 32, 16 / W) adjoint_batch(const __grid_con
       T.sync();
       const long long tRev = global_ns();
       tRecompute += tRev - tSeg;
-      bool staged = false;  // the record of step st is in the raw buffer (copied while step st + 1 was reversed)
+      // the record of step st is reversed where it was copied: into the tape's place, or (stageRecords) by turns there and
+      // into the raw buffer, each while the step after it is reversed
+      unsigned char* here = A.tape;
+      copy_record(ring + off[s1 - 1] % static_cast<long long>(B.arenaBytes), rb[s1 - 1], here, T);
       for (long long st = s1 - 1; st >= s0; --st) {
-        if (staged) {
-          asm volatile("cp.async.wait_all;" ::: "memory");  // this thread's copies; the barrier makes all of them visible
-          T.sync();
-          load_record(A.raw, sp, M.nn, T);
-        } else {
-          load_record(ring + off[st] % static_cast<long long>(B.arenaBytes), sp, M.nn, T);
-        }
-        staged = false;
+        copies_done();
+        T.sync();
+        const adj::Tape tp = packed_tape(here, TL, M.nn);
         if (st > s0) {
           const unsigned char* next = ring + off[st - 1] % static_cast<long long>(B.arenaBytes);
           if (B.stageRecords) {
-            // the next step's record (the one before this) into shared memory while this one is reversed: 16-byte
-            // asynchronous copies spread over the team (records and the buffer are 16-byte aligned, their sizes whole
-            // numbers of 16 bytes)
-            const int chunks = rb[st - 1] / 16;
-            for (int k = T.rank; k < chunks; k += 32 * W) {
-              const auto dst = static_cast<unsigned>(__cvta_generic_to_shared(A.raw + 16 * k));
-              asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(next + 16 * k) : "memory");
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            staged = true;
+            here = here == A.tape ? A.raw : A.tape;
+            copy_record(next, rb[st - 1], here, T);
           } else if (T.leader()) {
             // or at least into L2
             asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(next), "r"(static_cast<unsigned>(rb[st - 1])) : "memory");
           }
         }
-        adj::reverse_step(AT, M, sp, I.en(), I.area(), I.tOn(), A.rs, A.as, aSc, A.grad, &err);
+        adj::reverse_step(AT, M, tp, I.en(), I.area(), I.tOn(), A.rs, A.as, aSc, A.grad, &err);
         for (int q = 0; q < NS; ++q)
           if (static_cast<long long>(A.sampleS[q]) == st) {
             const double tr = B.trim[static_cast<std::size_t>(inst) * NS + q], hv = B.heave[static_cast<std::size_t>(inst) * NS + q];
-            add_sample_adjoint(M, sp.d[TL.scal + 1], sp.d[TL.scal + 2], sp.d[TL.scal + 3], 2 * (tr - trimT[q]), 2 * (hv - heaveT[q]), aSc);
+            add_sample_adjoint(M, tp.d[TL.scal + 1], tp.d[TL.scal + 2], tp.d[TL.scal + 3], 2 * (tr - trimT[q]), 2 * (hv - heaveT[q]), aSc);
           }
         T.sync();
+        if (!B.stageRecords && st > s0) copy_record(ring + off[st - 1] % static_cast<long long>(B.arenaBytes), rb[st - 1], here, T);
       }
       tReverse += global_ns() - tRev;
       if (--g < 0) break;
@@ -528,7 +546,7 @@ AdjLayout adjoint_layout(int nn, int nc, int ng, int nsamples, int W, bool withR
   A.aVol = take16(N); A.aLevel = take16(N); A.aCx = take16(N); A.aCy = take16(N); A.aCz = take16(N);
   A.grad = take16(C);
   A.sampleS = take16(sizeof(double) * static_cast<std::size_t>(std::max(nsamples, 1)));
-  A.tape = take16(adj::tape_layout(nn, ng).bytes);
+  A.tape = take16(std::max(adj::tape_layout(nn, ng).bytes, record_bytes(adj::tape_layout(nn, ng), nn, nn * adj::kMaxPasses)));
   A.poff = take16(sizeof(std::int32_t) * (static_cast<std::size_t>(std::max(nn, 1)) + 1));
   A.bytes = off;
   return A;

@@ -92,12 +92,17 @@ SSB_HD TapeLayout tape_layout(int nn, int ng) {
   return L;
 }
 
-// A step's tape in memory: doubles, then int32.
+// A step's tape in memory: doubles, then int32, with kMaxPasses places for every node's passes; or, with first set, a
+// packed record, in which node n's passes start at the first[n]-th (adjoint_kernel.cu).
 struct Tape {
   double* d;
   std::int32_t* i;
   TapeLayout L;
-  SSB_HD double* pass(int n, int k) const { return d + L.passes + (static_cast<std::size_t>(n) * kMaxPasses + k) * kPassFields; }
+  const std::int32_t* first = nullptr;
+  SSB_HD double* pass(int n, int k) const {
+    const std::size_t at = (first ? static_cast<std::size_t>(first[n]) : static_cast<std::size_t>(n) * kMaxPasses) + k;
+    return d + L.passes + at * kPassFields;
+  }
 };
 
 SSB_HD Tape tape_at(unsigned char* base, const TapeLayout& L) {
@@ -180,6 +185,33 @@ SSB_HD void trim_heave_reverse(const DevModel& M, double a_trim, double a_heave,
   aP.tz -= 2 * a_d;
 }
 
+// Calls f(xy, lo-hi pair, footprint) for the entries first, first + stride, ... below end of a table, in order; the loads
+// of four entries go out before the first is used: a team's L1 is small beside its tables, so every round of loads waits
+// for L2 (on B200 a 64-point gradient on the liner, two at a time: see adjoint_kernel.cu).
+template <class F>
+SSB_HD void each_entry(const double2* xy, const double2* ab, const double* area, int first, int end, int stride, F f) {
+  constexpr int kAhead = 4;
+  SSB_ROLLED
+  for (int j = first; j < end; j += kAhead * stride) {
+    double2 p[kAhead], q[kAhead];
+    double A[kAhead];
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+    for (int k = 0; k < kAhead; ++k) {
+      const int i = j + k * stride < end ? j + k * stride : j;
+      p[k] = xy[i];
+      q[k] = ab[i];
+      A[k] = area[i];
+    }
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+    for (int k = 0; k < kAhead; ++k)
+      if (j + k * stride < end) f(p[k], q[k], A[k], j + k * stride);
+  }
+}
+
 // ----------------------------------------------------------------------------- reductions over lanes
 
 // Inclusive prefix sum of v over the lanes 0 .. lane of the warp (width 1: v itself).
@@ -224,20 +256,12 @@ SSB_CALLED int pass_extreme(const DevModel& M, const PoseD& F, int n, bool want_
   if (width == 32) {
     double best = want_min ? 1e9 : -1e9;
     int idx = -1;
-    auto seg = [&](const double2 xy, const double2 ab, int j) {
+    auto seg = [&](const double2 xy, const double2 ab, double, int j) {
       const double base = F.R20 * xy.x + F.R21 * xy.y + F.tz;
       const double w = want_min ? base + F.R22 * ab.x : base + F.R22 * ab.y;
       if (want_min ? (w < best) : (w > best)) { best = w; idx = j; }
     };
-    // two segments per round, both loaded before either is compared; each lane keeps its segments' order
-    int j = s0 + lane;
-    SSB_ROLLED
-    for (; j + 32 < s1; j += 64) {
-      const double2 xy0 = M.segXY[j], ab0 = M.segLH[j], xy1 = M.segXY[j + 32], ab1 = M.segLH[j + 32];
-      seg(xy0, ab0, j);
-      seg(xy1, ab1, j + 32);
-    }
-    if (j < s1) seg(M.segXY[j], M.segLH[j], j);
+    each_entry(M.segXY, M.segLH, M.segAr, s0 + lane, s1, 32, seg);
     for (int off = 16; off > 0; off >>= 1) {
       const double ob = __shfl_xor_sync(0xffffffffu, best, off);
       const int oi = __shfl_xor_sync(0xffffffffu, idx, off);
@@ -290,7 +314,7 @@ SSB_CALLED double pass_sweep1(const DevModel& M, const PoseD& F, int n, double h
   const int s0 = M.segStart[n], s1 = s0 + M.segCount[n];
   const double mu = M.mu[n];
   double aR20 = 0, aR21 = 0, atz = 0, aiR = 0, ah = 0;
-  auto seg = [&](const double2 xy, const double2 ab, const double A) {
+  auto seg = [&](const double2 xy, const double2 ab, const double A, int) {
     const double base = F.R20 * xy.x + F.R21 * xy.y + F.tz;
     const double zp = (h - base) * F.iR;
     if (!(zp > ab.x && zp < ab.y)) return;
@@ -301,16 +325,7 @@ SSB_CALLED double pass_sweep1(const DevModel& M, const PoseD& F, int n, double h
     const double abase = -aL * F.iR;
     aR20 += abase * xy.x; aR21 += abase * xy.y; atz += abase;
   };
-  // two segments per round, both loaded before either is used; each lane still visits its segments in order
-  int j = s0 + lane;
-  SSB_ROLLED
-  for (; j + width < s1; j += 2 * width) {
-    const double2 xy0 = M.segXY[j], ab0 = M.segLH[j], xy1 = M.segXY[j + width], ab1 = M.segLH[j + width];
-    const double A0 = M.segAr[j], A1 = M.segAr[j + width];
-    seg(xy0, ab0, A0);
-    seg(xy1, ab1, A1);
-  }
-  if (j < s1) seg(M.segXY[j], M.segLH[j], M.segAr[j]);
+  each_entry(M.segXY, M.segLH, M.segAr, s0 + lane, s1, width, seg);
   aP.R20 += aR20; aP.R21 += aR21; aP.tz += atz; aP.iR += aiR;
   return ah;
 }
@@ -322,7 +337,7 @@ SSB_CALLED void pass_sweep_levels(const DevModel& M, const PoseD& F, int n, int 
   const int s0 = M.segStart[n], s1 = s0 + M.segCount[n];
   const double mu = M.mu[n];
   double aR20 = 0, aR21 = 0, atz = 0, aiR = 0;
-  auto seg = [&](const double2 xy, const double2 ab, const double A) {
+  auto seg = [&](const double2 xy, const double2 ab, const double A, int) {
     const double base = F.R20 * xy.x + F.R21 * xy.y + F.tz;
     SSB_ROLLED
     for (int i = 0; i < np; ++i) {
@@ -334,15 +349,7 @@ SSB_CALLED void pass_sweep_levels(const DevModel& M, const PoseD& F, int n, int 
       aR20 += abase * xy.x; aR21 += abase * xy.y; atz += abase;
     }
   };
-  int j = s0 + lane;
-  SSB_ROLLED
-  for (; j + width < s1; j += 2 * width) {
-    const double2 xy0 = M.segXY[j], ab0 = M.segLH[j], xy1 = M.segXY[j + width], ab1 = M.segLH[j + width];
-    const double A0 = M.segAr[j], A1 = M.segAr[j + width];
-    seg(xy0, ab0, A0);
-    seg(xy1, ab1, A1);
-  }
-  if (j < s1) seg(M.segXY[j], M.segLH[j], M.segAr[j]);
+  each_entry(M.segXY, M.segLH, M.segAr, s0 + lane, s1, width, seg);
   aP.R20 += aR20; aP.R21 += aR21; aP.tz += atz; aP.iR += aiR;
 }
 
@@ -351,7 +358,7 @@ SSB_CALLED void pass_sweep_levels(const DevModel& M, const PoseD& F, int n, int 
 SSB_CALLED void buoyancy_sweep(const DevModel& M, const PoseD& F, double aV, double aMx, double aMy, double aMz, int first, int stride,
                            AdjPose& aP) {
   double aR20 = 0, aR21 = 0, atz = 0, aiR = 0;
-  auto col = [&](const double2 xy, const double2 lh, const double A) {
+  auto col = [&](const double2 xy, const double2 lh, const double A, int) {
     const double base = F.R20 * xy.x + F.R21 * xy.y + F.tz;
     const double zp = -base * F.iR;
     if (!(zp > lh.x && zp < lh.y)) return;
@@ -361,16 +368,7 @@ SSB_CALLED void buoyancy_sweep(const DevModel& M, const PoseD& F, double aV, dou
     const double abase = -as * F.iR;
     aR20 += abase * xy.x; aR21 += abase * xy.y; atz += abase;
   };
-  // two columns per round, both loaded before either is used; each thread keeps its columns' order
-  int i = first;
-  SSB_ROLLED
-  for (; i + stride < M.ncol; i += 2 * stride) {
-    const double2 xy0 = M.colXY[i], lh0 = M.colLH[i], xy1 = M.colXY[i + stride], lh1 = M.colLH[i + stride];
-    const double A0 = M.colA[i], A1 = M.colA[i + stride];
-    col(xy0, lh0, A0);
-    col(xy1, lh1, A1);
-  }
-  if (i < M.ncol) col(M.colXY[i], M.colLH[i], M.colA[i]);
+  each_entry(M.colXY, M.colLH, M.colA, first, M.ncol, stride, col);
   aP.R20 += aR20; aP.R21 += aR21; aP.tz += atz; aP.iR += aiR;
 }
 
@@ -986,6 +984,35 @@ SSB_HD void loads_node_reverse(const DevModel& M, const PoseD& F, double zO, dou
   aZo -= aWz;
 }
 
+// Group g's members, their number and the first two: on the device from the model's list entry (one load), where it holds
+// them.
+struct Members {
+  int N, n0, n1;
+  const int* m;
+  SSB_HD int operator[](int k) const { return k == 0 ? n0 : (k == 1 ? n1 : m[k]); }
+};
+
+SSB_HD Members members_of(const DevModel& M, int g) {
+  Members r;
+  r.m = M.gNodes;
+#if defined(__CUDA_ARCH__)
+  const uint2 e = *reinterpret_cast<const uint2*>(M.groupEntry + g);
+  r.n0 = static_cast<int>(e.x >> 16);
+  r.n1 = static_cast<int>(e.y & 0xffff);
+  r.N = static_cast<int>((e.y >> 16) & 0xff);
+  if (r.N > 2) {
+    r.m = M.gNodes + M.gStart[g];
+    r.N = M.gCount[g];
+  }
+#else
+  r.m = M.gNodes + M.gStart[g];
+  r.N = M.gCount[g];
+  r.n0 = r.N > 0 ? r.m[0] : 0;
+  r.n1 = r.N > 1 ? r.m[1] : r.n0;
+#endif
+  return r;
+}
+
 // ----------------------------------------------------------------------------- the reverse of one step
 
 #if defined(__CUDACC__)
@@ -1168,9 +1195,9 @@ SSB_HDT bool reverse_step(const T& team, const DevModel& M, const Tape& tp, cons
         if (merged[g]) {
           c = 1;
         } else {
-          const int* mem = M.gNodes + M.gStart[g];
+          const Members mem = members_of(M, g);
           SSB_ROLLED
-          for (int k = 0; k < M.gCount[g]; ++k) {
+          for (int k = 0; k < mem.N; ++k) {
             const int n = mem[k];
             S.plain[n] = tp.d[L.volIn + n] <= kEmptyVolume && tp.i[L.npass + n] == 1 && tp.pass(n, 0)[0] == tp.d[L.levelIn + n] &&
                          S.aLs[n] == 0 && S.aZmx[n] == 0;
@@ -1190,9 +1217,9 @@ SSB_HDT bool reverse_step(const T& team, const DevModel& M, const Tape& tp, cons
         if (merged[g]) {
           S.units[at] = (g << 16) | 0xffff;
         } else {
-          const int* mem = M.gNodes + M.gStart[g];
+          const Members mem = members_of(M, g);
           SSB_ROLLED
-          for (int k = 0; k < M.gCount[g]; ++k)
+          for (int k = 0; k < mem.N; ++k)
             if (!S.plain[mem[k]]) S.units[at++] = (g << 16) | k;
         }
       }
