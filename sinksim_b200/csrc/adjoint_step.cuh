@@ -36,7 +36,8 @@
 // Loops whose bodies the compiler would copy four times over, and functions called from several places: the reverse
 // issues a long straight run of code once per step, which has to come from the instruction caches. With one call site of
 // the forward step (adjoint_kernel.cu) the kernel is 310 KB of code instead of 940; on B200 a 64-point gradient on the
-// liner to 400 s takes 107 ms against 111, 3 points on titanic64 51 against 58.
+// liner to 400 s takes 107 ms against 111, 3 points on titanic64 51 against 58. What adds to the pose adjoint is inlined all
+// the same: called, it keeps the adjoint's 14 sums in local memory (105 ms against 98 with the other steps since).
 #if defined(__CUDA_ARCH__)
 #define SSB_ROLLED _Pragma("unroll 1")
 #else
@@ -187,7 +188,7 @@ SSB_HD void trim_heave_reverse(const DevModel& M, double a_trim, double a_heave,
 
 // Calls f(xy, lo-hi pair, footprint) for the entries first, first + stride, ... below end of a table, in order; the loads
 // of four entries go out before the first is used: a team's L1 is small beside its tables, so every round of loads waits
-// for L2 (on B200 a 64-point gradient on the liner, two at a time: see adjoint_kernel.cu).
+// for L2 (on B200 a 64-point gradient on the liner to 400 s 98.4 ms, 99.0 with two at a time).
 template <class F>
 SSB_HD void each_entry(const double2* xy, const double2* ab, const double* area, int first, int end, int stride, F f) {
   constexpr int kAhead = 4;
@@ -309,7 +310,7 @@ SSB_HD void extreme_reverse(const DevModel& M, int j, bool bottom, double a_w, A
 // moments: adds the pose adjoint to aP and returns this lane's share of d(outputs)/d h (sum over the warp's lanes for
 // the total). Only segments the level cuts contribute (kernel/reduce.hpp:52-71: a full segment's height is b - a, a dry
 // one adds nothing).
-SSB_CALLED double pass_sweep1(const DevModel& M, const PoseD& F, int n, double h, double av, double amx, double amy, double amz, int lane, int width,
+SSB_HD double pass_sweep1(const DevModel& M, const PoseD& F, int n, double h, double av, double amx, double amy, double amz, int lane, int width,
                           AdjPose& aP) {
   const int s0 = M.segStart[n], s1 = s0 + M.segCount[n];
   const double mu = M.mu[n];
@@ -332,7 +333,7 @@ SSB_CALLED double pass_sweep1(const DevModel& M, const PoseD& F, int n, double h
 
 // The pose adjoint of np passes of node n at levels h[i] whose vol has the adjoint av[i] and whose moments have none
 // (their level adjoints are not needed).
-SSB_CALLED void pass_sweep_levels(const DevModel& M, const PoseD& F, int n, int np, const double* h, const double* av, int lane, int width,
+SSB_HD void pass_sweep_levels(const DevModel& M, const PoseD& F, int n, int np, const double* h, const double* av, int lane, int width,
                               AdjPose& aP) {
   const int s0 = M.segStart[n], s1 = s0 + M.segCount[n];
   const double mu = M.mu[n];
@@ -355,7 +356,7 @@ SSB_CALLED void pass_sweep_levels(const DevModel& M, const PoseD& F, int n, int 
 
 // Reverse of the buoyancy integral (kernel/reduce.hpp:39-49) over this thread's columns first, first + stride, ...: the
 // adjoints of V, Mx, My, Mz into the pose adjoint. A column cut by the waterplane contributes through its wet height.
-SSB_CALLED void buoyancy_sweep(const DevModel& M, const PoseD& F, double aV, double aMx, double aMy, double aMz, int first, int stride,
+SSB_HD void buoyancy_sweep(const DevModel& M, const PoseD& F, double aV, double aMx, double aMy, double aMz, int first, int stride,
                            AdjPose& aP) {
   double aR20 = 0, aR21 = 0, atz = 0, aiR = 0;
   auto col = [&](const double2 xy, const double2 lh, const double A, int) {
@@ -740,6 +741,106 @@ SSB_HD bool unit_reverse(const DevModel& M, const PoseD& F, const Tape& t, UnitW
     for (int k = 0; k < N; ++k) u.oVol[k] += w.aV;
   }
   return true;
+}
+
+// Whether single_reverse covers a unit: a node alone, empty, full or solved by Newton steps only.
+SSB_HD bool is_plain_single(const Replay& r) {
+  if (!r.single) return false;
+  if (r.cs == 2)
+    SSB_ROLLED
+    for (int j = r.base; j < r.K; ++j)
+      if (!r.newton[j]) return false;
+  return true;
+}
+
+// unit_reverse for a node alone without a bisection, operation for operation, but with the chain in every lane's registers:
+// unit_reverse keeps it in shared memory, where lane 0 works alone between warp syncs and each operation waits for the
+// last one's store (on B200, with the sweeps inlined: 64 points on the liner to 400 s 98 ms against 105, 320 points to
+// 150 s 105 against 117). in holds the solved values' adjoints (level, area, cx, cy, cz, vol, zmax), out receives the start's
+// (vol, level, cx, cy, cz).
+SSB_HD void single_reverse(const DevModel& M, const PoseD& F, const Tape& t, const Replay& r, UnitWork& w, const double* in, double* out, int lane,
+                           int width, AdjPose& aP) {
+  const int n = r.members[0], K = r.K;
+  double aV = 0, aLo = 0, aHi = 0, aH0 = 0, aZmin = 0, aZmax = in[6];
+  double av = 0, amx = 0, amy = 0, amz = 0, aArea = 0;
+  double oCx = 0, oCy = 0, oCz = 0;
+  int np = 0;
+  if (r.cs == 0) {
+    aZmin += in[0];
+    aV += in[5];
+    oCx += in[2]; oCy += in[3]; oCz += in[4];
+  } else {
+    const double* p = rec(t, n, r.cs == 1 ? 1 : K);
+    double ah = 0;
+    if (r.cs == 1) {
+      double aSum = 0, aDh = 0;
+      aSum += M.aov[n];
+      aDh += in[0];
+      aHi += in[0];
+      aV = in[5];
+      if (r.V - r.Vmax > 0) aV += aDh / aSum;
+    } else {
+      ah += in[0];
+      aArea += in[1];
+      aV += in[5];
+    }
+    centroid_reverse(p, in[2], in[3], in[4], av, amx, amy, amz, oCx, oCy, oCz);
+    const double a1 = lane_sum(pass_sweep1(M, F, n, p[0], av, amx, amy, amz, lane, width, aP), width);
+    if (r.cs == 1) {
+      aHi += a1;
+    } else {
+      ah += a1;
+      // the Newton updates, last first
+      SSB_ROLLED
+      for (int j = K - 1; j >= r.base; --j) {
+        const double* q = rec(t, n, j);
+        double e = 0, dvs = 0;
+        e += q[1]; dvs += q[2];
+        e = e - r.V;
+        const double aErr = -ah / dvs;
+        const double aDvs = ah * e / (dvs * dvs);
+        aV -= aErr;
+        if (lane == 0) { w.av[0][j] = aErr; w.adv[0][j] = aDvs; }
+        ah += aErr * q[2];
+      }
+      if (r.base == 1) {
+        if (r.startSrc == kSrcLo) aLo += ah; else aHi += ah;
+      } else {
+        aH0 += ah;
+      }
+      if (K > r.base) {
+        // the passes before the final one whose volume the chain reached, for the sweep of their pose adjoints
+        warp_sync();
+        SSB_ROLLED
+        for (int j = r.base; j < K; ++j) {
+          const double a = w.av[0][j];
+          if (a == 0) continue;
+          if (lane == 0) { w.hs[0][np] = rec(t, n, j)[0]; w.pv[0][np] = a; }
+          ++np;
+        }
+        warp_sync();
+      }
+    }
+    aZmin += aLo;
+    aZmax += aHi;
+  }
+  if (np) pass_sweep_levels(M, F, n, np, w.hs[0], w.pv[0], lane, width, aP);
+  if (aZmin != 0) {
+    const int j = pass_extreme(M, F, n, true, lane, width);
+    if (lane == 0) extreme_reverse(M, j, true, aZmin, aP);
+  }
+  if (aZmax != 0) {
+    const int j = pass_extreme(M, F, n, false, lane, width);
+    if (lane == 0) extreme_reverse(M, j, false, aZmax, aP);
+  }
+  if (lane == 0 && r.cs == 2) {
+    SSB_ROLLED
+    for (int j = r.base; j <= K; ++j) {
+      const double a = j == K ? aArea : w.adv[0][j];
+      if (a != 0) aP.iR += a * rec(t, n, j)[2] / F.iR;
+    }
+  }
+  out[0] = 0.0 + aV; out[1] = 0.0 + aH0; out[2] = oCx; out[3] = oCy; out[4] = oCz;
 }
 
 // ----------------------------------------------------------------------------- flows
@@ -1259,6 +1360,15 @@ SSB_HDT bool reverse_step(const T& team, const DevModel& M, const Tape& tp, cons
       const int* um = isMerged ? mem : mem + u;
       const int un = isMerged ? N : 1;
       if (un > kMaxMembers) { ok = false; *err |= kErrGroupSize; continue; }
+      if (S.replays[i].ok && is_plain_single(S.replays[i])) {
+        const int n = um[0];
+        const double in[7] = {S.aLs[n], S.aAs[n], S.aCxs[n], S.aCys[n], S.aCzs[n], S.aVs[n], S.aZmx[n]};
+        double out[5];
+        single_reverse(M, F, tp, S.replays[i], w, in, out, team.lane, team.width, aP);
+        if (team.lane == 0) { a.aVol[n] = out[0]; a.aLevel[n] = out[1]; a.aCx[n] = out[2]; a.aCy[n] = out[3]; a.aCz[n] = out[4]; }
+        warp_sync();  // every lane is done with the work area
+        continue;
+      }
       // the unit's replay into the warp's work area, a word per lane
       {
         const auto* src = reinterpret_cast<const std::int32_t*>(&S.replays[i]);
