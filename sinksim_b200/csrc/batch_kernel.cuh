@@ -29,7 +29,7 @@ constexpr int kStageWaitLimit = 1 << 20;
 // units; the rest, under 16 bytes, by plain copies) completing on an mbarrier after the table, and every thread waits
 // for the barrier's phase with a bounded number of try_wait rounds. Returns dst, or null when the wait ran out (the
 // health bit kHealthStageTimeout is set and the block reads the table from global memory). Every thread of the block
-// calls it once, before the teams diverge. The sources are cudaMalloc'd arrays, so 256-byte aligned.
+// calls it once, before the teams diverge. The sources are 256-byte aligned (TablePack).
 template <class T>
 __device__ const unsigned char* stage_column_table(const typename Vec2<T>::type* xy, const typename Vec2<T>::type* lh, const T* area, int ncol,
                                                    unsigned char* dst, std::int32_t* error) {

@@ -5,9 +5,11 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <memory>
 #include <stdexcept>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -97,6 +99,29 @@ inline SlotLayout slot_layout(std::int32_t NN, std::int32_t NC, std::int32_t NG,
   return L;
 }
 
+// Tables of one model put together on the host and copied to the device in one piece (a model has some fifty, and an
+// allocation and a copy of each cost more than building them); every table starts at a multiple of 256 bytes.
+class TablePack {
+ public:
+  template <class T>
+  void add(const T*& slot, const std::vector<T>& v) {
+    const std::size_t at = (host_.size() + 255) & ~static_cast<std::size_t>(255);
+    host_.resize(at + std::max<std::size_t>(v.size() * sizeof(T), 1));
+    if (!v.empty()) std::memcpy(host_.data() + at, v.data(), v.size() * sizeof(T));
+    places_.push_back({reinterpret_cast<const void**>(&slot), at});
+  }
+  // Copies the tables into `to` and points the slots at them.
+  void upload(DevBuf<unsigned char>& to, cudaStream_t s) {
+    to.upload(host_, s);
+    check(cudaStreamSynchronize(s), "model upload");
+    for (const auto& p : places_) *p.first = to.get() + p.second;
+  }
+
+ private:
+  std::vector<unsigned char> host_;
+  std::vector<std::pair<const void**, std::size_t>> places_;
+};
+
 // One compiled model on the device: its geometry in the kernel's layout (paired fields, the segment -> column gather
 // resolved, float copies), its node, group, connection, incidence, monitor and mark tables, and the DevModel that
 // points into them.
@@ -106,15 +131,7 @@ struct ModelDev {
   Incidence inc;
   MonitorLists mons;
   std::int32_t NN = 0, NC = 0, NG = 0, nmon = 0, nmark = 0, evCap = 0, maxGroup = 0;
-  DevBuf<double2> colXY, colLH, segXY, segLH, exXY;
-  DevBuf<float2> colXYf, colLHf, segXYf, segLHf, exXYf;
-  DevBuf<float> colAf, segArf, exZf;
-  DevBuf<double> colA, segAr, exZ, mu, vmax, amin, aov;
-  DevBuf<std::int32_t> exStart, incEdge, segStart, segCount, gStart, gCount, gNodes, ca, cb, skip, incStart, incCount, incConn, sea, monStart, monCount, monConn;
-  DevBuf<int2> nodeSeg;
-  DevBuf<Listed> groupEntry;
-  DevBuf<std::uint8_t> gMode, law, incSide, mkWhen;
-  DevBuf<double> gpx, gpy, gpz, kx, ky, kz, coef, mkx, mky, mkz;
+  DevBuf<unsigned char> tables;
   DevModel dm{};
 
   ModelDev(std::shared_ptr<const CompiledShip> s, const CompiledSim& m) : ship(std::move(s)), sim(m) {
@@ -128,6 +145,8 @@ struct ModelDev {
 
   void upload(cudaStream_t s) {
     const CompiledShip& S = *ship;
+    DevModel& d = dm;
+    TablePack pack;
     const CompiledSim& M = sim;
     {
       const std::size_t nc = S.x.size(), ns = S.segCol.size();
@@ -151,10 +170,10 @@ struct ModelDev {
         slhf[j] = float2{static_cast<float>(S.segA[j]), static_cast<float>(S.segE[j])};
         saf[j] = static_cast<float>(S.dxdy[c]);
       }
-      colXY.upload(cxy, s); colLH.upload(clh, s); colA.upload(S.dxdy, s);
-      colXYf.upload(cxyf, s); colLHf.upload(clhf, s); colAf.upload(caf, s);
-      segXY.upload(sxy, s); segLH.upload(slh, s); segAr.upload(sa, s);
-      segXYf.upload(sxyf, s); segLHf.upload(slhf, s); segArf.upload(saf, s);
+      pack.add(d.colXY, cxy); pack.add(d.colLH, clh); pack.add(d.colA, S.dxdy);
+      pack.add(d.colXYf, cxyf); pack.add(d.colLHf, clhf); pack.add(d.colAf, caf);
+      pack.add(d.segXY, sxy); pack.add(d.segLH, slh); pack.add(d.segAr, sa);
+      pack.add(d.segXYf, sxyf); pack.add(d.segLHf, slhf); pack.add(d.segArf, saf);
       // extent lists: set n < NN the segments of node n, set NN the hull's columns (points ns and up; tops only)
       std::vector<std::int32_t> first(S.segStart), number(S.segCount);
       first.push_back(static_cast<std::int32_t>(ns));
@@ -177,15 +196,14 @@ struct ModelDev {
           ezf[k] = static_cast<float>(ez[k]);
         }
       }
-      exStart.upload(lists.start, s); exXY.upload(exy, s); exZ.upload(ez, s); exXYf.upload(exyf, s); exZf.upload(ezf, s);
-      check(cudaStreamSynchronize(s), "stream sync");
+      pack.add(d.exStart, lists.start); pack.add(d.exXY, exy); pack.add(d.exZ, ez); pack.add(d.exXYf, exyf); pack.add(d.exZf, ezf);
     }
-    mu.upload(S.mu, s); vmax.upload(S.vmax, s); amin.upload(S.amin, s); aov.upload(S.aov, s);
+    pack.add(d.mu, S.mu); pack.add(d.vmax, S.vmax); pack.add(d.amin, S.amin); pack.add(d.aov, S.aov);
     std::vector<int2> ns(static_cast<std::size_t>(NN));
     for (std::size_t n = 0; n < ns.size(); ++n) ns[n] = int2{S.segStart[n], S.segCount[n]};
-    nodeSeg.upload(ns, s);
-    segStart.upload(S.segStart, s); segCount.upload(S.segCount, s);
-    gStart.upload(M.gNodeStart, s); gCount.upload(M.gNodeCount, s); gNodes.upload(M.gNodes, s); gMode.upload(M.gMode, s);
+    pack.add(d.nodeSeg, ns);
+    pack.add(d.segStart, S.segStart); pack.add(d.segCount, S.segCount);
+    pack.add(d.gStart, M.gNodeStart); pack.add(d.gCount, M.gNodeCount); pack.add(d.gNodes, M.gNodes); pack.add(d.gMode, M.gMode);
     std::vector<Listed> entry(static_cast<std::size_t>(NG));
     for (std::size_t g = 0; g < entry.size(); ++g) {
       const std::int32_t* m = M.gNodes.data() + M.gNodeStart[g];
@@ -194,46 +212,28 @@ struct ModelDev {
       entry[g] = Listed{static_cast<std::uint16_t>(g), static_cast<std::uint16_t>(first), static_cast<std::uint16_t>(N > 1 ? m[1] : first),
                         static_cast<std::uint8_t>(std::min(N, 255)), M.gMode[g]};
     }
-    groupEntry.upload(entry, s);
-    gpx.upload(M.gpx, s); gpy.upload(M.gpy, s); gpz.upload(M.gpz, s);
-    ca.upload(M.ca, s); cb.upload(M.cb, s); skip.upload(M.cSkipGroup, s); law.upload(M.cLaw, s);
-    kx.upload(M.cx, s); ky.upload(M.cy, s); kz.upload(M.cz, s); coef.upload(M.cCoef, s);
-    incStart.upload(inc.start, s); incCount.upload(inc.count, s); incConn.upload(inc.conn, s); incSide.upload(inc.side, s);
+    pack.add(d.groupEntry, entry);
+    pack.add(d.gpx, M.gpx); pack.add(d.gpy, M.gpy); pack.add(d.gpz, M.gpz);
+    pack.add(d.ca, M.ca); pack.add(d.cb, M.cb); pack.add(d.skip, M.cSkipGroup); pack.add(d.law, M.cLaw);
+    pack.add(d.kx, M.cx); pack.add(d.ky, M.cy); pack.add(d.kz, M.cz); pack.add(d.coef, M.cCoef);
+    pack.add(d.incStart, inc.start); pack.add(d.incCount, inc.count); pack.add(d.incConn, inc.conn); pack.add(d.incSide, inc.side);
     std::vector<std::int32_t> edge(inc.conn.size());
     for (std::size_t k = 0; k < edge.size(); ++k) edge[k] = 2 * inc.conn[k] + (inc.side[k] ? 1 : 0);
-    incEdge.upload(edge, s);
-    sea.upload(inc.sea.empty() ? std::vector<std::int32_t>{0} : inc.sea, s);
-    monStart.upload(mons.start.empty() ? std::vector<std::int32_t>{0} : mons.start, s);
-    monCount.upload(mons.count.empty() ? std::vector<std::int32_t>{0} : mons.count, s);
-    monConn.upload(mons.conn.empty() ? std::vector<std::int32_t>{0} : mons.conn, s);
-    mkx.upload(M.mkx.empty() ? std::vector<double>{0} : M.mkx, s);
-    mky.upload(M.mky.empty() ? std::vector<double>{0} : M.mky, s);
-    mkz.upload(M.mkz.empty() ? std::vector<double>{0} : M.mkz, s);
-    mkWhen.upload(M.mkWhen.empty() ? std::vector<std::uint8_t>{0} : M.mkWhen, s);
-    check(cudaStreamSynchronize(s), "model upload");
+    pack.add(d.incEdge, edge);
+    pack.add(d.sea, inc.sea.empty() ? std::vector<std::int32_t>{0} : inc.sea);
+    pack.add(d.monStart, mons.start.empty() ? std::vector<std::int32_t>{0} : mons.start);
+    pack.add(d.monCount, mons.count.empty() ? std::vector<std::int32_t>{0} : mons.count);
+    pack.add(d.monConn, mons.conn.empty() ? std::vector<std::int32_t>{0} : mons.conn);
+    pack.add(d.mkx, M.mkx.empty() ? std::vector<double>{0} : M.mkx);
+    pack.add(d.mky, M.mky.empty() ? std::vector<double>{0} : M.mky);
+    pack.add(d.mkz, M.mkz.empty() ? std::vector<double>{0} : M.mkz);
+    pack.add(d.mkWhen, M.mkWhen.empty() ? std::vector<std::uint8_t>{0} : M.mkWhen);
+    pack.upload(tables, s);
 
-    DevModel& d = dm;
-    d.ncol = S.columns();
-    d.colXY = colXY.get(); d.colLH = colLH.get(); d.colA = colA.get();
-    d.colXYf = colXYf.get(); d.colLHf = colLHf.get(); d.colAf = colAf.get();
-    d.nseg = S.segments();
-    d.segXY = segXY.get(); d.segLH = segLH.get(); d.segAr = segAr.get();
-    d.segXYf = segXYf.get(); d.segLHf = segLHf.get(); d.segArf = segArf.get();
-    d.exStart = exStart.get(); d.exXY = exXY.get(); d.exZ = exZ.get(); d.exXYf = exXYf.get(); d.exZf = exZf.get();
-    d.nn = NN;
-    d.mu = mu.get(); d.vmax = vmax.get(); d.amin = amin.get(); d.aov = aov.get();
-    d.segStart = segStart.get(); d.segCount = segCount.get(); d.nodeSeg = nodeSeg.get();
-    d.ng = NG;
-    d.gStart = gStart.get(); d.gCount = gCount.get(); d.gNodes = gNodes.get(); d.gMode = gMode.get(); d.groupEntry = groupEntry.get();
-    d.gpx = gpx.get(); d.gpy = gpy.get(); d.gpz = gpz.get(); d.gMargin = M.gMargin; d.maxGroup = maxGroup;
-    d.nc = NC;
-    d.ca = ca.get(); d.cb = cb.get(); d.skip = skip.get(); d.law = law.get();
-    d.kx = kx.get(); d.ky = ky.get(); d.kz = kz.get(); d.coef = coef.get();
-    d.incStart = incStart.get(); d.incCount = incCount.get(); d.incConn = incConn.get(); d.incSide = incSide.get(); d.incEdge = incEdge.get();
-    d.nsea = static_cast<std::int32_t>(inc.sea.size()); d.sea = sea.get();
-    d.nmon = nmon; d.monThreshold = M.monitorThreshold;
-    d.monStart = monStart.get(); d.monCount = monCount.get(); d.monConn = monConn.get();
-    d.nmark = nmark; d.mkx = mkx.get(); d.mky = mky.get(); d.mkz = mkz.get(); d.mkWhen = mkWhen.get();
+    d.ncol = S.columns(); d.nseg = S.segments(); d.nn = NN; d.ng = NG; d.nc = NC;
+    d.gMargin = M.gMargin; d.maxGroup = maxGroup;
+    d.nsea = static_cast<std::int32_t>(inc.sea.size());
+    d.nmon = nmon; d.monThreshold = M.monitorThreshold; d.nmark = nmark;
     d.hullTopBelow = M.hullTopBelow; d.pitchAbsAbove = M.pitchAbsAbove; d.buoyancyBelow = M.buoyancyBelow; d.minT = M.minT;
     d.rho = M.rho; d.g = M.g; d.sq2g = std::sqrt(2 * M.g); d.dt = M.dt;
     d.ms = M.body[0]; d.g0x = M.body[2]; d.g0y = M.body[3]; d.g0z = M.body[4]; d.XO = M.body[5]; d.YO = M.body[6];
