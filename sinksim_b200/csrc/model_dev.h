@@ -182,7 +182,8 @@ struct ModelDev {
       auto lh = [&](std::int32_t i) { const auto k = static_cast<std::size_t>(i); return k < ns ? slh[k] : clh[k - ns]; };
       const ExtentLists lists = extent_lists(
           first, number, [&](std::int32_t i) { return xy(i).x; }, [&](std::int32_t i) { return xy(i).y; },
-          [&](std::int32_t i) { return lh(i).x; }, [&](std::int32_t i) { return lh(i).y; });
+          [&](std::int32_t i) { return lh(i).x; }, [&](std::int32_t i) { return lh(i).y; },
+          static_cast<std::size_t>(NN));
       std::vector<double2> exy(lists.idx.size());
       std::vector<float2> exyf(lists.idx.size());
       std::vector<double> ez(lists.idx.size());
