@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(W * 32, 16 / W) adjoint_batch(const __grid_con
     if (T.leader()) {
       const int q = atomicAdd(B.queue, 1);
       S.misc[kMiscInstance] = B.order == nullptr || q >= B.count ? q : B.order[q];
-      S.misc[kMiscTaken] = W * (32 / kLevelLanes<false>);  // the level solve's list counter for the first step (team_step resets it)
+      S.misc[kMiscTaken] = W * (32 / kLevelLanes<false, W>);  // the level solve's list counter for the first step (team_step resets it)
     }
     T.sync();
     const int inst = S.misc[kMiscInstance];

@@ -88,12 +88,12 @@ __device__ __forceinline__ void write_record(double* rec, const SimRegs& R, cons
     rec[0] = R.t; rec[1] = R.zO; rec[2] = R.pitch; rec[3] = R.roll; rec[4] = R.vz; rec[5] = R.wth; rec[6] = R.wph;
     rec[7] = R.inflow; rec[8] = R.Vb; rec[9] = R.hullTop;
   }
-  constexpr int LANES = kLevelLanes<MIXED>, GROUPS = 32 / LANES * W;
-  const LevelLanes L = level_lanes<MIXED>(T.lane);
+  constexpr int LANES = kLevelLanes<MIXED, W>, GROUPS = 32 / LANES * W;
+  const LevelLanes L = level_lanes<MIXED, W>(T.lane);
   double* p = rec + 10;
 #pragma unroll 1
   for (int n = T.rank / LANES; n < nn; n += GROUPS) {
-    const double level = group_level<MIXED>(M, S, n, L);
+    const double level = group_level<MIXED, W>(M, S, n, L);
     if (L.sub == 0) {
       p[n] = S.vol[n];
       p[nn + n] = level;
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, kMinBlocksPerSM) run_b
     if (T.leader()) {
       const int q = atomicAdd(B.queue, 1);
       S.misc[kMiscInstance] = B.order == nullptr ? q : (q < *B.orderCount ? B.order[q] : B.count);
-      S.misc[kMiscTaken] = W * (32 / kLevelLanes<MIXED>);  // the level solve's list counter for the first step (team_step resets it)
+      S.misc[kMiscTaken] = W * (32 / kLevelLanes<MIXED, W>);  // the level solve's list counter for the first step (team_step resets it)
     }
     T.sync();
     const int inst = S.misc[kMiscInstance];

@@ -198,23 +198,17 @@ struct Parked {
   int foundered;
 };
 
-// Lanes that solve one group of nodes' free-surface levels together (8, 16 or 32), per numerics: a warp works on
-// 32 / kLevelLanes groups at once. Each lane forms the partials of 32 / kLevelLanes lanes of the 32-lane node-pass tree
+// Lanes that solve one group of nodes' free-surface levels together (8, 16 or 32), per numerics and team size: a warp works
+// on 32 / kLevelLanes groups at once. Each lane forms the partials of 32 / kLevelLanes lanes of the 32-lane node-pass tree
 // and combines them in the tree's order, so the results do not depend on this choice. Fewer lanes per group give more
-// groups in flight but more partials per lane (registers); on B200 (titanic64 batches) 16 was the fastest for double
-// precision partials and 8 for single precision ones.
-#ifndef SSB_LEVEL_LANES_F64
-#define SSB_LEVEL_LANES_F64 16
-#endif
-#ifndef SSB_LEVEL_LANES_F32
-#define SSB_LEVEL_LANES_F32 8
-#endif
-template <bool MIXED>
-constexpr int kLevelLanes = MIXED ? SSB_LEVEL_LANES_F32 : SSB_LEVEL_LANES_F64;
-static_assert(kLevelLanes<false> == 8 || kLevelLanes<false> == 16 || kLevelLanes<false> == 32, "level lanes must be 8, 16 or 32");
-static_assert(kLevelLanes<true> == 8 || kLevelLanes<true> == 16 || kLevelLanes<true> == 32, "level lanes must be 8, 16 or 32");
-// the slot's node-pass buffers are sized for the numerics with the most groups per warp
-constexpr int kMaxLevelGroupsPerWarp = 32 / (kLevelLanes<false> < kLevelLanes<true> ? kLevelLanes<false> : kLevelLanes<true>);
+// groups in flight and fewer shuffles, more lanes a shorter chain per pass. On B200 (16 lanes against the other choice):
+// double precision, 8-warp teams, 264 liner runs to 15 min 95.0 ms, 88.6 with 32; 16-warp teams, 192 titanic64 runs to
+// 1 h 266, 273 with 32; 1- and 2-warp teams, 2,048 uneven runs 348, 371 with 32, 359 with 8. Single precision, small
+// teams, 1,021 uneven runs 143, 161 with 8, 145 with 32; large teams, 48 runs 49.7, 45.7 with 32.
+template <bool MIXED, int W>
+constexpr int kLevelLanes = MIXED ? (W >= 8 ? 32 : 16) : (W == 8 ? 32 : 16);
+// the slot's node-pass buffers are sized for the most groups a warp works on
+constexpr int kMaxLevelGroupsPerWarp = 2;
 
 // Byte offsets of one simulation slot (one team of warps) in dynamic shared memory; `bytes` is the slot stride.
 // passes holds maxGroup node-pass results per level lane group of the team (up to kMaxLevelGroupsPerWarp per warp); hydro the

@@ -370,16 +370,16 @@ struct PassR {
   double vol, dv, mx, my, mz;
 };
 
-// The kLevelLanes<MIXED> consecutive lanes of a warp that solve one group of nodes: `lane` is the lane in the warp, `sub` the
+// The kLevelLanes<MIXED, W> consecutive lanes of a warp that solve one group of nodes: `lane` is the lane in the warp, `sub` the
 // lane in the group, `mask` the group's lanes.
 struct LevelLanes {
   int lane, sub;
   unsigned mask;
 };
 
-template <bool MIXED>
+template <bool MIXED, int W>
 __device__ __forceinline__ LevelLanes level_lanes(int lane) {
-  constexpr int LANES = kLevelLanes<MIXED>;
+  constexpr int LANES = kLevelLanes<MIXED, W>;
   return LevelLanes{lane, lane % LANES, (LANES == 32 ? kFull : (1u << (LANES & 31)) - 1u) << (lane / LANES * LANES)};
 }
 
@@ -420,7 +420,8 @@ template <bool MIXED, int W>
 __device__ __forceinline__ PassR node_pass(const DevModel& M, const Pose& F, int s0, int s1, double mu, double h, const LevelLanes& L) {
   using P = Prec<MIXED>;
   using T = typename P::T;
-  constexpr int LANES = kLevelLanes<MIXED>;
+  constexpr int LANES = kLevelLanes<MIXED, W>;
+  static_assert(LANES == 16 || LANES == 32, "a lane forms one or two of the tree's partials");
   constexpr int AHEAD = W >= 8 ? 2 : 1;  // large teams are bound by the loads' latency, small ones by issue slots
   const T hT = static_cast<T>(h);
   const int f = s0 + L.sub;
@@ -433,12 +434,6 @@ __device__ __forceinline__ PassR node_pass(const DevModel& M, const Pose& F, int
   } else {
     segment_partials<T, true, AHEAD>(xy, ab, area, f, s1, R20, R21, tz, iR, hT, p, b);  // tree lanes sub and sub + 16
     tree_pair(p, b);
-    if constexpr (LANES == 8) {
-      SegPartial<T> q;
-      segment_partials<T, true, AHEAD>(xy, ab, area, f + 8, s1, R20, R21, tz, iR, hT, q, b);  // sub + 8 and sub + 24
-      tree_pair(q, b);
-      tree_pair(p, q);
-    }
   }
 #pragma unroll
   for (int off = LANES / 2; off > 0; off >>= 1) {
@@ -594,9 +589,9 @@ __device__ __forceinline__ void list_groups(const DevModel& M, Slot& S, int lane
 }
 
 // A group's combined value of node_extreme over its lanes.
-template <bool MIXED>
+template <bool MIXED, int W>
 __device__ __forceinline__ double group_extreme(const DevModel& M, const Pose& F, int n, bool top, const LevelLanes& L) {
-  constexpr int LANES = kLevelLanes<MIXED>;
+  constexpr int LANES = kLevelLanes<MIXED, W>;
   auto v = node_extreme<MIXED>(M, F, n, top, L.sub, LANES);
 #pragma unroll
   for (int off = LANES / 2; off > 0; off >>= 1) {
@@ -612,9 +607,9 @@ __device__ __forceinline__ double stale_level(const DevModel& M, const Slot& S, 
   return (S.dry[n] & kStale) ? static_cast<double>(node_extreme<MIXED>(M, *S.prev, n, false, 0, 1)) : S.level[n];
 }
 
-template <bool MIXED>
+template <bool MIXED, int W>
 __device__ __forceinline__ double group_level(const DevModel& M, const Slot& S, int n, const LevelLanes& L) {
-  return (S.dry[n] & kStale) ? group_extreme<MIXED>(M, *S.prev, n, false, L) : S.level[n];
+  return (S.dry[n] & kStale) ? group_extreme<MIXED, W>(M, *S.prev, n, false, L) : S.level[n];
 }
 
 // A first look at the world extents of one node, or of two side by side, by a lane group: z[0] and z[1] the lowest bottom
@@ -625,9 +620,9 @@ struct Extents {
   bool whole;
 };
 
-template <bool MIXED>
+template <bool MIXED, int W>
 __device__ __forceinline__ Extents first_extents(const DevModel& M, const Pose& F, int n0, int n1, bool two, const LevelLanes& L) {
-  constexpr int LANES = kLevelLanes<MIXED>, Q = LANES / 4;
+  constexpr int LANES = kLevelLanes<MIXED, W>, Q = LANES / 4;
   const int quarter = L.sub / Q, at = L.sub % Q;
   const bool top = quarter & 1;
   bool whole = true;
@@ -720,7 +715,7 @@ __device__ __forceinline__ void share_pair(Slot& S, const PassR& p0, const PassR
 }
 
 // The level solve of the listed groups (levels.hpp:13-194). Groups are independent (a group's solve reads and writes only
-// its members), so the team's level lane groups (32 / kLevelLanes<MIXED> per warp) take them as they come: each starts
+// its members), so the team's level lane groups (32 / kLevelLanes<MIXED, W> per warp) take them as they come: each starts
 // with the list entry of its own index, then takes the next one from the team's counter (S.misc[kMiscTaken]); groups
 // take different numbers of passes, and a node's results do not depend on which lane group computes them. In 16-warp teams
 // the upper warps, which have no buoyancy tree, start with the first entries.
@@ -732,9 +727,9 @@ __device__ __forceinline__ void share_pair(Slot& S, const PassR& p0, const PassR
 // solver is a small machine (Phase) around one place for each of its parts.
 template <bool MIXED, int W, class Tape>
 __device__ __forceinline__ void solve_levels(const DevModel& M, const Pose& F, Slot& S, const Team<W>& T, const Tape& tape) {
-  constexpr int LANES = kLevelLanes<MIXED>, PER_WARP = 32 / LANES;
+  constexpr int LANES = kLevelLanes<MIXED, W>, PER_WARP = 32 / LANES;
   enum Phase { kIdle, kStart, kUpdate, kPass };
-  const LevelLanes L = level_lanes<MIXED>(T.lane);
+  const LevelLanes L = level_lanes<MIXED, W>(T.lane);
   const int grp = T.lane / LANES;
   PassR* const P = S.passes + static_cast<std::size_t>(T.warp * PER_WARP + grp) * M.maxGroup;
   const int listed = S.misc[kMiscListed];
@@ -780,7 +775,7 @@ __device__ __forceinline__ void solve_levels(const DevModel& M, const Pose& F, S
 #pragma unroll 1
             for (int q = 0; q < N; ++q) {
               const int n = q == 0 ? e.n0 : (q == 1 ? e.n1 : __ldg(m + q));
-              if (!(S.vol[n] > kEmptyVolume && group_level<MIXED>(M, S, n, L) > zMw + M.gMargin)) { merged = false; break; }
+              if (!(S.vol[n] > kEmptyVolume && group_level<MIXED, W>(M, S, n, L) > zMw + M.gMargin)) { merged = false; break; }
             }
           }
         }
@@ -822,12 +817,12 @@ __device__ __forceinline__ void solve_levels(const DevModel& M, const Pose& F, S
       const int q0 = allWet ? 0 : (firstWet >= 0 ? firstWet : nm - 1), q1 = allWet ? nm : q0 + 1;
       h = 0;
 #pragma unroll 1
-      for (int q = q0; q < q1; ++q) h += group_level<MIXED>(M, S, member(q), L);
+      for (int q = q0; q < q1; ++q) h += group_level<MIXED, W>(M, S, member(q), L);
       if (merged && allWet) h = nm == 2 ? 0.5 * h : h / static_cast<double>(nm);
       full = V >= Vmax * kFullFraction;
       inside = aKnown = bKnown = false;
       if (nm <= 2) {
-        const Extents x = first_extents<MIXED>(M, F, n0, n1, nm == 2, L);
+        const Extents x = first_extents<MIXED, W>(M, F, n0, n1, nm == 2, L);
         a = nm == 2 && x.z[2] < x.z[0] ? x.z[2] : x.z[0];
         b = nm == 2 && x.z[3] > x.z[1] ? x.z[3] : x.z[1];
         inside = Tape::kLazy && !full && h >= a && h <= b;
@@ -865,7 +860,7 @@ __device__ __forceinline__ void solve_levels(const DevModel& M, const Pose& F, S
         double zlo = 0, zhi = 0;
 #pragma unroll 1
         for (int top = 0; top < 2; ++top) {
-          const double z = group_extreme<MIXED>(M, F, n, top != 0, L);
+          const double z = group_extreme<MIXED, W>(M, F, n, top != 0, L);
           if (top) zhi = z; else zlo = z;
         }
         if (q == 0 || zlo < lo) lo = zlo;
@@ -1347,7 +1342,7 @@ __device__ __forceinline__ void team_step(const DevModel& M, SimRegs& R, Slot& S
   T.sync();
   // the list counter for the next step's level solve (read after this step's later barriers)
   if (T.leader()) {
-    S.misc[kMiscTaken] = W * (32 / kLevelLanes<MIXED>);
+    S.misc[kMiscTaken] = W * (32 / kLevelLanes<MIXED, W>);
     S.misc[kMiscFront] = 0;
     S.misc[kMiscBack] = 0;
   }
