@@ -209,12 +209,15 @@ void Batch::init(std::vector<std::pair<std::shared_ptr<const CompiledShip>, Comp
   };
   int W1 = opt_.teamWarps;
   if (W1 <= 0) {
-    // About 16 warps per SM in all. A batch that all fits at once in single-warp teams runs there; a larger one
-    // starts in two-warp teams: with 16 slots per SM the slots leave too little of the SM's shared storage to L1 for
-    // the geometry that every simulation reads (uneven titanic64 batches of 4096 and 8192 instances on B200: 7.3 and
-    // 7.8 M steps/s in two-warp teams, 6.4 and 5.5 M in single-warp teams).
+    // About 16 warps per SM in all. Up to one simulation per SM each has a whole 16-warp block from the start (on B200:
+    // one titanic64 run to 5 min 15.4 ms against 19.8 in 8-warp teams, 48 portable32 runs to 15 min 36 against 45, 140
+    // liner runs to 400 s 31 against 37, a fleet of 96 ships 22.6 against 32.2; 192 runs to 1 h 272 against 262 and 264
+    // liner runs 126 against 92, so not beyond one per SM). A batch that all fits at once in single-warp teams runs there;
+    // a larger one starts in two-warp teams: with 16 slots per SM the slots leave too little of the SM's shared storage
+    // to L1 for the geometry that every simulation reads, and fewer simulations wait for their first step (2,048 uneven
+    // titanic64 runs 348 ms in single-warp teams, 372 in two-warp ones; batches of 4,096 and more the other way round).
     const int fit = (sms * 16) / std::max(opt_.count, 1);
-    W1 = fit >= 8 ? 8 : fit >= 4 ? 4 : fit >= 2 ? 2 : fit >= 1 ? 1 : 2;
+    W1 = fit >= 16 && I.layout_for(16).bytes <= optin ? 16 : fit >= 8 ? 8 : fit >= 4 ? 4 : fit >= 2 ? 2 : fit >= 1 ? 1 : 2;
     // Large slots (a fleet's largest hull sets the slot) fit few simulations per SM: start with teams big enough that
     // the simulations that fit carry about 16 warps (a fleet of 2,048 hulls up to 256 spaces: 5 slots of 41.7 KB
     // per SM, so 4-warp teams).
@@ -722,10 +725,10 @@ void Batch::run_noalloc(const NoAllocRun& run, cudaStream_t stream) const {
   r.tMax = opt_.tMax;
   r.rule = opt_.rule;
   r.stopWhenStable = opt_.stopWhenStable;
-  // one launch, teams sized so that about 16 warps per SM carry the instances
+  // one launch, teams sized so that about 16 warps per SM carry the instances (as a batch's first phase, see init)
   const int sms = I.info.multiprocessors;
   const int fit = std::max(1, (sms * 16) / r.count);
-  r.teamWarps = fit >= 8 ? 8 : fit >= 4 ? 4 : fit >= 2 ? 2 : 1;
+  r.teamWarps = fit >= 16 && I.layout_for(16).bytes <= I.info.sharedPerBlockOptIn ? 16 : fit >= 8 ? 8 : fit >= 4 ? 4 : fit >= 2 ? 2 : 1;
   const SlotLayout L = I.layout_for(r.teamWarps);
   const int maxTeams = std::min(static_cast<int>(I.info.sharedPerBlockOptIn / L.bytes), kMaxWarpsPerBlock / r.teamWarps);
   r.teamsPerBlock = std::max(1, std::min(maxTeams, (r.count + sms - 1) / sms));
