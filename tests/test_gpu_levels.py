@@ -1,6 +1,8 @@
 """The level solve over the listed groups with extent lists (csrc/warp_step.cuh) against the C restatement, from restored
 states that put the spaces at the edges of its cases: dry, below the empty volume, partly flooded with the level inside
 and outside the space, full, overfull; upright, heeled and beyond a quarter turn."""
+import json
+
 import numpy as np
 import pytest
 
@@ -26,11 +28,33 @@ def _records(ship, sim):
         yield rec
 
 
+def _grouped_liner(out):
+    """The generated liner with its spaces in groups of 3, 1, 4 and 2, always merged or merged above a sill by turns."""
+    ship_p, sim_p = hullgen.write(out)
+    sim = json.load(open(sim_p))
+    n, start, count, mode = len(sim["state0"]["vol"]), [], [], []
+    while sum(count) < n:
+        start.append(sum(count))
+        count.append(min((3, 1, 4, 2)[len(count) % 4], n - sum(count)))
+        mode.append(1 + len(mode) % 2)
+    g = len(count)
+    sim["groups"] = dict(sim["groups"], n=g, nodeStart=start, nodeCount=count, mode=mode, px=[0.0] * g, py=[0.0] * g, pz=[4.0] * g)
+    kinds = dict(nodeStart="i32", nodeCount="i32", nodes="i32", mode="u8", a="i32", b="i32", type="u8", kind="u8", idx="i32", en="u8", skipGroup="i32",
+                 monitor="i32", when="u8")
+    order = [("groups", ("nodeStart", "nodeCount", "nodes", "mode", "px", "py", "pz")),
+             ("connections", ("a", "b", "type", "x", "y", "z", "area", "coef", "kind", "idx", "en", "tOn", "skipGroup", "monitor")),
+             ("marks", ("x", "y", "z", "when")), ("state0", ("vol", "level", "cx", "cy", "cz"))]
+    sim["hash"] = hullgen.hash_arrays([(f"{part}.{k}", kinds.get(k, "f64"), sim[part][k]) for part, keys in order for k in keys])
+    with open(sim_p, "w") as f:
+        json.dump(sim, f)
+    return ship_p, sim_p
+
+
 @pytest.mark.parametrize("warps", [1, 2, 8, 16])
 @pytest.mark.parametrize("numerics,mixed", [("portable", False), ("portable32", True)])
-@pytest.mark.parametrize("model", ["titanic64", "liner"])
+@pytest.mark.parametrize("model", ["titanic64", "liner", "grouped"])
 def test_restored_states_step_like_the_restatement(tmp_path, model, numerics, mixed, warps):
-    ship_p, sim_p = titanic() if model == "titanic64" else hullgen.write(str(tmp_path))
+    ship_p, sim_p = titanic() if model == "titanic64" else (hullgen.write if model == "liner" else _grouped_liner)(str(tmp_path))
     ship, sim = load_model(ship_p, sim_p)
     records = list(_records(ship, sim))
     b = ssb.Batch(ship_p, sim_p, count=len(records), numerics=numerics, t_max=STEPS * sim["dt"], team_warps=warps, tail_team_warps=0,
