@@ -40,7 +40,9 @@ sys.path.insert(0, ROOT)
 # and min/max not counted), from the exact per-step unit counts of the C restatement over a full run
 # (tests/test_oracle.py::test_work_counts_titanic64): 4,408 column clips (7 ops dry, 18 wet; 4,058 wet), 9,422
 # segment visits (10 ops dry, 21.5 wet; 4,174 wet), 71 node-pass trees (31), the buoyancy tree (191), 27 weir pows
-# (75), 290 connection flows (30), 64 node updates and loads (40).
+# (75), 290 connection flows (30), 64 node updates and loads (40). This is the reference algorithm's work; the engine leaves
+# out part of it (passes over dry spaces, extents and the hull's top from short lists), so a fraction of the peak by this
+# count says how fast it gets through steps, not how busy the FP64 units are.
 FP64_OPS_PER_STEP = 7 * 4408 + 11 * 4058 + 10 * 9422 + 11.5 * 4174 + 71 * 31 + 191 + 75 * 27 + 30 * 290 + 40 * 64
 
 # DRAM bytes (read + write) of one main-phase launch over the 4,096 instances, from ncu (dram__bytes per second x
@@ -223,6 +225,14 @@ def make_batch(ssb, ship_p, sim_p, sim, rule, count, first, args, device, total=
     return b
 
 
+def reference_unavailable():
+    """Why the reference CPU engine cannot be run here (its build from its own sources is not there), or None."""
+    ref = os.path.join(ROOT, "oracle", "_ref")
+    if all(os.path.exists(os.path.join(ref, f)) for f in ("libsinksim_ref.so", "sinksim_sweep")):
+        return None
+    return "the reference CPU engine is not built (make -C oracle REF=<reference tree>)"
+
+
 def cpu_fleet_rate(hulls, numerics, threads, t_max):
     """The reference CPU engine on the fleet's first `threads` hulls, one sinksim_sweep process per hull in parallel;
     returns (aggregate steps/s, steps, s, hulls): the steps of all processes over the longest of their own run times
@@ -344,6 +354,10 @@ def cpu_gradient_rate(ship_p, sim_p, space, thetas, h_rel, numerics, threads):
 def reference_arm(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return 0
+    why = reference_unavailable()
+    if why:
+        print(json.dumps({"impl": "reference", "unavailable": why}))
         return 0
     ship_p, sim_p = model_paths(args.model)
     from sinksim_b200.files import load_model
@@ -562,7 +576,10 @@ def gradient_bench(args):
                             "peak_source": "measured on this GPU: separately rounded FP64 add+mul microbenchmark (no FMA, as the bits require)",
                             "ops_per_sim_step": ops_per_step},
                "clocks": clk}
-        if world == 1 and not args.no_cpu_baseline:
+        why = reference_unavailable()
+        if why:
+            out["cpu_baseline"] = {"unavailable": why}
+        elif world == 1 and not args.no_cpu_baseline:
             threads = os.cpu_count() or 1
             k = max(1, threads // 2)
             v, s, secs = cpu_gradient_rate(ship_p, sim_p, space, thetas[:k], DEFAULT_FD_STEP, "portable", threads)
@@ -691,7 +708,10 @@ def main():
                             "fp32_peak": fp32_peak / 1e12, "ops_per_sim_step": ops_per_step,
                             "note": "the step is issue/latency bound; HBM traffic is negligible (L2-resident working set)"},
                "clocks": clk}
-        if world == 1 and not args.no_cpu_baseline and args.workload == "fleet":
+        why = reference_unavailable()
+        if why:
+            out["cpu_baseline"] = {"unavailable": why}
+        elif world == 1 and not args.no_cpu_baseline and args.workload == "fleet":
             threads = os.cpu_count() or 1
             v, s, secs, n = cpu_fleet_rate(hulls, args.numerics, threads, 1800.0)
             out["cpu_baseline"] = {"value": v, "unit": "sim-steps/s", "cores": threads, "kind": "reference",
