@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include "adjoint_kernel.h"
+#include "adjoint_layout.h"
 #include "batch.h"
 #include "model_dev.h"
 
@@ -41,7 +42,7 @@ struct AdjointBatch::Impl {
   int ringTeams = 0;
 
   // the forward slot of a team of W warps, as the batch kernel lays it out for one model
-  SlotLayout slot_for(int W) const { return slot_layout(model->NN, model->NC, model->NG, model->maxGroup, W, false); }
+  SlotLayout slot_for(int W) const { return slot_layout(model->NN, model->NC, model->NG, model->maxGroup, false, W, false); }
 };
 
 AdjointBatch::AdjointBatch(std::shared_ptr<const CompiledShip> ship, const CompiledSim& sim, const AdjointOptions& opt)

@@ -25,6 +25,7 @@
 #include <climits>
 
 #include "adjoint_kernel.h"
+#include "adjoint_layout.h"
 #include "adjoint_step.cuh"
 #include "warp_step.cuh"
 
@@ -193,7 +194,7 @@ __device__ __forceinline__ void load_state(const double* c, SimRegs& R, Slot& S,
   const int nn = M.nn;
   for (int n = T.rank; n < nn; n += 32 * W) {
     S.vol[n] = c[7 + n]; S.level[n] = c[7 + nn + n]; S.cx[n] = c[7 + 2 * nn + n]; S.cy[n] = c[7 + 3 * nn + n]; S.cz[n] = c[7 + 4 * nn + n];
-    S.area[n] = 0; S.zmax[n] = 0; S.hEff[n] = 0; S.aEff[n] = 0; S.acc[n] = 0; S.deg[n] = 0;
+    S.area[n] = 0; S.zmax[n] = 0; S.hEff[n] = 0; S.aEff[n] = 0; S.acc[n] = 0;
     S.dry[n] = 0;
   }
   for (int g = T.rank; g < M.ng; g += 32 * W) S.merged[g] = 0;
@@ -201,20 +202,6 @@ __device__ __forceinline__ void load_state(const double* c, SimRegs& R, Slot& S,
   T.sync();
   if (T.warp == W - 1) list_groups<false>(M, S, T.lane);  // every group, for the whole run
   T.sync();
-}
-
-// A packed step record: the tape's int32 (pass counts, merged flags), each node's first pass record in the packed
-// order and their total (nn + 1 int32; padded to 8 bytes), the tape's doubles up to the pass records, then only the
-// pass records the step used, node by node (min(count, kMaxPasses) per node), the whole rounded up to 16 bytes. The
-// pass records dominate the unpacked tape (kMaxPasses slots per node), and a node takes about 1.2 passes per step, so a
-// record is about a third of the tape; the stored offsets let its reader place every pass without a scan.
-__host__ __device__ __forceinline__ std::size_t record_ints_bytes(const adj::TapeLayout& L, int nn) {
-  return ((L.ints + static_cast<std::size_t>(nn) + 1) * sizeof(std::int32_t) + 7) & ~static_cast<std::size_t>(7);
-}
-
-__host__ __device__ __forceinline__ std::size_t record_bytes(const adj::TapeLayout& L, int nn, int records) {
-  return (record_ints_bytes(L, nn) + (L.passes + static_cast<std::size_t>(records) * adj::kPassFields) * sizeof(double) + 15) &
-         ~static_cast<std::size_t>(15);
 }
 
 // poff[n] = the first pass record of node n in the packed order, poff[nn] = their total (warp 0 scans the counts).
@@ -518,39 +505,6 @@ __global__ void __launch_bounds__(W * 32, 16 / W) adjoint_batch(const __grid_con
 }
 
 }  // namespace
-
-AdjLayout adjoint_layout(int nn, int nc, int ng, int nsamples, int W, bool withRaw) {
-  AdjLayout A{};
-  std::uint32_t off = 0;
-  auto take16 = [&](std::size_t bytes) {
-    const std::uint32_t at = off;
-    off = static_cast<std::uint32_t>((off + bytes + 15) & ~static_cast<std::size_t>(15));
-    return at;
-  };
-  const std::size_t N = sizeof(double) * static_cast<std::size_t>(std::max(nn, 1));
-  const std::size_t C = sizeof(double) * static_cast<std::size_t>(std::max(nc, 1));
-  A.hEff = take16(N); A.aEff = take16(N); A.dV = take16(C); A.volPost = take16(N);
-  A.deg = take16(sizeof(int) * static_cast<std::size_t>(std::max(nn, 1)));
-  A.clip = take16(sizeof(std::int32_t) * static_cast<std::size_t>(std::max(nn, 1)));
-  A.aVolPost = take16(N); A.aCxs = take16(N); A.aCys = take16(N); A.aCzs = take16(N); A.aVs = take16(N); A.aAcc = take16(N);
-  A.aZmx = take16(N); A.aLs = take16(N); A.aAs = take16(N);
-  A.faHA = take16(C); A.faHB = take16(C); A.faAA = take16(C); A.faAB = take16(C);
-  A.red = take16(sizeof(double) * 16 * static_cast<std::size_t>(W));
-  A.work = take16(sizeof(adj::UnitWork) * static_cast<std::size_t>(W));
-  A.plain = take16(static_cast<std::size_t>(std::max(nn, 1)));
-  A.units = take16(sizeof(std::int32_t) * static_cast<std::size_t>(std::max(nn, 1)));
-  A.nunits = take16(sizeof(std::int32_t));
-  A.pw = take16(2 * C);
-  A.replays = take16(sizeof(adj::Replay) * static_cast<std::size_t>(std::max(nn, 1)));
-  A.raw = withRaw ? take16(record_bytes(adj::tape_layout(nn, ng), nn, nn * adj::kMaxPasses)) : 0;
-  A.aVol = take16(N); A.aLevel = take16(N); A.aCx = take16(N); A.aCy = take16(N); A.aCz = take16(N);
-  A.grad = take16(C);
-  A.sampleS = take16(sizeof(double) * static_cast<std::size_t>(std::max(nsamples, 1)));
-  A.tape = take16(std::max(adj::tape_layout(nn, ng).bytes, record_bytes(adj::tape_layout(nn, ng), nn, nn * adj::kMaxPasses)));
-  A.poff = take16(sizeof(std::int32_t) * (static_cast<std::size_t>(std::max(nn, 1)) + 1));
-  A.bytes = off;
-  return A;
-}
 
 std::size_t adjoint_tape_bytes(int nn, int ng) { return record_bytes(adj::tape_layout(nn, ng), nn, nn * adj::kMaxPasses); }
 std::size_t adjoint_record_bytes(int nn, int ng, int passRecords) { return record_bytes(adj::tape_layout(nn, ng), nn, passRecords); }

@@ -57,8 +57,6 @@ struct AdjLayout {
   std::uint32_t aVol, aLevel, aCx, aCy, aCz, grad, sampleS, tape, poff, bytes;
 };
 
-// withRaw: room for one packed step record of the largest size (the reverse's asynchronous copy of the next record)
-AdjLayout adjoint_layout(int nn, int nc, int ng, int nsamples, int teamWarps, bool withRaw = false);
 std::size_t adjoint_tape_bytes(int nn, int ng);  // the largest packed step record
 std::size_t adjoint_record_bytes(int nn, int ng, int passRecords);  // a packed step record holding passRecords passes
 cudaError_t configure_adjoint_kernel(int teamWarps, std::size_t smem);

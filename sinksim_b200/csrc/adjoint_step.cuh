@@ -1098,9 +1098,9 @@ SSB_HD Members members_of(const DevModel& M, int g) {
   r.m = M.gNodes;
 #if defined(__CUDA_ARCH__)
   const uint2 e = *reinterpret_cast<const uint2*>(M.groupEntry + g);
-  r.n0 = static_cast<int>(e.x >> 16);
-  r.n1 = static_cast<int>(e.y & 0xffff);
-  r.N = static_cast<int>((e.y >> 16) & 0xff);
+  r.n0 = static_cast<int>(e.x & 0xffff);
+  r.n1 = static_cast<int>(e.x >> 16);
+  r.N = static_cast<int>(e.y & 0xff);
   if (r.N > 2) {
     r.m = M.gNodes + M.gStart[g];
     r.N = M.gCount[g];

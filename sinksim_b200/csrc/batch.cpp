@@ -56,7 +56,8 @@ struct Batch::Impl {
   const ModelDev& m0() const { return *models.front(); }
   const ModelDev& model(std::size_t inst) const { return *models[static_cast<std::size_t>(instModel[inst])]; }
 
-  SlotLayout layout_for(int W) const { return slot_layout(NN, NC, NG, maxGroup, W, fleet()); }
+  bool mixed = false;  // single-precision column arithmetic
+  SlotLayout layout_for(int W) const { return slot_layout(NN, NC, NG, maxGroup, mixed, W, fleet()); }
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   std::vector<cudaEvent_t> phaseEv;           // launch phase k ends at phaseEv[k + 1]; phaseEv[0] starts a round
@@ -167,6 +168,7 @@ void Batch::init(std::vector<std::pair<std::shared_ptr<const CompiledShip>, Comp
     I.nodeOff[i + 1] = I.nodeOff[i] + d.NN; I.connOff[i + 1] = I.connOff[i] + d.NC; I.evOff[i + 1] = I.evOff[i] + d.evCap;
     I.monOff[i + 1] = I.monOff[i] + d.nmon; I.markOff[i + 1] = I.markOff[i] + d.nmark;
   }
+  I.mixed = opt_.mixedPrecision;
   for (const auto& d : I.models) {
     I.NN = std::max(I.NN, d->NN); I.NC = std::max(I.NC, d->NC); I.NG = std::max(I.NG, d->NG); I.maxGroup = std::max(I.maxGroup, d->maxGroup);
   }

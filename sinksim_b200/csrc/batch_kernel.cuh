@@ -126,7 +126,7 @@ __device__ bool run_instance(const DevModel& M, const DevBatch& B, Slot& S, int 
   for (int n = rank; n < M.nn; n += kStride) {
     S.vol[n] = B.vol[iN + n]; S.level[n] = B.level[iN + n];
     S.cx[n] = B.cx[iN + n]; S.cy[n] = B.cy[iN + n]; S.cz[n] = B.cz[iN + n];
-    S.area[n] = 0; S.zmax[n] = 0; S.hEff[n] = 0; S.aEff[n] = 0; S.acc[n] = 0; S.deg[n] = 0;
+    S.area[n] = 0; S.zmax[n] = 0; S.hEff[n] = 0; S.aEff[n] = 0; S.acc[n] = 0;
     S.dry[n] = 0;
   }
 #pragma unroll 1

@@ -20,10 +20,10 @@
 
 namespace ssb {
 
-// A group as a step's level solve lists it: its index, its first two members (a group of one: that one twice), their number
+// A group as a step's level solve takes it, in one load: its first two members (a group of one: that one twice), their number
 // (255: at least that many) and its merge mode.
-struct alignas(8) Listed {
-  std::uint16_t g, n0, n1;
+struct alignas(8) GroupEntry {
+  std::uint16_t n0, n1;
   std::uint8_t N, mode;
 };
 
@@ -58,7 +58,7 @@ struct DevModel {
   std::int32_t ng;
   const std::int32_t *gStart, *gCount, *gNodes;
   const std::uint8_t* gMode;
-  const Listed* groupEntry;
+  const GroupEntry* groupEntry;
   const double *gpx, *gpy, *gpz;
   double gMargin;
   std::int32_t maxGroup;
@@ -198,29 +198,32 @@ struct Parked {
   int foundered;
 };
 
-// Lanes that solve one group of nodes' free-surface levels together (8, 16 or 32), per numerics and team size: a warp works
+// Lanes that solve one group of nodes' free-surface levels together (16 or 32), per numerics and team size: a warp works
 // on 32 / kLevelLanes groups at once. Each lane forms the partials of 32 / kLevelLanes lanes of the 32-lane node-pass tree
 // and combines them in the tree's order, so the results do not depend on this choice. Fewer lanes per group give more
 // groups in flight and fewer shuffles, more lanes a shorter chain per pass. On B200 (16 lanes against the other choice):
 // double precision, 8-warp teams, 264 liner runs to 15 min 95.0 ms, 88.6 with 32; 16-warp teams, 192 titanic64 runs to
 // 1 h 266, 273 with 32; 1- and 2-warp teams, 2,048 uneven runs 348, 371 with 32, 359 with 8. Single precision, small
 // teams, 1,021 uneven runs 143, 161 with 8, 145 with 32; large teams, 48 runs 49.7, 45.7 with 32.
+constexpr int level_lanes_of(bool mixed, int W) { return mixed ? (W >= 8 ? 32 : 16) : (W == 8 ? 32 : 16); }
 template <bool MIXED, int W>
-constexpr int kLevelLanes = MIXED ? (W >= 8 ? 32 : 16) : (W == 8 ? 32 : 16);
-// the slot's node-pass buffers are sized for the most groups a warp works on
-constexpr int kMaxLevelGroupsPerWarp = 2;
+constexpr int kLevelLanes = level_lanes_of(MIXED, W);
 
-// Byte offsets of one simulation slot (one team of warps) in dynamic shared memory; `bytes` is the slot stride.
-// passes holds maxGroup node-pass results per level lane group of the team (up to kMaxLevelGroupsPerWarp per warp); hydro the
-// eight buoyancy tree results and the hull's top; misc the team's small broadcast values and counters (MiscSlot); dry a
-// flag byte per node, wet the numbers of load terms, list the groups the next level solve visits and flow the connections that can flow
-// (warp_step.cuh); pose this step's pose and the last one's, which every phase reads (kept here rather than in each
-// thread's registers); parked the run's values; model (fleets only) the team's copy of its instance's model. area, zmax,
-// hEff, aEff, tmp and term5 become the six columns of the loads' per-node terms (a fixed stride apart); between the level
-// solve and the heads, acc, hEff, aEff and tmp hold the passes' sums.
+// A slot's small team values: the claimed instance, the yield flag, the level solve's counter of list entries taken, the
+// list's length, the numbers of flows at the front and at the back of their list.
+enum MiscSlot { kMiscInstance = 0, kMiscYield = 1, kMiscTaken = 2, kMiscListed = 3, kMiscFront = 4, kMiscBack = 5, kMiscSlots = 6 };
+
+// Byte offsets of one simulation slot (one team of warps) in dynamic shared memory; `bytes` is the slot stride
+// (slot_layout.h lays it out). passes holds maxGroup node-pass results per level lane group of the team, in models that have
+// groups of more than one; hydro the eight buoyancy tree results and the hull's top; misc the team's small broadcast values
+// and counters (MiscSlot); dry a flag byte per node, wet the numbers of load terms, list the groups the next level solve
+// visits (warp_step.cuh); pose this step's pose and the last one's, which every phase reads (kept here rather than in each
+// thread's registers); parked the run's values; model (fleets only) the team's copy of its instance's model. Arrays serve
+// more than one phase of a step: between the level solve and the heads acc, hEff, aEff and tmp hold the passes' sums; then,
+// until the volume update, acc holds the nodes' degrees and tmp's place the list of the connections that can flow; then acc
+// holds the excess, and area, zmax, hEff, aEff and tmp are the five columns of the loads' terms (a fixed stride apart).
 struct SlotLayout {
-  std::uint32_t vol, level, cx, cy, cz, area, zmax, hEff, aEff, tmp, term5, acc, deg, dV, flow, passes, hydro, misc, merged, dry, wet, list, pose, parked,
-      model, bytes;
+  std::uint32_t vol, level, cx, cy, cz, area, zmax, hEff, aEff, tmp, acc, dV, passes, hydro, misc, merged, dry, wet, list, pose, parked, model, bytes;
 };
 
 }  // namespace ssb

@@ -17,6 +17,7 @@
 #include "device_model.h"
 #include "extents.h"
 #include "model.h"
+#include "slot_layout.h"
 
 namespace ssb {
 
@@ -61,44 +62,6 @@ class DevBuf {
   }
 };
 
-
-inline std::uint32_t take(std::uint32_t& off, std::size_t bytes) {
-  const std::uint32_t at = off;
-  off = static_cast<std::uint32_t>((off + bytes + 15) & ~static_cast<std::size_t>(15));
-  return at;
-}
-
-// The shared-memory slot of one simulation of a model of these sizes, stepped by a team of W warps: per-node state and
-// scratch, the connections' flows and their list, the group-pass buffers, the buoyancy tree results, the poses and
-// parked run values, and in a fleet the team's copy of its instance's model.
-inline SlotLayout slot_layout(std::int32_t NN, std::int32_t NC, std::int32_t NG, std::int32_t maxGroup, int W, bool fleet) {
-  SlotLayout L{};
-  std::uint32_t off = 0;
-  const std::size_t nb = sizeof(double) * static_cast<std::size_t>(NN);
-  const std::size_t cb = sizeof(double) * static_cast<std::size_t>(std::max(NC, 1));
-  L.vol = take(off, nb); L.level = take(off, nb); L.cx = take(off, nb); L.cy = take(off, nb); L.cz = take(off, nb);
-  // six columns that the loads' terms are summed down side by side, so a stride that puts them in different banks
-  const std::size_t column = sizeof(double) * ((static_cast<std::size_t>(NN) + 5) / 8 * 8 + 2);
-  L.area = take(off, column); L.zmax = take(off, column); L.hEff = take(off, column); L.aEff = take(off, column); L.tmp = take(off, column);
-  L.term5 = take(off, column);
-  L.acc = take(off, nb);
-  L.deg = take(off, sizeof(std::int32_t) * static_cast<std::size_t>(NN));
-  L.dV = take(off, cb);
-  L.flow = take(off, sizeof(std::uint16_t) * static_cast<std::size_t>(std::max(NC, 1)));
-  L.passes = take(off, 5 * sizeof(double) * static_cast<std::size_t>(maxGroup) * static_cast<std::size_t>(W * kMaxLevelGroupsPerWarp));
-  L.hydro = take(off, 33 * sizeof(double));
-  L.misc = take(off, 8 * sizeof(std::int32_t));
-  L.merged = take(off, static_cast<std::size_t>(std::max(NG, 1)));
-  L.dry = take(off, static_cast<std::size_t>(std::max(NN, 1)));
-  L.wet = take(off, static_cast<std::size_t>(NN) / 32 + 1);
-  L.list = take(off, sizeof(Listed) * static_cast<std::size_t>(std::max(NG, 1)));
-  L.pose = take(off, 2 * sizeof(Pose));
-  L.parked = take(off, sizeof(Parked));
-  L.model = fleet ? take(off, sizeof(DevModel)) : 0u;
-  L.bytes = off;
-  return L;
-}
-
 // Tables of one model put together on the host and copied to the device in one piece (a model has some fifty, and an
 // allocation and a copy of each cost more than building them); every table starts at a multiple of 256 bytes.
 class TablePack {
@@ -141,6 +104,7 @@ struct ModelDev {
     mons = build_monitor_lists(sim);
     NN = ship->nodes(); NC = sim.connections(); NG = sim.groups();
     nmon = sim.monitors(); nmark = sim.marks(); evCap = nmon + nmark + 1; maxGroup = sim.maxGroupSize();
+    if (NG >= 32768) throw std::runtime_error("simulation " + sim.id + " has " + std::to_string(NG) + " groups, the level solve lists up to 32767");
   }
 
   void upload(cudaStream_t s) {
@@ -205,13 +169,13 @@ struct ModelDev {
     pack.add(d.nodeSeg, ns);
     pack.add(d.segStart, S.segStart); pack.add(d.segCount, S.segCount);
     pack.add(d.gStart, M.gNodeStart); pack.add(d.gCount, M.gNodeCount); pack.add(d.gNodes, M.gNodes); pack.add(d.gMode, M.gMode);
-    std::vector<Listed> entry(static_cast<std::size_t>(NG));
+    std::vector<GroupEntry> entry(static_cast<std::size_t>(NG));
     for (std::size_t g = 0; g < entry.size(); ++g) {
       const std::int32_t* m = M.gNodes.data() + M.gNodeStart[g];
       const std::int32_t N = M.gNodeCount[g];
       const std::int32_t first = N > 0 ? m[0] : 0;
-      entry[g] = Listed{static_cast<std::uint16_t>(g), static_cast<std::uint16_t>(first), static_cast<std::uint16_t>(N > 1 ? m[1] : first),
-                        static_cast<std::uint8_t>(std::min(N, 255)), M.gMode[g]};
+      entry[g] = GroupEntry{static_cast<std::uint16_t>(first), static_cast<std::uint16_t>(N > 1 ? m[1] : first),
+                            static_cast<std::uint8_t>(std::min(N, 255)), M.gMode[g]};
     }
     pack.add(d.groupEntry, entry);
     pack.add(d.gpx, M.gpx); pack.add(d.gpy, M.gpy); pack.add(d.gpz, M.gpz);

@@ -450,13 +450,12 @@ __device__ __forceinline__ PassR node_pass(const DevModel& M, const Pose& F, int
 // ----------------------------------------------------------------------------- per-warp view of the slot in shared memory
 
 struct Slot {
-  double *vol, *level, *cx, *cy, *cz, *area, *zmax, *hEff, *aEff, *tmp, *term5, *acc, *dV, *hydro;
-  int* deg;
+  double *vol, *level, *cx, *cy, *cz, *area, *zmax, *hEff, *aEff, *tmp, *acc, *dV, *hydro;
   int* misc;
   PassR* passes;
   std::uint8_t* merged;
   std::uint8_t* dry;          // NodeFlag bits
-  Listed* list;               // the groups the next level solve visits, misc[kMiscListed] of them
+  std::uint16_t* list;        // the groups the next level solve visits, misc[kMiscListed] of them (list_groups)
   std::uint8_t* wet;          // per 32 nodes, the flooded ones among them (their load terms)
   std::uint16_t* flow;        // the connections that can flow in this step (sort_connections)
   Pose* pose;                 // the current step's pose, and
@@ -478,17 +477,15 @@ __device__ __forceinline__ Slot carve_slot(unsigned char* base, const SlotLayout
   s.aEff = reinterpret_cast<double*>(base + L.aEff);
   s.acc = reinterpret_cast<double*>(base + L.acc);
   s.dV = reinterpret_cast<double*>(base + L.dV);
-  s.flow = reinterpret_cast<std::uint16_t*>(base + L.flow);
   s.tmp = reinterpret_cast<double*>(base + L.tmp);
-  s.term5 = reinterpret_cast<double*>(base + L.term5);
-  s.deg = reinterpret_cast<int*>(base + L.deg);
+  s.flow = reinterpret_cast<std::uint16_t*>(base + L.tmp);
   s.hydro = reinterpret_cast<double*>(base + L.hydro);
   s.misc = reinterpret_cast<int*>(base + L.misc);
   s.passes = reinterpret_cast<PassR*>(base + L.passes);
   s.merged = base + L.merged;
   s.dry = base + L.dry;
   s.wet = base + L.wet;
-  s.list = reinterpret_cast<Listed*>(base + L.list);
+  s.list = reinterpret_cast<std::uint16_t*>(base + L.list);
   s.pose = reinterpret_cast<Pose*>(base + L.pose);
   s.prev = s.pose + 1;
   s.parked = reinterpret_cast<Parked*>(base + L.parked);
@@ -521,10 +518,6 @@ enum NodeFlag : std::uint8_t {
   kNoTop = 16      // ... without its highest point: S.zmax[n] is not formed
 };
 
-// S.misc: the claimed instance, the yield flag, the level solve's counter of list entries taken, the list's length, the
-// numbers of flows at the front and at the back of their list.
-enum MiscSlot { kMiscInstance = 0, kMiscYield = 1, kMiscTaken = 2, kMiscListed = 3, kMiscFront = 4, kMiscBack = 5, kMiscSlots = 8 };
-
 // Where a step's forward computation records what its reverse (the adjoint, adjoint_kernel.cu) needs: every unit's start
 // (starting level and world extent), every node pass of the level solve (node, pass number within the node's solve,
 // level, result) and the solved levels. kLazy: empty nodes are left out of the solve, their levels formed on demand.
@@ -539,8 +532,11 @@ struct NoTape {
 
 // Lists the groups the next level solve visits, in increasing order, and flags the nodes of the others; one warp calls
 // it. A group is left out (kLazy) when neither its members nor their sum exceed the empty volume: then the solve would
-// find it empty merged or not. An entry, made with the model, carries what the solve would otherwise fetch in three
-// dependent loads.
+// find it empty merged or not. A group of one is listed as its node, which is all the solve needs of it (its merged flag
+// stays 0); a larger one as kListedGroup + its index, and its taker loads the entry made with the model. (The whole entry in
+// the list, 8 bytes a group, kept hulls of few connections from fitting a block.)
+constexpr int kListedGroup = 0x8000;
+
 template <bool LAZY>
 __device__ __forceinline__ void list_groups(const DevModel& M, Slot& S, int lane) {
   int count = 0;
@@ -549,7 +545,7 @@ __device__ __forceinline__ void list_groups(const DevModel& M, Slot& S, int lane
     const bool any = g0 + lane < M.ng;
     const int g = any ? g0 + lane : g0;
     const uint2 bits = __ldg(reinterpret_cast<const uint2*>(M.groupEntry) + g);
-    const int n0 = bits.x >> 16, n1 = bits.y & 0xffff, N = (bits.y >> 16) & 0xff;
+    const int n0 = bits.x & 0xffff, n1 = bits.x >> 16, N = bits.y & 0xff, mode = (bits.y >> 8) & 0xff;
     const double v0 = S.vol[n0], v1 = S.vol[n1];  // (n1 is n0 in a group of one)
     double V = v0;
     bool live = !LAZY || !(v0 <= kEmptyVolume);
@@ -569,7 +565,7 @@ __device__ __forceinline__ void list_groups(const DevModel& M, Slot& S, int lane
     }
     live = any && (live || !(V <= kEmptyVolume));
     if (any && !live) {
-      const bool merged = N >= 2 && (bits.y >> 24) == 1;
+      const bool merged = N >= 2 && mode == 1;
       const int flags = kEmptyNode | (merged ? kZeroVolume : 0);
       S.merged[g] = merged ? 1 : 0;
       S.dry[n0] |= flags;
@@ -582,7 +578,7 @@ __device__ __forceinline__ void list_groups(const DevModel& M, Slot& S, int lane
       }
     }
     const unsigned mask = __ballot_sync(kFull, live);
-    if (live) reinterpret_cast<uint2*>(S.list)[count + __popc(mask & ((1u << lane) - 1u))] = bits;
+    if (live) S.list[count + __popc(mask & ((1u << lane) - 1u))] = static_cast<std::uint16_t>(N == 1 ? n0 : kListedGroup + g);
     count += __popc(mask);
   }
   if (lane == 0) S.misc[kMiscListed] = count;
@@ -734,8 +730,8 @@ __device__ __forceinline__ void solve_levels(const DevModel& M, const Pose& F, S
   PassR* const P = S.passes + static_cast<std::size_t>(T.warp * PER_WARP + grp) * M.maxGroup;
   const int listed = S.misc[kMiscListed];
   int i = (W == 16 ? T.warp ^ 8 : T.warp) * PER_WARP + grp;   // the next list entry
-  Listed e{};                                  // the current group,
-  const int* m = nullptr;                      // its members when there are more than two,
+  int g0 = 0, g1 = 0;                          // the current group's first two members,
+  const int* m = nullptr;                      // all of them when there are more than two,
   int N = 0, j = 0, units = 0;                 // their number, its next unit and its units
   bool merged = false;
   // the current unit: nm members, n0 and n1 first (the others from m) with their segments
@@ -755,38 +751,43 @@ __device__ __forceinline__ void solve_levels(const DevModel& M, const Pose& F, S
 #pragma unroll 1
     while (phase == kIdle && (j < units || i < listed)) {
       if (j >= units) {
-        e = S.list[i];
+        g0 = g1 = S.list[i];
         int next = 0;
         if (L.sub == 0) next = atomicAdd(&S.misc[kMiscTaken], 1);
         i = __shfl_sync(L.mask, next, grp * LANES);
-        N = e.N;
+        N = 1;
         m = nullptr;
-        if (N > 2) {
-          if (N == 255) N = __ldg(M.gCount + e.g);
-          m = M.gNodes + __ldg(M.gStart + e.g);
-        }
         merged = false;
-        if (N >= 2) {
-          if (e.mode == 1) {
+        if (g0 >= kListedGroup) {
+          const int g = g0 - kListedGroup;
+          const uint2 bits = __ldg(reinterpret_cast<const uint2*>(M.groupEntry) + g);
+          g0 = bits.x & 0xffff;
+          g1 = bits.x >> 16;
+          N = bits.y & 0xff;
+          const int mode = (bits.y >> 8) & 0xff;
+          if (N > 2) {
+            if (N == 255) N = __ldg(M.gCount + g);
+            m = M.gNodes + __ldg(M.gStart + g);
+          }
+          if (mode == 1) {
             merged = true;
-          } else if (e.mode == 2) {
-            const double zMw = world_z(F, __ldg(M.gpx + e.g), __ldg(M.gpy + e.g), __ldg(M.gpz + e.g));
+          } else if (mode == 2) {
+            const double zMw = world_z(F, __ldg(M.gpx + g), __ldg(M.gpy + g), __ldg(M.gpz + g));
             merged = true;
 #pragma unroll 1
             for (int q = 0; q < N; ++q) {
-              const int n = q == 0 ? e.n0 : (q == 1 ? e.n1 : __ldg(m + q));
+              const int n = q == 0 ? g0 : (q == 1 ? g1 : __ldg(m + q));
               if (!(S.vol[n] > kEmptyVolume && group_level<MIXED, W>(M, S, n, L) > zMw + M.gMargin)) { merged = false; break; }
             }
           }
+          if (L.sub == 0) S.merged[g] = merged ? 1 : 0;
         }
-        if (L.sub == 0) S.merged[e.g] = merged ? 1 : 0;
         units = merged ? 1 : N;
         j = 0;
-        if (units == 0) continue;  // a group without members
       }
-      n0 = j == 0 ? e.n0 : (j == 1 ? e.n1 : __ldg(m + j));
+      n0 = j == 0 ? g0 : (j == 1 ? g1 : __ldg(m + j));
       nm = merged ? N : 1;
-      n1 = nm > 1 ? e.n1 : n0;
+      n1 = nm > 1 ? g1 : n0;
       ++j;
       // everything the unit needs of its nodes' table, in one round of loads
       seg0 = __ldg(M.nodeSeg + n0); seg1 = __ldg(M.nodeSeg + n1);
@@ -989,6 +990,9 @@ __device__ __forceinline__ FlowHeads flow_heads(const DevModel& M, const Pose& F
   return f;
 }
 
+// Node n's degree, in the first half of its place in S.acc (zeroed with the heads, dead with the volume update).
+__device__ __forceinline__ int* degree(const Slot& S, int n) { return reinterpret_cast<int*>(S.acc + n); }
+
 // A node's degree is the number of its incident connections that are enabled and not between two empty spaces. Each such
 // connection counts once at each of its nodes (the incidence lists hold it once at a when a >= 0 and once at b), counted
 // per connection with shared-memory atomics: an integer count, the same in any order, and one round of independent loads
@@ -999,8 +1003,8 @@ __device__ __forceinline__ bool count_degrees(const DevModel& M, double t, Slot&
   if (!__ldg(I.en() + c)) return false;
   const int a = __ldg(M.ca + c), b = __ldg(M.cb + c);
   if (a >= 0 && S.hEff[a] < kNoHeadTest && S.hEff[b] < kNoHeadTest) return false;
-  if (a >= 0) atomicAdd(&S.deg[a], 1);
-  atomicAdd(&S.deg[b], 1);
+  if (a >= 0) atomicAdd(degree(S, a), 1);
+  atomicAdd(degree(S, b), 1);
   const int sk = __ldg(M.skip + c);
   return !(__ldg(I.tOn() + c) > t) && !(sk >= 0 && S.merged[sk]);
 }
@@ -1033,7 +1037,8 @@ __device__ __forceinline__ double limit_volume(const Slot& S, const FlowHeads& f
   const double hs = src < 0 ? 0.0 : S.hEff[src];
   const double hd = dst < 0 ? 0.0 : S.hEff[dst];
   const double inv = (src < 0 ? 0.0 : S.aEff[src]) + (dst < 0 ? 0.0 : S.aEff[dst]);
-  const int degRef = src < 0 ? S.deg[dst] : (dst < 0 ? S.deg[src] : (S.deg[src] > S.deg[dst] ? S.deg[src] : S.deg[dst]));
+  const int degSrc = src < 0 ? 0 : *degree(S, src), degDst = dst < 0 ? 0 : *degree(S, dst);
+  const int degRef = degSrc > degDst ? degSrc : degDst;
   const double share = kLimiterShare / static_cast<double>(degRef > 1 ? degRef : 1);
   double lim = inv > 0 ? share * (hs - jmax(hd, f.zo)) / inv : fabs(dV);
   if (lim < 0) lim = 0;
@@ -1296,9 +1301,10 @@ __device__ __forceinline__ double3 integrate_motion(const DevModel& M, Parked& P
 }
 
 // The load sums, the motion and the next pose (body.hpp:11-57, events.hpp:30-38), by one warp. The load terms of the
-// flooded nodes are in six columns a fixed stride apart from S.area, in node order, 32 nodes' at the front of their 32
-// places and their number in S.wet (team_step). Lanes 0 .. 5 each add one column: a lane reading all six, node by node,
-// took a dependent load and six adds for each of all the nodes, and an add takes 23 cycles.
+// flooded nodes are in five columns a fixed stride apart from S.area, in node order, 32 nodes' at the front of their 32
+// places and their number in S.wet (team_step). Lanes 0 .. 5 each add one column: a lane reading all of them, node by node,
+// took a dependent load and six adds for each of all the nodes, and an add takes 23 cycles. The third column holds volumes,
+// of which lane 2 adds the weights and lane 3 the masses; the others' factor of one leaves their terms as they are.
 __device__ __forceinline__ void move_body(const DevModel& M, const Pose& F, Slot& S, int lane) {
   Parked& P = *S.parked;
   const Buoy hb = buoyancy_finish(S.hydro);
@@ -1311,12 +1317,14 @@ __device__ __forceinline__ void move_body(const DevModel& M, const Pose& F, Slot
   if (lane == 1) sum = -(bxw - M.XO) * Fb;
   if (lane == 2) sum = Fb - M.g * M.ms;
   {
-    const double* t = S.area + (lane < 6 ? lane : 5) * (S.zmax - S.area);
+    // (min, not nested choices: those cost the 16-warp fleet kernel 248 bytes of spills, 96 ships to 5 min 32 ms against 24.4)
+    const double* t = S.area + min(lane - (lane >= 3 ? 1 : 0), 4) * (S.zmax - S.area);
+    const double factor = lane == 2 ? -Wg : (lane == 3 ? M.rho : 1.0);
 #pragma unroll 1
     for (int n0 = 0; n0 < M.nn; n0 += kLanes) {
       const int wet = S.wet[n0 / kLanes];
 #pragma unroll 4
-      for (int k = 0; k < wet; ++k) sum += t[n0 + k];
+      for (int k = 0; k < wet; ++k) sum += factor * t[n0 + k];
     }
   }
   const double tauX = __shfl_sync(kFull, sum, 0), tauY = __shfl_sync(kFull, sum, 1), Fz = __shfl_sync(kFull, sum, 2);
@@ -1362,7 +1370,7 @@ __device__ __forceinline__ void team_step(const DevModel& M, SimRegs& R, Slot& S
     const double v = S.vol[n];
     S.hEff[n] = v > kEmptyVolume ? S.level[n] : kNoHead;
     S.aEff[n] = 1 / (v >= __ldg(M.vmax + n) ? __ldg(M.aov + n) : jmax(S.area[n], __ldg(M.amin + n)));
-    S.deg[n] = 0;
+    S.acc[n] = 0;  // the degree
   }
   tape.solved(M, S, T);  // a thread reads the nodes it has just finished
   T.sync();
@@ -1428,10 +1436,9 @@ __device__ __forceinline__ void team_step(const DevModel& M, SimRegs& R, Slot& S
         const int at = n0 + __popc(mask & ((1u << lane) - 1u));
         S.area[at] = wy * f;
         S.zmax[at] = -(wx * f);
-        S.hEff[at] = f;
-        S.aEff[at] = m;
-        S.tmp[at] = m * (wx * wx + wz * wz);
-        S.term5[at] = m * (wy * wy + wz * wz);
+        S.hEff[at] = v;
+        S.aEff[at] = m * (wx * wx + wz * wz);
+        S.tmp[at] = m * (wy * wy + wz * wz);
       }
     }
   }
