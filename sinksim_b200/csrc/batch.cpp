@@ -209,6 +209,8 @@ void Batch::init(std::vector<std::pair<std::shared_ptr<const CompiledShip>, Comp
     p.blocks = std::min((count + tpb - 1) / tpb, p.blocksPerSM * sms);
     return p;
   };
+  // team sizes that the caller does not ask for stop at the largest that fits
+  auto fitting = [&](int W) { return fitting_team(W, optin, [&](int w) { return I.layout_for(w); }); };
   int W1 = opt_.teamWarps;
   if (W1 <= 0) {
     // About 16 warps per SM in all. Up to one simulation per SM each has a whole 16-warp block from the start (on B200:
@@ -219,18 +221,18 @@ void Batch::init(std::vector<std::pair<std::shared_ptr<const CompiledShip>, Comp
     // to L1 for the geometry that every simulation reads, and fewer simulations wait for their first step (2,048 uneven
     // titanic64 runs 348 ms in single-warp teams, 372 in two-warp ones; batches of 4,096 and more the other way round).
     const int fit = (sms * 16) / std::max(opt_.count, 1);
-    W1 = fit >= 16 && I.layout_for(16).bytes <= optin ? 16 : fit >= 8 ? 8 : fit >= 4 ? 4 : fit >= 2 ? 2 : fit >= 1 ? 1 : 2;
+    W1 = fitting(fit >= 16 ? 16 : fit >= 8 ? 8 : fit >= 4 ? 4 : fit >= 2 ? 2 : fit >= 1 ? 1 : 2);
     // Large slots (a fleet's largest hull sets the slot) fit few simulations per SM: start with teams big enough that
     // the simulations that fit carry about 16 warps (a fleet of 2,048 hulls up to 256 spaces: 5 slots of 41.7 KB
     // per SM, so 4-warp teams).
     const int slotsPerSM = std::max(1, static_cast<int>(optin / cfg_.slotBytes));
-    while (W1 < 8 && W1 * slotsPerSM < 16) W1 *= 2;
+    while (W1 < 8 && W1 * slotsPerSM < 16 && fitting(2 * W1) == 2 * W1) W1 *= 2;
   }
   cfg_.phases.push_back(plan(W1, opt_.teamsPerBlock, opt_.count));
   if (opt_.blocks > 0) cfg_.phases[0].blocks = opt_.blocks;
   // the last phase: a whole 16-warp block per simulation (the uneven titanic64 bench batch on B200: 4.12 s against
   // 4.25 s with 8-warp teams last, same bits; the lone simulations of the tail step faster in larger teams)
-  const int Wlast = opt_.tailTeamWarps < 0 ? 16 : opt_.tailTeamWarps;
+  const int Wlast = opt_.tailTeamWarps < 0 ? fitting(16) : opt_.tailTeamWarps;
   if (Wlast > W1 && opt_.stepsPerLaunch <= 0) {
     for (int W = W1 * 2; W <= Wlast; W *= 2) {
       PhaseConfig p = plan(W, 0, opt_.count);
@@ -730,7 +732,8 @@ void Batch::run_noalloc(const NoAllocRun& run, cudaStream_t stream) const {
   // one launch, teams sized so that about 16 warps per SM carry the instances (as a batch's first phase, see init)
   const int sms = I.info.multiprocessors;
   const int fit = std::max(1, (sms * 16) / r.count);
-  r.teamWarps = fit >= 16 && I.layout_for(16).bytes <= I.info.sharedPerBlockOptIn ? 16 : fit >= 8 ? 8 : fit >= 4 ? 4 : fit >= 2 ? 2 : 1;
+  r.teamWarps = fitting_team(fit >= 16 ? 16 : fit >= 8 ? 8 : fit >= 4 ? 4 : fit >= 2 ? 2 : 1, I.info.sharedPerBlockOptIn,
+                             [&](int w) { return I.layout_for(w); });
   const SlotLayout L = I.layout_for(r.teamWarps);
   const int maxTeams = std::min(static_cast<int>(I.info.sharedPerBlockOptIn / L.bytes), kMaxWarpsPerBlock / r.teamWarps);
   r.teamsPerBlock = std::max(1, std::min(maxTeams, (r.count + sms - 1) / sms));

@@ -49,4 +49,12 @@ inline SlotLayout slot_layout(std::int32_t NN, std::int32_t NC, std::int32_t NG,
   return L;
 }
 
+// The largest team, of up to W warps, whose slot fits `room` bytes: the pass buffers of a large group grow with the team (a
+// merged group of 180 spaces fits teams of up to 8 warps). 1 when none larger does.
+template <class LayoutFor>
+int fitting_team(int W, std::size_t room, LayoutFor layout_for) {
+  while (W > 1 && layout_for(W).bytes > room) W /= 2;
+  return W;
+}
+
 }  // namespace ssb

@@ -43,7 +43,8 @@ int main(int, char** a) {
   if (A.poff < A.tape + T.doubles * 8 + T.ints * 4 || A.poff + 4ul * (nn + 1) > A.bytes || A.tape + record_bytes(T, nn, nn * adj::kMaxPasses) > A.bytes ||
       A.tape < A.sampleS + 64)
     return 1;
-  std::printf("%u %zu\n", L.bytes, L.bytes + static_cast<std::size_t>(A.bytes));
+  const int fits = fitting_team(16, 232448, [&](int w) { return slot_layout(nn, nc, ng, mg, mixed, w, fleet); });
+  std::printf("%u %zu %d\n", L.bytes, L.bytes + static_cast<std::size_t>(A.bytes), fits);
 }
 """
 
@@ -93,3 +94,11 @@ def test_the_places_do_not_overlap(sizes, nn, nc, per_group):
         for mixed in (0, 1):
             for fleet in (0, 1):
                 sizes(nn, nc, (nn + per_group - 1) // per_group, per_group, warps, mixed, fleet)
+
+
+@pytest.mark.parametrize("group,mixed,warps", [(100, 0, 16), (184, 0, 8), (184, 1, 16), (600, 0, 2), (600, 1, 2), (1200, 0, 1)])
+def test_the_largest_team_that_fits_a_large_group(sizes, group, mixed, warps):
+    """A merged group's pass buffers: 40 bytes a member, lane group and team."""
+    bytes_of = lambda w: sizes(group, 0, 1, group, w, mixed, 0)[0]
+    assert sizes(group, 0, 1, group, 1, mixed, 0)[2] == warps
+    assert bytes_of(warps) <= BLOCK and (warps == 16 or bytes_of(2 * warps) > BLOCK)
