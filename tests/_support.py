@@ -331,10 +331,24 @@ def tangent_gradient(ship, sim, en, area, t_on, conns, steps, sample_steps, trim
 _ref_lib = None
 
 
+def _from_reference(name):
+    """Path of a part of the checker that is built from the reference's own sources. Where it was not built (oracle/Makefile
+    needs those sources), the rest of the test that asks for it is skipped; what the test checked before that stands."""
+    path = os.path.join(REF_DIR, name)
+    if not os.path.exists(path):
+        why = f"oracle/_ref/{name} is not built (make -C oracle REF=<reference tree>)"
+        if "PYTEST_CURRENT_TEST" in os.environ:
+            import pytest
+
+            pytest.skip(why)
+        raise FileNotFoundError(why)
+    return path
+
+
 def ref_lib():
     global _ref_lib
     if _ref_lib is None:
-        lib = C.CDLL(os.path.join(REF_DIR, "libsinksim_ref.so"))
+        lib = C.CDLL(_from_reference("libsinksim_ref.so"))
         lib.ssref_last_error.restype = C.c_char_p
         lib.ssref_open.restype = C.c_void_p
         lib.ssref_open.argtypes = [C.c_char_p, C.c_char_p, C.c_char_p]
@@ -434,11 +448,11 @@ def ref_time_steps(ship_path, sim_path, numerics, count, max_steps, threads):
 
 
 def ref_tool(name):
-    return os.path.join(REF_DIR, name)
+    return _from_reference(name)
 
 
 def fdlibm_ref():
-    lib = C.CDLL(os.path.join(REF_DIR, "libfdlibm_ref.so"))
+    lib = C.CDLL(_from_reference("libfdlibm_ref.so"))
     for fn in ("fdlibm_sin", "fdlibm_cos"):
         getattr(lib, fn).restype = C.c_double
         getattr(lib, fn).argtypes = [C.c_double]
