@@ -28,7 +28,7 @@ struct HostModel {
   std::vector<double2> colXY, colLH, segXY, segLH;
   std::vector<double> colA, segAr, mu, vmax, amin, aov, gpx, gpy, gpz, kx, ky, kz, coef;
   std::vector<std::int32_t> segStart, segCount, gStart, gCount, gNodes, ca, cb, skip, incStart, incCount, incConn, sea;
-  std::vector<std::uint8_t> gMode, law, incSide;
+  std::vector<std::uint8_t> law, incSide;
   DevModel dm{};
 
   HostModel(const sso_ship* S, const sso_sim* M) {
@@ -47,7 +47,7 @@ struct HostModel {
     mu.assign(S->mu, S->mu + nn); vmax.assign(S->vmax, S->vmax + nn); amin.assign(S->amin, S->amin + nn); aov.assign(S->aov, S->aov + nn);
     segStart.assign(S->segStart, S->segStart + nn); segCount.assign(S->segCount, S->segCount + nn);
     const int ng = M->ngroup;
-    gStart.assign(M->gStart, M->gStart + ng); gCount.assign(M->gCount, M->gCount + ng); gMode.assign(M->gMode, M->gMode + ng);
+    gStart.assign(M->gStart, M->gStart + ng); gCount.assign(M->gCount, M->gCount + ng);
     gpx.assign(M->gpx, M->gpx + ng); gpy.assign(M->gpy, M->gpy + ng); gpz.assign(M->gpz, M->gpz + ng);
     int members = 0, maxGroup = 1;
     for (int g = 0; g < ng; ++g) { members = std::max(members, gStart[g] + gCount[g]); maxGroup = std::max(maxGroup, gCount[g]); }
@@ -73,7 +73,7 @@ struct HostModel {
     d.nseg = ns; d.segXY = segXY.data(); d.segLH = segLH.data(); d.segAr = segAr.data();
     d.nn = nn; d.mu = mu.data(); d.vmax = vmax.data(); d.amin = amin.data(); d.aov = aov.data();
     d.segStart = segStart.data(); d.segCount = segCount.data();
-    d.ng = ng; d.gStart = gStart.data(); d.gCount = gCount.data(); d.gNodes = gNodes.data(); d.gMode = gMode.data();
+    d.ng = ng; d.gStart = gStart.data(); d.gCount = gCount.data(); d.gNodes = gNodes.data();
     d.gpx = gpx.data(); d.gpy = gpy.data(); d.gpz = gpz.data(); d.gMargin = M->gMargin; d.maxGroup = maxGroup;
     d.nc = k; d.ca = ca.data(); d.cb = cb.data(); d.skip = skip.data(); d.law = law.data();
     d.kx = kx.data(); d.ky = ky.data(); d.kz = kz.data(); d.coef = coef.data();

@@ -57,7 +57,6 @@ struct DevModel {
   // groups
   std::int32_t ng;
   const std::int32_t *gStart, *gCount, *gNodes;
-  const std::uint8_t* gMode;
   const GroupEntry* groupEntry;
   const double *gpx, *gpy, *gpz;
   double gMargin;

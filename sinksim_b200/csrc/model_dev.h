@@ -168,7 +168,7 @@ struct ModelDev {
     for (std::size_t n = 0; n < ns.size(); ++n) ns[n] = int2{S.segStart[n], S.segCount[n]};
     pack.add(d.nodeSeg, ns);
     pack.add(d.segStart, S.segStart); pack.add(d.segCount, S.segCount);
-    pack.add(d.gStart, M.gNodeStart); pack.add(d.gCount, M.gNodeCount); pack.add(d.gNodes, M.gNodes); pack.add(d.gMode, M.gMode);
+    pack.add(d.gStart, M.gNodeStart); pack.add(d.gCount, M.gNodeCount); pack.add(d.gNodes, M.gNodes);
     std::vector<GroupEntry> entry(static_cast<std::size_t>(NG));
     for (std::size_t g = 0; g < entry.size(); ++g) {
       const std::int32_t* m = M.gNodes.data() + M.gNodeStart[g];
