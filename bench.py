@@ -45,11 +45,12 @@ sys.path.insert(0, ROOT)
 # count says how fast it gets through steps, not how busy the FP64 units are.
 FP64_OPS_PER_STEP = 7 * 4408 + 11 * 4058 + 10 * 9422 + 11.5 * 4174 + 71 * 31 + 191 + 75 * 27 + 30 * 290 + 40 * 64
 
-# DRAM bytes (read + write) of one main-phase launch over the 4,096 instances, from ncu (dram__bytes per second x
-# duration of run_batch<portable, 2-warp teams> on the same batch run to 600 s: python bench.py --count 4096 --tmax 600).
+# DRAM bytes (read + write) of one main-phase launch over the 4,096 instances, from ncu (dram__bytes_read.sum +
+# dram__bytes_write.sum of run_batch<portable, 2-warp teams> on the same batch run to 600 s: python bench.py --count 4096
+# --tmax 600).
 # The traffic is the instances' state going in and out: the geometry and the running state stay on chip, so the figure
 # does not grow with the steps a launch takes.
-KERNEL_DRAM_BYTES_PER_LAUNCH = 24.6e6
+KERNEL_DRAM_BYTES_PER_LAUNCH = 21.5e6
 
 
 def parse():

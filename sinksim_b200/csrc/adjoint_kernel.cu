@@ -10,8 +10,8 @@
 //      goes to shared memory and from there, packed, into the team's ring of step records in global memory;
 //   2. reverse: segment by segment, last first. A segment whose records the ring still holds is reversed from them;
 //      any other is recomputed from its checkpoint with the tape hooks on, into the ring, first. Each step's record is
-//      unpacked into shared memory and reversed (adjoint_step.cuh), adding the objective's adjoint at the sample
-//      states.
+//      copied into shared memory as it is and reversed there (adjoint_step.cuh), adding the objective's adjoint at the
+//      sample states.
 // Memory per team: the checkpoints of one run and the ring; the adjoint of the state lives in shared memory. When the
 // ring holds a whole run (the usual case: a packed record is about 12 KB on a 64-node model) nothing is recomputed;
 // with a ring of K records every segment is recomputed once, which costs one more forward pass.
@@ -140,12 +140,12 @@ struct AdjInst {
 
 // Per-team shared memory: the forward slot, then the reverse's arrays.
 struct AdjSmem {
-  unsigned char* raw;   // one packed step record (stageRecords), or null
+  unsigned char* raw;   // another packed record (stageRecords), or null
   adj::RevSlot rs;
   adj::AdjState as;
   double* grad;      // [nc]
   double* sampleS;   // [nsamples] state index of each sample (as doubles)
-  unsigned char* tape;  // one step's tape: written by the step's hooks, or unpacked from its record for its reverse
+  unsigned char* tape;  // one step's tape, written by the step's hooks; in the reverse a packed record
   std::int32_t* poff;   // [nn + 1] first pass record of each node in a packed record, then their total
 };
 

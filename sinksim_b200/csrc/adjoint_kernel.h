@@ -42,8 +42,9 @@ struct AdjRun {
   long long* stepOff;
   std::int32_t* recBytes;                       // [teams x (maxSteps + 1)] each step record's bytes
   std::int32_t tapeForward;
-  std::int32_t stageRecords;                    // 1: the layout has a raw record buffer (AdjLayout::raw): the reverse
-                                                // copies the next step's record into it while it reverses this one
+  std::int32_t stageRecords;                    // 1: the layout has a second record buffer (AdjLayout::raw): the reverse
+                                                // copies the next step's record into the one while it reverses this
+                                                // step's in the other (the tape's place), by turns
   double* sink;                                 // [teams x (evCap + nmon + nmark + 1)]
   std::int32_t* isink;                          // [teams x (evCap + 1)]
   long long* phaseNs;                           // [count x 3] the team's time on the instance (globaltimer ns):

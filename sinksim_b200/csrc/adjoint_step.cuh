@@ -35,8 +35,9 @@
 
 // Loops whose bodies the compiler would copy four times over, and functions called from several places: the reverse
 // issues a long straight run of code once per step, which has to come from the instruction caches. With one call site of
-// the forward step (adjoint_kernel.cu) the kernel is 310 KB of code instead of 940; on B200 a 64-point gradient on the
-// liner to 400 s takes 107 ms against 111, 3 points on titanic64 51 against 58. What adds to the pose adjoint is inlined all
+// the forward step (adjoint_kernel.cu) the kernel is 345 KB of code instead of 940 (128 registers, 316 to 348 bytes of
+// spills); when that came, on B200, a 64-point gradient on the liner to 400 s took 107 ms against 111, 3 points on
+// titanic64 51 against 58. What adds to the pose adjoint is inlined all
 // the same: called, it keeps the adjoint's 14 sums in local memory (105 ms against 98 with the other steps since).
 #if defined(__CUDA_ARCH__)
 #define SSB_ROLLED _Pragma("unroll 1")

@@ -9,7 +9,7 @@
 
 namespace ssb {
 
-// Warps per block at most (teams of 1, 2, 4 or 8 warps; teams per block x warps per team <= kMaxWarpsPerBlock) and the
+// Warps per block at most (teams of 1, 2, 4, 8 or 16 warps; teams per block x warps per team <= kMaxWarpsPerBlock) and the
 // blocks of that size the kernel is compiled to fit on one SM (which sets its register budget: 65,536 registers
 // over kMaxWarpsPerBlock x 32 x kMinBlocksPerSM threads).
 #ifndef SSB_BLOCK_WARPS

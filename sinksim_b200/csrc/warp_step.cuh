@@ -33,9 +33,11 @@ constexpr int kLanes = 32;
 // What a step issues must come from the instruction caches: with everything inlined and unrolled the kernel was 396 KB
 // of code, and once the level solve issued a third of its instructions the warps waited for code most of the time (8.8 of
 // 15.8 warps per issue, 1-warp teams). So the portable math, the extremes and the buoyancy are called, and loops that need
-// no overlap are not unrolled: 140 KB, most of it outside the step. Together with the sums a lane per column and one warp
-// for the motion (move_body), on B200: 2,048 uneven titanic64 runs to 20 min 371 ms against 469, a fleet of 96 ships to
-// 5 min 36.5 against 62.4, one run to 5 min 29.1 against 32.2, 48 portable32 runs to 15 min 68 against 83.
+// no overlap are not unrolled: 152 to 155 KB in double precision and 138 to 141 in single precision, half of it outside the
+// step. When that came, together with the sums a lane per column and one warp for the motion (move_body), on B200: 2,048
+// uneven titanic64 runs to 20 min 371 ms against 469, a fleet of 96 ships to 5 min 36.5 against 62.4, one run to 5 min 29.1
+// against 32.2, 48 portable32 runs to 15 min 68 against 83. At 128 registers a thread (16 warps an SM) the double precision
+// kernels spill 68 to 192 bytes and the fleets' up to 192; what a build spills does not order its times.
 static __device__ __noinline__ double2 trig_of(double x) {
   double s, c;
   pm::sin_cos(x, s, c);
@@ -259,8 +261,11 @@ __device__ __forceinline__ P load_col(const P* p) {
 }
 
 // Lane `lane`'s partial of tree w: columns w*32 + lane + 256 k in increasing k, AT_ONCE at a time (the loads of
-// all issue before the first is clipped; the clips stay in order). Large teams wait for the loads and take four; small
-// ones share an SM with others that fill the wait, and two need less code and pad less.
+// all issue before the first is clipped; the clips stay in order). Teams of 8 and 16 warps wait for the loads: they take
+// four, past L1. Smaller ones share an SM with others that fill the wait and that read the same columns from L1, and two
+// need less code and pad less. On B200: 16 warps, one run to 5 min 21.7 ms, cached 25.8; 8 warps, 250 titanic64 runs to 1 min
+// 4.11, cached in twos 4.54 (portable32 3.50, 3.46); 4 warps, 500 runs to 5 min 38.3, past L1 in fours 39.9 (portable32, 401
+// runs to 61 s 4.72, 5.02).
 template <class T, ColumnSource SRC, int AT_ONCE>
 __device__ __forceinline__ ColPartial<T> column_partial(const typename Vec2<T>::type* xy, const typename Vec2<T>::type* lh, const T* area,
                                                         int ncol, int first, T R20, T R21, T tz, T iR) {
@@ -970,8 +975,10 @@ __device__ __forceinline__ void solve_levels(const DevModel& M, const Pose& F, S
 // Larger teams have a thread for every connection of such a hull and are bound by the chain of dependent steps: they
 // form every flow while they count the degrees, and limit it after the barrier (team_step). A node's reciprocal area is
 // divided once, and a monitor divides the flows it sums itself (the step kept every connection's quotient before).
-// On B200: 2,048 uneven titanic64 runs to 20 min 469 ms against 493 (two-warp teams); one run to 5 min 32.2 against 33.4
-// (the sorted form in its 16-warp team: 35.4), 264 liner runs to 15 min 113 against 114 (sorted: 123).
+// On B200, when it came: 2,048 uneven titanic64 runs to 20 min 469 ms against 493 (two-warp teams); one run to 5 min 32.2
+// against 33.4 (the sorted form in its 16-warp team: 35.4), 264 liner runs to 15 min 113 against 114 (sorted: 123). With the
+// present step the two forms are level in between: 4 warps, 500 titanic64 runs to 5 min 38.3 sorted, 38.2 not; 8 warps, 250
+// runs to 1 min 4.13 sorted, 4.11 not.
 
 // The heads over connection c's opening at its two ends.
 struct FlowHeads {
