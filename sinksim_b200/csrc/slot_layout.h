@@ -19,7 +19,7 @@ inline std::uint32_t take(std::uint32_t& off, std::size_t bytes) {
 // (one slot has to fit a block's shared memory) and how much of an SM's shared storage a full load leaves to L1: 92 bytes a
 // space that is a group of its own and 8 a connection, so the 232,448 bytes of a B200 block hold 2,314 spaces with as many
 // connections, 2,144 with twice and 1,994 with three times as many.
-// A titanic64 slot is 9.2 KB in one-warp teams. With 10.6 KB (a degree array, a sixth column of load terms and 8-byte list
+// A titanic64 slot is 9.1 KB in one-warp teams. With 10.6 KB (a degree array, a sixth column of load terms and 8-byte list
 // entries of their own) hulls of 1,929 to 2,292 spaces were refused that had run before, and 2,048 uneven titanic64 runs to
 // 20 min took 350 ms on B200, 343 as it is; 264 liner runs to 15 min 91.7 and 89.3.
 inline SlotLayout slot_layout(std::int32_t NN, std::int32_t NC, std::int32_t NG, std::int32_t maxGroup, bool mixed, int W, bool fleet) {
