@@ -332,7 +332,7 @@ _ref_lib = None
 
 
 def _from_reference(name):
-    """Path of a part of the checker that is built from the reference's own sources. Where it was not built (oracle/Makefile
+    """Path of a part of the oracle that is built from the reference's own sources. Where it was not built (oracle/Makefile
     needs those sources), the rest of the test that asks for it is skipped; what the test checked before that stands."""
     path = os.path.join(REF_DIR, name)
     if not os.path.exists(path):
